@@ -194,7 +194,7 @@ def algorithmic_bytes(kernel, n, k, d_pad):
     a second, labelled figure beside the stage-level formulas below."""
     if kernel == "knn_kernel":
         # read every point once (padded coordinates + caller index); write the
-        # Morton-order rows (squared distance + position), the caller-order
+        # index-order rows (squared distance + position), the caller-order
         # neighbour matrix (k - 1 columns) and the one-byte boundary-tie flag
         return n * (4 * d_pad + 4) + n * k * 8 + n * (k - 1) * 4 + n
     if kernel == "search_kernel":

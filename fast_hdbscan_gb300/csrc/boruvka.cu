@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(kSW * 32) search_kernel(
         for (int lv = 0; lv < lvl_lo && x > 0; ++lv) x = (x - 1) >> 1;
     for (int lv = lvl_lo; sparse ? lv == lvl_lo : (lv < lvl_hi && x > 0); ++lv) {
         const int32_t sib = sparse ? 0 : (int32_t)((x & 1) ? x + 1 : x - 1);
-        // children nearer the home bucket in Morton order first
+        // children nearer the home bucket in index order first
         const bool right_side = (x & 1) != 0;
         if (!sparse) x = (x - 1) >> 1;
         {
@@ -1149,7 +1149,7 @@ int boruvka_mst(Workspace& ws, const fhg_index& ix, int min_samples, MstResult* 
     FHG_CUDA(cudaStreamSynchronize(s));
     int64_t m = h_cnt;
 
-    // representatives (component ids) in Morton order
+    // representatives (component ids) in index order
     FHG_TRY(ws.alloc(&reps, (size_t)n));
     FHG_TRY(ws.alloc(&reps2, (size_t)n));
     LAUNCH(rep_flags_kernel, n, n, comp, flag);

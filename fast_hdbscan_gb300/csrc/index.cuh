@@ -1,11 +1,11 @@
 // The spatial index shared by the kNN and Boruvka kernels.
 //
 // HBM layout (n points, p = 4 floats per point for d <= 4, 8 for d <= 8):
-//   pts   [n][p]  float32  points in Morton order, padded with zeros
-//   orig  [n]     int32    Morton position -> caller index
-//   rank  [n]     int32    caller index -> Morton position
+//   pts   [n][p]  float32  points in index order, padded with zeros
+//   orig  [n]     int32    index position -> caller index
+//   rank  [n]     int32    caller index -> index position
 //   box   [nodes][2][p]    float32 lower / upper corner of every tree node
-// Buckets of kLeaf = 32 consecutive Morton positions are the leaves of an
+// Buckets of kLeaf = 32 consecutive index positions are the leaves of an
 // implicit complete binary tree with `slots` (a power of two) leaf slots:
 // node i has children 2i+1 and 2i+2, and leaf slot s is node slots-1+s.
 // Slots past the last bucket carry an empty box (lo = +inf, hi = -inf).
@@ -107,14 +107,14 @@ int index_build(const float* X, int64_t n, int32_t d, cudaStream_t s, fhg_index*
 int index_free(fhg_index* ix, cudaStream_t s);
 
 // kNN over the index.  Outputs (all nullable):
-//   d_s/i_s : rows in Morton order, neighbour ids as Morton positions
+//   d_s/i_s : rows in index order, neighbour ids as index positions
 //   d_o/i_o : rows in caller order, neighbour ids as caller indices (i_o may
 //             be given alone; then its rows may have their own stride and
 //             drop their first io_skip columns -- the neighbours[:, 1:]
 //             matrix of the fit)
-//   tie_s   : per point (Morton order), 1 when some point outside its list
+//   tie_s   : per point (index order), 1 when some point outside its list
 //             lies at exactly its k-th distance
-// A capped kNN pass (all members nullable, Morton order): cap2 = every
+// A capped kNN pass (all members nullable, index order): cap2 = every
 // query's squared search radius; queries with fewer than k points within it
 // get fail = 1 (and fail_count, if given, counts them) and no output.
 // redo: only these queries search (uncapped).  scan_count (nullable, any

@@ -1,6 +1,6 @@
 // Exact k-nearest-neighbour search (core distances), warp-cooperative.
 //
-// One warp owns one bucket of 32 Morton-consecutive query points (lane =
+// One warp owns one bucket of 32 index-consecutive query points (lane =
 // query).  It first scans its own bucket -- which contains the queries
 // themselves -- to get a tight k-th distance, then walks up the bucket tree to
 // the root: at every ancestor it searches the sibling subtree depth-first
@@ -11,7 +11,7 @@
 // shared-memory load and marks it if it is within the lane's k-th distance;
 // then each lane inserts its own marked candidates.  Each lane keeps its
 // sorted top-K list (squared distance, caller index) in registers: exact
-// distance ties are broken without a memory access, and the Morton positions
+// distance ties are broken without a memory access, and the index positions
 // of the result are looked up once at the end.
 //
 // Ordering: (squared distance, caller index), ascending -- the reference's
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kKnnWarps * 32, knn_min_blocks<DIM, K>()) knn_
     // overlap, so no ancestor box bounds the search; but near subtrees come
     // first, and a far sibling whose box is out of every lane's reach costs a
     // single box test.  Inside a sibling subtree the child nearer the home
-    // bucket in Morton order goes first: the left child of a subtree to the
+    // bucket in index order goes first: the left child of a subtree to the
     // right of the home path, the right child of one to its left.
     int32_t* st = s_stack[warp];
     const int64_t first_leaf_node = ix.slots - 1;
@@ -475,7 +475,7 @@ int index_knn(const fhg_index& ix, int k, float* d_s, int32_t* i_s, float* d_o, 
     }
     if ((d_s == nullptr) != (i_s == nullptr) || (d_o != nullptr && i_o == nullptr) ||
         (d_o != nullptr && (io_stride != k || io_skip != 0))) {
-        set_error("knn: Morton-order outputs come in pairs; caller-order distances need ids");
+        set_error("knn: index-order outputs come in pairs; caller-order distances need ids");
         return FHG_ERR_INVALID;
     }
     Stage stage(s, "knn");

@@ -50,7 +50,7 @@ __device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
 }
 
 // ------------------------------------------------------------- features
-// Per Morton position p; written to row orig[p] when orig is given, else p.
+// Per index position p; written to row orig[p] when orig is given, else p.
 template <int SP>
 __global__ void features_kernel(IndexView ix, int d, const int32_t* __restrict__ orig,
                                 float* __restrict__ feat) {
@@ -547,7 +547,7 @@ int radius_train(float* prm, const float* feat, const float* tgt, int64_t n, int
 }
 
 // Certified kNN with a learned radius: features and the predicted radius per
-// Morton position, a capped pass, then the uncapped pass over the queries the
+// index position, a capped pass, then the uncapped pass over the queries the
 // capped pass could not certify.  Same outputs as index_knn.
 int knn_with_radius(const fhg_index& ix, int k, const RadiusUse& use, float* d_s, int32_t* i_s,
                     float* d_o, int32_t* i_o, cudaStream_t s, int8_t* tie_s, int io_stride,

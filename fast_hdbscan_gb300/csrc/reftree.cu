@@ -211,7 +211,7 @@ __global__ void keys_level_kernel(int64_t n, int64_t first, int pad,
     keys[p] = ((uint64_t)ordered_bits(x) << 32) | (uint32_t)c;
 }
 
-// The index's points (Morton order) back in caller order.
+// The index's points (index order) back in caller order.
 __global__ void caller_order_kernel(int64_t n, int pad, const int32_t* __restrict__ orig,
                                     const float* __restrict__ pts, float* __restrict__ out) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

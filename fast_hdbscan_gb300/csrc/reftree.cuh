@@ -42,8 +42,8 @@ int ref_tree_export(const RefTree& t, int32_t* idx_array, float* node_bounds, cu
 // of k (squared distance, index) entries and its heap sort, so that equal
 // distances come out in the reference's order.  With sqrt_order the sort
 // runs on the square roots (the query without output_rdist, boruvka.py:567).
-// d_s / s_s hold the engine's lists (Morton-order rows of kk = min(k, n)
-// squared distances and Morton positions, (distance, index) order) and tie
+// d_s / s_s hold the engine's lists (index-order rows of kk = min(k, n)
+// squared distances and index positions, (distance, index) order) and tie
 // (nullable) its flags of a point outside the list at the k-th distance; the
 // rows that can differ from the reference's -- equal distances inside, or a
 // tie at the k-th -- are recomputed by the reference's query and written

@@ -3,7 +3,7 @@
 Mirrors fast_hdbscan/numba_kdtree.py: ``build_kdtree`` returns a tree object
 whose ``data`` attribute is the float32 copy of the input (the only field the
 fit path reads), and ``parallel_tree_query`` returns the k nearest neighbours
-of every point, itself included.  The index itself is a Morton-ordered bucket
+of every point, itself included.  The index itself is a Hilbert-ordered bucket
 tree on the GPU (see include/fhg.h).
 """
 import numpy as np

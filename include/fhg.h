@@ -87,7 +87,7 @@ int fhg_set_tie_rule(int rule);
  * to the driver. */
 int fhg_release_cached_memory(void);
 
-/* Opaque spatial index: points sorted along a Morton curve into buckets of
+/* Opaque spatial index: points sorted along a Hilbert curve into buckets of
  * 32 with a complete binary tree of bounding boxes over the buckets. */
 typedef struct fhg_index fhg_index;
 

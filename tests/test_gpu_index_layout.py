@@ -1,0 +1,29 @@
+"""The spatial index at the edges of its chunks and levels: the kNN over it
+equals the oracle's whatever order the points are laid out in."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 64, 1023, 1024, 1025, 2047, 2048, 2049, 3000, 4097,
+                               33_000])
+@pytest.mark.parametrize("d", [1, 2, 3, 4, 5, 6, 8, 9, 17])
+@pytest.mark.parametrize("kind", ["normal", "grid"])
+def test_knn_over_layout_vs_oracle(engine, n, d, kind):
+    from fast_hdbscan_gb300.numba_kdtree import build_kdtree, parallel_tree_query
+    from oracle import oracle as O
+
+    if n == 33_000 and (kind == "grid" or d > 5):
+        pytest.skip("covered by the smaller sizes")
+    rng = np.random.default_rng(100 * n + d)
+    if kind == "grid":  # equal coordinates on both sides of every median
+        X = rng.integers(-2, 3, size=(n, d)).astype(np.float32)
+    else:
+        X = (rng.normal(size=(n, d)) * np.exp(rng.normal(size=(n, 1)))).astype(np.float32)
+    k = 5
+    tree = build_kdtree(X)
+    rd, ix = parallel_tree_query(tree, tree.data, k=k, output_rdist=True)
+    ord_, oix = O.tree_query(O.build_kdtree(X), k, mode=1)
+    np.testing.assert_array_equal(rd, ord_)
+    np.testing.assert_array_equal(ix, oix)
