@@ -59,9 +59,8 @@ __device__ __forceinline__ float box_lb(const float* __restrict__ box, const flo
 #pragma unroll
     for (int j = 0; j < P; ++j) {
         float lo = box[j], hi = box[P + j];
-        float dlo = lo > q[j] ? __fsub_rn(lo, q[j]) : 0.0f;
-        float dhi = q[j] > hi ? __fsub_rn(q[j], hi) : 0.0f;
-        float dd = __fadd_rn(dlo, dhi);
+        // at most one of the two differences is positive
+        const float dd = fmaxf(fmaxf(__fsub_rn(lo, q[j]), __fsub_rn(q[j], hi)), 0.0f);
         r = __fadd_rn(r, __fmul_rn(dd, dd));
     }
     return r;
@@ -75,9 +74,8 @@ __device__ __forceinline__ float box_lb_n(const float* __restrict__ box, const f
 #pragma unroll
     for (int j = 0; j < DIM; ++j) {
         float lo = box[j], hi = box[SP + j];
-        float dlo = lo > q[j] ? __fsub_rn(lo, q[j]) : 0.0f;
-        float dhi = q[j] > hi ? __fsub_rn(q[j], hi) : 0.0f;
-        float dd = __fadd_rn(dlo, dhi);
+        // at most one of the two differences is positive
+        const float dd = fmaxf(fmaxf(__fsub_rn(lo, q[j]), __fsub_rn(q[j], hi)), 0.0f);
         r = __fadd_rn(r, __fmul_rn(dd, dd));
     }
     return r;

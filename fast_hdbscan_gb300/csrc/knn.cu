@@ -6,10 +6,8 @@
 // the root: at every ancestor it searches the sibling subtree depth-first
 // (shared-memory stack; a node is entered when ANY lane's lower bound is
 // within that lane's current k-th distance).  At a
-// leaf the warp stages the bucket's points in shared memory with one
-// coalesced load per lane, and every lane reads candidate t with a broadcast
-// shared-memory load and marks it if it is within the lane's k-th distance;
-// then each lane inserts its own marked candidates.  Each lane keeps its
+// leaf the warp loads the bucket's points (one coalesced load per lane) and
+// every lane collects those within its k-th distance.  Each lane keeps its
 // sorted top-K list (squared distance, caller index) in registers: exact
 // distance ties are broken without a memory access, and the index positions
 // of the result are looked up once at the end.
@@ -23,14 +21,25 @@
 namespace fhg {
 namespace {
 
-constexpr int kKnnWarps = 4;
-// Buckets needed by at most this many lanes are scanned query by query.
-constexpr int kTransposeMax = 20;
+// Warps of a block: their shared memory stays within the static 48 KB.
+template <int SP>
+__host__ __device__ constexpr int knn_warps() { return SP <= 8 ? 4 : 2; }
+// Buckets needed by at most this many lanes are scanned query by query, each
+// lane with its own candidate; otherwise candidate by candidate, each lane for
+// its own query.  (Two, four or eight lanes to a query instead, with shared
+// counters for the queues: 13.3 against 13.2 ms at 10M x 3-D, 11.7 against 9.3
+// at 2M x 5-D.)
+constexpr int kTransposeMax = 16;
 // Resident blocks asked of the register allocator: small lists fit in 80
-// registers, which keeps 24 warps per SM; larger lists take what they need.
+// registers (100 above four dimensions), which keeps 24 (20) warps per SM;
+// larger lists take what they need.
 template <int DIM, int K>
-constexpr int knn_min_blocks() { return (K <= 16 && DIM <= 8) ? 6 : 1; }
+constexpr int knn_min_blocks() { return K > 16 || DIM > 8 ? 1 : DIM <= 4 ? 6 : 5; }
 constexpr int kStack = 64;
+// A lane's queue of candidates not yet in its list (see knn_kernel): the fill
+// at which the warp empties its queues, and the row stride (odd, in 8-byte
+// words: no bank conflicts across lanes).
+constexpr int kQueueFull = 16, kQueue = kQueueFull + 8, kQueueStride = kQueue + 1;
 
 __device__ __forceinline__ unsigned long long pack_entry(float d, int32_t o) {
     return ((unsigned long long)__float_as_uint(d) << 32) | (uint32_t)o;
@@ -40,31 +49,92 @@ __device__ __forceinline__ float entry_dist(unsigned long long e) {
 }
 __device__ __forceinline__ int32_t entry_orig(unsigned long long e) { return (int32_t)(uint32_t)e; }
 
+__device__ __forceinline__ void compare_exchange(unsigned long long& a, unsigned long long& b) {
+    const bool swap = a > b;
+    const unsigned long long lo = swap ? b : a;
+    b = swap ? a : b;
+    a = lo;
+}
+// Ascending sort of 8 keys (Batcher's odd-even merge sort, 19 exchanges).
+__device__ __forceinline__ void sort8(unsigned long long* v) {
+#define FHG_CE(i, j) compare_exchange(v[i], v[j])
+    FHG_CE(0, 1); FHG_CE(2, 3); FHG_CE(4, 5); FHG_CE(6, 7);
+    FHG_CE(0, 2); FHG_CE(1, 3); FHG_CE(4, 6); FHG_CE(5, 7);
+    FHG_CE(1, 2); FHG_CE(5, 6);
+    FHG_CE(0, 4); FHG_CE(1, 5); FHG_CE(2, 6); FHG_CE(3, 7);
+    FHG_CE(2, 4); FHG_CE(3, 5);
+    FHG_CE(1, 2); FHG_CE(3, 4); FHG_CE(5, 6);
+#undef FHG_CE
+}
+// Merges the ascending v[8] into the ascending key[K], keeping the K smallest
+// in order; out = min(out, every key left out).
+template <int K>
+__device__ __forceinline__ void merge8(unsigned long long (&key)[K],
+                                       const unsigned long long* v, unsigned long long& out) {
+    constexpr bool kPow2 = (K & (K - 1)) == 0;
+    constexpr int M = kPow2 ? K : 32;  // K = 24 merges as 32
+    unsigned long long c[M];
+#pragma unroll
+    for (int j = 0; j < K; ++j) c[j] = key[j];
+    if constexpr (kPow2) {
+        // the K smallest of key ++ reverse(v, +inf...) form a bitonic run
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            unsigned long long x = v[j];
+            compare_exchange(c[K - 1 - j], x);
+            out = x < out ? x : out;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) c[M - 1 - j] = v[j];
+    }
+#pragma unroll
+    for (int stride = M / 2; stride > 0; stride >>= 1) {
+#pragma unroll
+        for (int i = 0; i < M; ++i)
+            if ((i & stride) == 0) compare_exchange(c[i], c[i + stride]);
+    }
+#pragma unroll
+    for (int j = 0; j < K; ++j) key[j] = c[j];
+    if constexpr (!kPow2) out = c[K] < out ? c[K] : out;
+}
+
+// What bounds this kernel is instruction issue.  A bucket's candidates within
+// a lane's k-th distance go into that lane's queue in shared memory; when some
+// lane's queue fills up, every lane sorts its queue eight at a time and merges
+// it into its sorted list, by networks that run the same instructions on all
+// lanes.  (Inserting each candidate as it came made the warp wait for its
+// busiest lane in every bucket: about 150 insertions per warp at 1M x 3-D, k =
+// 16, where a lane inserts 41; now about 20 merges.)  Until its queue is
+// emptied a lane's k-th distance is out of date, i.e. larger: it queues some
+// more candidates, and no result changes.  Measured (one GB300, lists inserted
+// one by one -> this): 10M x 3-D, k = 16: 15.3 -> 13.2 ms; 2M x 5-D, k = 11:
+// 10.4 -> 9.3; 60k x 13-D, k = 11: 2.3 -> 1.8; 1M x 3-D, k = 31: 5.9 -> 3.6
+// (this one before the index order changed), 63 % of issue slots busy.
 template <int DIM, int SP, int K>
-__global__ void __launch_bounds__(kKnnWarps * 32, knn_min_blocks<DIM, K>()) knn_kernel(IndexView ix, int k,
-                                                              float* __restrict__ d_s,
-                                                              int32_t* __restrict__ i_s,
-                                                              float* __restrict__ d_o,
-                                                              int32_t* __restrict__ i_o,
-                                                              int8_t* __restrict__ tie_s,
-                                                              int io_stride, int io_skip,
-                                                              const float* __restrict__ cap2,
-                                                              const uint8_t* __restrict__ redo,
-                                                              uint8_t* __restrict__ fail,
-                                                              unsigned long long* fail_count,
-                                                              unsigned long long* scan_count) {
-    __shared__ int32_t s_stack[kKnnWarps][kStack];
+__global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>())
+    knn_kernel(IndexView ix, int k, float* __restrict__ d_s, int32_t* __restrict__ i_s,
+               float* __restrict__ d_o, int32_t* __restrict__ i_o, int8_t* __restrict__ tie_s,
+               int io_stride, int io_skip, const float* __restrict__ cap2,
+               const uint8_t* __restrict__ redo, uint8_t* __restrict__ fail,
+               unsigned long long* fail_count, unsigned long long* scan_count, int split) {
+    constexpr int kKnnWarps = knn_warps<SP>();
     __shared__ float4 s_cand[kKnnWarps][32 * (SP / 4)];
+    __shared__ float4 s_query[kKnnWarps][32 * (SP / 4)];
     __shared__ int32_t s_corig[kKnnWarps][32];
+    __shared__ unsigned long long s_queue[kKnnWarps][32 * kQueueStride];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t leaf = (int64_t)blockIdx.x * kKnnWarps + warp;
+    // `split` warps share a bucket's queries, 32 / split each (knn_split).
+    const int64_t part = (int64_t)blockIdx.x * kKnnWarps + warp;
+    const int64_t leaf = part / split;
     if (leaf >= ix.nleaves) return;
     const int64_t qi = leaf * kLeaf + lane;
+    const bool own_part = lane * split / 32 == (int)(part % split);
     // redo (nullable): only these queries search (the fallback of a capped
     // pass); cap2 (nullable): every query's list starts full of sentinels at
     // its squared search radius, so only points within it are considered.
-    const bool valid = qi < ix.n && (!redo || redo[qi]);
-    if (redo && !__any_sync(kFull, valid)) return;
+    const bool valid = own_part && qi < ix.n && (!redo || redo[qi]);
+    if (!__any_sync(kFull, valid)) return;
     float q[DIM];
     {
         float t[SP];
@@ -74,7 +144,12 @@ __global__ void __launch_bounds__(kKnnWarps * 32, knn_min_blocks<DIM, K>()) knn_
             for (int j = 0; j < SP; ++j) t[j] = 0.0f;
 #pragma unroll
         for (int j = 0; j < DIM; ++j) q[j] = t[j];
+#pragma unroll
+        for (int h = 0; h < SP / 4; ++h)
+            s_query[warp][lane * (SP / 4) + h] =
+                make_float4(t[4 * h], t[4 * h + 1], t[4 * h + 2], t[4 * h + 3]);
     }
+    __syncwarp();
     // Each list entry is one 64-bit key: squared distance bits above the
     // caller index.  Non-negative floats order like their bit patterns, so
     // one unsigned compare orders entries by (distance, caller index).
@@ -87,144 +162,203 @@ __global__ void __launch_bounds__(kKnnWarps * 32, knn_min_blocks<DIM, K>()) knn_
     for (int j = 0; j < K; ++j) key[j] = (j < K - k) ? 0ull : kEmptyKey;
     float4* cand = s_cand[warp];
     int32_t* corig = s_corig[warp];
+    unsigned long long* queue = s_queue[warp];
     const int32_t* __restrict__ orig = ix.orig;
 
-    // Smallest distance of a point examined but left out of the list: equal to
-    // the final k-th distance exactly when another point ties with the k-th.
-    float rejmin = INFINITY;
-    // Inserts (dd, o) into this lane's sorted list if it precedes the k-th.
-    // Every slot's new value depends only on the old list (no chain of
-    // compare-and-swap steps): slot j takes slot j-1's entry if that entry
-    // follows (dd, o), else (dd, o) if slot j's own entry follows it.
-    auto insert = [&](float dd, int32_t o) {
-        const unsigned long long nk = pack_entry(dd, o);
-        if (!(nk < key[K - 1])) {
-            rejmin = fminf(rejmin, dd);
-            return;
-        }
-        // (a sentinel of a capped list leaving is no point)
-        if (entry_orig(key[K - 1]) != INT32_MAX) rejmin = fminf(rejmin, entry_dist(key[K - 1]));
-        bool gt_hi = true;
-#pragma unroll
-        for (int j = K - 1; j > 0; --j) {
-            const bool gt_lo = key[j - 1] > nk;
-            key[j] = gt_lo ? key[j - 1] : (gt_hi ? nk : key[j]);
-            gt_hi = gt_lo;
-        }
-        if (gt_hi) key[0] = nk;
-    };
-
-    // One bucket: first every lane marks the candidates within its current
-    // k-th distance (one bit each), then each lane inserts only its own
-    // marked candidates -- the warp pays for the busiest lane, not for every
-    // candidate some lane wants.
+    // Least key of a point examined but left out of the list: its distance
+    // equals the final k-th exactly when another point ties with the k-th.
+    // (A capped list's sentinels follow every queued point: as this minimum
+    // one stands for "no point".)
+    unsigned long long rejected = ~0ull;
+    int waiting = 0;  // entries in this lane's queue
+    float thr = valid ? entry_dist(key[K - 1]) : -1.0f;  // (no distance is within -1)
     int scans = 0;  // buckets this warp scanned
-    auto scan_leaf = [&](int64_t lf, bool need) {
-        ++scans;
-        const int64_t base = lf * kLeaf;
-        const int cnt = (int)(ix.n - base < kLeaf ? ix.n - base : kLeaf);
-        float own[SP];  // this lane's candidate (lane t holds candidate t)
-#pragma unroll
-        for (int j = 0; j < SP; ++j) own[j] = 0.0f;
-        if (lane < cnt) {
-            const float4* src = reinterpret_cast<const float4*>(ix.pts) + (base + lane) * (SP / 4);
-#pragma unroll
-            for (int h = 0; h < SP / 4; ++h) {
-                const float4 v = __ldg(src + h);
-                cand[lane * (SP / 4) + h] = v;
-                own[4 * h] = v.x; own[4 * h + 1] = v.y; own[4 * h + 2] = v.z; own[4 * h + 3] = v.w;
-            }
-            corig[lane] = __ldg(orig + base + lane);
-        }
-        __syncwarp();
-        const float thr = need ? entry_dist(key[K - 1]) : -INFINITY;
-        uint32_t acc = 0u;
-        const unsigned needy = __ballot_sync(kFull, need);
-        if (__popc(needy) <= kTransposeMax) {
-            // Few lanes need the bucket: each lane takes its own candidate and
-            // the warp visits only the needing queries; the ballot over the
-            // candidates is that query's mask.  Same distances bit for bit.
-            unsigned mq = needy;
-            while (mq) {
-                const int i = __ffs(mq) - 1;
-                mq &= mq - 1u;
-                float qi[DIM];
-#pragma unroll
-                for (int j = 0; j < DIM; ++j) qi[j] = __shfl_sync(kFull, q[j], i);
-                const float ti = __shfl_sync(kFull, thr, i);
-                const unsigned bits = __ballot_sync(kFull, lane < cnt && rdist_rn<DIM>(qi, own) <= ti);
-                if (lane == i) acc = bits;
-            }
-        } else {
-#pragma unroll 4
-            for (int t = 0; t < cnt; ++t) {
-                float c[SP];
-#pragma unroll
-                for (int h = 0; h < SP / 4; ++h) {
-                    float4 v = cand[t * (SP / 4) + h];
-                    c[4 * h] = v.x; c[4 * h + 1] = v.y; c[4 * h + 2] = v.z; c[4 * h + 3] = v.w;
-                }
-                acc |= (rdist_rn<DIM>(q, c) <= thr ? 1u : 0u) << t;
-            }
-        }
-        while (acc) {
-            const int t = __ffs(acc) - 1;
-            acc &= acc - 1u;
-            float c[SP];
-#pragma unroll
-            for (int h = 0; h < SP / 4; ++h) {
-                float4 v = cand[t * (SP / 4) + h];
-                c[4 * h] = v.x; c[4 * h + 1] = v.y; c[4 * h + 2] = v.z; c[4 * h + 3] = v.w;
-            }
-            insert(rdist_rn<DIM>(q, c), corig[t]);
-        }
-        __syncwarp();
-    };
 
-    // Seed with the warp's own bucket (it holds the queries themselves), so
-    // that the walk below starts with a tight k-th distance; the walk then
-    // skips this bucket.
-    scan_leaf(leaf, valid);
-
-    // Walk up from the home bucket to the root: at each ancestor search the
-    // sibling subtree depth first, pruned by lower bounds.  Subtrees' boxes
-    // overlap, so no ancestor box bounds the search; but near subtrees come
-    // first, and a far sibling whose box is out of every lane's reach costs a
-    // single box test.  Inside a sibling subtree the child nearer the home
-    // bucket in index order goes first: the left child of a subtree to the
-    // right of the home path, the right child of one to its left.
-    int32_t* st = s_stack[warp];
+    // The walk: the home bucket first (it holds the queries themselves and
+    // gives a tight k-th distance), then up to the root, searching at each
+    // ancestor the sibling subtree depth first, pruned by lower bounds.
+    // Subtrees' boxes overlap, so no ancestor box bounds the search; but near
+    // subtrees come first, and a far sibling whose box is out of every lane's
+    // reach costs a single box test.  Inside a sibling subtree the child
+    // nearer the home bucket in index order goes first: the left child of a
+    // subtree to the right of the home path, the right child of one to its
+    // left.  Both children are tested when their parent is expanded; only
+    // needed ones are followed, the nearer at once, the farther by way of the
+    // stack (lane j holds entry j: at most one entry per level) or, for a
+    // bucket, of `later` with its bounds.
+    //
+    // Every bucket is scanned, and every queue emptied, at one place in the
+    // code each: with the scan and the merges inlined where they are needed,
+    // the kernel ran out of the instruction cache (3.1 of 10 stall cycles per
+    // instruction at 2M x 3-D, k = 16).
     const int64_t first_leaf_node = ix.slots - 1;
     int64_t x = first_leaf_node + leaf;
-    while (x > 0) {
-        const int32_t sib = (int32_t)((x & 1) ? x + 1 : x - 1);
-        const bool right_side = (x & 1) != 0;
-        int sp = 1;
-        if (lane == 0) st[0] = sib;
-        __syncwarp();
-        while (sp > 0) {
-            --sp;
-            const int32_t node = st[sp];
+    int32_t stack = 0, later = -1;
+    int sp = 0;
+    bool right_side = false;
+    float later_lb = 0.0f;
+    int64_t lf = leaf;  // the bucket to scan, -1 when the walk has ended
+    bool need = valid;
+    for (bool home = true;; home = false) {
+        // ---- scan: the bucket's candidates within the k-th distance of each
+        // lane that needs it join that lane's queue
+        const int64_t base = lf * kLeaf;
+        const int cnt = lf < 0 ? 0 : (int)(ix.n - base < kLeaf ? ix.n - base : kLeaf);
+        unsigned todo = lf < 0 ? 0u : __ballot_sync(kFull, need);
+        // (the home bucket fills every list: its lanes go through it together)
+        const bool by_query = !home && __popc(todo) <= kTransposeMax;
+        float own[SP];  // this lane's candidate (lane t holds candidate t)
+        int32_t own_o = 0;
+#pragma unroll
+        for (int j = 0; j < SP; ++j) own[j] = INFINITY;  // (within no distance but +inf)
+        if (lane < cnt) {
+            load_pt<SP>(ix.pts, base + lane, own);
+            own_o = __ldg(orig + base + lane);
+        }
+        if (lf >= 0) ++scans;
+        if (!by_query) {
             __syncwarp();
-            float b[2 * SP];
-            load_box<SP>(ix.box, node, b);
-            const float lb = box_lb_n<DIM, SP>(b, q);
-            const bool need = valid && lb <= entry_dist(key[K - 1]);
-            if (!__any_sync(kFull, need)) continue;
-            if (node >= first_leaf_node) {
-                scan_leaf(node - first_leaf_node, need);
-            } else {
-                const int32_t l = 2 * node + 1, r = l + 1;
-                const int32_t near = right_side ? l : r, far = right_side ? r : l;
-                if (lane == 0) {
-                    st[sp] = far;
-                    st[sp + 1] = near;
+#pragma unroll
+            for (int h = 0; h < SP / 4; ++h)
+                cand[lane * (SP / 4) + h] =
+                    make_float4(own[4 * h], own[4 * h + 1], own[4 * h + 2], own[4 * h + 3]);
+            corig[lane] = own_o;
+            __syncwarp();
+        }
+        unsigned open = cnt >= 32 ? kFull : (1u << cnt) - 1u;  // candidates of the current query
+        const unsigned every = open;
+        int t0 = 0;
+        // the queues are emptied at a fill of kQueueFull; after the home
+        // bucket and at the end always
+        const int full = home || lf < 0 ? 1 : kQueueFull;
+        for (;;) {
+            bool room = true;  // false: a queue must be emptied to go on
+            if (by_query) {
+                // Few lanes need the bucket: each lane takes its own candidate
+                // and the warp visits only the needing queries.
+                while (todo) {
+                    const int i = __ffs(todo) - 1;
+                    float y[SP];
+#pragma unroll
+                    for (int h = 0; h < SP / 4; ++h) {
+                        const float4 v = s_query[warp][i * (SP / 4) + h];
+                        y[4 * h] = v.x; y[4 * h + 1] = v.y; y[4 * h + 2] = v.z; y[4 * h + 3] = v.w;
+                    }
+                    const float lim = __shfl_sync(kFull, thr, i);
+                    const float dd = rdist_rn<DIM>(y, own);
+                    unsigned in = __ballot_sync(kFull, dd <= lim) & open;
+                    if (in) {
+                        const int have = __shfl_sync(kFull, waiting, i);
+                        if (have + __popc(in) > kQueue) {
+                            room = false;
+                            if (have > 0) break;
+                            if (in & 0xffffu) in &= 0xffffu;  // at most 16 at a time
+                        }
+                        if ((in >> lane) & 1u)
+                            queue[i * kQueueStride + have + __popc(in & ((1u << lane) - 1u))] =
+                                pack_entry(dd, own_o);
+                        if (lane == i) waiting += __popc(in);
+                        if (!room) {
+                            open &= ~in;
+                            break;
+                        }
+                    }
+                    open = every;
+                    todo &= todo - 1u;
                 }
-                sp += 2;
+            } else {
+                // Every lane reads candidate t from shared memory.
+                const float lim = need ? thr : -1.0f;
+                for (; t0 < cnt; t0 += 8) {
+                    room = !__any_sync(kFull, waiting >= kQueueFull);
+                    if (!room) break;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const int t = t0 + u;
+                        float c[SP];
+#pragma unroll
+                        for (int h = 0; h < SP / 4; ++h) {
+                            const float4 v = cand[t * (SP / 4) + h];
+                            c[4 * h] = v.x; c[4 * h + 1] = v.y;
+                            c[4 * h + 2] = v.z; c[4 * h + 3] = v.w;
+                        }
+                        const float dd = rdist_rn<DIM>(q, c);
+                        if (dd <= lim && t < cnt)
+                            queue[lane * kQueueStride + waiting++] = pack_entry(dd, corig[t]);
+                    }
+                }
+            }
+            // ---- queues into lists
+            if (!room || __any_sync(kFull, waiting >= full)) {
+                __syncwarp();
+                const int most = __reduce_max_sync(kFull, waiting);
+                for (int b = 0; b < most; b += 8) {
+                    unsigned long long v[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        v[j] = b + j < waiting ? queue[lane * kQueueStride + b + j] : ~0ull;
+                    sort8(v);
+                    merge8<K>(key, v, rejected);
+                }
+                waiting = 0;
+                if (valid) thr = entry_dist(key[K - 1]);
                 __syncwarp();
             }
+            if (room) break;
         }
-        x = (x - 1) >> 1;
+        if (lf < 0) break;
+
+        // ---- on to the next bucket some lane needs
+        lf = -1;
+        if (later >= 0) {
+            need = later_lb <= thr;
+            if (__any_sync(kFull, need)) lf = later;
+            later = -1;
+        }
+        while (lf < 0) {
+            int32_t node;
+            if (sp == 0) {
+                if (x == 0) break;
+                node = (int32_t)((x & 1) ? x + 1 : x - 1);
+                right_side = (x & 1) != 0;
+                x = (x - 1) >> 1;
+                float b[2 * SP];
+                load_box<SP>(ix.box, node, b);
+                need = box_lb_n<DIM, SP>(b, q) <= thr;
+                if (!__any_sync(kFull, need)) continue;
+                if (node >= first_leaf_node) {
+                    lf = node - first_leaf_node;
+                    break;
+                }
+            } else {
+                node = __shfl_sync(kFull, stack, --sp);
+            }
+            // down to a bucket, or until no child is needed
+            for (;;) {
+                const int32_t l = 2 * node + 1, r = l + 1;
+                const int32_t nearc = right_side ? l : r, farc = right_side ? r : l;
+                float bn[2 * SP], bf[2 * SP];
+                load_box<SP>(ix.box, nearc, bn);
+                load_box<SP>(ix.box, farc, bf);
+                const float lbn = box_lb_n<DIM, SP>(bn, q), lbf = box_lb_n<DIM, SP>(bf, q);
+                const bool an = __any_sync(kFull, lbn <= thr), af = __any_sync(kFull, lbf <= thr);
+                if (!an && !af) break;
+                if (l >= first_leaf_node) {
+                    lf = (an ? nearc : farc) - first_leaf_node;
+                    need = (an ? lbn : lbf) <= thr;
+                    if (an && af) {
+                        later = farc - (int32_t)first_leaf_node;
+                        later_lb = lbf;
+                    }
+                    break;
+                }
+                if (an && af) {
+                    if (lane == sp) stack = farc;
+                    ++sp;
+                }
+                node = an ? nearc : farc;
+            }
+        }
     }
     if (scan_count && lane == 0) atomicAdd(scan_count, (unsigned long long)scans);
     if (!valid) return;
@@ -237,6 +371,8 @@ __global__ void __launch_bounds__(kKnnWarps * 32, knn_min_blocks<DIM, K>()) knn_
         if (fail_count) atomicAdd(fail_count, 1ull);
         return;
     }
+    const float rejmin =
+        rejected == ~0ull || entry_orig(rejected) == INT32_MAX ? INFINITY : entry_dist(rejected);
     if (tie_s) tie_s[qi] = rejmin == entry_dist(key[K - 1]) ? 1 : 0;
     const int64_t o_row = orig[qi];
 #pragma unroll
@@ -437,19 +573,35 @@ int launch_knn_large(const fhg_index& ix, int k, float* d_s, int32_t* i_s, float
     return FHG_OK;
 }
 
+// Warps per bucket.  A walk is one long dependent chain, so with few buckets
+// its latency is the kernel's time (3,000 points, k = 16: 94 warps, 150 us of
+// which a few per cent issue): the queries of a bucket then go to several
+// warps, whose other lanes still share the work on candidates, until the GPU
+// has 20 warps per SM.  Measured (us at 1 / 4 / 8 / 16 warps per bucket): 94
+// buckets, 3-D, k = 16: 154 / 90 / 73 / 72; 313, 2-D: 123 / 91 / 79 / 82; 625,
+// 5-D: 370 / 297 / 269 / 297; 1,875, 3-D, k = 31: 512 / 591 / 708 / 1,028.
+constexpr int64_t kKnnWarpsWanted = 20 * 152;
+int knn_split(int64_t nleaves) {
+    int split = 1;
+    while (split < 32 && 2 * split * nleaves <= kKnnWarpsWanted) split *= 2;
+    return split;
+}
+
 template <int DIM, int K>
 int launch_knn(const fhg_index& ix, int k, float* d_s, int32_t* i_s, float* d_o, int32_t* i_o,
                int8_t* tie_s, int io_stride, int io_skip, const KnnCap& cap, cudaStream_t s) {
     // padded width; for d > 8 the kernels run over all SP = DIM padded
     // coordinates (the padding is zero and adds exact zeros to distances)
     constexpr int SP = DIM <= 4 ? 4 : (DIM <= 8 ? 8 : DIM);
-    unsigned g = grid_for(ix.nleaves, kKnnWarps);
+    constexpr int kKnnWarps = knn_warps<SP>();
+    const int split = knn_split(ix.nleaves);
+    const unsigned g = grid_for(ix.nleaves * split, kKnnWarps);
     Stage stage(s, "knn_kernel");
     ::fhg::note_launch();
     knn_kernel<DIM, SP, K><<<g, kKnnWarps * 32, 0, s>>>(view_of(ix), k, d_s, i_s, d_o, i_o,
                                                          tie_s, io_stride, io_skip, cap.cap2,
                                                          cap.redo, cap.fail, cap.fail_count,
-                                                         cap.scan_count);
+                                                         cap.scan_count, split);
     FHG_CUDA(cudaGetLastError());
     return FHG_OK;
 }

@@ -27,3 +27,27 @@ def test_knn_over_layout_vs_oracle(engine, n, d, kind):
     ord_, oix = O.tree_query(O.build_kdtree(X), k, mode=1)
     np.testing.assert_array_equal(rd, ord_)
     np.testing.assert_array_equal(ix, oix)
+
+
+@pytest.mark.parametrize("n", [5, 31, 95, 1000, 20_001, 97_281, 120_000])
+@pytest.mark.parametrize("k", [1, 2, 8, 9, 16, 17, 24, 25, 32, 33, 64])
+@pytest.mark.parametrize("kind", ["normal", "grid"])
+def test_knn_list_lengths_vs_oracle(engine, n, k, kind):
+    """Every list length's kernel, with several warps per bucket and with one,
+    and with many points at the k-th distance (grid)."""
+    from fast_hdbscan_gb300.numba_kdtree import build_kdtree, parallel_tree_query
+    from oracle import oracle as O
+
+    if n > 90_000 and (kind == "grid" or k not in (2, 16, 33)):
+        pytest.skip("covered by the smaller sizes")
+    rng = np.random.default_rng(n + 7 * k)
+    d = 2 + k % 3
+    if kind == "grid":
+        X = rng.integers(0, 9, size=(n, d)).astype(np.float32)
+    else:
+        X = (rng.normal(size=(n, d)) * np.exp(rng.normal(size=(n, 1)))).astype(np.float32)
+    tree = build_kdtree(X)
+    rd, ix = parallel_tree_query(tree, tree.data, k=k, output_rdist=True)
+    ord_, oix = O.tree_query(O.build_kdtree(X), k, mode=1)
+    np.testing.assert_array_equal(rd, ord_)
+    np.testing.assert_array_equal(ix, oix)
