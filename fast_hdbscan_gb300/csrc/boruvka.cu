@@ -25,6 +25,7 @@
 // Components merge with a lock-free union-find; edges of a round are written
 // in order of each component's lowest point index (the reference's dict
 // insertion order).
+#include "compact.cuh"
 #include "mst.cuh"
 #include "radius.cuh"
 #include "primitives.cuh"
@@ -63,11 +64,8 @@ __device__ __forceinline__ float key_weight(unsigned long long k) {
 __device__ __forceinline__ int8_t seed_open(float c, float kth, int8_t tie) {
     return (!(c < kth) && (c > kth || tie)) ? 1 : 0;
 }
-__global__ void core_from_knn_kernel(int64_t n, int kk, int k, int ms,
-                                     const float* __restrict__ knn_d_s, float* __restrict__ core2,
-                                     int8_t* __restrict__ open) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
+__device__ __forceinline__ void core_body(int64_t p, int kk, int k, int ms, const float* knn_d_s,
+                                          float* core2, int8_t* open) {
     const float kth = knn_d_s[p * kk + kk - 1];
     const float c = ms <= 1 ? 0.0f : (k > kk ? INFINITY : kth);
     core2[p] = c;
@@ -107,72 +105,121 @@ __global__ void gather_weights_kernel(int64_t n, const int32_t* __restrict__ ori
 // Core distances in caller order; neighbour columns past the kNN list (the
 // reference's padding when k exceeds the point count) are -1.  The kNN kernel
 // writes the other neighbour columns itself.
-__global__ void outputs_kernel(int64_t n, int kk, int k, const int32_t* __restrict__ orig,
-                               const float* __restrict__ core2, float* __restrict__ core_o,
-                               int32_t* __restrict__ nbr_o) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    int64_t o = orig[p];
+__device__ __forceinline__ void outputs_body(int64_t p, int kk, int k, const int32_t* orig,
+                                             const float* core2, float* core_o, int32_t* nbr_o) {
+    const int64_t o = orig[p];
     if (core_o) core_o[o] = __fsqrt_rn(core2[p]);
     if (nbr_o)
         for (int j = kk > 1 ? kk : 1; j < k; ++j) nbr_o[o * (k - 1) + j - 1] = -1;
 }
+// core_from_knn: the unweighted core distances first.
+__global__ void core_outputs_kernel(int64_t n, int kk, int k, int ms, int core_from_knn,
+                                    const float* __restrict__ knn_d_s, float* core2,
+                                    int8_t* open, const int32_t* __restrict__ orig, float* core_o,
+                                    int32_t* nbr_o) {
+    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    if (core_from_knn) core_body(p, kk, k, ms, knn_d_s, core2, open);
+    outputs_body(p, kk, k, orig, core2, core_o, nbr_o);
+}
+
+// ------------------------------------------------------- state of the rounds
+// Everything a round reads and writes, in index order unless noted.  The
+// bodies below take it by value and are run by one kernel each, or -- for few
+// points, where the launches themselves are the time -- one after the other
+// inside a single block (small_*_kernel).  No pointer is __restrict__: a block
+// reads what it wrote a barrier earlier.
+// Counts and flags kept on the device: edges and components so far, edges of
+// the round, flags, rounds and the components at the start of each.
+enum : int { kStEdges = 0, kStComps, kStAdded, kStMissing, kStEqual, kStRounds, kStHistory };
+constexpr int kStWords = kStHistory + kMaxRounds;
+struct BorState {
+    int64_t n, nleaves, slots;
+    int k, ref_ties, plain_d;
+    const int32_t *orig, *rank;
+    const float* knn_d;
+    const int32_t* knn_s;
+    float* core2;
+    int32_t *target, *par, *comp;  // par: union-find over points, then components
+    float* w0;
+    // cmin: a component's lowest caller index.  The components in its order
+    // (the reference's dict order): representative and cmin; next round's.
+    int32_t *cmin, *reps, *rep_cmin, *next_reps, *next_cmin;
+    unsigned long long* keyA;
+    uint32_t* keyB;
+    int32_t *winner, *tgt;
+    float* cand_w;
+    int32_t* cand_q;
+    int8_t* exhausted;
+    int2* nc;
+    int32_t *src, *dst;
+    float* w2;
+    uint32_t* stat;  // [kStWords]
+};
 
 // ----------------------------------------------------------------- round 0
 // plain_d: the weighted path's round 0 works on plain (not squared) distances.
-__global__ void round0_kernel(int64_t n, int k, const int32_t* __restrict__ knn_s,
-                              const float* __restrict__ knn_d, const float* __restrict__ core2,
-                              int plain_d, int32_t* __restrict__ target, float* __restrict__ w0,
-                              int* __restrict__ eq_flag) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const float cp = core2[p];
+__device__ __forceinline__ void round0_body(const BorState& S, int64_t p) {
+    const int k = S.k;
+    const float cp = S.core2[p];
     int32_t t = -1;
     float w = 0.0f;
     for (int j = 1; j < k; ++j) {
-        int32_t q = knn_s[p * k + j];
+        const int32_t q = S.knn_s[p * k + j];
         if (q < 0) break;
-        float cq = core2[q];
+        const float cq = S.core2[q];
         if (cp >= cq) {
             if (q != p) {
                 t = q;
-                const float d = knn_d[p * k + j];
-                w = fmaxf(cp, plain_d ? __fsqrt_rn(d) : d);
-                if (cq == cp) atomicOr(eq_flag, 1);
+                const float d = S.knn_d[p * k + j];
+                w = fmaxf(cp, S.plain_d ? __fsqrt_rn(d) : d);
+                if (cq == cp) S.stat[kStEqual] = 1u;
             }
             break;
         }
     }
-    target[p] = t;
-    w0[p] = w;
+    S.target[p] = t;
+    S.w0[p] = w;
+    S.par[p] = (int32_t)p;
+    S.cmin[p] = INT32_MAX;
+    S.cand_q[p] = -1;  // no candidate yet
+    S.exhausted[p] = 0;
+}
+__global__ void round0_kernel(BorState S) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < S.n) round0_body(S, p);
 }
 
-__global__ void iota_kernel(int32_t* a, int64_t n) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = (int32_t)i;
+__device__ __forceinline__ void union_target_body(const BorState& S, int64_t p) {
+    const int32_t t = S.target[p];
+    if (t >= 0) uf_union(S.par, (int32_t)p, t);
 }
-
-__global__ void union_targets_kernel(int32_t* par, const int32_t* __restrict__ target, int64_t n) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    int32_t t = target[p];
-    if (t >= 0) uf_union(par, (int32_t)p, t);
+__global__ void union_targets_kernel(BorState S) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < S.n) union_target_body(S, p);
 }
-
-__global__ void flatten_kernel(int32_t* par, int32_t* __restrict__ comp, int64_t n) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    comp[p] = uf_find(par, (int32_t)p);
+__device__ __forceinline__ void flatten_body(const BorState& S, int64_t p) {
+    const int32_t c = uf_find(S.par, (int32_t)p);
+    S.comp[p] = c;
+    // most points find their component's minimum already at or below theirs
+    const int32_t o = S.orig[p];
+    if (o < *(volatile int32_t*)&S.cmin[c]) atomicMin(&S.cmin[c], o);
+}
+__global__ void flatten_kernel(BorState S) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < S.n) flatten_body(S, p);
 }
 
 // Functional-graph cycle detection by pointer doubling (only run when some
 // round-0 link joins two equal core distances).
-__global__ void cyc_init_kernel(int64_t n, const int32_t* __restrict__ target,
-                                const int32_t* __restrict__ orig, int32_t* nxt, int32_t* mx) {
+__device__ __forceinline__ void cyc_init_body(const BorState& S, int64_t p, int32_t* nxt,
+                                              int32_t* mx) {
+    nxt[p] = S.target[p] >= 0 ? S.target[p] : (int32_t)p;
+    mx[p] = S.orig[p];
+}
+__global__ void cyc_init_kernel(BorState S, int32_t* nxt, int32_t* mx) {
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    nxt[p] = target[p] >= 0 ? target[p] : (int32_t)p;
-    mx[p] = orig[p];
+    if (p < S.n) cyc_init_body(S, p, nxt, mx);
 }
 // `changed` (nullable) is set when some node's window maximum grew.  A step
 // that grows none has converged: every node's maximum is then at least the
@@ -188,101 +235,104 @@ __global__ void cyc_step_kernel(int64_t n, const int32_t* __restrict__ nxt,
     mx2[p] = max(a, b);
     if (changed && b > a) *changed = 1;
 }
-__global__ void cyc_drop_kernel(int64_t n, const int32_t* __restrict__ nxt,
-                                const int32_t* __restrict__ mx, const int32_t* __restrict__ orig,
-                                int32_t* __restrict__ target) {
+__device__ __forceinline__ void cyc_drop_body(const BorState& S, int64_t p, const int32_t* nxt,
+                                              const int32_t* mx) {
+    if (S.target[p] >= 0 && mx[nxt[p]] == S.orig[p]) S.target[p] = -1;
+}
+__global__ void cyc_drop_kernel(BorState S, const int32_t* nxt, const int32_t* mx) {
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    if (target[p] >= 0 && mx[nxt[p]] == orig[p]) target[p] = -1;
+    if (p < S.n) cyc_drop_body(S, p, nxt, mx);
 }
 
-// `by` (nullable) numbers the points for the edge order: caller indices, or
-// NULL for the index positions themselves.
-__global__ void r0_flags_kernel(int64_t n, const int32_t* __restrict__ target,
-                                const int32_t* __restrict__ by, uint32_t* __restrict__ flag) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    flag[by ? by[p] : p] = target[p] >= 0 ? 1u : 0u;
-}
-__global__ void r0_emit_kernel(int64_t n, const int32_t* __restrict__ target,
-                               const float* __restrict__ w0, const int32_t* __restrict__ orig,
-                               const int32_t* __restrict__ by, const uint32_t* __restrict__ pos,
-                               int32_t* __restrict__ src, int32_t* __restrict__ dst,
-                               float* __restrict__ w2) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    int32_t t = target[p];
-    if (t < 0) return;
-    int32_t op = orig[p];
-    uint32_t i = pos[by ? by[p] : p];
-    src[i] = op;
-    dst[i] = orig[t];
-    w2[i] = w0[p];
-}
+// Round-0 edges, by caller index of the choosing point (the reference's
+// order), or in index order when the order does not matter.
+struct Round0Edges {
+    BorState S;
+    int by_caller;
+    __device__ int32_t point(int64_t i) const { return by_caller ? S.rank[i] : (int32_t)i; }
+    __device__ bool test(int64_t i) const { return S.target[point(i)] >= 0; }
+    __device__ void emit(int64_t i, uint32_t at) const {
+        const int32_t p = point(i);
+        S.src[at] = S.orig[p];
+        S.dst[at] = S.orig[S.target[p]];
+        S.w2[at] = S.w0[p];
+    }
+    __device__ void each(int64_t) const {}
+};
 
-__global__ void cmin_init_kernel(int64_t n, int32_t* cmin) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < n) cmin[p] = INT32_MAX;
+__device__ __forceinline__ void reset_component(const BorState& S, int32_t c) {
+    S.keyA[c] = ~0ull;
+    S.keyB[c] = 0xffffffffu;
+    S.winner[c] = -1;
 }
-__global__ void cmin_points_kernel(int64_t n, const int32_t* __restrict__ comp,
-                                   const int32_t* __restrict__ orig, int32_t* cmin) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < n) atomicMin(&cmin[comp[p]], orig[p]);
-}
-__global__ void rep_flags_kernel(int64_t n, const int32_t* __restrict__ comp,
-                                 uint32_t* __restrict__ flag) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < n) flag[p] = comp[p] == (int32_t)p ? 1u : 0u;
-}
-__global__ void compact_kernel(int64_t n, const uint32_t* __restrict__ flag,
-                               const uint32_t* __restrict__ pos, const int32_t* __restrict__ src,
-                               int32_t* __restrict__ out) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && flag[i]) out[pos[i]] = src ? src[i] : (int32_t)i;
-}
+// The components in the order of their lowest caller index i.
+struct FirstComponents {
+    BorState S;
+    __device__ bool test(int64_t i) const { return S.cmin[S.comp[S.rank[i]]] == (int32_t)i; }
+    __device__ void emit(int64_t i, uint32_t at) const {
+        const int32_t c = S.comp[S.rank[i]];
+        S.reps[at] = c;
+        S.rep_cmin[at] = (int32_t)i;
+        reset_component(S, c);
+    }
+    __device__ void each(int64_t) const {}
+};
 
 // ---------------------------------------------------------- per round: nodes
 // Per node: x = its single component (node_comp, boruvka.py:98-124), kMixed
 // or kEmpty; y = bits of the least core distance of its points.  Every edge
 // into the node weighs at least that core distance, so a node whose least
 // core distance exceeds a query's threshold is skipped like a distant one.
-__global__ void node_comp_leaf_kernel(const int32_t* __restrict__ comp,
-                                      const float* __restrict__ core2, int64_t n,
-                                      int64_t nleaves, int64_t slots, int2* __restrict__ nc) {
-    int64_t leaf = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (leaf >= slots) return;
-    int64_t i = leaf * kLeaf + lane;
-    bool valid = leaf < nleaves && i < n;
-    int32_t c = valid ? comp[i] : 0;
+// The kernels cover the tree in pieces: a block joins the kNodeLeaves leaves of
+// its chunk up to the chunk's root, then blocks of kNodeTop nodes go on.  A
+// leaf's points take their new component first (relabel).
+constexpr int kNodeLeaves = 64, kNodeThreads = 256, kNodeTop = 512;
+__device__ __forceinline__ void leaf_node_body(const BorState& S, int64_t leaf, int lane,
+                                               int relabel) {
+    const int64_t i = leaf * kLeaf + lane;
+    const bool valid = leaf < S.nleaves && i < S.n;
+    int32_t c = 0;
+    if (valid) {
+        c = S.comp[i];
+        if (relabel) {
+            c = uf_find(S.par, c);
+            S.comp[i] = c;
+        }
+    }
     // non-negative floats order like their bit patterns
-    int32_t kb = valid ? __float_as_int(core2[i]) : INT32_MAX;
-    int32_t c0 = __shfl_sync(kFull, c, 0);
-    bool same = __all_sync(kFull, !valid || c == c0);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) kb = min(kb, __shfl_xor_sync(kFull, kb, o));
+    int32_t kb = valid ? __float_as_int(S.core2[i]) : INT32_MAX;
+    const int32_t c0 = __shfl_sync(kFull, c, 0);
+    const bool same = __all_sync(kFull, !valid || c == c0);
+    kb = __reduce_min_sync(kFull, kb);
     if (lane == 0)
-        nc[slots - 1 + leaf] = make_int2(leaf >= nleaves ? kEmpty : (same ? c0 : kMixed), kb);
+        S.nc[S.slots - 1 + leaf] =
+            make_int2(leaf >= S.nleaves ? kEmpty : (same ? c0 : kMixed), kb);
 }
-__global__ void node_comp_level_kernel(int2* __restrict__ nc, int64_t first, int64_t count) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    int64_t node = first + t;
+__device__ __forceinline__ void join_node_body(int2* nc, int64_t node) {
     const int2 l = nc[2 * node + 1], r = nc[2 * node + 2];
     nc[node] = make_int2(l.x == kEmpty ? r.x : (r.x == kEmpty ? l.x : (l.x == r.x ? l.x : kMixed)),
                          min(l.y, r.y));
 }
-
-__global__ void reset_keys_kernel(const int32_t* __restrict__ reps, int64_t nrep,
-                                  unsigned long long* keyA, uint32_t* keyB, int32_t* winner,
-                                  int32_t* par) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nrep) return;
-    int32_t c = reps[i];
-    keyA[c] = ~0ull;
-    keyB[c] = 0xffffffffu;
-    winner[c] = -1;
-    par[c] = c;
+__global__ void __launch_bounds__(kNodeThreads) node_chunk_kernel(BorState S, int relabel) {
+    const int leaves = (int)min(S.slots, (int64_t)kNodeLeaves);
+    for (int l = threadIdx.x >> 5; l < leaves; l += kNodeThreads / 32)
+        leaf_node_body(S, (int64_t)blockIdx.x * kNodeLeaves + l, threadIdx.x & 31, relabel);
+    int64_t level = S.slots - 1;
+    for (int width = leaves / 2; width >= 1; width >>= 1) {
+        __syncthreads();
+        level = (level - 1) / 2;
+        if (threadIdx.x < width)
+            join_node_body(S.nc, level + (int64_t)blockIdx.x * width + threadIdx.x);
+    }
+}
+__global__ void __launch_bounds__(kNodeTop / 2) node_top_kernel(int2* nc, int64_t width) {
+    const int span = (int)min(width, (int64_t)kNodeTop);
+    int64_t level = width - 1;
+    for (int wd = span / 2; wd >= 1; wd >>= 1) {
+        level = (level - 1) / 2;
+        if (threadIdx.x < wd) join_node_body(nc, level + (int64_t)blockIdx.x * wd + threadIdx.x);
+        __syncthreads();
+    }
 }
 
 // ------------------------------------------------------- per round: seeds
@@ -291,15 +341,9 @@ __global__ void reset_keys_kernel(const int32_t* __restrict__ reps, int64_t nrep
 // search starts from every component's seed bound.
 // exhausted[p]: every kNN neighbour of p was already in p's component in an
 // earlier round -- it stays so, as components only merge.
-__global__ void seed_kernel(int64_t n, int k, const int32_t* __restrict__ knn_s,
-                            const float* __restrict__ knn_d, const float* __restrict__ core2,
-                            const int32_t* __restrict__ comp, const int32_t* __restrict__ orig,
-                            unsigned long long* keyA, float* __restrict__ cand_w,
-                            int32_t* __restrict__ cand_q, int8_t* __restrict__ exhausted,
-                            int ref_ties) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const int32_t c = comp[p];
+__device__ __forceinline__ void seed_body(const BorState& S, int64_t p) {
+    const int k = S.k;
+    const int32_t c = S.comp[p];
     // The previous round's candidate of this point is still an edge out of
     // its component when its target has not been merged in: it seeds the
     // point's best (when it beats the kNN seed) and its component's key
@@ -308,38 +352,43 @@ __global__ void seed_kernel(int64_t n, int k, const int32_t* __restrict__ knn_s,
     // weight equals the core distance only for a target inside the kNN
     // radius, which the kNN seed has already met, so the seed-finality rule
     // below is unaffected.)
-    const int32_t oq = cand_q[p];
-    const float ow = cand_w[p];
-    const int32_t oo = (oq >= 0 && comp[oq] != c) ? orig[oq] : -1;
+    const int32_t oq = S.cand_q[p];
+    const float ow = S.cand_w[p];
+    const int32_t oo = (oq >= 0 && S.comp[oq] != c) ? S.orig[oq] : -1;
     float bw = INFINITY;
     int32_t bq = -1, bo = INT32_MAX;
-    if (!exhausted[p]) {
-        const float cp = core2[p];
+    if (!S.exhausted[p]) {
+        const float cp = S.core2[p];
         for (int j = 1; j < k; ++j) {
-            int32_t qs = knn_s[p * k + j];
+            const int32_t qs = S.knn_s[p * k + j];
             if (qs < 0) break;
-            if (comp[qs] == c) continue;
-            float w = fmaxf(fmaxf(knn_d[p * k + j], cp), core2[qs]);
-            int32_t o = orig[qs];
+            if (S.comp[qs] == c) continue;
+            const float w = fmaxf(fmaxf(S.knn_d[p * k + j], cp), S.core2[qs]);
+            const int32_t o = S.orig[qs];
             if (w < bw || (w == bw && o < bo)) {
                 bw = w;
                 bq = qs;
                 bo = o;
             }
         }
-        if (bq < 0) exhausted[p] = 1;  // no other component in the kNN list
+        if (bq < 0) S.exhausted[p] = 1;  // no other component in the kNN list
     }
     if (oo >= 0 && (ow < bw || (ow == bw && oo < bo))) {
         bw = ow;
         bq = oq;
         bo = oo;
     }
-    cand_w[p] = bw;
-    cand_q[p] = bq;
+    S.cand_w[p] = bw;
+    S.cand_q[p] = bq;
     if (bq >= 0) {
-        unsigned long long key = pack_key(bw, ref_ties ? orig[p] : min(orig[p], bo));
-        if (key < *(volatile unsigned long long*)&keyA[c]) atomicMin(&keyA[c], key);
+        const unsigned long long key =
+            pack_key(bw, S.ref_ties ? S.orig[p] : min(S.orig[p], bo));
+        if (key < *(volatile unsigned long long*)&S.keyA[c]) atomicMin(&S.keyA[c], key);
     }
+}
+__global__ void seed_kernel(BorState S) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < S.n) seed_body(S, p);
 }
 
 // ------------------------------------------------------- per round: search
@@ -361,7 +410,7 @@ __global__ void __launch_bounds__(kSW * 32) search_kernel(
     const float* __restrict__ core2, const int32_t* __restrict__ comp,
     const int2* __restrict__ nc, unsigned long long* keyA, float* __restrict__ cand_w,
     int32_t* __restrict__ cand_q, int lvl_lo, int lvl_hi, const int32_t* __restrict__ plist,
-    int64_t plen, int ref_ties) {
+    int64_t plen, int ref_ties, int split, const uint32_t* __restrict__ stat) {
     __shared__ int32_t s_stack[kSW][kStack];
     __shared__ float4 s_xyz[kSW][32 * (SP / 4)];
     __shared__ int2 s_cc[kSW][32];      // (component, core bits)
@@ -370,12 +419,16 @@ __global__ void __launch_bounds__(kSW * 32) search_kernel(
     // Dense: warp = bucket, lane = point.  Sparse (plist): warp = 32
     // consecutive entries of a list of the points still searching (in index
     // order), each searching from the root.
+    // `split` warps share a bucket's points, 32 / split each.
     const bool sparse = plist != nullptr;
-    const int64_t leaf = (int64_t)blockIdx.x * kSW + warp;
+    const int64_t part = (int64_t)blockIdx.x * kSW + warp;
+    const int64_t leaf = part / split;
     if (sparse ? leaf * 32 >= plen : leaf >= ix.nleaves) return;
+    if (stat[kStComps] <= 1) return;  // (a round launched after the last)
     const int64_t li = leaf * 32 + lane;
     const int64_t p = sparse ? (li < plen ? plist[li] : 0) : leaf * kLeaf + lane;
-    const bool valid = sparse ? li < plen : p < ix.n;
+    const bool valid =
+        lane * split / 32 == (int)(part % split) && (sparse ? li < plen : p < ix.n);
     int32_t c = -3;
     float cp = 0.0f, bw = INFINITY;
     int32_t bq = -1, bo = INT32_MAX;
@@ -565,125 +618,237 @@ __global__ void __launch_bounds__(kSW * 32) search_kernel(
     if (key < *(volatile unsigned long long*)&keyA[c]) atomicMin(&keyA[c], key);
 }
 
-// The points that start the global pass searching (as search_kernel decides).
-__global__ void searching_flags_kernel(int64_t n, const int8_t* __restrict__ knn_open,
-                                       const float* __restrict__ core2,
-                                       const int32_t* __restrict__ comp,
-                                       const unsigned long long* __restrict__ keyA,
-                                       const float* __restrict__ cand_w,
-                                       const int32_t* __restrict__ cand_q,
-                                       uint32_t* __restrict__ flag) {
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const float cp = core2[p], bw = cand_w[p];
-    const bool settled = cand_q[p] >= 0 && bw == cp && !knn_open[p];
-    const float thr0 = fminf(bw, key_weight(keyA[comp[p]]));
-    flag[p] = (!settled && !(cp > thr0)) ? 1u : 0u;
-}
-__global__ void iota_list_kernel(int64_t n, const uint32_t* __restrict__ flag,
-                                 const uint32_t* __restrict__ pos, int32_t* __restrict__ list) {
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < n && flag[p]) list[pos[p]] = (int32_t)p;
-}
-
-__global__ void stage_b_kernel(int64_t n, const int32_t* __restrict__ comp,
-                               const int32_t* __restrict__ orig, const float* __restrict__ cand_w,
-                               const int32_t* __restrict__ cand_q,
-                               const unsigned long long* __restrict__ keyA, uint32_t* keyB) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    int32_t q = cand_q[p];
-    if (q < 0) return;
-    int32_t c = comp[p], op = orig[p], oq = orig[q];
-    if (keyA[c] == pack_key(cand_w[p], min(op, oq))) atomicMin(&keyB[c], (uint32_t)max(op, oq));
-}
-__global__ void stage_c_kernel(int64_t n, const int32_t* __restrict__ comp,
-                               const int32_t* __restrict__ orig, const float* __restrict__ cand_w,
-                               const int32_t* __restrict__ cand_q,
-                               const unsigned long long* __restrict__ keyA,
-                               const uint32_t* __restrict__ keyB, int32_t* winner) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    int32_t q = cand_q[p];
-    if (q < 0) return;
-    int32_t c = comp[p], op = orig[p], oq = orig[q];
-    if (keyA[c] == pack_key(cand_w[p], min(op, oq)) && keyB[c] == (uint32_t)max(op, oq))
-        winner[c] = (int32_t)p;
-}
-
-__global__ void select_kernel(const int32_t* __restrict__ reps, int64_t nrep,
-                              const int32_t* __restrict__ winner,
-                              const int32_t* __restrict__ cand_q,
-                              const int32_t* __restrict__ comp, int32_t* __restrict__ tgt,
-                              int* __restrict__ missing) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nrep) return;
-    int32_t c = reps[i], p = winner[c];
-    if (p < 0) {
-        tgt[c] = -1;
-        atomicOr(missing, 1);
-        return;
+// The points that start the search searching (as search_kernel decides).
+struct SearchingPoints {
+    BorState S;
+    const int8_t* knn_open;
+    int32_t* list;
+    __device__ bool test(int64_t p) const {
+        const float cp = S.core2[p], bw = S.cand_w[p];
+        const bool settled = S.cand_q[p] >= 0 && bw == cp && !knn_open[p];
+        const float thr0 = fminf(bw, key_weight(S.keyA[S.comp[p]]));
+        return !settled && !(cp > thr0);
     }
-    tgt[c] = comp[cand_q[p]];
+    __device__ void emit(int64_t p, uint32_t at) const { list[at] = (int32_t)p; }
+    __device__ void each(int64_t) const {}
+};
+
+// ---------------------------------------------------- per round: the merge
+// Every component's winner: the point that holds its least (weight, lowest
+// index) with, among those, the least highest index.
+__device__ __forceinline__ void stage_b_body(const BorState& S, int64_t p) {
+    const int32_t q = S.cand_q[p];
+    if (q < 0) return;
+    const int32_t c = S.comp[p], op = S.orig[p], oq = S.orig[q];
+    if (S.keyA[c] == pack_key(S.cand_w[p], min(op, oq)))
+        atomicMin(&S.keyB[c], (uint32_t)max(op, oq));
+}
+__device__ __forceinline__ void stage_c_body(const BorState& S, int64_t p) {
+    const int32_t q = S.cand_q[p];
+    if (q < 0) return;
+    const int32_t c = S.comp[p], op = S.orig[p], oq = S.orig[q];
+    if (S.keyA[c] == pack_key(S.cand_w[p], min(op, oq)) && S.keyB[c] == (uint32_t)max(op, oq))
+        S.winner[c] = (int32_t)p;
+}
+__global__ void stage_b_kernel(BorState S) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < S.n) stage_b_body(S, p);
+}
+__global__ void stage_c_kernel(BorState S) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < S.n) stage_c_body(S, p);
 }
 
-__global__ void emit_flags_kernel(const int32_t* __restrict__ reps, int64_t nrep,
-                                  const int32_t* __restrict__ tgt,
-                                  const int32_t* __restrict__ cmin, uint32_t* __restrict__ flag) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nrep) return;
-    int32_t c = reps[i], t = tgt[c];
-    if (t < 0) return;
-    bool mutual = tgt[t] == c;
-    if (!mutual || cmin[c] < cmin[t]) flag[cmin[c]] = 1u;
+__device__ __forceinline__ void select_body(const BorState& S, int64_t i) {
+    const int32_t c = S.reps[i], p = S.winner[c];
+    S.tgt[c] = p < 0 ? -1 : S.comp[S.cand_q[p]];
+    if (p < 0) S.stat[kStMissing] = 1u;
+}
+// The round's edges, in the order of the components' lowest caller indices:
+// of a pair that chose each other, the first one's.  (In the reference tie
+// mode the cycles have been dropped from tgt already.)
+struct RoundEdges {
+    BorState S;
+    __device__ bool test(int64_t i) const {
+        const int32_t c = S.reps[i], t = S.tgt[c];
+        if (t < 0) return false;
+        return S.ref_ties || S.tgt[t] != c || S.cmin[c] < S.cmin[t];
+    }
+    __device__ void emit(int64_t i, uint32_t at) const {
+        const int32_t p = S.winner[S.reps[i]];
+        const uint32_t e = S.stat[kStEdges] + at;
+        S.src[e] = S.orig[p];
+        S.dst[e] = S.orig[S.cand_q[p]];
+        S.w2[e] = S.cand_w[p];
+    }
+    __device__ void each(int64_t i) const {
+        const int32_t c = S.reps[i], t = S.tgt[c];
+        if (t >= 0) uf_union(S.par, c, t);
+    }
+};
+__device__ __forceinline__ void merge_cmin_body(const BorState& S, int64_t i) {
+    const int32_t c = S.reps[i], r = uf_find(S.par, c);
+    if (r != c) atomicMin(&S.cmin[r], S.rep_cmin[i]);
+}
+// The merged components, each at the place of the old one whose cmin it has.
+struct MergedComponents {
+    BorState S;
+    __device__ bool test(int64_t i) const {
+        return S.cmin[uf_find(S.par, S.reps[i])] == S.rep_cmin[i];
+    }
+    __device__ void emit(int64_t i, uint32_t at) const {
+        const int32_t r = uf_find(S.par, S.reps[i]);
+        S.next_reps[at] = r;
+        S.next_cmin[at] = S.rep_cmin[i];
+        reset_component(S, r);
+    }
+    __device__ void each(int64_t) const {}
+};
+__global__ void select_kernel(BorState S, int64_t ncomp) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < ncomp) select_body(S, i);
+}
+__global__ void merge_cmin_kernel(BorState S, int64_t ncomp) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) S.stat[kStEdges] += S.stat[kStAdded];
+    if (i < ncomp) merge_cmin_body(S, i);
 }
 
-__global__ void emit_write_kernel(const int32_t* __restrict__ reps, int64_t nrep,
-                                  const int32_t* __restrict__ tgt,
-                                  const int32_t* __restrict__ cmin,
-                                  const uint32_t* __restrict__ flag, const uint32_t* __restrict__ pos,
-                                  const int32_t* __restrict__ winner,
-                                  const int32_t* __restrict__ cand_q,
-                                  const float* __restrict__ cand_w,
-                                  const int32_t* __restrict__ orig, int64_t base,
-                                  int32_t* __restrict__ src, int32_t* __restrict__ dst,
-                                  float* __restrict__ w2) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nrep) return;
-    int32_t c = reps[i];
-    if (tgt[c] < 0 || !flag[cmin[c]]) return;
-    int32_t p = winner[c];
-    int64_t e = base + pos[cmin[c]];
-    src[e] = orig[p];
-    dst[e] = orig[cand_q[p]];
-    w2[e] = cand_w[p];
+// ------------------------------------------------- phases inside one block
+// compact() by one block.
+template <class F>
+__device__ __forceinline__ uint32_t block_compact(const F& f, int64_t n) {
+    __shared__ uint32_t s_warp[33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    uint32_t base = 0;
+    for (int64_t i0 = 0; i0 < n; i0 += blockDim.x) {
+        const int64_t i = i0 + threadIdx.x;
+        const bool on = i < n && f.test(i);
+        const unsigned b = __ballot_sync(kFull, on);
+        if (lane == 0) s_warp[w] = __popc(b);
+        __syncthreads();
+        if (w == 0) {
+            const uint32_t v = lane < nw ? s_warp[lane] : 0u;
+            uint32_t x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane < nw) s_warp[lane] = x - v;
+            if (lane == 31) s_warp[32] = x;
+        }
+        __syncthreads();
+        if (on) f.emit(i, base + s_warp[w] + __popc(b & ((1u << lane) - 1u)));
+        if (i < n) f.each(i);
+        base += s_warp[32];
+        __syncthreads();
+    }
+    return base;
+}
+// From tgt to the merged components (kStEdges, kStComps and the list updated).
+__device__ __forceinline__ void block_merge(const BorState& S, int64_t ncomp) {
+    const uint32_t added = block_compact(RoundEdges{S}, ncomp);
+    for (int64_t i = threadIdx.x; i < ncomp; i += blockDim.x) merge_cmin_body(S, i);
+    __syncthreads();
+    const uint32_t left = block_compact(MergedComponents{S}, ncomp);
+    if (threadIdx.x == 0) {
+        S.stat[kStEdges] += added;
+        S.stat[kStComps] = left;
+        S.stat[kStAdded] = added;
+    }
+    for (int64_t i = threadIdx.x; i < left; i += blockDim.x) {
+        S.reps[i] = S.next_reps[i];
+        S.rep_cmin[i] = S.next_cmin[i];
+    }
+    __syncthreads();
+}
+constexpr int kSmallThreads = 1024;
+// Components of one round that a single block merges in one launch.
+constexpr int64_t kBlockMerge = 8192;
+__global__ void __launch_bounds__(kSmallThreads) merge_kernel(BorState S, int64_t ncomp) {
+    if (!S.ref_ties)
+        for (int64_t i = threadIdx.x; i < ncomp; i += blockDim.x) select_body(S, i);
+    __syncthreads();
+    block_merge(S, ncomp);
 }
 
-__global__ void emit_clear_kernel(const int32_t* __restrict__ reps, int64_t nrep,
-                                  const int32_t* __restrict__ cmin, uint32_t* __restrict__ flag) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nrep) flag[cmin[reps[i]]] = 0u;
+// Few points: whole phases in one block.  A launch costs about 2 us however
+// little it does, the host's read of a count 12 us; a phase over 8,192 points
+// costs one block a microsecond or two.
+constexpr int64_t kSmallPoints = 8192, kSmallEntries = 32 * 8192;  // points, list entries
+__device__ __forceinline__ void block_nodes_and_seeds(const BorState& S, int relabel) {
+    for (int64_t l = threadIdx.x >> 5; l < S.slots; l += blockDim.x >> 5)
+        leaf_node_body(S, l, threadIdx.x & 31, relabel);
+    __syncthreads();
+    for (int64_t width = S.slots / 2; width >= 1; width /= 2) {
+        for (int64_t t = threadIdx.x; t < width; t += blockDim.x)
+            join_node_body(S.nc, width - 1 + t);
+        __syncthreads();
+    }
+    for (int64_t p = threadIdx.x; p < S.n; p += blockDim.x) seed_body(S, p);
 }
-
-__global__ void union_reps_kernel(const int32_t* __restrict__ reps, int64_t nrep,
-                                  const int32_t* __restrict__ tgt, int32_t* par) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nrep) return;
-    int32_t c = reps[i], t = tgt[c];
-    if (t >= 0) uf_union(par, c, t);
+// Core distances and outputs (as core_outputs_kernel), round 0, and the nodes
+// and seeds of round 1.
+__global__ void __launch_bounds__(kSmallThreads) small_round0_kernel(
+    BorState S, int kq, int ms, int core_from_knn, int8_t* open, float* core_o, int32_t* nbr_o,
+    int by_caller, int32_t* nxt, int32_t* mx, int32_t* nxt2, int32_t* mx2) {
+    const int64_t n = S.n;
+    if (threadIdx.x < kStWords) S.stat[threadIdx.x] = 0u;
+    for (int64_t p = threadIdx.x; p < n; p += blockDim.x) {
+        if (core_from_knn) core_body(p, S.k, kq, ms, S.knn_d, S.core2, open);
+        outputs_body(p, S.k, kq, S.orig, S.core2, core_o, nbr_o);
+    }
+    __syncthreads();
+    for (int64_t p = threadIdx.x; p < n; p += blockDim.x) round0_body(S, p);
+    __syncthreads();
+    if (S.stat[kStEqual]) {
+        for (int64_t p = threadIdx.x; p < n; p += blockDim.x) cyc_init_body(S, p, nxt, mx);
+        __syncthreads();
+        for (bool grew = true; grew;) {
+            bool more = false;
+            for (int64_t p = threadIdx.x; p < n; p += blockDim.x) {
+                const int32_t q = nxt[p], a = mx[p], b = mx[q];
+                nxt2[p] = nxt[q];
+                mx2[p] = max(a, b);
+                more |= b > a;
+            }
+            grew = __syncthreads_or(more);
+            int32_t* t = nxt; nxt = nxt2; nxt2 = t;
+            t = mx; mx = mx2; mx2 = t;
+        }
+        for (int64_t p = threadIdx.x; p < n; p += blockDim.x) cyc_drop_body(S, p, nxt, mx);
+        __syncthreads();
+    }
+    const uint32_t edges = block_compact(Round0Edges{S, by_caller}, n);
+    for (int64_t p = threadIdx.x; p < n; p += blockDim.x) union_target_body(S, p);
+    __syncthreads();
+    for (int64_t p = threadIdx.x; p < n; p += blockDim.x) flatten_body(S, p);
+    __syncthreads();
+    const uint32_t comps = block_compact(FirstComponents{S}, n);
+    if (threadIdx.x == 0) {
+        S.stat[kStEdges] = edges;
+        S.stat[kStComps] = comps;
+    }
+    if (comps > 1) block_nodes_and_seeds(S, 0);
 }
-__global__ void relabel_points_kernel(int64_t n, int32_t* par, int32_t* __restrict__ comp) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < n) comp[p] = uf_find(par, comp[p]);
-}
-__global__ void merge_cmin_kernel(const int32_t* __restrict__ reps, int64_t nrep, int32_t* par,
-                                  int32_t* cmin, uint32_t* __restrict__ keep) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nrep) return;
-    int32_t c = reps[i];
-    int32_t r = uf_find(par, c);
-    keep[i] = r == c ? 1u : 0u;
-    if (r != c) atomicMin(&cmin[r], cmin[c]);
+// After a round's search: the merge, and the nodes and seeds of the next.
+__global__ void __launch_bounds__(kSmallThreads) small_round_kernel(BorState S) {
+    const int64_t ncomp = S.stat[kStComps];
+    if (ncomp <= 1) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const uint32_t r = S.stat[kStRounds]++;
+        if (r < kMaxRounds) S.stat[kStHistory + r] = (uint32_t)ncomp;
+    }
+    for (int64_t p = threadIdx.x; p < S.n; p += blockDim.x) stage_b_body(S, p);
+    __syncthreads();
+    for (int64_t p = threadIdx.x; p < S.n; p += blockDim.x) stage_c_body(S, p);
+    __syncthreads();
+    for (int64_t i = threadIdx.x; i < ncomp; i += blockDim.x) select_body(S, i);
+    __syncthreads();
+    block_merge(S, ncomp);
+    if (S.stat[kStComps] > 1) block_nodes_and_seeds(S, 1);
 }
 
 // ------------------------------------------- reference tie mode, per round
@@ -845,15 +1010,6 @@ __global__ void crep_drop_kernel(const int32_t* __restrict__ reps, int64_t nrep,
     const int32_t c = reps[i];
     if (tgt[c] >= 0 && mx[nxt[c]] == cmin[c]) tgt[c] = -1;
 }
-__global__ void ref_emit_flags_kernel(const int32_t* __restrict__ reps, int64_t nrep,
-                                      const int32_t* __restrict__ tgt,
-                                      const int32_t* __restrict__ cmin, uint32_t* __restrict__ flag) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nrep) return;
-    const int32_t c = reps[i];
-    if (tgt[c] >= 0) flag[cmin[c]] = 1u;
-}
-
 __global__ void finalize_edges_kernel(int64_t m, const int32_t* __restrict__ src,
                                       const int32_t* __restrict__ dst,
                                       const float* __restrict__ w2, double* __restrict__ edges) {
@@ -864,63 +1020,58 @@ __global__ void finalize_edges_kernel(int64_t m, const int32_t* __restrict__ src
     edges[3 * e + 2] = __dsqrt_rn((double)w2[e]);
 }
 
+// Warps per bucket (or per 32 listed points), as for the kNN: with few of
+// them the latency of one walk is the search's time.
+constexpr int64_t kSearchWarpsWanted = 20 * 152;
+int search_split(int64_t groups) {
+    int split = 1;
+    while (split < 32 && 2 * split * groups <= kSearchWarpsWanted) split *= 2;
+    return split;
+}
+
 template <int DIM>
-int launch_search(const fhg_index& ix, const int8_t* knn_open,
-                  const float* core2, const int32_t* comp, const int2* nc,
-                  unsigned long long* keyA, float* cand_w, int32_t* cand_q, bool* try_sparse,
-                  int ref_ties, cudaStream_t s) {
+int launch_search(Workspace& ws, const fhg_index& ix, const int8_t* knn_open, const BorState& S,
+                  bool one_pass, bool* try_sparse) {
     constexpr int SP = DIM <= 4 ? 4 : (DIM <= 8 ? 8 : DIM);  // as in the kNN kernel
     const int64_t n = ix.n;
+    cudaStream_t s = ws.stream();
+    auto run = [&](int lo, int hi, const int32_t* list, int64_t len) -> int {
+        const int64_t groups = list ? (len + 31) / 32 : ix.nleaves;
+        const int split = search_split(groups);
+        Stage stage(s, "search_kernel");
+        ::fhg::note_launch();
+        search_kernel<DIM, SP><<<grid_for(groups * split, kSW), kSW * 32, 0, s>>>(
+            view_of(ix), knn_open, S.core2, S.comp, S.nc, S.keyA, S.cand_w, S.cand_q, lo, hi, list,
+            len, S.ref_ties, split, S.stat);
+        FHG_CUDA(cudaGetLastError());
+        return FHG_OK;
+    };
     // When few points search (early rounds: most points' best edge is settled
     // by the seeds), one pass runs on a list of them, 32 to a warp, each from
     // the root -- instead of a warp per bucket walking for one or two of its
     // lanes.  Searching only grows with the components, so after the first
     // dense round the list is not made again.
     if (*try_sparse) {
-        Workspace tmp(s);
-        uint32_t *flag, *pos, *cnt;
+        Workspace tmp(ws);
+        uint32_t* cnt;
         int32_t* list;
-        FHG_TRY(tmp.alloc(&flag, (size_t)n));
-        FHG_TRY(tmp.alloc(&pos, (size_t)n));
         FHG_TRY(tmp.alloc(&list, (size_t)n));
         FHG_TRY(tmp.alloc(&cnt, 1));
-        ::fhg::note_launch();
-        searching_flags_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, knn_open, core2, comp, keyA,
-                                                                  cand_w, cand_q, flag);
-        FHG_CUDA(cudaGetLastError());
-        FHG_TRY(scan_exclusive_u32(tmp, flag, pos, n, cnt));
+        FHG_TRY(compact(tmp, SearchingPoints{S, knn_open, list}, n, cnt));
         uint32_t h_cnt = 0;
         FHG_CUDA(cudaMemcpyAsync(&h_cnt, cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         FHG_CUDA(cudaStreamSynchronize(s));
         const int64_t ns = h_cnt;
         if (ns == 0) return FHG_OK;
         *try_sparse = ns * kSparseDen < n * kSparseNum;
-        if (*try_sparse) {
-            ::fhg::note_launch();
-            iota_list_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, flag, pos, list);
-            FHG_CUDA(cudaGetLastError());
-            Stage stage(s, "search_kernel");
-            ::fhg::note_launch();
-            search_kernel<DIM, SP><<<grid_for((ns + 31) / 32, kSW), kSW * 32, 0, s>>>(
-                view_of(ix), knn_open, core2, comp, nc, keyA, cand_w, cand_q, 0, 64, list, ns,
-                ref_ties);
-            FHG_CUDA(cudaGetLastError());
-            return FHG_OK;
-        }
+        if (*try_sparse) return run(0, 64, list, ns);
     }
     // Dense: a local pass (home bucket and the kLocalLevels nearest sibling
     // subtrees), then the rest of the walk -- every component's bound from
     // its nearby candidates is published before any point searches far away.
-    const int spans[2][2] = {{0, kLocalLevels}, {kLocalLevels, 64}};
-    for (const auto& sp : spans) {
-        Stage stage(s, "search_kernel");
-        ::fhg::note_launch();
-        search_kernel<DIM, SP><<<grid_for(ix.nleaves, kSW), kSW * 32, 0, s>>>(
-            view_of(ix), knn_open, core2, comp, nc, keyA, cand_w, cand_q, sp[0], sp[1],
-            nullptr, 0, ref_ties);
-        FHG_CUDA(cudaGetLastError());
-    }
-    return FHG_OK;
+    if (one_pass) return run(0, 64, nullptr, 0);
+    FHG_TRY(run(0, kLocalLevels, nullptr, 0));
+    return run(kLocalLevels, 64, nullptr, 0);
 }
 
 template <int DIM>
@@ -960,31 +1111,20 @@ int tie_walk(const fhg_index& ix, const RefTree& rt, const int32_t* reps, int64_
 #undef FHG_TW
 }
 
-int search_round(const fhg_index& ix, int k, const int32_t* knn_s, const float* knn_d,
-                 const int8_t* knn_open, int8_t* exhausted, const float* core2,
-                 const int32_t* comp,
-                 const int2* nc, unsigned long long* keyA, float* cand_w, int32_t* cand_q,
-                 bool* try_sparse, int ref_ties, cudaStream_t s) {
-    const int64_t n = ix.n;
-    if (n > 0) {
-        ::fhg::note_launch();
-        seed_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, k, knn_s, knn_d, core2, comp, ix.orig,
-                                                       keyA, cand_w, cand_q, exhausted, ref_ties);
-        FHG_CUDA(cudaGetLastError());
-    }
+int search_round(Workspace& ws, const fhg_index& ix, const int8_t* knn_open, const BorState& S,
+                 bool one_pass, bool* try_sparse) {
     switch (ix.d) {
-        case 1: return launch_search<1>(ix, knn_open, core2, comp, nc, keyA, cand_w, cand_q, try_sparse, ref_ties, s);
-        case 2: return launch_search<2>(ix, knn_open, core2, comp, nc, keyA, cand_w, cand_q, try_sparse, ref_ties, s);
-        case 3: return launch_search<3>(ix, knn_open, core2, comp, nc, keyA, cand_w, cand_q, try_sparse, ref_ties, s);
-        case 4: return launch_search<4>(ix, knn_open, core2, comp, nc, keyA, cand_w, cand_q, try_sparse, ref_ties, s);
-        case 5: return launch_search<5>(ix, knn_open, core2, comp, nc, keyA, cand_w, cand_q, try_sparse, ref_ties, s);
-        case 6: return launch_search<6>(ix, knn_open, core2, comp, nc, keyA, cand_w, cand_q, try_sparse, ref_ties, s);
-        case 7: return launch_search<7>(ix, knn_open, core2, comp, nc, keyA, cand_w, cand_q, try_sparse, ref_ties, s);
-        case 8: return launch_search<8>(ix, knn_open, core2, comp, nc, keyA, cand_w, cand_q, try_sparse, ref_ties, s);
+        case 1: return launch_search<1>(ws, ix, knn_open, S, one_pass, try_sparse);
+        case 2: return launch_search<2>(ws, ix, knn_open, S, one_pass, try_sparse);
+        case 3: return launch_search<3>(ws, ix, knn_open, S, one_pass, try_sparse);
+        case 4: return launch_search<4>(ws, ix, knn_open, S, one_pass, try_sparse);
+        case 5: return launch_search<5>(ws, ix, knn_open, S, one_pass, try_sparse);
+        case 6: return launch_search<6>(ws, ix, knn_open, S, one_pass, try_sparse);
+        case 7: return launch_search<7>(ws, ix, knn_open, S, one_pass, try_sparse);
+        case 8: return launch_search<8>(ws, ix, knn_open, S, one_pass, try_sparse);
         default:
-            if (ix.d <= 16)
-                return launch_search<16>(ix, knn_open, core2, comp, nc, keyA, cand_w, cand_q, try_sparse, ref_ties, s);
-            return launch_search<32>(ix, knn_open, core2, comp, nc, keyA, cand_w, cand_q, try_sparse, ref_ties, s);
+            if (ix.d <= 16) return launch_search<16>(ws, ix, knn_open, S, one_pass, try_sparse);
+            return launch_search<32>(ws, ix, knn_open, S, one_pass, try_sparse);
     }
 }
 
@@ -1047,13 +1187,8 @@ int boruvka_mst(Workspace& ws, const fhg_index& ix, int min_samples, MstResult* 
     FHG_TRY(ws.alloc(&out->dst, (size_t)m_cap));
     FHG_TRY(ws.alloc(&out->w2, (size_t)m_cap));
 
-    float *knn_d, *core2, *knn_d_o = nullptr, *w0, *cand_w;
-    int32_t *knn_s, *target, *par, *comp, *cmin, *reps, *reps2, *winner, *tgt,
-        *cand_q;
-    int2* nc;
-    uint32_t *flag, *pos, *keyB, *cnt;
-    unsigned long long* keyA;
-    int* iflag;
+    float *knn_d, *core2;
+    int32_t* knn_s;
     FHG_TRY(ws.alloc(&knn_d, (size_t)(n * k)));
     FHG_TRY(ws.alloc(&knn_s, (size_t)(n * k)));
     int8_t* knn_open;  // the kNN kernel's tie flags, then "seed not provably final"
@@ -1061,9 +1196,9 @@ int boruvka_mst(Workspace& ws, const fhg_index& ix, int min_samples, MstResult* 
     // the neighbours[:, 1:] matrix (kq - 1 columns) straight from the kNN kernel
     const RadiusUse* ru = k <= 64 ? radius_in_use() : nullptr;  // (radius passes: k <= 64)
     if (ru)
-        FHG_TRY(knn_with_radius(ix, k, *ru, knn_d, knn_s, knn_d_o, nbr_o, s, knn_open, kq - 1, 1));
+        FHG_TRY(knn_with_radius(ix, k, *ru, knn_d, knn_s, nullptr, nbr_o, s, knn_open, kq - 1, 1));
     else
-        FHG_TRY(index_knn(ix, k, knn_d, knn_s, knn_d_o, nbr_o, s, knn_open, kq - 1, 1));
+        FHG_TRY(index_knn(ix, k, knn_d, knn_s, nullptr, nbr_o, s, knn_open, kq - 1, 1));
     // the reference tie mode breaks ties in the order of the reference's own
     // KD-tree, built here exactly; its kNN lists (and so round 0 and the
     // neighbour matrix) list equal distances in the order of the reference's
@@ -1084,189 +1219,195 @@ int boruvka_mst(Workspace& ws, const fhg_index& ix, int min_samples, MstResult* 
         FHG_CUDA(cudaStreamSynchronize(s));
         LAUNCH(weighted_core_kernel, n, n, k, kq, min_samples, knn_d, knn_s, w_s, w_last, core2,
                knn_open);
-    } else {
-        LAUNCH(core_from_knn_kernel, n, n, k, kq, min_samples, knn_d, core2, knn_open);
     }
-    if (core_o || nbr_o)
-        LAUNCH(outputs_kernel, n, n, k, kq, ix.orig, core2, core_o, nbr_o);
+    const int core_from_knn = weighted ? 0 : 1;
+    const bool small = n > 1 && !ref_ties && n <= kSmallPoints && n * k <= kSmallEntries;
+    if (!small && (core_from_knn || core_o || nbr_o))
+        LAUNCH(core_outputs_kernel, n, n, k, kq, min_samples, core_from_knn, knn_d, core2,
+               knn_open, ix.orig, core_o, nbr_o);
     if (n < 2) return FHG_OK;
 
-    FHG_TRY(ws.alloc(&target, (size_t)n));
-    FHG_TRY(ws.alloc(&w0, (size_t)n));
-    FHG_TRY(ws.alloc(&par, (size_t)n));
-    FHG_TRY(ws.alloc(&comp, (size_t)n));
-    FHG_TRY(ws.alloc(&cmin, (size_t)n));
-    FHG_TRY(ws.alloc(&flag, (size_t)n));
-    FHG_TRY(ws.alloc(&pos, (size_t)n));
-    FHG_TRY(ws.alloc(&cnt, 2));
-    FHG_TRY(ws.alloc(&iflag, 2));
-    FHG_CUDA(cudaMemsetAsync(iflag, 0, 2 * sizeof(int), s));
-
-    // ---- round 0: kNN-seeded links (boruvka.py:474)
-    std::unique_ptr<Stage> r0_stage(new Stage(s, "boruvka_round0"));
-    LAUNCH(round0_kernel, n, n, k, knn_s, knn_d, core2, weighted ? 1 : 0, target, w0, iflag);
-    int h_flag[2] = {0, 0};
-    FHG_CUDA(cudaMemcpyAsync(h_flag, iflag, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-    FHG_CUDA(cudaStreamSynchronize(s));
-    if (h_flag[0]) {
-        int32_t *nxt, *mx, *nxt2, *mx2;
-        FHG_TRY(ws.alloc(&nxt, (size_t)n));
-        FHG_TRY(ws.alloc(&mx, (size_t)n));
-        FHG_TRY(ws.alloc(&nxt2, (size_t)n));
-        FHG_TRY(ws.alloc(&mx2, (size_t)n));
-        LAUNCH(cyc_init_kernel, n, n, target, ix.orig, nxt, mx);
-        // link chains are short: every fourth step reports whether it changed
-        // anything, and the doubling stops at the first that did not
-        int R = bits_for(n) + 1;
-        for (int r = 0; r < R; ++r) {
-            const bool check = (r & 3) == 3 && r + 1 < R;
-            if (check) FHG_CUDA(cudaMemsetAsync(iflag, 0, sizeof(int), s));
-            LAUNCH(cyc_step_kernel, n, n, nxt, mx, nxt2, mx2, check ? iflag : nullptr);
-            int32_t* t1 = nxt; nxt = nxt2; nxt2 = t1;
-            t1 = mx; mx = mx2; mx2 = t1;
-            if (check) {
-                int h_changed = 1;
-                FHG_CUDA(cudaMemcpyAsync(&h_changed, iflag, sizeof(int), cudaMemcpyDeviceToHost, s));
-                FHG_CUDA(cudaStreamSynchronize(s));
-                if (!h_changed) break;
-            }
-        }
-        LAUNCH(cyc_drop_kernel, n, n, nxt, mx, ix.orig, target);
-    }
+    BorState S;
+    S.n = n;
+    S.nleaves = ix.nleaves;
+    S.slots = ix.slots;
+    S.k = k;
+    S.ref_ties = ref_ties;
+    S.plain_d = weighted ? 1 : 0;
+    S.orig = ix.orig;
+    S.rank = ix.rank;
+    S.knn_d = knn_d;
+    S.knn_s = knn_s;
+    S.core2 = core2;
+    S.src = out->src;
+    S.dst = out->dst;
+    S.w2 = out->w2;
+    for (int32_t** p : {&S.target, &S.par, &S.comp, &S.cmin, &S.reps, &S.rep_cmin, &S.next_reps,
+                        &S.next_cmin, &S.winner, &S.tgt, &S.cand_q})
+        FHG_TRY(ws.alloc(p, (size_t)n));
+    FHG_TRY(ws.alloc(&S.w0, (size_t)n));
+    FHG_TRY(ws.alloc(&S.keyA, (size_t)n));
+    FHG_TRY(ws.alloc(&S.keyB, (size_t)n));
+    FHG_TRY(ws.alloc(&S.cand_w, (size_t)n));
+    FHG_TRY(ws.alloc(&S.exhausted, (size_t)n));
+    FHG_TRY(ws.alloc(&S.nc, (size_t)ix.nnodes));
+    FHG_TRY(ws.alloc(&S.stat, (size_t)kStWords));
+    uint32_t st[kStWords];
+    auto read_stat = [&]() -> int {
+        FHG_CUDA(cudaMemcpyAsync(st, S.stat, sizeof st, cudaMemcpyDeviceToHost, s));
+        FHG_CUDA(cudaStreamSynchronize(s));
+        return FHG_OK;
+    };
+    // the pointer-doubling buffers of round 0 (points) and of the reference
+    // tie mode's rounds (components)
+    int32_t *nxt, *mx, *nxt2, *mx2;
+    for (int32_t** p : {&nxt, &mx, &nxt2, &mx2}) FHG_TRY(ws.alloc(p, (size_t)n));
     // round-0 edges by caller index of the choosing point (the reference's
     // order), or by index position when the order does not matter
-    const int32_t* by = any_order ? nullptr : ix.orig;
-    LAUNCH(r0_flags_kernel, n, n, target, by, flag);
-    FHG_TRY(scan_exclusive_u32(ws, flag, pos, n, cnt));
-    LAUNCH(r0_emit_kernel, n, n, target, w0, ix.orig, by, pos, out->src, out->dst, out->w2);
-    uint32_t h_cnt = 0;
-    FHG_CUDA(cudaMemcpyAsync(&h_cnt, cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    LAUNCH(iota_kernel, n, par, n);
-    LAUNCH(union_targets_kernel, n, par, target, n);
-    LAUNCH(flatten_kernel, n, par, comp, n);
-    LAUNCH(cmin_init_kernel, n, n, cmin);
-    LAUNCH(cmin_points_kernel, n, n, comp, ix.orig, cmin);
-    FHG_CUDA(cudaStreamSynchronize(s));
-    int64_t m = h_cnt;
+    const int by_caller = any_order ? 0 : 1;
 
-    // representatives (component ids) in index order
-    FHG_TRY(ws.alloc(&reps, (size_t)n));
-    FHG_TRY(ws.alloc(&reps2, (size_t)n));
-    LAUNCH(rep_flags_kernel, n, n, comp, flag);
-    FHG_TRY(scan_exclusive_u32(ws, flag, pos, n, cnt));
-    LAUNCH(compact_kernel, n, n, flag, pos, (const int32_t*)nullptr, reps);
-    uint32_t h_ncomp = 0;
-    FHG_CUDA(cudaMemcpyAsync(&h_ncomp, cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    r0_stage.reset();
-    FHG_CUDA(cudaStreamSynchronize(s));
-    int64_t ncomp = h_ncomp;
-
-    FHG_TRY(ws.alloc(&keyA, (size_t)n));
-    FHG_TRY(ws.alloc(&keyB, (size_t)n));
-    FHG_TRY(ws.alloc(&winner, (size_t)n));
-    FHG_TRY(ws.alloc(&tgt, (size_t)n));
-    FHG_TRY(ws.alloc(&nc, (size_t)ix.nnodes));
-    FHG_TRY(ws.alloc(&cand_w, (size_t)n));
-    FHG_TRY(ws.alloc(&cand_q, (size_t)n));
-    FHG_CUDA(cudaMemsetAsync(cand_q, 0xff, sizeof(int32_t) * n, s));  // no candidate yet (-1)
-    int8_t* exhausted;
-    FHG_TRY(ws.alloc(&exhausted, (size_t)n));
-    FHG_CUDA(cudaMemsetAsync(exhausted, 0, (size_t)n, s));
-    uint32_t* kpos;
-    FHG_TRY(ws.alloc(&kpos, (size_t)n));
-    FHG_CUDA(cudaMemsetAsync(flag, 0, sizeof(uint32_t) * n, s));
-
-    // the reference tie mode's pointer-doubling buffers
-    int32_t *cy_nxt = nullptr, *cy_mx = nullptr, *cy_nxt2 = nullptr, *cy_mx2 = nullptr;
-    if (ref_ties && ncomp > 1) {
-        FHG_TRY(ws.alloc(&cy_nxt, (size_t)n));
-        FHG_TRY(ws.alloc(&cy_mx, (size_t)n));
-        FHG_TRY(ws.alloc(&cy_nxt2, (size_t)n));
-        FHG_TRY(ws.alloc(&cy_mx2, (size_t)n));
+    // ---- round 0: kNN-seeded links (boruvka.py:474)
+    {
+        Stage stage(s, "boruvka_round0");
+        if (small) {
+            ::fhg::note_launch();
+            small_round0_kernel<<<1, kSmallThreads, 0, s>>>(S, kq, min_samples, core_from_knn,
+                                                            knn_open, core_o, nbr_o, by_caller, nxt,
+                                                            mx, nxt2, mx2);
+            FHG_CUDA(cudaGetLastError());
+        } else {
+            FHG_CUDA(cudaMemsetAsync(S.stat, 0, sizeof st, s));
+            LAUNCH(round0_kernel, n, S);
+            FHG_TRY(read_stat());
+            if (st[kStEqual]) {
+                LAUNCH(cyc_init_kernel, n, S, nxt, mx);
+                // link chains are short: every fourth step reports whether it
+                // changed anything, and the doubling stops at the first that
+                // did not
+                int* grew = reinterpret_cast<int*>(S.stat + kStEqual);
+                const int R = bits_for(n) + 1;
+                for (int r = 0; r < R; ++r) {
+                    const bool check = (r & 3) == 3 && r + 1 < R;
+                    if (check) FHG_CUDA(cudaMemsetAsync(grew, 0, sizeof(int), s));
+                    LAUNCH(cyc_step_kernel, n, n, nxt, mx, nxt2, mx2, check ? grew : nullptr);
+                    std::swap(nxt, nxt2);
+                    std::swap(mx, mx2);
+                    if (check) {
+                        FHG_TRY(read_stat());
+                        if (!st[kStEqual]) break;
+                    }
+                }
+                LAUNCH(cyc_drop_kernel, n, S, nxt, mx);
+            }
+            FHG_TRY(compact(ws, Round0Edges{S, by_caller}, n, S.stat + kStEdges));
+            LAUNCH(union_targets_kernel, n, S);
+            LAUNCH(flatten_kernel, n, S);
+            FHG_TRY(compact(ws, FirstComponents{S}, n, S.stat + kStComps));
+        }
     }
 
     int rounds = 0;
+    bool dense = false;  // small inputs never make a list of the searching points
     bool try_sparse = true;  // until a round's global pass is dense
-    while (ncomp > 1) {
-        if (rounds >= kMaxRounds) {
-            set_error("boruvka: no convergence after %d rounds (%lld components left)", rounds,
-                      (long long)ncomp);
-            return FHG_ERR_NO_CONVERGENCE;
+    if (small) {
+        // two rounds between the host's reads: a round after the last costs
+        // less than a read
+        for (;;) {
+            FHG_TRY(read_stat());
+            if (st[kStComps] <= 1 || st[kStMissing] || st[kStRounds] >= kMaxRounds) break;
+            for (int r = 0; r < 2; ++r) {
+                {
+                    Stage stage(s, "boruvka_search");
+                    FHG_TRY(search_round(ws, ix, knn_open, S, /*one_pass=*/true, &dense));
+                }
+                Stage stage(s, "boruvka_merge");
+                ::fhg::note_launch();
+                small_round_kernel<<<1, kSmallThreads, 0, s>>>(S);
+                FHG_CUDA(cudaGetLastError());
+            }
         }
-        profile_count("boruvka_components", (double)ncomp);  // C_r of the round
-        {  // node_comp (boruvka.py:98-124), bottom-up
-            Stage stage(s, "boruvka_nodes");
-            LAUNCH(node_comp_leaf_kernel, ix.slots * 32, comp, core2, n, ix.nleaves, ix.slots, nc);
-            for (int64_t width = ix.slots / 2; width >= 1; width /= 2)
-                LAUNCH(node_comp_level_kernel, width, nc, width - 1, width);
-            LAUNCH(reset_keys_kernel, ncomp, reps, ncomp, keyA, keyB, winner, par);
-        }
-        {
-            Stage stage(s, "boruvka_search");
-            FHG_TRY(search_round(ix, k, knn_s, knn_d, knn_open, exhausted, core2, comp, nc, keyA,
-                                 cand_w, cand_q, &try_sparse, ref_ties, s));
-        }
-        Stage merge_stage(s, "boruvka_merge");
-        FHG_CUDA(cudaMemsetAsync(iflag + 1, 0, sizeof(int), s));
-        if (ref_ties) {
-            LAUNCH(ref_winner_kernel, ncomp, reps, ncomp, keyA, ix.rank, winner);
-            FHG_TRY(tie_walk(ix, rt, reps, ncomp, comp, core2, nc, winner, cand_w, cand_q, tgt,
-                             iflag + 1, s));
-            LAUNCH(crep_init_kernel, ncomp, reps, ncomp, tgt, cmin, cy_nxt, cy_mx);
-            const int R = bits_for(ncomp) + 1;
-            for (int r = 0; r < R; ++r) {
-                const bool check = (r & 3) == 3 && r + 1 < R;
-                if (check) FHG_CUDA(cudaMemsetAsync(iflag, 0, sizeof(int), s));
-                LAUNCH(crep_step_kernel, ncomp, reps, ncomp, cy_nxt, cy_mx, cy_nxt2, cy_mx2,
-                       check ? iflag : nullptr);
-                int32_t* t1 = cy_nxt; cy_nxt = cy_nxt2; cy_nxt2 = t1;
-                t1 = cy_mx; cy_mx = cy_mx2; cy_mx2 = t1;
-                if (check) {
-                    int h_changed = 1;
-                    FHG_CUDA(cudaMemcpyAsync(&h_changed, iflag, sizeof(int),
-                                             cudaMemcpyDeviceToHost, s));
-                    FHG_CUDA(cudaStreamSynchronize(s));
-                    if (!h_changed) break;
+        rounds = (int)st[kStRounds];
+        for (int r = 0; r < rounds && r < kMaxRounds; ++r)  // C_r of the rounds
+            profile_count("boruvka_components", (double)st[kStHistory + r]);
+    } else {
+        FHG_TRY(read_stat());
+        while (st[kStComps] > 1) {
+            const int64_t ncomp = st[kStComps], edges = st[kStEdges];
+            if (rounds >= kMaxRounds) break;
+            profile_count("boruvka_components", (double)ncomp);  // C_r of the round
+            {  // node_comp (boruvka.py:98-124), bottom-up
+                Stage stage(s, "boruvka_nodes");
+                int64_t width = (ix.slots + kNodeLeaves - 1) / kNodeLeaves;
+                ::fhg::note_launch();
+                node_chunk_kernel<<<(unsigned)width, kNodeThreads, 0, s>>>(S, rounds > 0 ? 1 : 0);
+                FHG_CUDA(cudaGetLastError());
+                while (width > 1) {
+                    const int64_t blocks = (width + kNodeTop - 1) / kNodeTop;
+                    ::fhg::note_launch();
+                    node_top_kernel<<<(unsigned)blocks, kNodeTop / 2, 0, s>>>(S.nc, width);
+                    FHG_CUDA(cudaGetLastError());
+                    width = blocks;
                 }
             }
-            LAUNCH(crep_drop_kernel, ncomp, reps, ncomp, cy_nxt, cy_mx, cmin, tgt);
-            LAUNCH(ref_emit_flags_kernel, ncomp, reps, ncomp, tgt, cmin, flag);
-        } else {
-            LAUNCH(stage_b_kernel, n, n, comp, ix.orig, cand_w, cand_q, keyA, keyB);
-            LAUNCH(stage_c_kernel, n, n, comp, ix.orig, cand_w, cand_q, keyA, keyB, winner);
-            LAUNCH(select_kernel, ncomp, reps, ncomp, winner, cand_q, comp, tgt, iflag + 1);
-            LAUNCH(emit_flags_kernel, ncomp, reps, ncomp, tgt, cmin, flag);
+            {
+                Stage stage(s, "boruvka_search");
+                LAUNCH(seed_kernel, n, S);
+                FHG_TRY(search_round(ws, ix, knn_open, S, /*one_pass=*/false, &try_sparse));
+            }
+            Stage merge_stage(s, "boruvka_merge");
+            if (ref_ties) {
+                LAUNCH(ref_winner_kernel, ncomp, S.reps, ncomp, S.keyA, ix.rank, S.winner);
+                FHG_TRY(tie_walk(ix, rt, S.reps, ncomp, S.comp, core2, S.nc, S.winner, S.cand_w,
+                                 S.cand_q, S.tgt, reinterpret_cast<int*>(S.stat + kStMissing), s));
+                LAUNCH(crep_init_kernel, ncomp, S.reps, ncomp, S.tgt, S.cmin, nxt, mx);
+                int* grew = reinterpret_cast<int*>(S.stat + kStEqual);
+                const int R = bits_for(ncomp) + 1;
+                for (int r = 0; r < R; ++r) {
+                    const bool check = (r & 3) == 3 && r + 1 < R;
+                    if (check) FHG_CUDA(cudaMemsetAsync(grew, 0, sizeof(int), s));
+                    LAUNCH(crep_step_kernel, ncomp, S.reps, ncomp, nxt, mx, nxt2, mx2,
+                           check ? grew : nullptr);
+                    std::swap(nxt, nxt2);
+                    std::swap(mx, mx2);
+                    if (check) {
+                        FHG_TRY(read_stat());
+                        if (!st[kStEqual]) break;
+                    }
+                }
+                LAUNCH(crep_drop_kernel, ncomp, S.reps, ncomp, nxt, mx, S.cmin, S.tgt);
+            } else {
+                LAUNCH(stage_b_kernel, n, S);
+                LAUNCH(stage_c_kernel, n, S);
+            }
+            if (ncomp <= kBlockMerge) {
+                ::fhg::note_launch();
+                merge_kernel<<<1, kSmallThreads, 0, s>>>(S, ncomp);
+                FHG_CUDA(cudaGetLastError());
+            } else {
+                if (!ref_ties) LAUNCH(select_kernel, ncomp, S, ncomp);
+                FHG_TRY(compact(ws, RoundEdges{S}, ncomp, S.stat + kStAdded));
+                LAUNCH(merge_cmin_kernel, ncomp, S, ncomp);
+                FHG_TRY(compact(ws, MergedComponents{S}, ncomp, S.stat + kStComps));
+                std::swap(S.reps, S.next_reps);
+                std::swap(S.rep_cmin, S.next_cmin);
+            }
+            FHG_TRY(read_stat());
+            if (st[kStMissing] || st[kStEdges] - edges != ncomp - st[kStComps]) {
+                set_error("boruvka round %d: inconsistent merge (added %lld, components %lld -> "
+                          "%lld, missing=%d)", rounds, (long long)(st[kStEdges] - edges),
+                          (long long)ncomp, (long long)st[kStComps], (int)st[kStMissing]);
+                return FHG_ERR_NO_CONVERGENCE;
+            }
+            ++rounds;
         }
-        Workspace tmp(s);  // per-round scan scratch, released at the end of the round
-        FHG_TRY(scan_exclusive_u32(tmp, flag, pos, n, cnt));
-        LAUNCH(emit_write_kernel, ncomp, reps, ncomp, tgt, cmin, flag, pos, winner, cand_q, cand_w,
-               ix.orig, m, out->src, out->dst, out->w2);
-        LAUNCH(emit_clear_kernel, ncomp, reps, ncomp, cmin, flag);
-        LAUNCH(union_reps_kernel, ncomp, reps, ncomp, tgt, par);
-        LAUNCH(relabel_points_kernel, n, n, par, comp);
-        uint32_t* keep = pos;  // pos is free again after emit_write
-        LAUNCH(merge_cmin_kernel, ncomp, reps, ncomp, par, cmin, keep);
-        FHG_TRY(scan_exclusive_u32(tmp, keep, kpos, ncomp, cnt + 1));
-        LAUNCH(compact_kernel, ncomp, ncomp, keep, kpos, reps, reps2);
-        uint32_t h2[2] = {0, 0};
-        int h_missing = 0;
-        FHG_CUDA(cudaMemcpyAsync(h2, cnt, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        FHG_CUDA(cudaMemcpyAsync(&h_missing, iflag + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-        FHG_CUDA(cudaStreamSynchronize(s));
-        int32_t* tr = reps; reps = reps2; reps2 = tr;
-        int64_t new_ncomp = h2[1];
-        int64_t added = h2[0];
-        if (h_missing || added != ncomp - new_ncomp) {
-            set_error("boruvka round %d: inconsistent merge (added %lld, components %lld -> %lld, "
-                      "missing=%d)", rounds, (long long)added, (long long)ncomp,
-                      (long long)new_ncomp, h_missing);
-            return FHG_ERR_NO_CONVERGENCE;
-        }
-        m += added;
-        ncomp = new_ncomp;
-        ++rounds;
     }
-    out->m = m;
+    if (st[kStComps] > 1 || st[kStMissing] || (int64_t)st[kStEdges] + st[kStComps] != n) {
+        set_error("boruvka: no convergence after %d rounds (%lld components, %lld edges left, "
+                  "missing=%d)", rounds, (long long)st[kStComps],
+                  (long long)(n - 1 - (int64_t)st[kStEdges]), (int)st[kStMissing]);
+        return FHG_ERR_NO_CONVERGENCE;
+    }
+    out->m = st[kStEdges];
     out->rounds = rounds;
     return FHG_OK;
 }

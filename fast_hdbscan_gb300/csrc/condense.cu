@@ -366,7 +366,7 @@ int condense_tree(Workspace& ws, const Linkage& lk, int64_t mcs, double max_cs, 
     FHG_TRY(ws.alloc(&top, (size_t)m));
     FHG_TRY(ws.alloc(&bth, (size_t)m));
     {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         PjRec *R, *R2;
         int* moving;
         FHG_TRY(tmp.alloc(&R, (size_t)m));
@@ -406,7 +406,7 @@ int condense_tree(Workspace& ws, const Linkage& lk, int64_t mcs, double max_cs, 
     LAUNCH(reached_flags_kernel, m, m, top, flag);
     uint32_t h_cnt = 0;
     {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         FHG_TRY(scan_exclusive_u32(tmp, flag, pos, m, cnt_dev));
     }
     FHG_TRY(ws.alloc(&reached, (size_t)m));
@@ -414,7 +414,7 @@ int condense_tree(Workspace& ws, const Linkage& lk, int64_t mcs, double max_cs, 
     FHG_TRY(read1(cnt_dev, &h_cnt, s));
     const int64_t cnt = h_cnt;
     {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         uint32_t *kd, *kp;
         FHG_TRY(tmp.alloc(&kd, (size_t)cnt));
         FHG_TRY(tmp.alloc(&kp, (size_t)cnt));
@@ -434,7 +434,7 @@ int condense_tree(Workspace& ws, const Linkage& lk, int64_t mcs, double max_cs, 
     LAUNCH(reached_counts_kernel, cnt, cnt, reached, kase, lk.left, lk.right, lk.size, nrows, nnew,
            bfs_pos);
     {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         FHG_TRY(scan_exclusive_i64(tmp, nrows, roff, cnt, tot));
         FHG_TRY(scan_exclusive_i64(tmp, nnew, k6, cnt, tot + 1));
     }
@@ -452,7 +452,7 @@ int condense_tree(Workspace& ws, const Linkage& lk, int64_t mcs, double max_cs, 
     int32_t* items;
     FHG_TRY(ws.alloc(&items, (size_t)(rows > 0 ? rows : 1)));
     {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         FHG_TRY(scan_exclusive_u32(tmp, flag, pos, universe, cnt_dev));
     }
     {
@@ -465,7 +465,7 @@ int condense_tree(Workspace& ws, const Linkage& lk, int64_t mcs, double max_cs, 
     FHG_TRY(ws.alloc(&out->csize, (size_t)(rows > 0 ? rows : 1)));
     if (rows == 0) return FHG_OK;
     {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         uint32_t *kseg, *kdep, *kpre, *key;
         int32_t* order;
         FHG_TRY(tmp.alloc(&kseg, (size_t)rows));

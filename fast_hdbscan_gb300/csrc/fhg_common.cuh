@@ -68,43 +68,103 @@ struct Status {
 // returns the cached blocks.
 int device_pool(cudaMemPool_t* out);
 
-// Stream-ordered scratch allocation.  Every buffer of a call is released on
-// the same stream when the Workspace goes out of scope.
+// Stream-ordered scratch.  Every buffer of a call is released on the same
+// stream when the Workspace goes out of scope.
+//
+// Buffers of up to a quarter of a block are carved from blocks that the
+// Workspace takes from the pool (1 MiB, then twice the last, at most 16 MiB);
+// larger ones are their own allocation.  A fit has about a hundred buffers,
+// and an allocation with its release costs 0.5 us on one thread but 3.5 us
+// per call when 16 threads run fits side by side.
+//
+// A Workspace made from another one is scratch inside it: its small buffers
+// come from the same blocks and their room is used again when it ends, up to
+// the last buffer that its parent took meanwhile.  Such Workspaces nest.
 class Workspace {
   public:
-    explicit Workspace(cudaStream_t s) : stream_(s) {}
+    explicit Workspace(cudaStream_t s) : stream_(s), arena_(&own_) {}
+    explicit Workspace(Workspace& parent)
+        : stream_(parent.stream_), pool_(parent.pool_), arena_(parent.arena_) {
+        mark_block_ = arena_->blocks.size();
+        mark_ = arena_->used;
+        level_ = ++arena_->depth;
+    }
     ~Workspace() { release(); }
     Workspace(const Workspace&) = delete;
     Workspace& operator=(const Workspace&) = delete;
 
     template <class T>
     int alloc(T** out, size_t count) {
+        size_t bytes = (count * sizeof(T) + kAlign - 1) / kAlign * kAlign;
+        if (bytes == 0) bytes = kAlign;
         void* p = nullptr;
-        size_t bytes = count * sizeof(T);
-        if (bytes == 0) bytes = 16;
-        if (!pool_) {
-            int rc = device_pool(&pool_);
-            if (rc != FHG_OK) return rc;
+        if (bytes > kFirstBlock / 4 && bytes > arena_->size / 4) {
+            FHG_TRY(take(&p, bytes));
+            bufs_.push_back(p);
+        } else {
+            if (arena_->used + bytes > arena_->size) {
+                const size_t want = arena_->size == 0              ? kFirstBlock
+                                    : arena_->size < kLargestBlock ? 2 * arena_->size
+                                                                   : kLargestBlock;
+                FHG_TRY(take(&p, want));
+                arena_->blocks.push_back(p);
+                arena_->size = want;
+                arena_->used = 0;
+            }
+            p = static_cast<char*>(arena_->blocks.back()) + arena_->used;
+            arena_->used += bytes;
+            if (level_ < arena_->depth) {  // outlives the Workspaces inside this one
+                arena_->kept_block = arena_->blocks.size();
+                arena_->kept = arena_->used;
+            }
         }
-        cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool_, stream_);
-        if (e != cudaSuccess) {
-            set_error("cudaMallocFromPoolAsync(%zu bytes) failed: %s", bytes,
-                      cudaGetErrorString(e));
-            return e == cudaErrorMemoryAllocation ? FHG_ERR_OOM : FHG_ERR_CUDA;
-        }
-        bufs_.push_back(p);
         *out = static_cast<T*>(p);
         return FHG_OK;
     }
     void release() {
         for (size_t i = bufs_.size(); i-- > 0;) cudaFreeAsync(bufs_[i], stream_);
         bufs_.clear();
+        if (arena_ != &own_) {
+            if (level_ == 0) return;  // released already
+            --arena_->depth;
+            level_ = 0;
+            if (arena_->blocks.size() == mark_block_) {
+                const bool kept = arena_->kept_block == mark_block_ && arena_->kept > mark_;
+                arena_->used = kept ? arena_->kept : mark_;
+            }
+            return;
+        }
+        for (size_t i = own_.blocks.size(); i-- > 0;) cudaFreeAsync(own_.blocks[i], stream_);
+        own_ = Arena();
     }
     cudaStream_t stream() const { return stream_; }
 
   private:
+    static constexpr size_t kAlign = 256, kFirstBlock = size_t{1} << 20,
+                            kLargestBlock = size_t{1} << 24;
+    struct Arena {
+        std::vector<void*> blocks;      // the last one is being filled
+        size_t size = 0, used = 0;      // of the last block
+        int depth = 0;                  // Workspaces inside
+        size_t kept_block = 0, kept = 0;  // room up to here stays taken
+    };
+    int take(void** p, size_t bytes) {
+        if (!pool_) FHG_TRY(device_pool(&pool_));
+        cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool_, stream_);
+        if (e != cudaSuccess) {
+            set_error("cudaMallocFromPoolAsync(%zu bytes) failed: %s", bytes,
+                      cudaGetErrorString(e));
+            return e == cudaErrorMemoryAllocation ? FHG_ERR_OOM : FHG_ERR_CUDA;
+        }
+        return FHG_OK;
+    }
+
     cudaStream_t stream_;
     cudaMemPool_t pool_ = nullptr;
+    Arena own_;
+    Arena* arena_;
+    int level_ = 0;
+    size_t mark_block_ = 0, mark_ = 0;
     std::vector<void*> bufs_;
 };
 

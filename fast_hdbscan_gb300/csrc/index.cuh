@@ -17,6 +17,7 @@ struct fhg_index {
     int32_t d = 0;
     int32_t pad = 4;
     int64_t nleaves = 0, slots = 0, nnodes = 0;
+    void* base = nullptr;  // the allocation of all four
     float* pts = nullptr;
     int32_t* orig = nullptr;
     int32_t* rank = nullptr;

@@ -306,7 +306,7 @@ int kruskal_mst_of_lists(int64_t n, int min_samples, int query_k, const float* w
     LAUNCH(kr_compact_kernel, E, E, flag, pos, k0, key, eid);
     sub.reset(new Stage(s, "kruskal_sort"));
     if (m > 1) {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         FHG_TRY(radix_sort_u32(tmp, key, eid, m, 0, 32));
     }
 

@@ -478,7 +478,7 @@ int sort_and_link(Workspace& ws, int64_t n, const int32_t* src, const int32_t* d
     const int ibits = bits_for(n);
     if (!presorted) {
         Stage stage(s, "mst_sort");
-        Workspace tmp(s);
+        Workspace tmp(ws);
         LAUNCH(gather_key32_kernel, m, dst, perm, k32, m);
         FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, ibits));
         LAUNCH(gather_key32_kernel, m, src, perm, k32, m);
@@ -503,7 +503,7 @@ int sort_and_link(Workspace& ws, int64_t n, const int32_t* src, const int32_t* d
     FHG_TRY(ws.alloc(&newid, (size_t)n));
     FHG_TRY(ws.alloc(&inv, (size_t)n));
     {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         FHG_TRY(tmp.alloc(&slot_flag, (size_t)(2 * m)));
         FHG_TRY(tmp.alloc(&slot_pos, (size_t)(2 * m)));
         FHG_TRY(tmp.alloc(&slot_cnt, 1));

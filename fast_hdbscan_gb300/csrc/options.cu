@@ -565,7 +565,7 @@ static int linkage_preorder(Workspace& ws, const Linkage& lk, int32_t* par, int8
     }
     LAUNCH(cut_parents_kernel, m, m, n, lk.left, lk.right, par, side);
     const int R = bits_for(m) + 1;
-    Workspace tmp(s);
+    Workspace tmp(ws);
     int32_t *anc, *anc2;
     int64_t* pre2;
     FHG_TRY(tmp.alloc(&anc, (size_t)m));
@@ -590,7 +590,7 @@ int weighted_sizes(Workspace& ws, Linkage& lk, const float* weights) {
     FHG_TRY(ws.alloc(&lk.wsize, (size_t)nodes));
     FHG_CUDA(cudaMemcpyAsync(lk.wsize, weights, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
     if (m == 0) return FHG_OK;
-    Workspace tmp(s);
+    Workspace tmp(ws);
     int32_t* par;
     int8_t* side;
     int64_t* pre;
@@ -618,7 +618,7 @@ int linkage_leaf_counts(Workspace& ws, Linkage& lk) {
     FHG_TRY(ws.alloc(&src, (size_t)m));
     FHG_TRY(ws.alloc(&dst, (size_t)m));
     {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         FHG_TRY(tmp.alloc(&jmp, (size_t)m));
         FHG_TRY(tmp.alloc(&jmp2, (size_t)m));
         LAUNCH(rep_init_kernel, m, m, lk.left, jmp);
@@ -649,7 +649,7 @@ static int cluster_tree_of(Workspace& ws, const Condensed& ct, ClusterTree* out)
     *out = ClusterTree();
     if (ct.rows == 0) return FHG_OK;
     uint32_t *flag, *pos, *total;
-    Workspace tmp(s);
+    Workspace tmp(ws);
     FHG_TRY(tmp.alloc(&flag, (size_t)ct.rows));
     FHG_TRY(tmp.alloc(&pos, (size_t)ct.rows));
     FHG_TRY(tmp.alloc(&total, 1));
@@ -679,7 +679,7 @@ static int sort_rows_by(Workspace& ws, const ClusterTree& t, const int32_t* by,
                         int32_t* sorted_other, int32_t* rows_out) {
     cudaStream_t s = ws.stream();
     const int64_t R = t.R;
-    Workspace tmp(s);
+    Workspace tmp(ws);
     uint32_t* key;
     FHG_TRY(tmp.alloc(&key, (size_t)R));
     LAUNCH(keys_u32_kernel, R, R, by, base, key, rows_out);
@@ -831,7 +831,7 @@ int labelling_at_cut(Workspace& ws, const Linkage& lk, double cut, int64_t mcs,
         FHG_CUDA(cudaMemsetAsync(rk, 1, (size_t)m, s));
         const int64_t positions = 2 * n - 1;
         {
-            Workspace tmp(s);
+            Workspace tmp(ws);
             FHG_TRY(tmp.alloc(&flag, (size_t)positions));
             FHG_TRY(tmp.alloc(&pos, (size_t)positions));
             for (int r = 2; r < 127; ++r) {
@@ -846,7 +846,7 @@ int labelling_at_cut(Workspace& ws, const Linkage& lk, double cut, int64_t mcs,
         }
         // representatives and components
         {
-            Workspace tmp(s);
+            Workspace tmp(ws);
             FHG_TRY(tmp.alloc(&jmp2, (size_t)m));
             FHG_TRY(tmp.alloc(&up2, (size_t)m));
             LAUNCH(cut_dom_kernel, m, m, n, lk.left, lk.right, rk, jmp);
@@ -866,7 +866,7 @@ int labelling_at_cut(Workspace& ws, const Linkage& lk, double cut, int64_t mcs,
         }
     }
     LAUNCH(cut_point_rep_kernel, n, n, cut, par, lk.w, up, jmp, prep, count);
-    Workspace tmp(s);
+    Workspace tmp(ws);
     FHG_TRY(tmp.alloc(&flag, (size_t)n));
     FHG_TRY(tmp.alloc(&pos, (size_t)n));
     LAUNCH(cut_flags_kernel, n, n, mcs, count, flag);

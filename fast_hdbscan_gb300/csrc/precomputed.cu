@@ -203,7 +203,7 @@ int precomputed_mst(const int32_t* rows, const int32_t* cols, const double* data
     FHG_TRY(ws.alloc(&d0, mz));
     LAUNCH(pc_pairs_kernel, nnz, nnz, n, rows, cols, data, flag, pos, key, at, d0);
     if (m0 > 1) {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         const int kb = 2 * bits_for(n);
         FHG_TRY(radix_sort_u64(tmp, key, at, m0, 0, kb < 64 ? kb : 64));
     }
@@ -245,7 +245,7 @@ int precomputed_mst(const int32_t* rows, const int32_t* cols, const double* data
     FHG_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t) * n, s));
     LAUNCH(pc_sym_kernel, M, mu, gu, gv, rowkey, perm);
     if (M > 1) {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         FHG_TRY(radix_sort_u32(tmp, rowkey, perm, M, 0, bits_for(n)));
     }
     LAUNCH(pc_csr_kernel, M, M, mu, perm, gu, gv, gmin, srow, scol, sd, count);
@@ -257,12 +257,12 @@ int precomputed_mst(const int32_t* rows, const int32_t* cols, const double* data
         FHG_TRY(ws.alloc(&wkey, Mz));
         LAUNCH(pc_weight_keys_kernel, M, M, sd, wkey, perm);
         {
-            Workspace tmp(s);
+            Workspace tmp(ws);
             if (M > 1) FHG_TRY(radix_sort_u64(tmp, wkey, perm, M, 0, 64));
         }
         LAUNCH(pc_row_keys_kernel, M, M, perm, srow, rowkey);
         {
-            Workspace tmp(s);
+            Workspace tmp(ws);
             if (M > 1) FHG_TRY(radix_sort_u32(tmp, rowkey, perm, M, 0, bits_for(n)));
         }
         LAUNCH(pc_core_kernel, M, M, k, min_samples, perm, srow, scol, sd, indptr, neighbors,
@@ -278,7 +278,7 @@ int precomputed_mst(const int32_t* rows, const int32_t* cols, const double* data
     FHG_TRY(ws.alloc(&w, Mz));
     LAUNCH(pc_mrd_kernel, M, M, srow, scol, sd, core, mkey, perm);
     if (M > 1) {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         FHG_TRY(radix_sort_u64(tmp, mkey, perm, M, 0, 64));
     }
     LAUNCH(pc_ranks_kernel, M, M, perm, srow, scol, mkey, uv, w);

@@ -505,7 +505,7 @@ int prepare(Workspace& ws, const Condensed& ct, Prepared* P) {
     LAUNCH(fill_i32_kernel, C, P->row_of_cluster, C, -1);
     LAUNCH(row_of_child_kernel, rows, rows, n, ct.child, P->row_of_cluster, (int32_t*)nullptr);
     {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         FHG_TRY(tmp.alloc(&key, (size_t)rows));
         int64_t* cnt64;
         FHG_TRY(tmp.alloc(&cnt64, (size_t)C));
@@ -557,7 +557,7 @@ int prepare(Workspace& ws, const Condensed& ct, Prepared* P) {
     FHG_TRY(ws.alloc(&P->cstart, (size_t)C));
     FHG_TRY(ws.alloc(&P->ccnt, (size_t)C));
     {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         uint32_t *flag, *pos, *total;
         FHG_TRY(tmp.alloc(&flag, (size_t)rows));
         FHG_TRY(tmp.alloc(&pos, (size_t)rows));
@@ -737,7 +737,7 @@ int label_points(Workspace& ws, const Condensed& ct, const int32_t* sel, int64_t
     LAUNCH(fill_i32_kernel, C, label_of, C, -1);
     LAUNCH(sel_flags_kernel, n_sel, n_sel, n, C, sel, is_sel, key, val);
     {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         FHG_TRY(radix_sort_u32(tmp, key, val, n_sel, 0, 32));
     }
     LAUNCH(label_map_kernel, n_sel, n_sel, n, C, key, label_of, by_label);
@@ -792,7 +792,7 @@ int membership_strengths(Workspace& ws, const Condensed& ct, const int32_t* sel,
     LAUNCH(fill_i32_kernel, C, label_of, C, -1);
     LAUNCH(sel_flags_kernel, n_sel, n_sel, n, C, sel, is_sel, key, val);
     {
-        Workspace tmp(s);
+        Workspace tmp(ws);
         FHG_TRY(radix_sort_u32(tmp, key, val, n_sel, 0, 32));
     }
     LAUNCH(label_map_kernel, n_sel, n_sel, n, C, key, label_of, by_label);

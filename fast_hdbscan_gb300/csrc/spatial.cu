@@ -508,14 +508,21 @@ int fill_tree(fhg_index* ix, const float* X, bool iota, cudaStream_t s) {
     return fill_tree<32, 32, false>(ix, X, iota, s);
 }
 
+// One allocation holds the four arrays.
 int index_alloc(fhg_index* ix, cudaStream_t s) {
     cudaMemPool_t pool;
     FHG_TRY(device_pool(&pool));
-    FHG_CUDA(cudaMallocFromPoolAsync(&ix->pts, sizeof(float) * ix->n * ix->pad + 16, pool, s));
-    FHG_CUDA(cudaMallocFromPoolAsync(&ix->orig, sizeof(int32_t) * ix->n + 16, pool, s));
-    FHG_CUDA(cudaMallocFromPoolAsync(&ix->rank, sizeof(int32_t) * ix->n + 16, pool, s));
-    FHG_CUDA(cudaMallocFromPoolAsync(&ix->box, sizeof(float) * ix->nnodes * 2 * ix->pad + 16,
-                                     pool, s));
+    auto room = [](int64_t bytes) { return (size_t)((bytes + 16 + 255) / 256 * 256); };
+    const size_t pts = room((int64_t)sizeof(float) * ix->n * ix->pad);
+    const size_t ids = room((int64_t)sizeof(int32_t) * ix->n);
+    const size_t box = room((int64_t)sizeof(float) * ix->nnodes * 2 * ix->pad);
+    char* base = nullptr;
+    FHG_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&base), pts + 2 * ids + box, pool, s));
+    ix->base = base;
+    ix->pts = reinterpret_cast<float*>(base);
+    ix->orig = reinterpret_cast<int32_t*>(base + pts);
+    ix->rank = reinterpret_cast<int32_t*>(base + pts + ids);
+    ix->box = reinterpret_cast<float*>(base + pts + 2 * ids);
     return FHG_OK;
 }
 
@@ -557,10 +564,7 @@ int curve_order(fhg_index* ix, const float* X, cudaStream_t s) {
 
 int index_free(fhg_index* ix, cudaStream_t s) {
     if (!ix) return FHG_OK;
-    if (ix->pts) cudaFreeAsync(ix->pts, s);
-    if (ix->orig) cudaFreeAsync(ix->orig, s);
-    if (ix->rank) cudaFreeAsync(ix->rank, s);
-    if (ix->box) cudaFreeAsync(ix->box, s);
+    if (ix->base) cudaFreeAsync(ix->base, s);
     delete ix;
     return FHG_OK;
 }
