@@ -1,11 +1,16 @@
 // Exclusive scan and LSD radix sort (8-bit digits, stable) for sm_103a.
 //
-// Radix pass = histogram kernel (one 4096-item tile per block, shared-memory
-// counters) + exclusive scan of the digit-major [256][tiles] count table +
-// scatter kernel.  The scatter keeps LSD stability by letting each warp rank
-// its 512 items in order (warp match on the digit, per-warp running counters)
-// and adding the per-warp prefix of each digit.
+// Radix sort: one kernel counts every digit of every key, then one kernel per
+// digit ranks, places and writes its tiles.  A tile learns how many items of
+// each digit lie in the tiles before it from the words those tiles publish
+// (decoupled look-back: their own count first, then the count up to and
+// including them).  Tiles are numbered as blocks start, so every tile before
+// a running one has started; a wait that still goes on too long ends with the
+// block counting the keys of the tiles before it itself.
+//
+// Scan: the sums of tiles, then every block adds up the sums before its tile.
 #include <algorithm>
+#include <type_traits>
 
 #include "primitives.cuh"
 
@@ -48,32 +53,56 @@ __device__ T block_exclusive_scan(T v, T* total) {
 }
 
 template <class T>
-__global__ void __launch_bounds__(kScanThreads) scan_tile_kernel(const T* in, T* out,
-                                                                 T* tile_sums, int64_t n) {
+__device__ __forceinline__ void load_scan_items(const T* in, int64_t base, int64_t n, T* v) {
+#pragma unroll
+    for (int i = 0; i < kScanIPT; ++i) v[i] = (base + i < n) ? in[base + i] : T(0);
+}
+template <class T>
+__global__ void __launch_bounds__(kScanThreads) scan_sums_kernel(const T* in, T* sums, int64_t n) {
     const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanIPT;
-    T v[kScanIPT];
-    T s = 0;
+    T v[kScanIPT], s = 0;
+    load_scan_items(in, base, n, v);
 #pragma unroll
-    for (int i = 0; i < kScanIPT; ++i) {
-        v[i] = (base + i < n) ? in[base + i] : T(0);
-        s += v[i];
+    for (int i = 0; i < kScanIPT; ++i) s += v[i];
+    T tot = 0;
+    block_exclusive_scan<T>(s, &tot);
+    if (threadIdx.x == 0) sums[blockIdx.x] = tot;
+}
+// The tile's items after the sums of the tiles before it (added up by every
+// block in the same order), or after before[blockIdx.x] where that is given.
+template <class T>
+__global__ void __launch_bounds__(kScanThreads) scan_tile_kernel(const T* in, T* out,
+                                                                 const T* sums, const T* before,
+                                                                 T* total, int64_t n) {
+    const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanIPT;
+    T v[kScanIPT], s = 0;
+    T first = 0;
+    if (before) {
+        first = before[blockIdx.x];
+    } else if (blockIdx.x > 0) {
+        const int per = (int)((blockIdx.x + kScanThreads - 1) / kScanThreads);
+        const int b0 = (int)threadIdx.x * per;
+        T x = 0;
+        for (int b = b0; b < b0 + per && b < (int)blockIdx.x; ++b) x += sums[b];
+        block_exclusive_scan<T>(x, &first);
     }
-    __shared__ T tot;
-    T run = block_exclusive_scan<T>(s, threadIdx.x == 0 ? &tot : nullptr);
+    load_scan_items(in, base, n, v);
+#pragma unroll
+    for (int i = 0; i < kScanIPT; ++i) s += v[i];
+    T tot = 0;
+    T run = block_exclusive_scan<T>(s, &tot);
 #pragma unroll
     for (int i = 0; i < kScanIPT; ++i) {
-        if (base + i < n) out[base + i] = run;
+        if (base + i < n) out[base + i] = run + first;
         run += v[i];
     }
-    __syncthreads();
-    if (threadIdx.x == 0 && tile_sums) tile_sums[blockIdx.x] = tot;
+    if (threadIdx.x == 0 && total && blockIdx.x == gridDim.x - 1) *total = first + tot;
 }
 
-template <class T>
-__global__ void scan_add_kernel(T* out, const T* tile_offsets, int64_t n) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] += tile_offsets[i / kScanTile];
-}
+// Beyond this many tiles the tile sums are scanned themselves, as they always
+// are for float64 (the order of whose additions is the result); up to it every
+// block adds up those before it, a few words a thread.
+constexpr int64_t kScanDirect = 4096;
 
 template <class T>
 int scan_exclusive(Workspace& ws, const T* in, T* out, int64_t n, T* total) {
@@ -82,21 +111,21 @@ int scan_exclusive(Workspace& ws, const T* in, T* out, int64_t n, T* total) {
         if (total) FHG_CUDA(cudaMemsetAsync(total, 0, sizeof(T), s));
         return FHG_OK;
     }
-    int64_t tiles = (n + kScanTile - 1) / kScanTile;
-    if (tiles == 1) {
+    const int64_t tiles = (n + kScanTile - 1) / kScanTile;
+    Workspace tmp(ws);
+    T *sums = nullptr, *before = nullptr;
+    if (tiles > 1) {
+        FHG_TRY(tmp.alloc(&sums, (size_t)tiles));
         ::fhg::note_launch();
-        scan_tile_kernel<T><<<1, kScanThreads, 0, s>>>(in, out, total, n);
+        scan_sums_kernel<T><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, sums, n);
         FHG_CUDA(cudaGetLastError());
-        return FHG_OK;
+        if (tiles > kScanDirect || std::is_same<T, double>::value) {
+            FHG_TRY(tmp.alloc(&before, (size_t)tiles));
+            FHG_TRY(scan_exclusive<T>(tmp, sums, before, tiles, nullptr));
+        }
     }
-    T* sums;
-    FHG_TRY(ws.alloc(&sums, (size_t)tiles));
     ::fhg::note_launch();
-    scan_tile_kernel<T><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, out, sums, n);
-    FHG_CUDA(cudaGetLastError());
-    FHG_TRY(scan_exclusive<T>(ws, sums, sums, tiles, total));
-    ::fhg::note_launch();
-    scan_add_kernel<T><<<grid_for(n, 256), 256, 0, s>>>(out, sums, n);
+    scan_tile_kernel<T><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, out, sums, before, total, n);
     FHG_CUDA(cudaGetLastError());
     return FHG_OK;
 }
@@ -104,99 +133,175 @@ int scan_exclusive(Workspace& ws, const T* in, T* out, int64_t n, T* total) {
 // ---------------------------------------------------------------- radix sort
 constexpr int kRsThreads = 256;
 constexpr int kRsWarps = kRsThreads / 32;
-constexpr int kRsChunks = 8;                        // 32-item chunks per warp
-constexpr int kRsTile = kRsWarps * kRsChunks * 32;  // 2048 items per block
+constexpr int kRsSmall = 2048;  // items that one block sorts alone
+constexpr int kRsMaxPasses = 8;
+// 32-item rows of a warp: a tile's keys and values fit the static 48 KB.
+template <class K>
+__host__ __device__ constexpr int rs_rows() { return sizeof(K) == 8 ? 11 : 16; }
+template <class K>
+__host__ __device__ constexpr int rs_tile() { return kRsWarps * rs_rows<K>() * 32; }
 
+// Counts of every digit of all passes: hist[pass][256].
 template <class K>
 __global__ void __launch_bounds__(kRsThreads) rs_hist_kernel(const K* __restrict__ keys,
-                                                             int64_t n, int shift,
-                                                             uint32_t* __restrict__ hist,
-                                                             int64_t tiles) {
-    __shared__ uint32_t h[256];
-    h[threadIdx.x] = 0;
+                                                             int64_t n, int shift, int passes,
+                                                             uint32_t* __restrict__ hist) {
+    __shared__ uint32_t h[kRsMaxPasses][256];
+    for (int i = threadIdx.x; i < passes * 256; i += kRsThreads) (&h[0][0])[i] = 0;
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kRsTile;
-    for (int i = threadIdx.x; i < kRsTile; i += kRsThreads) {
-        int64_t idx = base + i;
-        if (idx < n) atomicAdd(&h[(unsigned)(keys[idx] >> shift) & 255u], 1u);
+    const int lane = threadIdx.x & 31;
+    const int64_t step = (int64_t)gridDim.x * kRsThreads;
+    for (int64_t i = (int64_t)blockIdx.x * kRsThreads + threadIdx.x; i - lane < n; i += step) {
+        const bool valid = i < n;
+        const K k = valid ? keys[i] : K(0);
+        const unsigned act = __ballot_sync(kFull, valid);
+        for (int p = 0; p < passes; ++p) {
+            const unsigned d = (unsigned)(k >> (shift + 8 * p)) & 255u;
+            // the high digits of a row are often all the same: one addition
+            const unsigned d0 = __shfl_sync(kFull, d, 0);
+            if (__all_sync(kFull, !valid || d == d0)) {
+                if (lane == 0) atomicAdd(&h[p][d0], (uint32_t)__popc(act));
+            } else if (valid) {
+                atomicAdd(&h[p][d], 1u);
+            }
+        }
     }
     __syncthreads();
-    hist[(int64_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
+    for (int i = threadIdx.x; i < passes * 256; i += kRsThreads) {
+        const uint32_t c = (&h[0][0])[i];
+        if (c) atomicAdd(&hist[i], c);
+    }
 }
 
-// Stable scatter of one 8-bit digit.  Each warp ranks its 16 chunks of 32
-// items per digit (lanes by __match_any_sync); the tile's items are then laid
-// out in digit order in shared memory and written out so that consecutive
-// threads store consecutive positions of one digit's run (coalesced), in the
-// same stable order as a direct scatter.
+// A published word: the pass and kind above 56 bits of count, so that one
+// zeroed array serves every pass.
+__device__ __forceinline__ unsigned long long rs_word(int pass, int kind, uint64_t count) {
+    return ((unsigned long long)(2 * pass + kind) << 56) | count;
+}
+constexpr int kRsOwn = 1, kRsUpTo = 2;         // the tile's own count; all up to it
+constexpr int kRsWaitPolls = 1 << 20;          // some tenths of a second
+
+// One stable pass.  Each warp ranks its rows in order (the lanes of equal
+// digit by eight ballots, per-warp running counts); the tile's items are then
+// laid out in digit order in shared memory and written so that consecutive
+// threads store consecutive positions of one digit's run.  What bounds it is
+// memory at the largest sizes and the launch at the smallest; against a
+// histogram, a scan and a scatter kernel per pass it reads the keys once less
+// and takes one launch instead of four.
 template <class K>
-__global__ void __launch_bounds__(kRsThreads) rs_scatter_kernel(
+__global__ void __launch_bounds__(kRsThreads, 3) rs_pass_kernel(
     const K* __restrict__ kin, const int32_t* __restrict__ vin, K* __restrict__ kout,
-    int32_t* __restrict__ vout, int64_t n, int shift, const uint32_t* __restrict__ offs,
-    int64_t tiles) {
+    int32_t* __restrict__ vout, int64_t n, int shift, int pass, const uint32_t* __restrict__ hist,
+    uint32_t* __restrict__ counter, unsigned long long* __restrict__ state) {
+    constexpr int kRows = rs_rows<K>(), kTile = rs_tile<K>();
     __shared__ uint32_t wcnt[kRsWarps][256];
     __shared__ uint32_t tstart[256];
-    __shared__ K skey[kRsTile];
-    __shared__ int32_t sval[kRsTile];
+    __shared__ int64_t gbase[256];
+    __shared__ K skey[kTile];
+    __shared__ int32_t sval[kTile];
+    __shared__ uint32_t s_tile;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
     for (int i = threadIdx.x; i < kRsWarps * 256; i += kRsThreads) (&wcnt[0][0])[i] = 0;
     __syncthreads();
+    const int64_t tile = s_tile;
     const unsigned lt_mask = (1u << lane) - 1u;
-    const int64_t tile0 = (int64_t)blockIdx.x * kRsTile;
-    const int64_t base = tile0 + (int64_t)w * (kRsChunks * 32);
-    K key[kRsChunks];
-    int32_t val[kRsChunks];
-    uint32_t pos[kRsChunks];
-    int dig[kRsChunks];
+    const int64_t tile0 = tile * kTile;
+    const int64_t base = tile0 + (int64_t)w * (kRows * 32);
+    K key[kRows];
+    uint32_t pos[kRows];
 #pragma unroll
-    for (int c = 0; c < kRsChunks; ++c) {
-        int64_t idx = base + c * 32 + lane;
-        bool valid = idx < n;
-        K k = valid ? kin[idx] : K(0);
-        int32_t v = valid ? vin[idx] : 0;
-        int d = valid ? (int)((unsigned)(k >> shift) & 255u) : 256;
-        unsigned peers = __match_any_sync(kFull, d);
-        int r = __popc(peers & lt_mask);
-        uint32_t pre = valid ? wcnt[w][d] : 0u;
-        __syncwarp();
-        if (valid && r == 0) wcnt[w][d] = pre + (uint32_t)__popc(peers);
-        __syncwarp();
-        key[c] = k;
-        val[c] = v;
-        pos[c] = pre + (uint32_t)r;
-        dig[c] = d;
+    for (int c = 0; c < kRows; ++c) {
+        const int64_t idx = base + c * 32 + lane;
+        key[c] = idx < n ? kin[idx] : K(0);
     }
-    __syncthreads();
-    {   // per digit: warps' offsets inside the digit, then the digit's start in the tile
-        uint32_t sum = 0;
-        for (int ww = 0; ww < kRsWarps; ++ww) {
-            uint32_t c = wcnt[ww][threadIdx.x];
-            wcnt[ww][threadIdx.x] = sum;
-            sum += c;
+    // The first lane of every digit in a row adds the row's lanes to the warp's
+    // count; the count it found is wanted only after all rows, so that their
+    // additions (in row order) do not wait for one another.
+    unsigned peers[kRows];
+#pragma unroll
+    for (int c = 0; c < kRows; ++c) {
+        const bool valid = base + c * 32 + lane < n;
+        const unsigned d = (unsigned)(key[c] >> shift) & 255u;
+        unsigned m = __ballot_sync(kFull, valid);
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            const bool bit = (d >> b) & 1u;
+            const unsigned on = __ballot_sync(kFull, bit);
+            m &= bit ? on : ~on;
         }
-        tstart[threadIdx.x] = block_exclusive_scan<uint32_t>(sum, nullptr);
+        peers[c] = m;
+        pos[c] = 0;
+        if (valid && (m & lt_mask) == 0) pos[c] = atomicAdd(&wcnt[w][d], (uint32_t)__popc(m));
+        __syncwarp();
     }
+#pragma unroll
+    for (int c = 0; c < kRows; ++c)
+        pos[c] = __shfl_sync(kFull, pos[c], max(__ffs(peers[c]) - 1, 0)) +
+                 __popc(peers[c] & lt_mask);
+    __syncthreads();
+    const int d = threadIdx.x;  // this thread's digit
+    uint32_t count = 0;
+    for (int ww = 0; ww < kRsWarps; ++ww) {  // the warps' offsets inside the digit
+        const uint32_t c = wcnt[ww][d];
+        wcnt[ww][d] = count;
+        count += c;
+    }
+    volatile unsigned long long* word = state + tile * 256 + d;
+    *word = rs_word(pass, tile == 0 ? kRsUpTo : kRsOwn, count);
+    tstart[d] = block_exclusive_scan<uint32_t>(count, nullptr);
+    const uint32_t first = block_exclusive_scan<uint32_t>(hist[d], nullptr);
     __syncthreads();
 #pragma unroll
-    for (int c = 0; c < kRsChunks; ++c) {
-        if (dig[c] < 256) {
-            const uint32_t lp = tstart[dig[c]] + wcnt[w][dig[c]] + pos[c];
+    for (int c = 0; c < kRows; ++c) {
+        if (base + c * 32 + lane < n) {
+            const unsigned dg = (unsigned)(key[c] >> shift) & 255u;
+            const uint32_t lp = tstart[dg] + wcnt[w][dg] + pos[c];
             skey[lp] = key[c];
-            sval[lp] = val[c];
+            sval[lp] = vin[base + c * 32 + lane];
         }
     }
+    // ---- the digit's items in the tiles before this one
+    uint64_t before = 0;
+    bool lost = false;
+    for (int64_t t = tile - 1; t >= 0 && !lost;) {
+        const volatile unsigned long long* from = state + t * 256 + d;
+        unsigned long long x = *from;
+        int polls = 0;
+        while ((int)(x >> 56) <= 2 * pass) {  // not published in this pass yet
+            if (++polls > kRsWaitPolls) {
+                lost = true;
+                break;
+            }
+            if (polls > 16) __nanosleep(64);
+            x = *from;
+        }
+        if (lost) break;
+        before += x & ((1ull << 56) - 1ull);
+        if ((int)(x >> 56) == 2 * pass + kRsUpTo) break;
+        --t;
+    }
+    if (__syncthreads_or(lost)) {  // count them from the keys
+        wcnt[0][d] = 0;
+        __syncthreads();
+        for (int64_t i = threadIdx.x; i < tile0; i += kRsThreads)
+            atomicAdd(&wcnt[0][(unsigned)(kin[i] >> shift) & 255u], 1u);
+        __syncthreads();
+        before = wcnt[0][d];
+    }
+    if (tile > 0) *word = rs_word(pass, kRsUpTo, before + count);
+    gbase[d] = (int64_t)(first + before) - (int64_t)tstart[d];
     __syncthreads();
-    const int cnt = (int)(n - tile0 < kRsTile ? n - tile0 : kRsTile);
+    const int cnt = (int)(n - tile0 < kTile ? n - tile0 : kTile);
     for (int i = threadIdx.x; i < cnt; i += kRsThreads) {
         const K k = skey[i];
-        const int d = (int)((unsigned)(k >> shift) & 255u);
-        const uint32_t dst = offs[(int64_t)d * tiles + blockIdx.x] + (uint32_t)i - tstart[d];
+        const int64_t dst = gbase[(unsigned)(k >> shift) & 255u] + i;
         kout[dst] = k;
         vout[dst] = sval[i];
     }
 }
 
-// The same sort for n <= kRsTile in one launch: a bitonic sort in shared
+// The same sort for n <= kRsSmall in one launch: a bitonic sort in shared
 // memory of (digits, position) pairs, where digits are the key bits the LSD
 // passes cover ([begin, end) rounded up to whole 8-bit digits), so the order
 // is the stable one the passes give.
@@ -204,9 +309,9 @@ constexpr int kRsSmallThreads = 1024;
 template <class K>
 __global__ void __launch_bounds__(kRsSmallThreads) rs_small_kernel(K* keys, int32_t* vals, int n,
                                                                    int shift, int bits) {
-    __shared__ K sk[kRsTile];
-    __shared__ uint16_t si[kRsTile];
-    __shared__ int32_t sv[kRsTile];
+    __shared__ K sk[kRsSmall];
+    __shared__ uint16_t si[kRsSmall];
+    __shared__ int32_t sv[kRsSmall];
     const K mask = bits >= (int)(8 * sizeof(K)) ? ~K(0) : ((K(1) << bits) - K(1));
     int m2 = 1;
     while (m2 < n) m2 <<= 1;
@@ -250,7 +355,7 @@ int radix_sort(Workspace& ws, K* keys, int32_t* vals, int64_t n, int begin_bit, 
         return FHG_ERR_INVALID;
     }
     cudaStream_t s = ws.stream();
-    if (n <= kRsTile) {
+    if (n <= kRsSmall) {
         const int bits = std::min(((end_bit - begin_bit + 7) / 8) * 8,
                                   (int)(8 * sizeof(K)) - begin_bit);
         ::fhg::note_launch();
@@ -258,30 +363,41 @@ int radix_sort(Workspace& ws, K* keys, int32_t* vals, int64_t n, int begin_bit, 
         FHG_CUDA(cudaGetLastError());
         return FHG_OK;
     }
-    const int64_t tiles = (n + kRsTile - 1) / kRsTile;
-    K* kalt;
-    int32_t* valt;
-    uint32_t* hist;
-    FHG_TRY(ws.alloc(&kalt, (size_t)n));
-    FHG_TRY(ws.alloc(&valt, (size_t)n));
-    FHG_TRY(ws.alloc(&hist, (size_t)(256 * tiles)));
-    K *ka = keys, *kb = kalt;
-    int32_t *va = vals, *vb = valt;
-    for (int shift = begin_bit; shift < end_bit; shift += 8) {
-        ::fhg::note_launch();
-        rs_hist_kernel<K><<<(unsigned)tiles, kRsThreads, 0, s>>>(ka, n, shift, hist, tiles);
-        FHG_CUDA(cudaGetLastError());
-        FHG_TRY(scan_exclusive<uint32_t>(ws, hist, hist, 256 * tiles, nullptr));
-        ::fhg::note_launch();
-        rs_scatter_kernel<K><<<(unsigned)tiles, kRsThreads, 0, s>>>(ka, va, kb, vb, n, shift,
-                                                                   hist, tiles);
-        FHG_CUDA(cudaGetLastError());
-        K* tk = ka; ka = kb; kb = tk;
-        int32_t* tv = va; va = vb; vb = tv;
+    const int passes = (end_bit - begin_bit + 7) / 8;
+    const int64_t tiles = (n + rs_tile<K>() - 1) / rs_tile<K>();
+    Workspace tmp(ws);
+    // an odd number of passes over two buffers would end in the other one
+    K* kb[3] = {keys, nullptr, nullptr};
+    int32_t* vb[3] = {vals, nullptr, nullptr};
+    const int spare = passes >= 3 && (passes & 1) ? 2 : 1;
+    for (int i = 1; i <= spare; ++i) {
+        FHG_TRY(tmp.alloc(&kb[i], (size_t)n));
+        FHG_TRY(tmp.alloc(&vb[i], (size_t)n));
     }
-    if (ka != keys) {
-        FHG_CUDA(cudaMemcpyAsync(keys, ka, sizeof(K) * n, cudaMemcpyDeviceToDevice, s));
-        FHG_CUDA(cudaMemcpyAsync(vals, va, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s));
+    // [tile counters][digit counts][published words], zeroed together
+    constexpr size_t kHead = kRsMaxPasses + kRsMaxPasses * 256;
+    uint32_t* head;
+    const size_t words = kHead + 2 * (size_t)tiles * 256;
+    FHG_TRY(tmp.alloc(&head, words));
+    unsigned long long* state = reinterpret_cast<unsigned long long*>(head + kHead);
+    FHG_CUDA(cudaMemsetAsync(head, 0, words * sizeof(uint32_t), s));
+    ::fhg::note_launch();
+    rs_hist_kernel<K><<<(unsigned)std::min<int64_t>(tiles, 4 * 152), kRsThreads, 0, s>>>(
+        keys, n, begin_bit, passes, head + kRsMaxPasses);
+    FHG_CUDA(cudaGetLastError());
+    int cur = 0;
+    for (int p = 0; p < passes; ++p) {
+        const int to = p + 1 == passes && passes > 1 ? 0 : (cur == 1 ? (spare == 2 ? 2 : 0) : 1);
+        ::fhg::note_launch();
+        rs_pass_kernel<K><<<(unsigned)tiles, kRsThreads, 0, s>>>(
+            kb[cur], vb[cur], kb[to], vb[to], n, begin_bit + 8 * p, p,
+            head + kRsMaxPasses + 256 * p, head + p, state);
+        FHG_CUDA(cudaGetLastError());
+        cur = to;
+    }
+    if (cur != 0) {
+        FHG_CUDA(cudaMemcpyAsync(keys, kb[cur], sizeof(K) * n, cudaMemcpyDeviceToDevice, s));
+        FHG_CUDA(cudaMemcpyAsync(vals, vb[cur], sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s));
     }
     return FHG_OK;
 }

@@ -14,6 +14,7 @@
 //                 point the nearest selected cluster above its row's parent,
 //                 computed here by pointer doubling over clusters.
 //   probabilities cluster_trees.py:999-1031.
+#include "compact.cuh"
 #include "primitives.cuh"
 #include "trees.cuh"
 
@@ -22,34 +23,63 @@ namespace {
 
 constexpr int kEomThreads = 1024;
 
-__global__ void parent_keys_kernel(int64_t rows, int64_t n, const int32_t* __restrict__ parent,
-                                   uint32_t* __restrict__ key, int32_t* __restrict__ cnt) {
-    int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    int32_t c = parent[r] - (int32_t)n;
-    key[r] = (uint32_t)c;
-    // rows of one parent come in runs: one atomic per parent per warp
-    const unsigned peers = __match_any_sync(__activemask(), c);
-    if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&cnt[c], __popc(peers));
+// Maximum of non-negative floats as bits, with an atomic only where it grows:
+// most warps find a value at or above theirs (reading first took this from
+// 1.25 to 0.1 ms at 10M rows, of which a few clusters have most).
+__device__ __forceinline__ void max_bits(unsigned int* to, unsigned int b) {
+    if (b > *(volatile unsigned int*)to) atomicMax(to, b);
 }
-__global__ void row_of_child_kernel(int64_t rows, int64_t n, const int32_t* __restrict__ child,
-                                    int32_t* __restrict__ row_of_cluster,
-                                    int32_t* __restrict__ row_of_point) {
-    int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// One pass over the rows: the row of every point and cluster, the largest
+// lambda under the root (root_max) and of every cluster's points (death), and
+// -- with key -- the parent keys and the row numbers to be sorted by them.
+__global__ void row_facts_kernel(int64_t rows, int64_t n, const int32_t* __restrict__ parent,
+                                 const int32_t* __restrict__ child, const float* __restrict__ lam,
+                                 const float* __restrict__ csize,
+                                 int32_t* __restrict__ row_of_point,
+                                 int32_t* __restrict__ row_of_cluster, unsigned int* root_max,
+                                 unsigned int* death, uint32_t* __restrict__ key,
+                                 int32_t* __restrict__ order) {
+    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= rows) return;
-    int32_t c = child[r];
-    if (c >= n) row_of_cluster[c - n] = (int32_t)r;
-    else if (row_of_point) row_of_point[c] = (int32_t)r;
+    const int32_t c = parent[r] - (int32_t)n, x = child[r];
+    if (x >= n) row_of_cluster[x - n] = (int32_t)r;
+    else row_of_point[x] = (int32_t)r;
+    if (key) {
+        key[r] = (uint32_t)c;
+        order[r] = (int32_t)r;
+    }
+    const unsigned int b = __float_as_uint(lam[r]);
+    const int lane = threadIdx.x & 31;
+    const unsigned act = __activemask();
+    // non-negative floats order like their bits; lanes combine first
+    const unsigned roots = __ballot_sync(act, c == 0);
+    if (c == 0) {
+        const unsigned m = __reduce_max_sync(roots, b);
+        if (lane == __ffs(roots) - 1) max_bits(root_max, m);
+    }
+    const bool pt = csize[r] == 1.0f;
+    const unsigned pts = __ballot_sync(act, pt);
+    if (pt) {
+        const unsigned peers = __match_any_sync(pts, c);
+        const unsigned m = __reduce_max_sync(peers, b);
+        if (lane == __ffs(peers) - 1) max_bits(&death[c], m);
+    }
 }
 // lambda * size of every row, in parent-grouped row order (contiguous per
 // cluster), so that each cluster's sequential sum below streams its addends.
-__global__ void products_kernel(int64_t rows, const int32_t* __restrict__ order,
+// The sorted keys' runs are the clusters' ranges [start, start + cnt).
+__global__ void products_kernel(int64_t rows, const uint32_t* __restrict__ key,
+                                const int32_t* __restrict__ order,
                                 const float* __restrict__ lam, const float* __restrict__ csize,
-                                float* __restrict__ prod) {
+                                float* __restrict__ prod, int64_t* __restrict__ start,
+                                int64_t* __restrict__ end) {
     int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= rows) return;
     int32_t r = order[j];
     prod[j] = __fmul_rn(lam[r], csize[r]);
+    const uint32_t c = key[j];
+    if (j == 0 || key[j - 1] != c) start[c] = j;
+    if (j + 1 == rows || key[j + 1] != c) end[c] = j + 1;
 }
 // One thread per cluster: the float32 sum of its rows' products, strictly in
 // row order (a float32 sum is not associative, so the order is the result).
@@ -66,14 +96,14 @@ __device__ __forceinline__ float score_start(int64_t c, const int32_t* __restric
     return s;
 }
 __global__ void score_kernel(int64_t C, const int64_t* __restrict__ start,
-                             const int32_t* __restrict__ cnt, const float* __restrict__ prod,
+                             const int64_t* __restrict__ end, const float* __restrict__ prod,
                              const int32_t* __restrict__ row_of_cluster,
                              const float* __restrict__ lam, const float* __restrict__ csize,
                              float* __restrict__ score) {
     int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C || cnt[c] >= kBigRows) return;
+    if (c >= C || end[c] - start[c] >= kBigRows) return;
     float s = score_start(c, row_of_cluster, lam, csize);
-    const int64_t b = start[c], e = b + cnt[c];
+    const int64_t b = start[c], e = end[c];
     int64_t j = b;
     for (; j + 8 <= e; j += 8) {
         float v[8];
@@ -92,13 +122,13 @@ __global__ void score_kernel(int64_t C, const int64_t* __restrict__ start,
 constexpr int kScoreThreads = 256;
 constexpr int kScoreChunk = 4096;
 __global__ void __launch_bounds__(kScoreThreads) score_big_kernel(
-    int64_t C, const int64_t* __restrict__ start, const int32_t* __restrict__ cnt,
+    int64_t C, const int64_t* __restrict__ start, const int64_t* __restrict__ end,
     const float* __restrict__ prod, const int32_t* __restrict__ row_of_cluster,
     const float* __restrict__ lam, const float* __restrict__ csize, float* __restrict__ score) {
     __shared__ float buf[2][kScoreChunk];
     for (int64_t c = blockIdx.x; c < C; c += gridDim.x) {
-        if (cnt[c] < kBigRows) continue;  // uniform over the block
-        const int64_t b = start[c], len = cnt[c];
+        const int64_t b = start[c], len = end[c] - b;
+        if (len < kBigRows) continue;  // uniform over the block
         const int64_t chunks = (len + kScoreChunk - 1) / kScoreChunk;
         for (int64_t j = threadIdx.x; j < kScoreChunk && j < len; j += blockDim.x)
             buf[0][j] = __ldg(prod + b + j);
@@ -131,32 +161,23 @@ __global__ void __launch_bounds__(kScoreThreads) score_big_kernel(
     }
 }
 
-// Cluster rows (child_size > 1) of every parent, kept in row order.
-__global__ void cluster_row_flags_kernel(int64_t rows, const int32_t* __restrict__ order,
-                                         const float* __restrict__ csize,
-                                         uint32_t* __restrict__ flag) {
-    int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < rows) flag[j] = csize[order[j]] > 1.0f ? 1u : 0u;
-}
-__global__ void cluster_row_compact_kernel(int64_t rows, const int32_t* __restrict__ order,
-                                           const uint32_t* __restrict__ flag,
-                                           const uint32_t* __restrict__ pos,
-                                           int32_t* __restrict__ corder) {
-    int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < rows && flag[j]) corder[pos[j]] = order[j];
-}
-__global__ void cluster_row_ranges_kernel(int64_t C, int64_t rows, const int64_t* __restrict__ start,
-                                          const int32_t* __restrict__ cnt,
-                                          const uint32_t* __restrict__ pos,
-                                          const uint32_t* __restrict__ total,
-                                          int64_t* __restrict__ cstart, int32_t* __restrict__ ccnt) {
-    int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
-    int64_t b = start[c], e = b + cnt[c];
-    uint32_t pb = b < rows ? pos[b] : *total, pe = e < rows ? pos[e] : *total;
-    cstart[c] = pb;
-    ccnt[c] = (int32_t)(pe - pb);
-}
+// Cluster rows (child_size > 1) in parent-grouped row order: corder, and every
+// parent's range of it [cstart, cstart + ccnt) (cstart starts as -1 unsigned).
+struct ClusterRows {
+    const uint32_t* key;
+    const int32_t* order;
+    const float* csize;
+    int32_t* corder;
+    uint32_t* cstart;
+    int32_t* ccnt;
+    __device__ bool test(int64_t j) const { return csize[order[j]] > 1.0f; }
+    __device__ void emit(int64_t j, uint32_t at) const {
+        corder[at] = order[j];
+        atomicMin(&cstart[key[j]], at);
+        atomicAdd(&ccnt[key[j]], 1);
+    }
+    __device__ void each(int64_t) const {}
+};
 
 // Cluster-tree structure: parent cluster (local id) and size of each cluster.
 __global__ void cluster_info_kernel(int64_t C, int64_t n, const int32_t* __restrict__ row_of_cluster,
@@ -211,9 +232,9 @@ __device__ void block_scan_excl(int32_t* a, int64_t len, int32_t* tmp_total) {
 __global__ void __launch_bounds__(kEomThreads) eom_kernel(
     int64_t C, const int32_t* __restrict__ cpar, const float* __restrict__ nsize,
     const int8_t* __restrict__ in_tree, const float* __restrict__ score,
-    const int64_t* __restrict__ start, const int32_t* __restrict__ cnt,
-    const int32_t* __restrict__ order, const float* __restrict__ csize,
-    const int32_t* __restrict__ child, int64_t n, double max_cs, int allow_single,
+    const uint32_t* __restrict__ start, const int32_t* __restrict__ cnt,
+    const int32_t* __restrict__ order, const int32_t* __restrict__ child, int64_t n,
+    double max_cs, int allow_single,
     int32_t* depth, int32_t* depth2, int32_t* jmp, int32_t* jmp2, int32_t* dcount, int32_t* byd,
     double* ret, int8_t* chose, int8_t* blocked, int32_t* flags, int32_t* sel, int64_t* n_sel) {
     const int t = threadIdx.x;
@@ -265,7 +286,8 @@ __global__ void __launch_bounds__(kEomThreads) eom_kernel(
             }
             const double cur = (double)score[c] > 0.0 ? (double)score[c] : 0.0;
             double tot = 0.0;
-            for (int64_t q = start[c]; q < start[c] + cnt[c]; ++q) tot += ret[child[order[q]] - n];
+            for (int32_t q = 0; q < cnt[c]; ++q)
+                tot += ret[child[order[start[c] + (uint32_t)q]] - n];
             if (tot > cur || (double)nsize[c] > max_cs) {
                 ret[c] = tot;
             } else {
@@ -327,6 +349,14 @@ __global__ void __launch_bounds__(kEomThreads) leaf_kernel(
 }
 
 // ---------------------------------------------------------------- labels
+// Membership strength of a point that leaves at lambda lx a cluster whose
+// largest point lambda is mx (cluster_trees.py:1011).
+__device__ __forceinline__ float strength(float lx, float mx) {
+    const double ml = (double)mx;
+    if (ml == 0.0 || !isfinite(lx)) return 1.0f;
+    const double lv = (double)lx < ml ? (double)lx : ml;
+    return (float)(lv / ml);
+}
 __global__ void sel_flags_kernel(int64_t n_sel, int64_t n, int64_t C, const int32_t* __restrict__ sel,
                                  int8_t* __restrict__ is_sel, uint32_t* __restrict__ key,
                                  int32_t* __restrict__ val) {
@@ -346,64 +376,54 @@ __global__ void label_map_kernel(int64_t n_sel, int64_t n, int64_t C,
     by_label[j] = c;
     if (c >= 0 && c < C) atomicMax(&label_of[c], (int32_t)j);  // last position wins
 }
-__global__ void anc_init_kernel(int64_t C, const int32_t* __restrict__ cpar,
-                                const int8_t* __restrict__ is_sel, int32_t* __restrict__ jmp,
-                                int32_t* __restrict__ sa) {
-    int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
-    jmp[c] = c == 0 ? 0 : (cpar[c] < 0 ? 0 : cpar[c]);
-    sa[c] = (is_sel[c] || c == 0) ? (int32_t)c : -1;
-}
-__global__ void anc_step_kernel(int64_t C, const int32_t* __restrict__ jmp,
-                                const int32_t* __restrict__ sa, int32_t* __restrict__ jmp2,
-                                int32_t* __restrict__ sa2) {
-    int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
-    int32_t a = jmp[c];
-    jmp2[c] = jmp[a];
-    sa2[c] = sa[c] != -1 ? sa[c] : sa[a];
-}
-__global__ void root_stats_kernel(int64_t rows, int64_t n, const int32_t* __restrict__ parent,
-                                  const float* __restrict__ lam, const float* __restrict__ csize,
-                                  unsigned int* __restrict__ root_max, unsigned int* __restrict__ death) {
-    int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    int32_t c = parent[r] - (int32_t)n;
-    unsigned int b = __float_as_uint(lam[r]);
-    const int lane = threadIdx.x & 31;
-    const unsigned act = __activemask();
-    // non-negative floats order like their bits; lanes combine first, then one
-    // atomic per target per warp
-    const unsigned roots = __ballot_sync(act, c == 0);
-    if (c == 0) {
-        const unsigned m = __reduce_max_sync(roots, b);
-        if (lane == __ffs(roots) - 1) atomicMax(root_max, m);
+// Nearest selected cluster at or above every cluster (or the root), by pointer
+// doubling, and the number of distinct selected clusters.  One block: the
+// cluster tree is small against the points, and its log2(C) steps are a
+// barrier each instead of a launch.
+__global__ void __launch_bounds__(kEomThreads) ancestors_kernel(
+    int64_t C, const int32_t* __restrict__ cpar, const int8_t* __restrict__ is_sel, int steps,
+    int32_t* jmp, int32_t* sa, int32_t* jmp2, int32_t* sa2, int32_t* n_distinct) {
+    int32_t mine = 0;
+    for (int64_t c = threadIdx.x; c < C; c += blockDim.x) {
+        jmp[c] = c == 0 ? 0 : (cpar[c] < 0 ? 0 : cpar[c]);
+        sa[c] = (is_sel[c] || c == 0) ? (int32_t)c : -1;
+        mine += is_sel[c] ? 1 : 0;
     }
-    const bool pt = csize[r] == 1.0f;
-    const unsigned pts = __ballot_sync(act, pt);
-    if (pt) {
-        const unsigned peers = __match_any_sync(pts, c);
-        const unsigned m = __reduce_max_sync(peers, b);
-        if (lane == __ffs(peers) - 1) atomicMax(&death[c], m);
+    if (mine) atomicAdd(n_distinct, mine);
+    __syncthreads();
+    for (int r = 0; r < steps; ++r) {
+        for (int64_t c = threadIdx.x; c < C; c += blockDim.x) {
+            const int32_t a = jmp[c];
+            jmp2[c] = jmp[a];
+            sa2[c] = sa[c] != -1 ? sa[c] : sa[a];
+        }
+        __syncthreads();
+        int32_t* t = jmp; jmp = jmp2; jmp2 = t;
+        t = sa; sa = sa2; sa2 = t;
     }
 }
-__global__ void point_labels_kernel(int64_t n, int64_t n_distinct, double eps,
+// Label and membership strength of every point (probs_kernel's expression).
+__global__ void point_labels_kernel(int64_t n, const int32_t* __restrict__ n_distinct, double eps,
                                     const int32_t* __restrict__ row_of_point,
                                     const int32_t* __restrict__ parent,
                                     const float* __restrict__ lam, const int32_t* __restrict__ sa,
                                     const int8_t* __restrict__ is_sel,
                                     const int32_t* __restrict__ label_of,
+                                    const int32_t* __restrict__ by_label,
                                     const unsigned int* __restrict__ root_max,
-                                    int64_t* __restrict__ labels, int* __restrict__ err) {
+                                    const unsigned int* __restrict__ death,
+                                    int64_t* __restrict__ labels, float* __restrict__ probs,
+                                    int* __restrict__ err) {
     int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= n) return;
     int32_t r = row_of_point[x];
     int64_t lab = -1;
+    float prob = 0.0f;
     if (r >= 0 && lam[r] != 0.0f) {
         int32_t a = sa[parent[r] - (int32_t)n];
         if (a != 0) {
             lab = label_of[a];
-        } else if (n_distinct == 1) {
+        } else if (*n_distinct == 1) {
             float lx = lam[r];
             bool take = eps > 0.0 ? ((double)lx >= 1.0 / eps) : (lx >= __uint_as_float(*root_max));
             if (take) {
@@ -412,7 +432,9 @@ __global__ void point_labels_kernel(int64_t n, int64_t n_distinct, double eps,
             }
         }
     }
+    if (lab >= 0) prob = strength(lam[r], __uint_as_float(death[by_label[lab]]));
     labels[x] = lab;
+    probs[x] = prob;
 }
 __global__ void probs_kernel(int64_t rows, int64_t n, const int32_t* __restrict__ child,
                              const float* __restrict__ lam, const int64_t* __restrict__ labels,
@@ -424,25 +446,9 @@ __global__ void probs_kernel(int64_t rows, int64_t n, const int32_t* __restrict_
     if (x >= n) return;
     int64_t lab = labels[x];
     if (lab < 0) return;
-    int32_t c = by_label[lab];
-    double ml = (double)__uint_as_float(death[c]);
-    float lx = lam[r];
-    if (ml == 0.0 || !isfinite(lx)) {
-        probs[x] = 1.0f;
-    } else {
-        double lv = (double)lx < ml ? (double)lx : ml;
-        probs[x] = (float)(lv / ml);
-    }
-}
-__global__ void widen_kernel(int64_t C, const int32_t* __restrict__ a, int64_t* __restrict__ b) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < C) b[i] = a[i];
+    probs[x] = strength(lam[r], __uint_as_float(death[by_label[lab]]));
 }
 __global__ void fill_i64_kernel(int64_t* a, int64_t n, int64_t v) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = v;
-}
-__global__ void fill_i32_kernel(int32_t* a, int64_t n, int32_t v) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) a[i] = v;
 }
@@ -456,21 +462,20 @@ __global__ void fill_i32_kernel(int32_t* a, int64_t n, int32_t v) {
         }                                                                   \
     } while (0)
 
-// Shared preparation: rows grouped by parent, scores, cluster tree.
+// What the EOM selection needs beside LabelPre: rows grouped by parent and
+// every cluster's score.
 //
 // The scores are one sequential float32 sum per cluster, so a large cluster's
-// sum is a long chain of dependent additions on a single thread.  They are
-// computed on a side stream while the stream goes on with the work that does
-// not read them; join() (also run by the destructor) orders the stream after
-// them.  Every buffer the side stream touches belongs to the caller's
-// Workspace, which outlives the join.
+// sum is a long chain of dependent additions on a single thread.  For many
+// rows they are computed on a side stream while the stream goes on with the
+// work that does not read them; join() (also run by the destructor) orders the
+// stream after them.  Every buffer the side stream touches belongs to the
+// caller's Workspace, which outlives the join.
 struct Prepared {
-    int64_t C = 0;
-    int32_t *order = nullptr, *cnt = nullptr, *row_of_cluster = nullptr, *cpar = nullptr;
-    int32_t *corder = nullptr, *ccnt = nullptr;
-    int64_t *start = nullptr, *cstart = nullptr;
-    float *score = nullptr, *nsize = nullptr, *prod = nullptr;
-    int8_t* in_tree = nullptr;
+    int32_t *order = nullptr, *corder = nullptr, *ccnt = nullptr;
+    uint32_t *key = nullptr, *cstart = nullptr;
+    int64_t *start = nullptr, *end = nullptr;
+    float *score = nullptr, *prod = nullptr;
     cudaStream_t main = nullptr, side = nullptr;
     cudaEvent_t done = nullptr;
 
@@ -487,42 +492,51 @@ struct Prepared {
         done = nullptr;
     }
 };
+// A stream and its events cost more than the sums of fewer rows.
+constexpr int64_t kSideRows = 1 << 18;
 
-int prepare(Workspace& ws, const Condensed& ct, Prepared* P) {
+// LabelPre of a tree; with P also what the EOM selection needs.
+int prepare(Workspace& ws, const Condensed& ct, LabelPre* pre, Prepared* P) {
     cudaStream_t s = ws.stream();
     const int64_t C = ct.n_clusters, rows = ct.rows, n = ct.n;
-    P->C = C;
-    uint32_t* key;
-    FHG_TRY(ws.alloc(&P->order, (size_t)rows));
-    FHG_TRY(ws.alloc(&P->cnt, (size_t)C));
-    FHG_TRY(ws.alloc(&P->start, (size_t)C));
-    FHG_TRY(ws.alloc(&P->row_of_cluster, (size_t)C));
-    FHG_TRY(ws.alloc(&P->score, (size_t)C));
-    FHG_TRY(ws.alloc(&P->cpar, (size_t)C));
-    FHG_TRY(ws.alloc(&P->nsize, (size_t)C));
-    FHG_TRY(ws.alloc(&P->in_tree, (size_t)C));
-    FHG_CUDA(cudaMemsetAsync(P->cnt, 0, sizeof(int32_t) * C, s));
-    LAUNCH(fill_i32_kernel, C, P->row_of_cluster, C, -1);
-    LAUNCH(row_of_child_kernel, rows, rows, n, ct.child, P->row_of_cluster, (int32_t*)nullptr);
-    {
-        Workspace tmp(ws);
-        FHG_TRY(tmp.alloc(&key, (size_t)rows));
-        int64_t* cnt64;
-        FHG_TRY(tmp.alloc(&cnt64, (size_t)C));
-        LAUNCH(parent_keys_kernel, rows, rows, n, ct.parent, key, P->cnt);
-        FHG_TRY(fill_iota_i32(P->order, rows, s));
-        FHG_TRY(radix_sort_u32(tmp, key, P->order, rows, 0, bits_for(C)));
-        // start = exclusive scan of counts
-        LAUNCH(widen_kernel, C, C, P->cnt, cnt64);
-        FHG_TRY(scan_exclusive_i64(tmp, cnt64, P->start, C, nullptr));
+    *pre = LabelPre();
+    // all arrays that start as -1, then all that start as 0
+    FHG_TRY(ws.alloc(&pre->row_of_point, (size_t)(n + 2 * C)));
+    pre->row_of_cluster = pre->row_of_point + n;
+    uint32_t* cstart = reinterpret_cast<uint32_t*>(pre->row_of_cluster + C);
+    FHG_CUDA(cudaMemsetAsync(pre->row_of_point, 0xff, sizeof(int32_t) * (n + 2 * C), s));
+    int64_t* zeroed;
+    FHG_TRY(ws.alloc(&zeroed, (size_t)(3 * C + 1)));
+    FHG_CUDA(cudaMemsetAsync(zeroed, 0, sizeof(int64_t) * (3 * C + 1), s));
+    pre->death = reinterpret_cast<unsigned int*>(zeroed + 2 * C);
+    int32_t* ccnt = reinterpret_cast<int32_t*>(pre->death + C);
+    pre->root_max = reinterpret_cast<unsigned int*>(zeroed + 3 * C);
+    FHG_TRY(ws.alloc(&pre->cpar, (size_t)C));
+    FHG_TRY(ws.alloc(&pre->nsize, (size_t)C));
+    FHG_TRY(ws.alloc(&pre->in_tree, (size_t)C));
+    if (P) {
+        P->start = zeroed;
+        P->end = zeroed + C;
+        P->ccnt = ccnt;
+        P->cstart = cstart;
+        FHG_TRY(ws.alloc(&P->key, (size_t)rows));
+        FHG_TRY(ws.alloc(&P->order, (size_t)rows));
+        FHG_TRY(ws.alloc(&P->prod, (size_t)rows));
+        FHG_TRY(ws.alloc(&P->corder, (size_t)rows));
+        FHG_TRY(ws.alloc(&P->score, (size_t)C));
     }
-    FHG_TRY(ws.alloc(&P->prod, (size_t)rows));
-    LAUNCH(products_kernel, rows, rows, P->order, ct.lambda, ct.csize, P->prod);
-    {
-        // the scores on a side stream (on the stream itself if none can be made)
-        cudaStream_t ss = s;
+    LAUNCH(row_facts_kernel, rows, rows, n, ct.parent, ct.child, ct.lambda, ct.csize,
+           pre->row_of_point, pre->row_of_cluster, pre->root_max, pre->death,
+           P ? P->key : (uint32_t*)nullptr, P ? P->order : (int32_t*)nullptr);
+    if (P) {
+        FHG_TRY(radix_sort_u32(ws, P->key, P->order, rows, 0, bits_for(C)));
+        LAUNCH(products_kernel, rows, rows, P->key, P->order, ct.lambda, ct.csize, P->prod,
+               P->start, P->end);
+        cudaStream_t ss = s;  // (the stream itself if no other can be made)
         cudaEvent_t fork = nullptr;
-        if (cudaStreamCreateWithFlags(&P->side, cudaStreamNonBlocking) == cudaSuccess) {
+        if (rows < kSideRows) {
+            P->side = nullptr;
+        } else if (cudaStreamCreateWithFlags(&P->side, cudaStreamNonBlocking) == cudaSuccess) {
             if (cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess &&
                 cudaEventCreateWithFlags(&P->done, cudaEventDisableTiming) == cudaSuccess &&
                 cudaEventRecord(fork, s) == cudaSuccess &&
@@ -541,35 +555,26 @@ int prepare(Workspace& ws, const Condensed& ct, Prepared* P) {
             cudaGetLastError();
         }
         if (C > 0) {
+            if (rows >= kBigRows) {
+                ::fhg::note_launch();
+                score_big_kernel<<<(unsigned)(C < 1024 ? C : 1024), kScoreThreads, 0, ss>>>(
+                    C, P->start, P->end, P->prod, pre->row_of_cluster, ct.lambda, ct.csize,
+                    P->score);
+                FHG_CUDA(cudaGetLastError());
+            }
             ::fhg::note_launch();
-            score_big_kernel<<<(unsigned)(C < 1024 ? C : 1024), kScoreThreads, 0, ss>>>(
-                C, P->start, P->cnt, P->prod, P->row_of_cluster, ct.lambda, ct.csize, P->score);
-            FHG_CUDA(cudaGetLastError());
-            ::fhg::note_launch();
-            score_kernel<<<grid_for(C, 256), 256, 0, ss>>>(C, P->start, P->cnt, P->prod,
-                                                           P->row_of_cluster, ct.lambda,
+            score_kernel<<<grid_for(C, 256), 256, 0, ss>>>(C, P->start, P->end, P->prod,
+                                                           pre->row_of_cluster, ct.lambda,
                                                            ct.csize, P->score);
             FHG_CUDA(cudaGetLastError());
         }
         if (P->side) FHG_CUDA(cudaEventRecord(P->done, P->side));
+        FHG_TRY(compact(ws, ClusterRows{P->key, P->order, ct.csize, P->corder, P->cstart, P->ccnt},
+                        rows, nullptr));
     }
-    FHG_TRY(ws.alloc(&P->corder, (size_t)rows));
-    FHG_TRY(ws.alloc(&P->cstart, (size_t)C));
-    FHG_TRY(ws.alloc(&P->ccnt, (size_t)C));
-    {
-        Workspace tmp(ws);
-        uint32_t *flag, *pos, *total;
-        FHG_TRY(tmp.alloc(&flag, (size_t)rows));
-        FHG_TRY(tmp.alloc(&pos, (size_t)rows));
-        FHG_TRY(tmp.alloc(&total, 1));
-        LAUNCH(cluster_row_flags_kernel, rows, rows, P->order, ct.csize, flag);
-        FHG_TRY(scan_exclusive_u32(tmp, flag, pos, rows, total));
-        LAUNCH(cluster_row_compact_kernel, rows, rows, P->order, flag, pos, P->corder);
-        LAUNCH(cluster_row_ranges_kernel, C, C, rows, P->start, P->cnt, pos, total, P->cstart,
-               P->ccnt);
-    }
-    LAUNCH(cluster_info_kernel, C, C, n, P->row_of_cluster, ct.parent, ct.csize, P->cpar, P->nsize,
-           P->in_tree);
+    LAUNCH(cluster_info_kernel, C, C, n, pre->row_of_cluster, ct.parent, ct.csize, pre->cpar,
+           pre->nsize, pre->in_tree);
+    pre->ready = true;
     return FHG_OK;
 }
 
@@ -620,11 +625,12 @@ int select_eom(Workspace& ws, const Condensed& ct, double max_cs, bool allow_sin
     *n_sel = 0;
     if (ct.rows == 0) return FHG_OK;
     Stage stage(s, "select");
+    LabelPre own;
+    if (!pre) pre = &own;
     Prepared P;
-    FHG_TRY(prepare(ws, ct, &P));
-    if (pre) FHG_TRY(label_prework(ws, ct, pre));
+    FHG_TRY(prepare(ws, ct, pre, &P));
     P.join();
-    const int64_t C = P.C;
+    const int64_t C = ct.n_clusters;
     int32_t *depth, *depth2, *jmp, *jmp2, *dcount, *byd, *flags;
     double* ret;
     int8_t *chose, *blocked;
@@ -641,8 +647,8 @@ int select_eom(Workspace& ws, const Condensed& ct, double max_cs, bool allow_sin
     FHG_TRY(ws.alloc(&blocked, (size_t)C));
     FHG_TRY(ws.alloc(&nsel_dev, 1));
     ::fhg::note_launch();
-    eom_kernel<<<1, kEomThreads, 0, s>>>(C, P.cpar, P.nsize, P.in_tree, P.score, P.cstart, P.ccnt,
-                                         P.corder, ct.csize, ct.child, ct.n, max_cs,
+    eom_kernel<<<1, kEomThreads, 0, s>>>(C, pre->cpar, pre->nsize, pre->in_tree, P.score, P.cstart,
+                                         P.ccnt, P.corder, ct.child, ct.n, max_cs,
                                          allow_single ? 1 : 0, depth, depth2, jmp, jmp2, dcount,
                                          byd, ret, chose, blocked, flags, sel, nsel_dev);
     FHG_CUDA(cudaGetLastError());
@@ -656,44 +662,19 @@ int select_leaf(Workspace& ws, const Condensed& ct, int32_t* sel, int64_t* n_sel
     cudaStream_t s = ws.stream();
     *n_sel = 0;
     if (ct.rows == 0) return FHG_OK;
-    Prepared P;
-    FHG_TRY(prepare(ws, ct, &P));
-    if (pre) FHG_TRY(label_prework(ws, ct, pre));
-    P.join();
+    LabelPre own;
+    if (!pre) pre = &own;
+    FHG_TRY(prepare(ws, ct, pre, nullptr));
     int32_t* flags;
     int64_t* nsel_dev;
-    FHG_TRY(ws.alloc(&flags, (size_t)P.C));
+    FHG_TRY(ws.alloc(&flags, (size_t)ct.n_clusters));
     FHG_TRY(ws.alloc(&nsel_dev, 1));
     ::fhg::note_launch();
-    leaf_kernel<<<1, kEomThreads, 0, s>>>(P.C, ct.n, P.cpar, P.in_tree, flags, sel, nsel_dev);
+    leaf_kernel<<<1, kEomThreads, 0, s>>>(ct.n_clusters, ct.n, pre->cpar, pre->in_tree, flags, sel,
+                                          nsel_dev);
     FHG_CUDA(cudaGetLastError());
     FHG_CUDA(cudaMemcpyAsync(n_sel, nsel_dev, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     FHG_CUDA(cudaStreamSynchronize(s));
-    return FHG_OK;
-}
-
-int label_prework(Workspace& ws, const Condensed& ct, LabelPre* pre) {
-    cudaStream_t s = ws.stream();
-    const int64_t n = ct.n, rows = ct.rows, C = ct.n_clusters;
-    *pre = LabelPre();
-    if (rows == 0) return FHG_OK;
-    FHG_TRY(ws.alloc(&pre->row_of_point, (size_t)n));
-    FHG_TRY(ws.alloc(&pre->row_of_cluster, (size_t)C));
-    FHG_TRY(ws.alloc(&pre->cpar, (size_t)C));
-    FHG_TRY(ws.alloc(&pre->nsize, (size_t)C));
-    FHG_TRY(ws.alloc(&pre->in_tree, (size_t)C));
-    FHG_TRY(ws.alloc(&pre->root_max, 1));
-    FHG_TRY(ws.alloc(&pre->death, (size_t)C));
-    FHG_CUDA(cudaMemsetAsync(pre->root_max, 0, sizeof(unsigned int), s));
-    FHG_CUDA(cudaMemsetAsync(pre->death, 0, sizeof(unsigned int) * C, s));
-    LAUNCH(fill_i32_kernel, n, pre->row_of_point, n, -1);
-    LAUNCH(fill_i32_kernel, C, pre->row_of_cluster, C, -1);
-    LAUNCH(row_of_child_kernel, rows, rows, n, ct.child, pre->row_of_cluster, pre->row_of_point);
-    LAUNCH(cluster_info_kernel, C, C, n, pre->row_of_cluster, ct.parent, ct.csize, pre->cpar,
-           pre->nsize, pre->in_tree);
-    LAUNCH(root_stats_kernel, rows, rows, n, ct.parent, ct.lambda, ct.csize, pre->root_max,
-           pre->death);
-    pre->ready = true;
     return FHG_OK;
 }
 
@@ -702,27 +683,26 @@ int label_points(Workspace& ws, const Condensed& ct, const int32_t* sel, int64_t
     cudaStream_t s = ws.stream();
     const int64_t n = ct.n, rows = ct.rows, C = ct.n_clusters;
     Stage stage(s, "labels");
-    FHG_CUDA(cudaMemsetAsync(probs, 0, sizeof(float) * n, s));
     if (rows == 0 || n_sel == 0) {
+        FHG_CUDA(cudaMemsetAsync(probs, 0, sizeof(float) * n, s));
         LAUNCH(fill_i64_kernel, n, labels, n, (int64_t)-1);
         return FHG_OK;
     }
     LabelPre own;
     const LabelPre* pre = pre_in;
     if (!pre || !pre->ready) {
-        FHG_TRY(label_prework(ws, ct, &own));
+        FHG_TRY(prepare(ws, ct, &own, nullptr));
         pre = &own;
     }
-    const int32_t* row_of_point = pre->row_of_point;
-    const int32_t* cpar = pre->cpar;
-    unsigned int* root_max = pre->root_max;
-    unsigned int* death = pre->death;
     int8_t* is_sel;
     int32_t *label_of, *by_label, *jmp, *sa, *jmp2, *sa2;
     uint32_t* key;
     int32_t* val;
     int* err;
-    FHG_TRY(ws.alloc(&is_sel, (size_t)C));
+    // [error flag, distinct selected clusters, is_sel], zeroed together
+    FHG_TRY(ws.alloc(&err, (size_t)(2 + (C + 3) / 4)));
+    int32_t* n_distinct = err + 1;
+    is_sel = reinterpret_cast<int8_t*>(err + 2);
     FHG_TRY(ws.alloc(&label_of, (size_t)C));
     FHG_TRY(ws.alloc(&by_label, (size_t)n_sel));
     FHG_TRY(ws.alloc(&jmp, (size_t)C));
@@ -731,34 +711,19 @@ int label_points(Workspace& ws, const Condensed& ct, const int32_t* sel, int64_t
     FHG_TRY(ws.alloc(&sa2, (size_t)C));
     FHG_TRY(ws.alloc(&key, (size_t)n_sel));
     FHG_TRY(ws.alloc(&val, (size_t)n_sel));
-    FHG_TRY(ws.alloc(&err, 1));
-    FHG_CUDA(cudaMemsetAsync(is_sel, 0, C, s));
-    FHG_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
-    LAUNCH(fill_i32_kernel, C, label_of, C, -1);
+    FHG_CUDA(cudaMemsetAsync(err, 0, 2 * sizeof(int) + C, s));
+    FHG_CUDA(cudaMemsetAsync(label_of, 0xff, sizeof(int32_t) * C, s));
     LAUNCH(sel_flags_kernel, n_sel, n_sel, n, C, sel, is_sel, key, val);
-    {
-        Workspace tmp(ws);
-        FHG_TRY(radix_sort_u32(tmp, key, val, n_sel, 0, 32));
-    }
+    FHG_TRY(radix_sort_u32(ws, key, val, n_sel, 0, 32));
     LAUNCH(label_map_kernel, n_sel, n_sel, n, C, key, label_of, by_label);
-    LAUNCH(anc_init_kernel, C, C, cpar, is_sel, jmp, sa);
-    for (int r = 0; r < bits_for(C) + 1; ++r) {
-        LAUNCH(anc_step_kernel, C, C, jmp, sa, jmp2, sa2);
-        std::swap(jmp, jmp2);
-        std::swap(sa, sa2);
-    }
-    // distinct selected count
-    int64_t n_distinct = 0;
-    {
-        int8_t* h = (int8_t*)malloc((size_t)C);
-        FHG_CUDA(cudaMemcpyAsync(h, is_sel, C, cudaMemcpyDeviceToHost, s));
-        FHG_CUDA(cudaStreamSynchronize(s));
-        for (int64_t c = 0; c < C; ++c) n_distinct += h[c] ? 1 : 0;
-        free(h);
-    }
-    LAUNCH(point_labels_kernel, n, n, n_distinct, eps, row_of_point, ct.parent, ct.lambda, sa,
-           is_sel, label_of, root_max, labels, err);
-    LAUNCH(probs_kernel, rows, rows, n, ct.child, ct.lambda, labels, by_label, death, probs);
+    const int steps = bits_for(C) + 1;
+    ::fhg::note_launch();
+    ancestors_kernel<<<1, kEomThreads, 0, s>>>(C, pre->cpar, is_sel, steps, jmp, sa, jmp2, sa2,
+                                               n_distinct);
+    FHG_CUDA(cudaGetLastError());
+    LAUNCH(point_labels_kernel, n, n, n_distinct, eps, pre->row_of_point, ct.parent, ct.lambda,
+           (steps & 1) ? sa2 : sa, is_sel, label_of, by_label, pre->root_max, pre->death, labels,
+           probs, err);
     int h_err = 0;
     FHG_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, s));
     FHG_CUDA(cudaStreamSynchronize(s));
@@ -779,25 +744,19 @@ int membership_strengths(Workspace& ws, const Condensed& ct, const int32_t* sel,
     int8_t* is_sel;
     int32_t *label_of, *by_label, *val;
     uint32_t* key;
-    unsigned int *root_max, *death;
     FHG_TRY(ws.alloc(&is_sel, (size_t)C));
     FHG_TRY(ws.alloc(&label_of, (size_t)C));
     FHG_TRY(ws.alloc(&by_label, (size_t)n_sel));
     FHG_TRY(ws.alloc(&key, (size_t)n_sel));
     FHG_TRY(ws.alloc(&val, (size_t)n_sel));
-    FHG_TRY(ws.alloc(&root_max, 1));
-    FHG_TRY(ws.alloc(&death, (size_t)C));
+    LabelPre pre;
+    FHG_TRY(prepare(ws, ct, &pre, nullptr));
     FHG_CUDA(cudaMemsetAsync(is_sel, 0, C, s));
-    FHG_CUDA(cudaMemsetAsync(death, 0, sizeof(unsigned int) * C, s));
-    LAUNCH(fill_i32_kernel, C, label_of, C, -1);
+    FHG_CUDA(cudaMemsetAsync(label_of, 0xff, sizeof(int32_t) * C, s));
     LAUNCH(sel_flags_kernel, n_sel, n_sel, n, C, sel, is_sel, key, val);
-    {
-        Workspace tmp(ws);
-        FHG_TRY(radix_sort_u32(tmp, key, val, n_sel, 0, 32));
-    }
+    FHG_TRY(radix_sort_u32(ws, key, val, n_sel, 0, 32));
     LAUNCH(label_map_kernel, n_sel, n_sel, n, C, key, label_of, by_label);
-    LAUNCH(root_stats_kernel, rows, rows, n, ct.parent, ct.lambda, ct.csize, root_max, death);
-    LAUNCH(probs_kernel, rows, rows, n, ct.child, ct.lambda, labels, by_label, death, probs);
+    LAUNCH(probs_kernel, rows, rows, n, ct.child, ct.lambda, labels, by_label, pre.death, probs);
     return FHG_OK;
 }
 

@@ -57,12 +57,9 @@ struct LabelPre {
     int8_t* in_tree = nullptr;
     unsigned int *root_max = nullptr, *death = nullptr;
 };
-int label_prework(Workspace& ws, const Condensed& ct, LabelPre* pre);
 
 // Cluster selection.  `sel` receives selected labels in the reference's
-// order; *n_sel its count (host).  With `pre`, label_prework runs on the
-// stream while the cluster stabilities (a sequential float32 sum per
-// cluster) are computed beside it.
+// order; *n_sel its count (host); *pre (nullable) what label_points can use.
 int select_eom(Workspace& ws, const Condensed& ct, double max_cluster_size, bool allow_single,
                int32_t* sel, int64_t* n_sel, LabelPre* pre = nullptr);
 int select_leaf(Workspace& ws, const Condensed& ct, int32_t* sel, int64_t* n_sel,

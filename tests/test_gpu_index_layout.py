@@ -51,3 +51,22 @@ def test_knn_list_lengths_vs_oracle(engine, n, k, kind):
     ord_, oix = O.tree_query(O.build_kdtree(X), k, mode=1)
     np.testing.assert_array_equal(rd, ord_)
     np.testing.assert_array_equal(ix, oix)
+
+
+@pytest.mark.parametrize("m", [2, 2048, 2049, 2816, 2817, 4096, 4097, 8192, 8193, 100_001,
+                               1_000_000])
+@pytest.mark.parametrize("weights", ["random", "few", "equal"])
+def test_mst_sort_sizes(engine, m, weights):
+    """The radix sort at the edges of its tiles, through the MST sort (float64
+    weights: keys of 64 and 32 bits), against np.lexsort."""
+    from fast_hdbscan_gb300.cluster_trees import sort_mst
+
+    rng = np.random.default_rng(m)
+    w = {"random": rng.normal(size=m) ** 2, "few": rng.integers(0, 5, size=m) / 4.0,
+         "equal": np.full(m, 0.5)}[weights]
+    # a spanning tree: every point past the first hangs from an earlier one
+    child = np.arange(1, m + 1)
+    mst = np.stack([(rng.random(m) * child).astype(np.int64), child, w], axis=1).astype(np.float64)
+    mst = mst[rng.permutation(m)]
+    expect = mst[np.lexsort((mst[:, 1], mst[:, 0], mst[:, 2]))]
+    np.testing.assert_array_equal(sort_mst(mst), expect)
