@@ -43,7 +43,9 @@ constexpr int kSW = 4;        // warps per block, search kernel
 constexpr int64_t kSparseNum = 1, kSparseDen = 4;
 constexpr int kStack = 64;
 constexpr int kMaxRounds = 64;
-constexpr int kLocalLevels = 4;  // first search pass: subtrees of up to 16 buckets
+// Levels that a dense search expands at once (32 nodes, one per lane), and its
+// stack: 31 nodes wait at every expanded depth of at most 26 / 5.
+constexpr int kWideLevels = 5, kWideStack = 6 * 32;
 constexpr int32_t kEmpty = -2;  // node_comp of a node with no points
 constexpr int32_t kMixed = -1;  // node_comp of a node spanning components
 
@@ -392,34 +394,178 @@ __global__ void seed_kernel(BorState S) {
 }
 
 // ------------------------------------------------------- per round: search
-// One warp per bucket of 32 query points, as in the kNN kernel.  A node is
-// entered when some lane's point lies outside the node's single component
-// (node_comp) and within that lane's threshold -- the smaller of its own best
-// weight and its component's running best (boruvka.py:182-191).  Candidates
-// of a leaf are staged in shared memory; a candidate in the query's own
-// component, or with a core distance above the threshold, costs one compare.
+// A node is entered when some lane's point lies outside the node's single
+// component (node_comp) and within that lane's threshold -- the smaller of its
+// own best weight and its component's running best (boruvka.py:182-191).
 //
 // A point whose seed already weighs its own core distance (the least weight
 // any of its edges can have) is settled without a search when every point
 // at that distance is in its kNN list: the core distance is below the k-th
 // distance, or no point outside the list lies exactly at the k-th distance
 // (knn_open clear).  Any other edge then weighs more than the seed.
+
+// Order-preserving map of float bits to uint32, and back.
+__device__ __forceinline__ uint32_t ordered_bits(float f) {
+    const uint32_t u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float ordered_float(uint32_t u) {
+    return __uint_as_float((u & 0x80000000u) ? u & 0x7fffffffu : ~u);
+}
+
+// One warp's searching points (one per lane) and a bucket scan for them.
+template <int DIM, int SP>
+struct Searcher {
+    const IndexView& ix;
+    const float* core2;
+    const int32_t* comp;
+    unsigned long long* keyA;
+    float4* xyz;     // [32 * SP / 4] a bucket's points
+    float4* queries; // [32 * SP / 4] the lanes' points
+    int2* cc;        // [32] (component, core bits) of the bucket
+    int32_t* co;     // [32] caller indices of the bucket
+    int lane;
+    float q[DIM];
+    int32_t c;       // this lane's component
+    float cp, bw;    // core distance, best weight so far
+    int32_t bq, bo;  // its far end: index position, caller index
+    float thr;       // min(bw, the component's running best)
+    bool active;
+
+    __device__ __forceinline__ void refresh() {
+        if (active) {
+            thr = fminf(thr, key_weight(*(volatile unsigned long long*)&keyA[c]));
+            active = !(cp > thr);
+        }
+    }
+
+    // The bucket's candidates for the lanes that need it.  Only candidates
+    // that can matter to some needing lane are considered: a core distance
+    // within the largest needing threshold, and -- when every needing lane is
+    // in one component -- outside it.  The best edge is a minimum over
+    // (weight, index), so the order of the visits does not change it.  Few
+    // needing lanes take the candidates one per lane and a warp minimum each;
+    // otherwise every candidate is read by all of them.
+    __device__ __forceinline__ void scan(int64_t lf, bool need) {
+        const int64_t base = lf * kLeaf;
+        const int cnt = (int)(ix.n - base < kLeaf ? ix.n - base : kLeaf);
+        float own[SP];
+        int2 mine = make_int2(0, 0);
+        int32_t own_o = 0;
+#pragma unroll
+        for (int j = 0; j < SP; ++j) own[j] = 0.0f;
+        if (lane < cnt) {
+            load_pt<SP>(ix.pts, base + lane, own);
+            mine = make_int2(comp[base + lane], __float_as_int(core2[base + lane]));
+            own_o = ix.orig[base + lane];
+        }
+        const unsigned needers = __ballot_sync(kFull, need);
+        const float mthr =
+            __uint_as_float(__reduce_max_sync(kFull, need ? __float_as_uint(thr) : 0u));
+        const int32_t c0 = __shfl_sync(kFull, c, __ffs(needers) - 1);
+        const bool one_comp = __all_sync(kFull, !need || c == c0);
+        const bool relevant =
+            lane < cnt && !(__int_as_float(mine.y) > mthr) && !(one_comp && mine.x == c0);
+        unsigned todo = __ballot_sync(kFull, relevant);
+        if (!todo) {
+            refresh();
+            return;
+        }
+        if (2 * __popc(needers) <= __popc(todo)) {
+            const float core = __int_as_float(mine.y);
+            for (unsigned m = needers; m; m &= m - 1u) {
+                const int i = __ffs(m) - 1;
+                float y[SP];
+#pragma unroll
+                for (int h = 0; h < SP / 4; ++h) {
+                    const float4 v = queries[i * (SP / 4) + h];
+                    y[4 * h] = v.x; y[4 * h + 1] = v.y; y[4 * h + 2] = v.z; y[4 * h + 3] = v.w;
+                }
+                const float cpi = __shfl_sync(kFull, cp, i), bwi = __shfl_sync(kFull, bw, i);
+                const int32_t ci = __shfl_sync(kFull, c, i);
+                const float w = fmaxf(fmaxf(rdist_rn<DIM>(y, own), cpi), core);
+                const bool in = relevant && mine.x != ci && w <= bwi;
+                if (!__any_sync(kFull, in)) continue;
+                // non-negative floats order like their bits
+                const uint32_t wm = __reduce_min_sync(kFull, in ? __float_as_uint(w) : 0xffffffffu);
+                const bool low = in && __float_as_uint(w) == wm;
+                const uint32_t om = __reduce_min_sync(kFull, low ? (uint32_t)own_o : 0xffffffffu);
+                const int t = __ffs(__ballot_sync(kFull, low && (uint32_t)own_o == om)) - 1;
+                if (lane == i) {
+                    const float wl = __uint_as_float(wm);
+                    if (wl < bw || (int32_t)om < bo) {
+                        bw = wl;
+                        bq = (int32_t)(base + t);
+                        bo = (int32_t)om;
+                        thr = fminf(thr, bw);
+                    }
+                }
+            }
+        } else {
+            __syncwarp();
+            if (lane < cnt) {
+#pragma unroll
+                for (int h = 0; h < SP / 4; ++h)
+                    xyz[lane * (SP / 4) + h] =
+                        make_float4(own[4 * h], own[4 * h + 1], own[4 * h + 2], own[4 * h + 3]);
+                cc[lane] = mine;
+                co[lane] = own_o;
+            }
+            __syncwarp();
+            for (; todo; todo &= todo - 1u) {
+                const int t = __ffs(todo) - 1;
+                const int2 tcc = cc[t];
+                const float tk = __int_as_float(tcc.y);
+                if (need && tcc.x != c && tk <= thr) {
+                    float x[SP];
+#pragma unroll
+                    for (int h = 0; h < SP / 4; ++h) {
+                        const float4 v = xyz[t * (SP / 4) + h];
+                        x[4 * h] = v.x; x[4 * h + 1] = v.y; x[4 * h + 2] = v.z; x[4 * h + 3] = v.w;
+                    }
+                    const float w = fmaxf(fmaxf(rdist_rn<DIM>(q, x), cp), tk);
+                    if (w <= bw) {
+                        const int32_t to = co[t];
+                        if (w < bw || to < bo) {
+                            bw = w;
+                            bq = (int32_t)(base + t);
+                            bo = to;
+                            thr = fminf(thr, bw);
+                        }
+                    }
+                }
+            }
+        }
+        refresh();
+    }
+};
+
+// Few points search: a warp takes 32 consecutive entries of a list of them (in
+// index order) and walks from the root, children of least bound over its
+// lanes first; both children are tested when their parent is expanded.
+// Many points search: a warp takes a bucket, and its lanes test up to 32 nodes
+// at once -- the descendants five levels down -- against the box and the
+// largest threshold of the bucket's searching points: no bound of a single
+// point to a node is below the bound between the two boxes (every operation
+// rounds monotonically).  A node left over is expanded in turn, a bucket left
+// over gets a test per lane before it is scanned.  (One node after another,
+// every lane testing its own point, took two thirds of this kernel's
+// instructions.)  pass 0 stays inside the 32 buckets around the home bucket,
+// pass 1 takes the others, so that every component's bound from its nearby
+// candidates is published before any point searches far away; pass 2 is both.
+// `split` warps share a bucket's (or 32 list entries') points, 32 / split each.
 template <int DIM, int SP>
 __global__ void __launch_bounds__(kSW * 32) search_kernel(
-    IndexView ix, const int8_t* __restrict__ knn_open,
-    const float* __restrict__ core2, const int32_t* __restrict__ comp,
-    const int2* __restrict__ nc, unsigned long long* keyA, float* __restrict__ cand_w,
-    int32_t* __restrict__ cand_q, int lvl_lo, int lvl_hi, const int32_t* __restrict__ plist,
-    int64_t plen, int ref_ties, int split, const uint32_t* __restrict__ stat) {
-    __shared__ int32_t s_stack[kSW][kStack];
-    __shared__ float4 s_xyz[kSW][32 * (SP / 4)];
-    __shared__ int2 s_cc[kSW][32];      // (component, core bits)
+    IndexView ix, const int8_t* __restrict__ knn_open, const float* __restrict__ core2,
+    const int32_t* __restrict__ comp, const int2* __restrict__ nc, unsigned long long* keyA,
+    float* __restrict__ cand_w, int32_t* __restrict__ cand_q, int pass,
+    const int32_t* __restrict__ plist, int64_t plen, int ref_ties, int split,
+    const uint32_t* __restrict__ stat) {
+    __shared__ int32_t s_stack[kSW][kWideStack];
+    __shared__ float4 s_xyz[kSW][32 * (SP / 4)], s_q[kSW][32 * (SP / 4)];
+    __shared__ int2 s_cc[kSW][32];
     __shared__ int32_t s_orig[kSW][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // Dense: warp = bucket, lane = point.  Sparse (plist): warp = 32
-    // consecutive entries of a list of the points still searching (in index
-    // order), each searching from the root.
-    // `split` warps share a bucket's points, 32 / split each.
     const bool sparse = plist != nullptr;
     const int64_t part = (int64_t)blockIdx.x * kSW + warp;
     const int64_t leaf = part / split;
@@ -429,138 +575,61 @@ __global__ void __launch_bounds__(kSW * 32) search_kernel(
     const int64_t p = sparse ? (li < plen ? plist[li] : 0) : leaf * kLeaf + lane;
     const bool valid =
         lane * split / 32 == (int)(part % split) && (sparse ? li < plen : p < ix.n);
-    int32_t c = -3;
-    float cp = 0.0f, bw = INFINITY;
-    int32_t bq = -1, bo = INT32_MAX;
-    bool active = false;
+    Searcher<DIM, SP> S{ix, core2, comp, keyA, s_xyz[warp], s_q[warp], s_cc[warp], s_orig[warp],
+                        lane};
+    S.c = -3;
+    S.cp = 0.0f;
+    S.bw = INFINITY;
+    S.bq = -1;
+    S.bo = INT32_MAX;
+    S.active = false;
+    S.thr = INFINITY;
     if (valid) {
-        c = comp[p];
-        cp = core2[p];
-        bw = cand_w[p];
-        bq = cand_q[p];
-        if (bq >= 0) bo = ix.orig[bq];
-        const bool settled = bq >= 0 && bw == cp && !knn_open[p];
-        const float thr0 = fminf(bw, key_weight(*(volatile unsigned long long*)&keyA[c]));
-        active = !settled && !(cp > thr0);
+        S.c = comp[p];
+        S.cp = core2[p];
+        S.bw = cand_w[p];
+        S.bq = cand_q[p];
+        if (S.bq >= 0) S.bo = ix.orig[S.bq];
+        const bool settled = S.bq >= 0 && S.bw == S.cp && !knn_open[p];
+        S.thr = fminf(S.bw, key_weight(*(volatile unsigned long long*)&keyA[S.c]));
+        S.active = !settled && !(S.cp > S.thr);
     }
-    if (!__any_sync(kFull, active)) return;
-    const int32_t seed_q = bq;
-    float thr = bw;
-    if (valid) thr = fminf(thr, key_weight(*(volatile unsigned long long*)&keyA[c]));
-    float q[DIM];
+    if (!__any_sync(kFull, S.active)) return;
+    const int32_t seed_q = S.bq;
     {
         float t[SP];
-        if (valid) {
-            load_pt<SP>(ix.pts, p, t);
-        } else {
 #pragma unroll
-            for (int j = 0; j < SP; ++j) t[j] = 0.0f;
-        }
+        for (int j = 0; j < SP; ++j) t[j] = 0.0f;
+        if (valid) load_pt<SP>(ix.pts, p, t);
 #pragma unroll
-        for (int j = 0; j < DIM; ++j) q[j] = t[j];
+        for (int j = 0; j < DIM; ++j) S.q[j] = t[j];
+#pragma unroll
+        for (int h = 0; h < SP / 4; ++h)
+            s_q[warp][lane * (SP / 4) + h] =
+                make_float4(t[4 * h], t[4 * h + 1], t[4 * h + 2], t[4 * h + 3]);
     }
-
-    float4* xyz = s_xyz[warp];
-    int2* cc = s_cc[warp];
-    int32_t* co = s_orig[warp];
-
-    auto scan_leaf = [&](int64_t lf, bool need) {
-        const int64_t base = lf * kLeaf;
-        const int cnt = (int)(ix.n - base < kLeaf ? ix.n - base : kLeaf);
-        if (lane < cnt) {
-            const float4* src = reinterpret_cast<const float4*>(ix.pts) + (base + lane) * (SP / 4);
-#pragma unroll
-            for (int h = 0; h < SP / 4; ++h) xyz[lane * (SP / 4) + h] = __ldg(src + h);
-            cc[lane] = make_int2(comp[base + lane], __float_as_int(core2[base + lane]));
-            co[lane] = ix.orig[base + lane];
-        }
-        __syncwarp();
-        // Only candidates that can matter to some needing lane are visited:
-        // a core distance within the largest needing threshold, and -- when
-        // every needing lane is in one component -- outside it.  The best
-        // edge is a minimum over (weight, index), so the order of the visits
-        // does not change it.
-        const unsigned needers = __ballot_sync(kFull, need);
-        const float mthr =
-            __uint_as_float(__reduce_max_sync(kFull, need ? __float_as_uint(thr) : 0u));
-        const int32_t c0 = __shfl_sync(kFull, c, __ffs(needers) - 1);
-        const bool one_comp = __all_sync(kFull, !need || c == c0);
-        bool relevant = false;
-        if (lane < cnt) {
-            const int2 mine = cc[lane];
-            relevant = !(__int_as_float(mine.y) > mthr) && !(one_comp && mine.x == c0);
-        }
-        for (unsigned todo = __ballot_sync(kFull, relevant); todo; todo &= todo - 1u) {
-            const int t = __ffs(todo) - 1;
-            const int2 tcc = cc[t];
-            const float tk = __int_as_float(tcc.y);
-            if (need && tcc.x != c && tk <= thr) {
-                float x[SP];
-#pragma unroll
-                for (int h = 0; h < SP / 4; ++h) {
-                    float4 v = xyz[t * (SP / 4) + h];
-                    x[4 * h] = v.x; x[4 * h + 1] = v.y; x[4 * h + 2] = v.z; x[4 * h + 3] = v.w;
-                }
-                const float w = fmaxf(fmaxf(rdist_rn<DIM>(q, x), cp), tk);
-                if (w <= bw) {
-                    const int32_t to = co[t];
-                    if (w < bw || to < bo) {
-                        bw = w;
-                        bq = (int32_t)(base + t);
-                        bo = to;
-                        thr = fminf(thr, bw);
-                    }
-                }
-            }
-        }
-        __syncwarp();
-        if (active) {
-            thr = fminf(thr, key_weight(*(volatile unsigned long long*)&keyA[c]));
-            active = !(cp > thr);
-        }
-    };
-
-    const int64_t first_leaf_node = ix.slots - 1;
-    const int64_t home_node = first_leaf_node + (sparse ? 0 : leaf);
-    // A home bucket spanning several components holds the nearest candidates.
-    const bool home_first = !sparse && lvl_lo == 0 && nc[home_node].x == kMixed;
-    if (home_first && __any_sync(kFull, active)) scan_leaf(leaf, active);
-
-    // Walk up from the home bucket to the root, searching the sibling subtree
-    // at every ancestor (nearest subtrees first).  As in the kNN walk,
-    // children are tested when their parent is expanded and only needed ones
-    // are pushed; a bucket's test is repeated from registers right before it
-    // is scanned.  A lane's key for a node is max(box bound, least core) when
-    // the node holds points of another component, else +inf; the node is
-    // needed when the key is within the lane's threshold.
+    __syncwarp();
     int32_t* st = s_stack[warp];
-    auto other = [&](int2 ncn) { return ncn.x != c && ncn.x != kEmpty; };
-    // (Sparse: one pass over the whole tree from the root, children of least
-    // bound over the searching lanes first.)
-    int64_t x = home_node;
-    if (!sparse)
-        for (int lv = 0; lv < lvl_lo && x > 0; ++lv) x = (x - 1) >> 1;
-    for (int lv = lvl_lo; sparse ? lv == lvl_lo : (lv < lvl_hi && x > 0); ++lv) {
-        const int32_t sib = sparse ? 0 : (int32_t)((x & 1) ? x + 1 : x - 1);
-        // children nearer the home bucket in index order first
-        const bool right_side = (x & 1) != 0;
-        if (!sparse) x = (x - 1) >> 1;
-        {
-            const int2 ncn = nc[sib];
-            bool need = active && other(ncn) && !(__int_as_float(ncn.y) > thr);
-            if (need) {
-                float b[2 * SP];
-                load_box<SP>(ix.box, sib, b);
-                need = box_lb_n<DIM, SP>(b, q) <= thr;
-            }
-            if (!__any_sync(kFull, need)) continue;
-            if (sib >= first_leaf_node) {
-                scan_leaf(sib - first_leaf_node, need);
-                continue;
+    const int64_t first_leaf_node = ix.slots - 1;
+    auto other = [&](int2 ncn) { return ncn.x != S.c && ncn.x != kEmpty; };
+    if (sparse) {
+        // A lane's key for a node is max(box bound, least core) when the node
+        // holds points of another component; the node is needed when the key
+        // is within the lane's threshold.
+        auto key_of = [&](int2 ncn, const float* b) {
+            return other(ncn) ? fmaxf(box_lb_n<DIM, SP>(b, S.q), __int_as_float(ncn.y)) : INFINITY;
+        };
+        float b0[2 * SP];
+        load_box<SP>(ix.box, 0, b0);
+        int sp = 0;
+        if (__any_sync(kFull, S.active && key_of(nc[0], b0) <= S.thr)) {
+            if (first_leaf_node == 0) {
+                S.scan(0, S.active && key_of(nc[0], b0) <= S.thr);
+            } else {
+                if (lane == 0) st[0] = 0;
+                sp = 1;
             }
         }
-        int sp = 1;
-        if (lane == 0) st[0] = sib;
         __syncwarp();
         while (sp > 0) {
             --sp;
@@ -568,54 +637,152 @@ __global__ void __launch_bounds__(kSW * 32) search_kernel(
             __syncwarp();
             const int32_t l = 2 * node + 1, r = l + 1;
             const int2 ncl = nc[l], ncr = nc[r];
-            bool nl = active && other(ncl) && !(__int_as_float(ncl.y) > thr);
-            bool nr = active && other(ncr) && !(__int_as_float(ncr.y) > thr);
-            const bool pl = __any_sync(kFull, nl), pr = __any_sync(kFull, nr);
-            if (!pl && !pr) continue;
+            bool nl = S.active && other(ncl) && !(__int_as_float(ncl.y) > S.thr);
+            bool nr = S.active && other(ncr) && !(__int_as_float(ncr.y) > S.thr);
+            if (!__any_sync(kFull, nl || nr)) continue;
             float bl[2 * SP], br[2 * SP];
-            float kl = INFINITY, kr = INFINITY;
-            if (pl) {
-                load_box<SP>(ix.box, l, bl);
-                if (other(ncl)) kl = fmaxf(box_lb_n<DIM, SP>(bl, q), __int_as_float(ncl.y));
-                nl = nl && kl <= thr;
-            }
-            if (pr) {
-                load_box<SP>(ix.box, r, br);
-                if (other(ncr)) kr = fmaxf(box_lb_n<DIM, SP>(br, q), __int_as_float(ncr.y));
-                nr = nr && kr <= thr;
-            }
+            load_box<SP>(ix.box, l, bl);
+            load_box<SP>(ix.box, r, br);
+            const float kl = key_of(ncl, bl), kr = key_of(ncr, br);
+            nl = nl && kl <= S.thr;
+            nr = nr && kr <= S.thr;
             const bool al = __any_sync(kFull, nl), ar = __any_sync(kFull, nr);
             if (!al && !ar) continue;
-            bool left_first = !(al && ar) ? al : right_side;
-            if (sparse && al && ar)  // non-negative floats order like their bits
+            bool left_first = al;
+            if (al && ar)  // non-negative floats order like their bits
                 left_first = __reduce_min_sync(kFull, nl ? __float_as_uint(kl) : 0x7f800000u) <=
                              __reduce_min_sync(kFull, nr ? __float_as_uint(kr) : 0x7f800000u);
             if (l >= first_leaf_node) {
                 // thresholds may shrink while the first bucket is scanned
-                const int32_t n1 = left_first ? l : r, n2 = left_first ? r : l;
-                if (left_first ? al : ar) scan_leaf(n1 - first_leaf_node, left_first ? nl : nr);
-                if (left_first ? ar : al) {
-                    const bool need2 = active && (left_first ? kr : kl) <= thr;
-                    if (__any_sync(kFull, need2)) scan_leaf(n2 - first_leaf_node, need2);
+                for (int turn = 0; turn < 2; ++turn) {
+                    const bool left = left_first == (turn == 0);
+                    const bool need = S.active && (left ? kl : kr) <= S.thr;
+                    if (__any_sync(kFull, need)) S.scan((left ? l : r) - first_leaf_node, need);
                 }
             } else {
-                const int32_t nearc = left_first ? l : r, farc = left_first ? r : l;
-                const bool an = left_first ? al : ar, af = left_first ? ar : al;
                 if (lane == 0) {
                     int t = sp;
-                    if (af) st[t++] = farc;
-                    if (an) st[t] = nearc;
+                    if (left_first ? ar : al) st[t++] = left_first ? r : l;
+                    st[t] = left_first ? l : r;
                 }
-                sp += (an ? 1 : 0) + (af ? 1 : 0);
+                sp += al && ar ? 2 : 1;
                 __syncwarp();
             }
         }
+    } else {
+        // One component after another: its searching points' box and largest
+        // threshold.  (Two components of one bucket can have thresholds far
+        // apart, and only the nodes that lie wholly inside the searching
+        // component fall away early.)
+        bool pending = S.active;
+        for (unsigned pm = __ballot_sync(kFull, pending); pm;
+             pm = __ballot_sync(kFull, pending)) {
+            const int32_t c0 = __shfl_sync(kFull, S.c, __ffs(pm) - 1);
+            S.active = pending && S.c == c0;
+            pending = pending && S.c != c0;
+            S.refresh();
+            if (!__any_sync(kFull, S.active)) continue;
+            float qlo[DIM], qhi[DIM];
+#pragma unroll
+            for (int j = 0; j < DIM; ++j) {
+                const uint32_t u = ordered_bits(S.q[j]);
+                qlo[j] = ordered_float(__reduce_min_sync(kFull, S.active ? u : 0xffffffffu));
+                qhi[j] = ordered_float(__reduce_max_sync(kFull, S.active ? u : 0u));
+            }
+            auto largest_thr = [&]() {
+                return __uint_as_float(
+                    __reduce_max_sync(kFull, S.active ? __float_as_uint(S.thr) : 0u));
+            };
+            float T = largest_thr();
+            auto box_key = [&](int64_t node, int2 ncn) {  // lane's node against the points' box
+                if (ncn.x == kEmpty || ncn.x == c0 || __int_as_float(ncn.y) > T) return INFINITY;
+                float b[2 * SP];
+                load_box<SP>(ix.box, node, b);
+                float r = 0.0f;
+#pragma unroll
+                for (int j = 0; j < DIM; ++j) {
+                    const float dd =
+                        fmaxf(fmaxf(__fsub_rn(b[j], qhi[j]), __fsub_rn(qlo[j], b[SP + j])), 0.0f);
+                    r = __fadd_rn(r, __fmul_rn(dd, dd));
+                }
+                return fmaxf(r, __int_as_float(ncn.y));
+            };
+            const int depth = 63 - __clzll(ix.slots);  // of the buckets
+            const int64_t home_group = leaf >> kWideLevels;
+            // the 32 buckets from 32 * group on, nearest first
+            auto scan_group = [&](int64_t group) {
+                const int size = ix.slots < 32 ? (int)ix.slots : 32;
+                const int64_t node = first_leaf_node + group * 32 + lane;
+                int2 ncn = make_int2(kEmpty, 0);
+                float key = INFINITY;
+                if (lane < size) {
+                    ncn = nc[node];
+                    key = box_key(node, ncn);
+                }
+                unsigned left = __ballot_sync(kFull, key <= T && key < INFINITY);
+                while (left) {
+                    const uint32_t mine = (left >> lane) & 1u ? __float_as_uint(key) : 0xffffffffu;
+                    const uint32_t least = __reduce_min_sync(kFull, mine);
+                    if (__uint_as_float(least) > T) break;
+                    const int t = __ffs(__ballot_sync(kFull, mine == least)) - 1;
+                    left &= ~(1u << t);
+                    const int64_t lf = group * 32 + t;
+                    const float core = __int_as_float(__shfl_sync(kFull, ncn.y, t));
+                    bool need = S.active && !(core > S.thr);
+                    if (need) {
+                        float b[2 * SP];
+                        load_box<SP>(ix.box, first_leaf_node + lf, b);
+                        need = box_lb_n<DIM, SP>(b, S.q) <= S.thr;
+                    }
+                    if (!__any_sync(kFull, need)) continue;
+                    S.scan(lf, need);
+                    T = largest_thr();
+                    if (!__any_sync(kFull, S.active)) break;
+                }
+            };
+            if (pass != 1) scan_group(home_group);
+            if (pass != 0 && depth > kWideLevels && __any_sync(kFull, S.active)) {
+                int sp = 0;
+                int64_t node = 0;  // the node to expand
+                int at = 0;        // its depth
+                for (;;) {
+                    const int step = at == 0 && depth % kWideLevels ? depth % kWideLevels : kWideLevels;
+                    const int64_t first = ((node + 1) << step) - 1;
+                    if (at + step == depth) {
+                        const int64_t group = (first - first_leaf_node) >> kWideLevels;
+                        if (group != home_group) scan_group(group);
+                    } else {
+                        const int64_t mine = first + lane;
+                        float key = INFINITY;
+                        if (lane < (1 << step)) key = box_key(mine, nc[mine]);
+                        const unsigned in = __ballot_sync(kFull, key <= T && key < INFINITY);
+                        if (in) {  // the nearest on top of the stack
+                            const bool on = (in >> lane) & 1u;
+                            const uint32_t bits = on ? __float_as_uint(key) : 0xffffffffu;
+                            const uint32_t least = __reduce_min_sync(kFull, bits);
+                            const int top = __ffs(__ballot_sync(kFull, on && bits == least)) - 1;
+                            const unsigned rest = in & ~(1u << top);
+                            if ((rest >> lane) & 1u)
+                                st[sp + __popc(rest & ((1u << lane) - 1u))] = (int32_t)mine;
+                            if (lane == top) st[sp + __popc(rest)] = (int32_t)mine;
+                            sp += __popc(in);
+                            __syncwarp();
+                        }
+                    }
+                    if (sp == 0 || !__any_sync(kFull, S.active)) break;
+                    node = st[--sp];
+                    at = 63 - __clzll(node + 1);
+                    __syncwarp();
+                }
+            }
+        }
     }
-    if (!valid || bq == seed_q) return;
-    cand_w[p] = bw;
-    cand_q[p] = bq;
-    unsigned long long key = pack_key(bw, ref_ties ? ix.orig[p] : min(ix.orig[p], bo));
-    if (key < *(volatile unsigned long long*)&keyA[c]) atomicMin(&keyA[c], key);
+    if (!valid || S.bq == seed_q) return;
+    cand_w[p] = S.bw;
+    cand_q[p] = S.bq;
+    const unsigned long long key =
+        pack_key(S.bw, ref_ties ? ix.orig[p] : min(ix.orig[p], S.bo));
+    if (key < *(volatile unsigned long long*)&keyA[S.c]) atomicMin(&keyA[S.c], key);
 }
 
 // The points that start the search searching (as search_kernel decides).
@@ -1035,14 +1202,14 @@ int launch_search(Workspace& ws, const fhg_index& ix, const int8_t* knn_open, co
     constexpr int SP = DIM <= 4 ? 4 : (DIM <= 8 ? 8 : DIM);  // as in the kNN kernel
     const int64_t n = ix.n;
     cudaStream_t s = ws.stream();
-    auto run = [&](int lo, int hi, const int32_t* list, int64_t len) -> int {
+    auto run = [&](int pass, const int32_t* list, int64_t len) -> int {
         const int64_t groups = list ? (len + 31) / 32 : ix.nleaves;
         const int split = search_split(groups);
         Stage stage(s, "search_kernel");
         ::fhg::note_launch();
         search_kernel<DIM, SP><<<grid_for(groups * split, kSW), kSW * 32, 0, s>>>(
-            view_of(ix), knn_open, S.core2, S.comp, S.nc, S.keyA, S.cand_w, S.cand_q, lo, hi, list,
-            len, S.ref_ties, split, S.stat);
+            view_of(ix), knn_open, S.core2, S.comp, S.nc, S.keyA, S.cand_w, S.cand_q, pass, list, len,
+            S.ref_ties, split, S.stat);
         FHG_CUDA(cudaGetLastError());
         return FHG_OK;
     };
@@ -1064,14 +1231,11 @@ int launch_search(Workspace& ws, const fhg_index& ix, const int8_t* knn_open, co
         const int64_t ns = h_cnt;
         if (ns == 0) return FHG_OK;
         *try_sparse = ns * kSparseDen < n * kSparseNum;
-        if (*try_sparse) return run(0, 64, list, ns);
+        if (*try_sparse) return run(2, list, ns);
     }
-    // Dense: a local pass (home bucket and the kLocalLevels nearest sibling
-    // subtrees), then the rest of the walk -- every component's bound from
-    // its nearby candidates is published before any point searches far away.
-    if (one_pass) return run(0, 64, nullptr, 0);
-    FHG_TRY(run(0, kLocalLevels, nullptr, 0));
-    return run(kLocalLevels, 64, nullptr, 0);
+    if (one_pass || ix.slots <= 32) return run(2, nullptr, 0);
+    FHG_TRY(run(0, nullptr, 0));
+    return run(1, nullptr, 0);
 }
 
 template <int DIM>
