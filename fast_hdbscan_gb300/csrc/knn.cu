@@ -108,9 +108,11 @@ __device__ __forceinline__ void merge8(unsigned long long (&key)[K],
 // 16, where a lane inserts 41; now about 20 merges.)  Until its queue is
 // emptied a lane's k-th distance is out of date, i.e. larger: it queues some
 // more candidates, and no result changes.  Measured (one GB300, lists inserted
-// one by one -> this): 10M x 3-D, k = 16: 15.3 -> 13.2 ms; 2M x 5-D, k = 11:
-// 10.4 -> 9.3; 60k x 13-D, k = 11: 2.3 -> 1.8; 1M x 3-D, k = 31: 5.9 -> 3.6
-// (this one before the index order changed), 63 % of issue slots busy.
+// one by one -> this): 10M x 3-D, k = 16: 15.3 -> 12.5 ms; 2M x 5-D, k = 11:
+// 10.4 -> 9.2; 60k x 13-D, k = 11: 2.3 -> 1.7; 1M x 3-D, k = 31: 5.9 -> 3.4
+// (this one before the index order changed), 63 % of issue slots busy.  (All
+// nodes of a level at once against the bucket's box, as the Boruvka search
+// does: 16.1 ms at 10M -- one outlying query makes its bucket walk everything.)
 template <int DIM, int SP, int K>
 __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>())
     knn_kernel(IndexView ix, int k, float* __restrict__ d_s, int32_t* __restrict__ i_s,
@@ -291,16 +293,18 @@ __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>()
             // ---- queues into lists
             if (!room || __any_sync(kFull, waiting >= full)) {
                 __syncwarp();
-                const int most = __reduce_max_sync(kFull, waiting);
-                for (int b = 0; b < most; b += 8) {
+                // whole eights of the fullest queue; the rest waits, unless the
+                // lists are wanted now or one query needs all its room
+                const int keep = full == 1 || (by_query && !room) ? 0 : 7;
+                for (int most = __reduce_max_sync(kFull, waiting); most > keep; most -= 8) {
                     unsigned long long v[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
-                        v[j] = b + j < waiting ? queue[lane * kQueueStride + b + j] : ~0ull;
+                        v[j] = j < waiting ? queue[lane * kQueueStride + waiting - 1 - j] : ~0ull;
+                    waiting = max(waiting - 8, 0);
                     sort8(v);
                     merge8<K>(key, v, rejected);
                 }
-                waiting = 0;
                 if (valid) thr = entry_dist(key[K - 1]);
                 __syncwarp();
             }
