@@ -571,7 +571,7 @@ FHG_API int fhg_mst_to_linkage_tree(const double* sorted_mst_dev, int64_t m,
     double* w;
     FHG_TRY(split_mst_f64(ws, sorted_mst_dev, m, &src, &dst, &w));
     Linkage lk;
-    FHG_TRY(sort_and_link(ws, m + 1, src, dst, w, nullptr, &lk, /*presorted=*/true));
+    FHG_TRY(sort_and_link(ws, m + 1, src, dst, w, nullptr, &lk, EdgeOrder::sorted));
     if (sample_weights_dev) FHG_TRY(weighted_sizes(ws, lk, sample_weights_dev));
     return linkage_to_f64(lk, linkage_dev, s);
 }
@@ -950,7 +950,7 @@ int fit_impl(const float* X_dev, int64_t n, int32_t d, int32_t min_samples,
         int32_t *src, *dst;
         double* w;
         FHG_TRY(split_mst_f64(ws, mst_in, n - 1, &src, &dst, &w));
-        FHG_TRY(sort_and_link(ws, n, src, dst, w, nullptr, &lk, false));
+        FHG_TRY(sort_and_link(ws, n, src, dst, w, nullptr, &lk));
     } else if (graph) {  // a precomputed sparse graph (precomputed.py:410 / :479)
         double *kedges, *core64 = core64_dev;
         int32_t* nb = neighbors_dev;
@@ -963,7 +963,8 @@ int fit_impl(const float* X_dev, int64_t n, int32_t d, int32_t min_samples,
         int32_t *src, *dst;
         double* w;
         FHG_TRY(split_mst_f64(ws, kedges, n - 1, &src, &dst, &w));
-        FHG_TRY(sort_and_link(ws, n, src, dst, w, nullptr, &lk, false));
+        // Kruskal's acceptance order: ascending weights
+        FHG_TRY(sort_and_link(ws, n, src, dst, w, nullptr, &lk, EdgeOrder::by_weight));
     } else if (knn_k > 0) {  // the kNN-graph Kruskal back-end (kruskal.py:950)
         double *kedges, *core64 = core64_dev;
         FHG_TRY(ws.alloc(&kedges, (size_t)(3 * (n - 1))));
@@ -978,7 +979,7 @@ int fit_impl(const float* X_dev, int64_t n, int32_t d, int32_t min_samples,
         int32_t *src, *dst;
         double* w;
         FHG_TRY(split_mst_f64(ws, kedges, n - 1, &src, &dst, &w));
-        FHG_TRY(sort_and_link(ws, n, src, dst, w, nullptr, &lk, false));
+        FHG_TRY(sort_and_link(ws, n, src, dst, w, nullptr, &lk, EdgeOrder::by_weight));
     } else {
         MstResult mst;
         FHG_TRY(boruvka_mst(ws, *ix, min_samples, &mst, core_dev, neighbors_dev,

@@ -14,10 +14,13 @@
 //   topmost non-continuing node -> whether a node is reached, and for a point
 //                                  the node that emits it
 //   nearest cluster birth       -> the condensed label of a reached node
-// Rows are then ordered by (emitting node's row offset, depth, preorder) --
-// the reference's emission order -- with a stable radix sort, and new cluster
+// Rows come in the reference's emission order: (emitting node's row offset,
+// depth, preorder).  A node's place in the preorder is a number below 2n - 1,
+// so the nodes are listed in preorder by writing each at its place, and the
+// points of one segment are neighbours in that list.  New cluster
 // labels are numbered by a prefix count of "both children large" nodes in
 // breadth-first order.
+#include "compact.cuh"
 #include "primitives.cuh"
 #include "trees.cuh"
 
@@ -111,35 +114,38 @@ __global__ void pj_init_kernel(int64_t m, int64_t n, const int32_t* __restrict__
     pj_store(R, i, r);
 }
 
-// One doubling step.  A node's state covers the path from it up to (not
-// including) its ancestor; the root's own contribution is an identity for
-// dep, pre and top and a default for bth, so a state stops changing one step
-// after its ancestor has become the root.  `moving` (nullable) is set when
-// some node's ancestor was not yet the root: a step that leaves it clear has
-// finished every node.
+// One step: four paths joined into one, i.e. two doublings (three gathers and
+// one record read and written, against two of each).  A node's state covers
+// the path from it up to (not including) its ancestor; the root's own
+// contribution is an identity for dep, pre and top and a default for bth, so a
+// state is final once its ancestor is the root and it has a birth.  `moving`
+// (nullable) is set when some state is not.
 __global__ void pj_step_kernel(int64_t m, const PjRec* __restrict__ R, PjRec* __restrict__ R2,
                                int* __restrict__ moving) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
-    const PjRec x = pj_load(R, i);
-    if (x.anc == (int32_t)i) {  // the root
-        pj_store(R2, i, x);
-        return;
+    const int32_t root = (int32_t)(m - 1);
+    PjRec x = pj_load(R, i);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        if (x.anc == root && x.bth != -1) break;
+        const PjRec y = pj_load(R, x.anc);
+        x.anc = y.anc;
+        x.dep += y.dep;
+        x.pre += y.pre;
+        x.top = y.top != -1 ? y.top : x.top;
+        x.bth = x.bth != -1 ? x.bth : y.bth;
     }
-    if (moving && x.anc != (int32_t)(m - 1)) *moving = 1;
-    const PjRec y = pj_load(R, x.anc);
-    PjRec z;
-    z.anc = y.anc;
-    z.dep = x.dep + y.dep;
-    z.pre = x.pre + y.pre;
-    z.top = y.top != -1 ? y.top : x.top;
-    z.bth = x.bth != -1 ? x.bth : y.bth;
-    pj_store(R2, i, z);
+    if (moving && (x.anc != root || x.bth == -1)) *moving = 1;
+    pj_store(R2, i, x);
 }
 
-__global__ void pj_split_kernel(int64_t m, const PjRec* __restrict__ R, int32_t* __restrict__ dep,
-                                int64_t* __restrict__ pre, int32_t* __restrict__ top,
-                                int32_t* __restrict__ bth) {
+// node_at: the node at every place of the preorder (-1 where the sizes given
+// with a linkage tree are not its own and leave or overstep a place).
+__global__ void pj_split_kernel(int64_t m, int64_t n, const PjRec* __restrict__ R,
+                                int32_t* __restrict__ dep, int64_t* __restrict__ pre,
+                                int32_t* __restrict__ top, int32_t* __restrict__ bth,
+                                int32_t* __restrict__ node_at) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     const PjRec x = pj_load(R, i);
@@ -147,6 +153,7 @@ __global__ void pj_split_kernel(int64_t m, const PjRec* __restrict__ R, int32_t*
     pre[i] = x.pre;
     top[i] = x.top;
     bth[i] = x.bth;
+    if (x.pre >= 0 && x.pre < n + m) node_at[x.pre] = (int32_t)(n + i);
 }
 
 // Points: derive from the parent node; decide the emitting node and segment.
@@ -156,12 +163,13 @@ __global__ void points_kernel(int64_t n, int64_t m, const int32_t* __restrict__ 
                               const int32_t* __restrict__ dep, const int64_t* __restrict__ pre,
                               const int32_t* __restrict__ top, int32_t* __restrict__ emit_u,
                               int8_t* __restrict__ emit_part, int32_t* __restrict__ pdep,
-                              int64_t* __restrict__ ppre) {
+                              int32_t* __restrict__ node_at) {
     int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= n) return;
     const int32_t p = par[x];
     pdep[x] = dep[p] + 1;
-    ppre[x] = pre[p] + (side[x] == 0 ? 1 : 2 * (int64_t)size[left[p]]);
+    const int64_t at = pre[p] + (side[x] == 0 ? 1 : 2 * (int64_t)size[left[p]]);
+    if (at >= 0 && at < n + m) node_at[at] = (int32_t)x;
     int32_t t = top[p];
     if (t == -1) t = cont[x] ? -1 : (int32_t)x;
     if (t == -1) {
@@ -173,33 +181,35 @@ __global__ void points_kernel(int64_t n, int64_t m, const int32_t* __restrict__ 
     emit_part[x] = side[t];
 }
 
-// Reached internal nodes (no non-continuing node on the path).
-__global__ void reached_flags_kernel(int64_t m, const int32_t* __restrict__ top,
-                                     uint32_t* __restrict__ flag) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m) flag[i] = top[i] == -1 ? 1u : 0u;
-}
-__global__ void compact_idx_kernel(int64_t m, const uint32_t* __restrict__ flag,
-                                   const uint32_t* __restrict__ pos, int32_t* __restrict__ out) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m && flag[i]) out[pos[i]] = (int32_t)i;
-}
-__global__ void gather_keys_kernel(int64_t cnt, const int32_t* __restrict__ items,
-                                   const int32_t* __restrict__ dep, const int64_t* __restrict__ pre,
-                                   uint32_t* __restrict__ kd, uint32_t* __restrict__ kp, int which) {
-    int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= cnt) return;
-    int32_t i = items[j];
-    if (which == 0) kp[j] = (uint32_t)pre[i];
-    else kd[j] = (uint32_t)dep[i];
-}
+// Reached internal nodes (no non-continuing node on the path), in preorder.
+struct ReachedNodes {
+    int64_t n;
+    const int32_t *node_at, *top, *dep;
+    int32_t* reached;
+    uint32_t* key;  // their depths
+    __device__ bool test(int64_t j) const {
+        const int32_t v = node_at[j];
+        return v >= n && top[v - n] == -1;
+    }
+    __device__ void emit(int64_t j, uint32_t at) const {
+        const int32_t i = (int32_t)(node_at[j] - n);
+        reached[at] = i;
+        key[at] = (uint32_t)dep[i];
+    }
+    __device__ void each(int64_t) const {}
+};
+// A reached node's rows and new clusters in one 64-bit word, so that one scan
+// gives both offsets.
+constexpr int kRowBits = 33;
+__device__ __forceinline__ int64_t row_part(int64_t v) { return v & (((int64_t)1 << kRowBits) - 1); }
+__device__ __forceinline__ int64_t new_part(int64_t v) { return v >> kRowBits; }
 // Row counts and "new clusters" flags of reached nodes in breadth-first order.
 __global__ void reached_counts_kernel(int64_t cnt, const int32_t* __restrict__ items,
                                       const int8_t* __restrict__ kase,
                                       const int32_t* __restrict__ left,
                                       const int32_t* __restrict__ right,
                                       const int32_t* __restrict__ size,
-                                      int64_t* __restrict__ nrows, int64_t* __restrict__ nnew,
+                                      int64_t* __restrict__ count,
                                       int32_t* __restrict__ bfs_pos) {
     int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= cnt) return;
@@ -211,8 +221,7 @@ __global__ void reached_counts_kernel(int64_t cnt, const int32_t* __restrict__ i
     else if (c == C3) r = size[right[i]];
     else if (c == C4) r = (int64_t)size[left[i]] + size[right[i]];
     else if (c == C6) r = 2;
-    nrows[j] = r;
-    nnew[j] = c == C6 ? 1 : 0;
+    count[j] = r | ((int64_t)(c == C6 ? 1 : 0) << kRowBits);
     bfs_pos[i] = (int32_t)j;
 }
 // Condensed label of every reached node (from its nearest birth).
@@ -221,7 +230,8 @@ __global__ void reached_labels_kernel(int64_t cnt, int64_t n, const int32_t* __r
                                       const int32_t* __restrict__ par,
                                       const int8_t* __restrict__ side,
                                       const int32_t* __restrict__ bfs_pos,
-                                      const int64_t* __restrict__ k6, int32_t* __restrict__ label) {
+                                      const int64_t* __restrict__ off,
+                                      int32_t* __restrict__ label) {
     int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= cnt) return;
     int32_t i = items[j];
@@ -231,78 +241,117 @@ __global__ void reached_labels_kernel(int64_t cnt, int64_t n, const int32_t* __r
     if (b == (int32_t)root_node) lab = (int32_t)n;
     else {
         int32_t u = par[b];
-        lab = (int32_t)(n + 1 + 2 * k6[bfs_pos[u]] + side[b]);
+        lab = (int32_t)(n + 1 + 2 * new_part(off[bfs_pos[u]]) + side[b]);
     }
     label[i] = lab;
 }
 
-// Sort items: points that are emitted, plus two rows per new-cluster node.
-// item ids: x in [0, n) for points; n + 2*j + s for the s-th row of reached
-// node j (breadth-first position) when that node creates clusters.
-__global__ void item_flags_kernel(int64_t n, int64_t cnt, const int32_t* __restrict__ emit_u,
-                                  const int64_t* __restrict__ nnew, uint32_t* __restrict__ flag) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) flag[t] = emit_u[t] >= 0 ? 1u : 0u;
-    else if (t < n + 2 * cnt) flag[t] = nnew[(t - n) >> 1] ? 1u : 0u;
-}
-__global__ void item_keys_kernel(int64_t nitems, int64_t n, const int32_t* __restrict__ items,
-                                 const int32_t* __restrict__ emit_u,
-                                 const int8_t* __restrict__ emit_part,
-                                 const int8_t* __restrict__ kase, const int32_t* __restrict__ left,
-                                 const int32_t* __restrict__ size,
-                                 const int32_t* __restrict__ bfs_pos,
-                                 const int64_t* __restrict__ roff, const int32_t* __restrict__ pdep,
-                                 const int64_t* __restrict__ ppre, uint32_t* __restrict__ kseg,
-                                 uint32_t* __restrict__ kdep, uint32_t* __restrict__ kpre) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nitems) return;
-    int32_t it = items[t];
-    if (it < n) {
-        int32_t u = emit_u[it];
-        int64_t base = roff[bfs_pos[u]];
-        if (emit_part[it] == 1 && kase[u] == C4) base += size[left[u]];
-        kseg[t] = (uint32_t)base;
-        kdep[t] = (uint32_t)pdep[it];
-        kpre[t] = (uint32_t)ppre[it];
-    } else {
-        int64_t r = it - n;
-        kseg[t] = (uint32_t)(roff[r >> 1] + (r & 1));
-        kdep[t] = 0;
-        kpre[t] = 0;
+// The points that get a row, in preorder, each with the row its segment (the
+// points eliminated under one child of one node) starts at and its depth.
+struct EmittedPoints {
+    int64_t n;
+    const int32_t *node_at, *emit_u;
+    const int8_t *emit_part, *kase;
+    const int32_t *left, *size, *bfs_pos, *pdep;
+    const int64_t* off;
+    int32_t* items;
+    uint32_t *kseg, *kdep;
+    int64_t room;
+    __device__ bool test(int64_t j) const {
+        const int32_t x = node_at[j];
+        return x >= 0 && x < n && emit_u[x] >= 0;
     }
+    __device__ void emit(int64_t j, uint32_t at) const {
+        if (at >= room) return;
+        const int32_t x = node_at[j], u = emit_u[x];
+        int64_t base = row_part(off[bfs_pos[u]]);
+        if (emit_part[x] == 1 && kase[u] == C4) base += size[left[u]];
+        items[at] = x;
+        kseg[at] = (uint32_t)base;
+        kdep[at] = (uint32_t)pdep[x];
+    }
+    __device__ void each(int64_t) const {}
+};
+__device__ __forceinline__ void point_row(int64_t r, int64_t rows, int32_t x, const int32_t* emit_u,
+                                          const int32_t* label, const float* lam,
+                                          int32_t* oparent, int32_t* ochild, float* olam,
+                                          float* osize) {
+    if (r < 0 || r >= rows) return;
+    const int32_t u = emit_u[x];
+    oparent[r] = label[u];
+    ochild[r] = x;
+    olam[r] = lam[u];
+    osize[r] = 1.0f;
 }
+// A segment is a run of the preorder, of fewer than min_cluster_size points:
+// every point counts the points of its run that precede it by (depth,
+// preorder), which is its row.
+__global__ void point_rows_kernel(int64_t items_n, int64_t rows, const int32_t* __restrict__ items,
+                                  const uint32_t* __restrict__ kseg,
+                                  const uint32_t* __restrict__ kdep,
+                                  const int32_t* __restrict__ emit_u,
+                                  const int32_t* __restrict__ label,
+                                  const float* __restrict__ lam, int32_t* __restrict__ oparent,
+                                  int32_t* __restrict__ ochild, float* __restrict__ olam,
+                                  float* __restrict__ osize) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= items_n) return;
+    const uint32_t seg = kseg[t], dep = kdep[t];
+    int64_t r = seg;
+    for (int64_t j = t - 1; j >= 0 && kseg[j] == seg; --j) r += kdep[j] <= dep ? 1 : 0;
+    for (int64_t j = t + 1; j < items_n && kseg[j] == seg; ++j) r += kdep[j] < dep ? 1 : 0;
+    point_row(r, rows, items[t], emit_u, label, lam, oparent, ochild, olam, osize);
+}
+// The same with the rank from a sort (order: items by segment, depth,
+// preorder): its place in its run of the sorted segments.
 __global__ void gather_u32_kernel(int64_t cnt, const uint32_t* __restrict__ src,
                                   const int32_t* __restrict__ perm, uint32_t* __restrict__ dst) {
     int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < cnt) dst[t] = src[perm[t]];
 }
-__global__ void rows_kernel(int64_t rows, int64_t n, const int32_t* __restrict__ order,
-                            const int32_t* __restrict__ items, const int32_t* __restrict__ reached,
-                            const int32_t* __restrict__ emit_u, const int32_t* __restrict__ label,
-                            const float* __restrict__ lam, const int32_t* __restrict__ left,
-                            const int32_t* __restrict__ right, const int32_t* __restrict__ size,
-                            const float* __restrict__ wsize, const int64_t* __restrict__ k6,
-                            int32_t* __restrict__ oparent,
-                            int32_t* __restrict__ ochild, float* __restrict__ olam,
-                            float* __restrict__ osize) {
-    int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    int32_t it = items[order[r]];
-    if (it < n) {
-        int32_t u = emit_u[it];
-        oparent[r] = label[u];
-        ochild[r] = it;
-        olam[r] = lam[u];
-        osize[r] = 1.0f;
-    } else {
-        int64_t q = it - n;
-        int64_t j = q >> 1;
-        int s = (int)(q & 1);
-        int32_t u = reached[j];
-        oparent[r] = label[u];
-        ochild[r] = (int32_t)(n + 1 + 2 * k6[j] + s);
-        olam[r] = lam[u];
+__global__ void run_starts_kernel(int64_t items_n, int64_t rows,
+                                  const uint32_t* __restrict__ seg, int32_t* __restrict__ start) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < items_n && seg[t] < rows && (t == 0 || seg[t - 1] != seg[t]))
+        start[seg[t]] = (int32_t)t;
+}
+__global__ void sorted_point_rows_kernel(int64_t items_n, int64_t rows, const int32_t* __restrict__ order,
+                                         const uint32_t* __restrict__ seg,
+                                         const int32_t* __restrict__ start,
+                                         const int32_t* __restrict__ items,
+                                         const int32_t* __restrict__ emit_u,
+                                         const int32_t* __restrict__ label,
+                                         const float* __restrict__ lam,
+                                         int32_t* __restrict__ oparent,
+                                         int32_t* __restrict__ ochild, float* __restrict__ olam,
+                                         float* __restrict__ osize) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= items_n || seg[t] >= rows) return;
+    const int64_t r = (int64_t)seg[t] + (t - start[seg[t]]);
+    point_row(r, rows, items[order[t]], emit_u, label, lam, oparent, ochild, olam, osize);
+}
+// The two rows of every node that starts clusters.
+__global__ void cluster_rows_kernel(int64_t cnt, int64_t n, const int32_t* __restrict__ reached,
+                                    const int8_t* __restrict__ kase,
+                                    const int64_t* __restrict__ off,
+                                    const int32_t* __restrict__ label,
+                                    const float* __restrict__ lam,
+                                    const int32_t* __restrict__ left,
+                                    const int32_t* __restrict__ right,
+                                    const int32_t* __restrict__ size,
+                                    const float* __restrict__ wsize,
+                                    int32_t* __restrict__ oparent, int32_t* __restrict__ ochild,
+                                    float* __restrict__ olam, float* __restrict__ osize) {
+    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= cnt) return;
+    const int32_t u = reached[j];
+    if (kase[u] != C6) return;
+    for (int s = 0; s < 2; ++s) {
+        const int64_t r = row_part(off[j]) + s;
         const int32_t v = s == 0 ? left[u] : right[u];
+        oparent[r] = label[u];
+        ochild[r] = (int32_t)(n + 1 + 2 * new_part(off[j]) + s);
+        olam[r] = lam[u];
         osize[r] = wsize ? wsize[v] : (float)size[v];
     }
 }
@@ -319,6 +368,11 @@ __global__ void condensed_out_kernel(int64_t rows, const int32_t* __restrict__ p
     ol[r] = l[r];
     oz[r] = z[r];
 }
+
+// Segments of at most this many points are ordered by counting: a point reads
+// its whole segment, so longer ones (and those of weighted trees, whose sizes
+// are no counts) are sorted.
+constexpr int64_t kCountedRun = 512;
 
 #define LAUNCH(kernel, count, ...)                                          \
     do {                                                                    \
@@ -349,8 +403,8 @@ int condense_tree(Workspace& ws, const Linkage& lk, int64_t mcs, double max_cs, 
 
     int8_t *kase, *cont, *birth, *side, *emit_part;
     float* lam;
-    int32_t *par, *dep, *top, *bth, *emit_u, *pdep;
-    int64_t *pre, *ppre;
+    int32_t *par, *dep, *top, *bth, *emit_u, *pdep, *node_at;
+    int64_t* pre;
     FHG_TRY(ws.alloc(&kase, (size_t)m));
     FHG_TRY(ws.alloc(&lam, (size_t)m));
     FHG_TRY(ws.alloc(&par, (size_t)nodes));
@@ -365,6 +419,8 @@ int condense_tree(Workspace& ws, const Linkage& lk, int64_t mcs, double max_cs, 
     FHG_TRY(ws.alloc(&pre, (size_t)m));
     FHG_TRY(ws.alloc(&top, (size_t)m));
     FHG_TRY(ws.alloc(&bth, (size_t)m));
+    FHG_TRY(ws.alloc(&node_at, (size_t)nodes));
+    FHG_CUDA(cudaMemsetAsync(node_at, 0xff, sizeof(int32_t) * nodes, s));
     {
         Workspace tmp(ws);
         PjRec *R, *R2;
@@ -373,11 +429,11 @@ int condense_tree(Workspace& ws, const Linkage& lk, int64_t mcs, double max_cs, 
         FHG_TRY(tmp.alloc(&R2, (size_t)m));
         FHG_TRY(tmp.alloc(&moving, 1));
         LAUNCH(pj_init_kernel, m, m, n, par, cont, birth, side, lk.left, lk.size, R);
-        // log2(height) + 1 steps finish every node; the height is not known,
-        // so from step 12 on every fourth step reports whether it was the last
-        const int steps = bits_for(m) + 1;
+        // log4(height) + 1 steps finish every node; the height is not known,
+        // so from step 6 on every second step reports whether it was the last
+        const int steps = (bits_for(m) + 1) / 2 + 1;
         for (int r = 0; r < steps; ++r) {
-            const bool check = r >= 11 && (r & 3) == 3 && r + 1 < steps;
+            const bool check = r >= 5 && (r & 1) == 1 && r + 1 < steps;
             if (check) FHG_CUDA(cudaMemsetAsync(moving, 0, sizeof(int), s));
             LAUNCH(pj_step_kernel, m, m, R, R2, check ? moving : nullptr);
             std::swap(R, R2);
@@ -387,104 +443,80 @@ int condense_tree(Workspace& ws, const Linkage& lk, int64_t mcs, double max_cs, 
                 if (!h_moving) break;
             }
         }
-        LAUNCH(pj_split_kernel, m, m, R, dep, pre, top, bth);
+        LAUNCH(pj_split_kernel, m, m, n, R, dep, pre, top, bth, node_at);
     }
 
     FHG_TRY(ws.alloc(&emit_u, (size_t)n));
     FHG_TRY(ws.alloc(&emit_part, (size_t)n));
     FHG_TRY(ws.alloc(&pdep, (size_t)n));
-    FHG_TRY(ws.alloc(&ppre, (size_t)n));
     LAUNCH(points_kernel, n, n, m, par, cont, side, lk.left, lk.size, dep, pre, top, emit_u,
-           emit_part, pdep, ppre);
+           emit_part, pdep, node_at);
 
-    // ---- reached internal nodes in breadth-first order
-    uint32_t *flag, *pos, *cnt_dev;
+    // ---- reached internal nodes in breadth-first order: by depth, stably from
+    // the preorder
+    uint32_t *cnt_dev, *kd;
     int32_t *reached, *bfs_pos, *label;
-    FHG_TRY(ws.alloc(&flag, (size_t)(n + 2 * m + 1)));
-    FHG_TRY(ws.alloc(&pos, (size_t)(n + 2 * m + 1)));
     FHG_TRY(ws.alloc(&cnt_dev, 2));
-    LAUNCH(reached_flags_kernel, m, m, top, flag);
-    uint32_t h_cnt = 0;
-    {
-        Workspace tmp(ws);
-        FHG_TRY(scan_exclusive_u32(tmp, flag, pos, m, cnt_dev));
-    }
     FHG_TRY(ws.alloc(&reached, (size_t)m));
-    LAUNCH(compact_idx_kernel, m, m, flag, pos, reached);
+    FHG_TRY(ws.alloc(&kd, (size_t)m));
+    FHG_TRY(compact(ws, ReachedNodes{n, node_at, top, dep, reached, kd}, nodes, cnt_dev));
+    uint32_t h_cnt = 0;
     FHG_TRY(read1(cnt_dev, &h_cnt, s));
     const int64_t cnt = h_cnt;
-    {
-        Workspace tmp(ws);
-        uint32_t *kd, *kp;
-        FHG_TRY(tmp.alloc(&kd, (size_t)cnt));
-        FHG_TRY(tmp.alloc(&kp, (size_t)cnt));
-        LAUNCH(gather_keys_kernel, cnt, cnt, reached, dep, pre, kd, kp, 0);
-        FHG_TRY(radix_sort_u32(tmp, kp, reached, cnt, 0, bits_for(2 * n)));
-        LAUNCH(gather_keys_kernel, cnt, cnt, reached, dep, pre, kd, kp, 1);
-        FHG_TRY(radix_sort_u32(tmp, kd, reached, cnt, 0, bits_for(n)));
-    }
-    int64_t *nrows, *nnew, *roff, *k6, *tot;
-    FHG_TRY(ws.alloc(&nrows, (size_t)cnt));
-    FHG_TRY(ws.alloc(&nnew, (size_t)cnt));
-    FHG_TRY(ws.alloc(&roff, (size_t)cnt));
-    FHG_TRY(ws.alloc(&k6, (size_t)cnt));
-    FHG_TRY(ws.alloc(&tot, 2));
+    // (every node above a reached one is reached: no depth is cnt or more)
+    FHG_TRY(radix_sort_u32(ws, kd, reached, cnt, 0, bits_for(cnt)));
+    int64_t *count, *off, *tot;
+    FHG_TRY(ws.alloc(&count, (size_t)cnt));
+    FHG_TRY(ws.alloc(&off, (size_t)cnt));
+    FHG_TRY(ws.alloc(&tot, 1));
     FHG_TRY(ws.alloc(&bfs_pos, (size_t)m));
     FHG_TRY(ws.alloc(&label, (size_t)m));
-    LAUNCH(reached_counts_kernel, cnt, cnt, reached, kase, lk.left, lk.right, lk.size, nrows, nnew,
+    LAUNCH(reached_counts_kernel, cnt, cnt, reached, kase, lk.left, lk.right, lk.size, count,
            bfs_pos);
-    {
-        Workspace tmp(ws);
-        FHG_TRY(scan_exclusive_i64(tmp, nrows, roff, cnt, tot));
-        FHG_TRY(scan_exclusive_i64(tmp, nnew, k6, cnt, tot + 1));
-    }
-    LAUNCH(reached_labels_kernel, cnt, cnt, n, reached, bth, par, side, bfs_pos, k6, label);
-    int64_t h_tot[2] = {0, 0};
-    FHG_CUDA(cudaMemcpyAsync(h_tot, tot, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    FHG_CUDA(cudaStreamSynchronize(s));
-    const int64_t rows = h_tot[0];
+    FHG_TRY(scan_exclusive_i64(ws, count, off, cnt, tot));
+    LAUNCH(reached_labels_kernel, cnt, cnt, n, reached, bth, par, side, bfs_pos, off, label);
+    int64_t h_tot = 0;
+    FHG_TRY(read1(tot, &h_tot, s));
+    const int64_t rows = h_tot & (((int64_t)1 << kRowBits) - 1), births = h_tot >> kRowBits;
     out->rows = rows;
-    out->n_clusters = 1 + 2 * h_tot[1];
-
-    // ---- row order: stable sort of items by (segment, depth, preorder)
-    const int64_t universe = n + 2 * cnt;
-    LAUNCH(item_flags_kernel, universe, n, cnt, emit_u, nnew, flag);
-    int32_t* items;
-    FHG_TRY(ws.alloc(&items, (size_t)(rows > 0 ? rows : 1)));
-    {
-        Workspace tmp(ws);
-        FHG_TRY(scan_exclusive_u32(tmp, flag, pos, universe, cnt_dev));
-    }
-    {
-        // compact: item id = its index in the universe
-        LAUNCH(compact_idx_kernel, universe, universe, flag, pos, items);
-    }
+    out->n_clusters = 1 + 2 * births;
     FHG_TRY(ws.alloc(&out->parent, (size_t)(rows > 0 ? rows : 1)));
     FHG_TRY(ws.alloc(&out->child, (size_t)(rows > 0 ? rows : 1)));
     FHG_TRY(ws.alloc(&out->lambda, (size_t)(rows > 0 ? rows : 1)));
     FHG_TRY(ws.alloc(&out->csize, (size_t)(rows > 0 ? rows : 1)));
     if (rows == 0) return FHG_OK;
-    {
-        Workspace tmp(ws);
-        uint32_t *kseg, *kdep, *kpre, *key;
-        int32_t* order;
-        FHG_TRY(tmp.alloc(&kseg, (size_t)rows));
-        FHG_TRY(tmp.alloc(&kdep, (size_t)rows));
-        FHG_TRY(tmp.alloc(&kpre, (size_t)rows));
-        FHG_TRY(tmp.alloc(&key, (size_t)rows));
-        FHG_TRY(tmp.alloc(&order, (size_t)rows));
-        LAUNCH(item_keys_kernel, rows, rows, n, items, emit_u, emit_part, kase, lk.left, lk.size,
-               bfs_pos, roff, pdep, ppre, kseg, kdep, kpre);
-        FHG_TRY(fill_iota_i32(order, rows, s));
-        LAUNCH(gather_u32_kernel, rows, rows, kpre, order, key);
-        FHG_TRY(radix_sort_u32(tmp, key, order, rows, 0, bits_for(2 * n)));
-        LAUNCH(gather_u32_kernel, rows, rows, kdep, order, key);
-        FHG_TRY(radix_sort_u32(tmp, key, order, rows, 0, bits_for(n)));
-        LAUNCH(gather_u32_kernel, rows, rows, kseg, order, key);
-        FHG_TRY(radix_sort_u32(tmp, key, order, rows, 0, bits_for(rows)));
-        LAUNCH(rows_kernel, rows, rows, n, order, items, reached, emit_u, label, lam, lk.left,
-               lk.right, lk.size, lk.wsize, k6, out->parent, out->child, out->lambda, out->csize);
+
+    // ---- rows: the clusters' own, and the points by (segment, depth, preorder)
+    LAUNCH(cluster_rows_kernel, cnt, cnt, n, reached, kase, off, label, lam, lk.left, lk.right,
+           lk.size, lk.wsize, out->parent, out->child, out->lambda, out->csize);
+    const int64_t pts = rows - 2 * births;
+    if (pts <= 0) return FHG_OK;
+    Workspace tmp(ws);
+    int32_t* items;
+    uint32_t *kseg, *kdep;
+    FHG_TRY(tmp.alloc(&items, (size_t)pts));
+    FHG_TRY(tmp.alloc(&kseg, (size_t)pts));
+    FHG_TRY(tmp.alloc(&kdep, (size_t)pts));
+    FHG_TRY(compact(tmp, EmittedPoints{n, node_at, emit_u, emit_part, kase, lk.left, lk.size,
+                                       bfs_pos, pdep, off, items, kseg, kdep, pts},
+                    nodes, nullptr));
+    if (!lk.wsize && mcs <= kCountedRun) {
+        LAUNCH(point_rows_kernel, pts, pts, rows, items, kseg, kdep, emit_u, label, lam, out->parent,
+               out->child, out->lambda, out->csize);
+        return FHG_OK;
     }
+    int32_t *order, *start;
+    uint32_t* key;
+    FHG_TRY(tmp.alloc(&order, (size_t)pts));
+    FHG_TRY(tmp.alloc(&start, (size_t)rows));
+    FHG_TRY(tmp.alloc(&key, (size_t)pts));
+    FHG_TRY(fill_iota_i32(order, pts, s));
+    FHG_TRY(radix_sort_u32(tmp, kdep, order, pts, 0, bits_for(n)));
+    LAUNCH(gather_u32_kernel, pts, pts, kseg, order, key);
+    FHG_TRY(radix_sort_u32(tmp, key, order, pts, 0, bits_for(rows)));
+    LAUNCH(run_starts_kernel, pts, pts, rows, key, start);
+    LAUNCH(sorted_point_rows_kernel, pts, pts, rows, order, key, start, items, emit_u, label, lam,
+           out->parent, out->child, out->lambda, out->csize);
     return FHG_OK;
 }
 

@@ -45,6 +45,55 @@ __global__ void gather_wkey_kernel(const double* __restrict__ w, const float* __
     if (w) k64[i] = f64_key(w[perm[i]]);
     else k32[i] = __float_as_uint(w2[perm[i]]);  // non-negative: bits are monotone
 }
+// The edges in weight order; their order among equal weights is settled next.
+__global__ void gather_ends_kernel(const int32_t* __restrict__ perm,
+                                   const int32_t* __restrict__ src,
+                                   const int32_t* __restrict__ dst, int32_t* __restrict__ s0,
+                                   int32_t* __restrict__ d0, int64_t m) {
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    s0[i] = src[perm[i]];
+    d0[i] = dst[perm[i]];
+}
+// Runs of equal weight ordered by (src, dst), then as they came: every edge
+// counts the edges of its run that precede it.  A run longer than `most` sets
+// *too_long and leaves the order unfinished.
+//
+// Equal weights come in short runs (one core distance shared by a few edges),
+// so this takes the place of the sorts by dst and src: six of ten digits.
+// Sort of 10M edges 1.41 -> 0.65 ms, of 20k 114 -> 70 us.
+template <class K>
+__global__ void order_ties_kernel(int64_t m, const K* __restrict__ key,
+                                  const int32_t* __restrict__ perm,
+                                  const int32_t* __restrict__ s0, const int32_t* __restrict__ d0,
+                                  const double* __restrict__ w, const float* __restrict__ w2,
+                                  int most, int32_t* __restrict__ ssrc,
+                                  int32_t* __restrict__ sdst, double* __restrict__ sw,
+                                  int32_t* __restrict__ A, int32_t* __restrict__ B,
+                                  int* __restrict__ too_long) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const K k = key[i];
+    const int32_t a = s0[i], b = d0[i];
+    int64_t at = i;
+    int seen = 0;
+    for (int64_t j = i - 1; j >= 0 && key[j] == k; --j) {
+        if (++seen > most) break;
+        if (s0[j] > a || (s0[j] == a && d0[j] > b)) --at;
+    }
+    for (int64_t j = i + 1; j < m && key[j] == k && seen <= most; ++j) {
+        ++seen;
+        if (s0[j] < a || (s0[j] == a && d0[j] < b)) ++at;
+    }
+    if (seen > most) {
+        *too_long = 1;
+        return;
+    }
+    const int32_t e = perm[i];
+    ssrc[at] = A[at] = a;
+    sdst[at] = B[at] = b;
+    sw[at] = w ? w[e] : __dsqrt_rn((double)w2[e]);
+}
 __global__ void apply_perm_kernel(const int32_t* __restrict__ perm, const int32_t* __restrict__ src,
                                   const int32_t* __restrict__ dst, const double* __restrict__ w,
                                   const float* __restrict__ w2, int32_t* __restrict__ ssrc,
@@ -418,6 +467,11 @@ __global__ void sorted_mst_f64_kernel(int64_t m, const int32_t* __restrict__ ssr
         }                                                                   \
     } while (0)
 
+// Longest run of equal weights ordered by counting, and the input size up to
+// which every run is.
+constexpr int kTieRun = 256;
+constexpr int64_t kTieRunSmall = 2048;
+
 // The whole contraction over m > 0 sorted edges with endpoint labels A, B.
 // The leaf interval length L = ceil(m / 2^K) <= kLeafRanks makes the top
 // interval L * 2^K just cover m, so every level splits its intervals at their
@@ -451,7 +505,7 @@ int contract_ranks(int64_t m, int64_t n, int32_t* A, int32_t* B, NodeRec* R, cud
 }  // namespace
 
 int sort_and_link(Workspace& ws, int64_t n, const int32_t* src, const int32_t* dst,
-                  const double* w, const float* w2, Linkage* out, bool presorted) {
+                  const double* w, const float* w2, Linkage* out, EdgeOrder order) {
     cudaStream_t s = ws.stream();
     const int64_t m = n - 1;
     *out = Linkage();
@@ -467,7 +521,9 @@ int sort_and_link(Workspace& ws, int64_t n, const int32_t* src, const int32_t* d
         return FHG_OK;
     }
 
-    // ---- sort by (weight, src, dst): stable LSD over dst, src, weight
+    // ---- sort by (weight, src, dst): a stable radix sort by weight (left out
+    // where the edges come in that order), then the runs of equal weight; a long
+    // run sends all of it to stable sorts over dst, src and weight instead
     int32_t* perm;
     uint32_t* k32;
     uint64_t* k64 = nullptr;
@@ -475,25 +531,57 @@ int sort_and_link(Workspace& ws, int64_t n, const int32_t* src, const int32_t* d
     FHG_TRY(ws.alloc(&k32, (size_t)m));
     if (w) FHG_TRY(ws.alloc(&k64, (size_t)m));
     LAUNCH(iota_kernel, m, perm, m);
-    const int ibits = bits_for(n);
-    if (!presorted) {
-        Stage stage(s, "mst_sort");
-        Workspace tmp(ws);
-        LAUNCH(gather_key32_kernel, m, dst, perm, k32, m);
-        FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, ibits));
-        LAUNCH(gather_key32_kernel, m, src, perm, k32, m);
-        FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, ibits));
-        LAUNCH(gather_wkey_kernel, m, w, w2, perm, k64, k32, m);
-        if (w) FHG_TRY(radix_sort_u64(tmp, k64, perm, m, 0, 64));
-        else FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, 32));
-    }
     int32_t *A, *B;
     FHG_TRY(ws.alloc(&out->ssrc, (size_t)m));
     FHG_TRY(ws.alloc(&out->sdst, (size_t)m));
     FHG_TRY(ws.alloc(&out->w, (size_t)m));
     FHG_TRY(ws.alloc(&A, (size_t)m));
     FHG_TRY(ws.alloc(&B, (size_t)m));
-    LAUNCH(apply_perm_kernel, m, perm, src, dst, w, w2, out->ssrc, out->sdst, out->w, A, B, m);
+    if (order == EdgeOrder::sorted) {
+        LAUNCH(apply_perm_kernel, m, perm, src, dst, w, w2, out->ssrc, out->sdst, out->w, A, B, m);
+    } else {
+        Stage stage(s, "mst_sort");
+        Workspace tmp(ws);
+        LAUNCH(gather_wkey_kernel, m, w, w2, perm, k64, k32, m);
+        if (order == EdgeOrder::any) {
+            if (w) FHG_TRY(radix_sort_u64(tmp, k64, perm, m, 0, 64));
+            else FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, 32));
+        }
+        int32_t *s0, *d0;
+        int* too_long;
+        FHG_TRY(tmp.alloc(&s0, (size_t)m));
+        FHG_TRY(tmp.alloc(&d0, (size_t)m));
+        FHG_TRY(tmp.alloc(&too_long, 1));
+        LAUNCH(gather_ends_kernel, m, perm, src, dst, s0, d0, m);
+        // (no run of a small input is too long, so its flag is not read)
+        const bool small = m <= kTieRunSmall;
+        const int most = small ? (int)kTieRunSmall : kTieRun;
+        if (!small) FHG_CUDA(cudaMemsetAsync(too_long, 0, sizeof(int), s));
+        if (w)
+            LAUNCH(order_ties_kernel<uint64_t>, m, m, k64, perm, s0, d0, w, w2, most, out->ssrc,
+                   out->sdst, out->w, A, B, too_long);
+        else
+            LAUNCH(order_ties_kernel<uint32_t>, m, m, k32, perm, s0, d0, w, w2, most, out->ssrc,
+                   out->sdst, out->w, A, B, too_long);
+        int h_long = 0;
+        if (!small) {
+            FHG_CUDA(cudaMemcpyAsync(&h_long, too_long, sizeof(int), cudaMemcpyDeviceToHost, s));
+            FHG_CUDA(cudaStreamSynchronize(s));
+        }
+        if (h_long) {
+            const int ibits = bits_for(n);
+            LAUNCH(iota_kernel, m, perm, m);
+            LAUNCH(gather_key32_kernel, m, dst, perm, k32, m);
+            FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, ibits));
+            LAUNCH(gather_key32_kernel, m, src, perm, k32, m);
+            FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, ibits));
+            LAUNCH(gather_wkey_kernel, m, w, w2, perm, k64, k32, m);
+            if (w) FHG_TRY(radix_sort_u64(tmp, k64, perm, m, 0, 64));
+            else FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, 32));
+            LAUNCH(apply_perm_kernel, m, perm, src, dst, w, w2, out->ssrc, out->sdst, out->w, A, B,
+                   m);
+        }
+    }
 
     Stage stage(s, "linkage");
     // ---- point renumbering by first edge rank

@@ -630,7 +630,7 @@ int linkage_leaf_counts(Workspace& ws, Linkage& lk) {
         LAUNCH(rep_edges_kernel, m, m, n, lk.left, lk.right, jmp, src, dst);
     }
     Linkage rebuilt;
-    FHG_TRY(sort_and_link(ws, n, src, dst, lk.w, nullptr, &rebuilt, /*presorted=*/true));
+    FHG_TRY(sort_and_link(ws, n, src, dst, lk.w, nullptr, &rebuilt, EdgeOrder::sorted));
     lk.size = rebuilt.size;
     return FHG_OK;
 }

@@ -135,11 +135,14 @@ constexpr int kRsThreads = 256;
 constexpr int kRsWarps = kRsThreads / 32;
 constexpr int kRsSmall = 2048;  // items that one block sorts alone
 constexpr int kRsMaxPasses = 8;
-// 32-item rows of a warp: a tile's keys and values fit the static 48 KB.
-template <class K>
-__host__ __device__ constexpr int rs_rows() { return sizeof(K) == 8 ? 11 : 16; }
-template <class K>
-__host__ __device__ constexpr int rs_tile() { return kRsWarps * rs_rows<K>() * 32; }
+// 32-item rows of a warp.  A tile is one block's latency, and every tile reads
+// the words of those before it that run beside it: few items want small tiles
+// (20k items, ten digits: 114 us at 8 rows, 140 at 12), many want few (16M
+// items, four digits: 914 and 764 us).  At 12 a tile fits the static 48 KB.
+constexpr int kRsRowsFew = 8, kRsRowsMany = 12;
+constexpr int64_t kRsMany = 1 << 19;
+template <int ROWS>
+__host__ __device__ constexpr int rs_tile() { return kRsWarps * ROWS * 32; }
 
 // Counts of every digit of all passes: hist[pass][256].
 template <class K>
@@ -180,6 +183,7 @@ __device__ __forceinline__ unsigned long long rs_word(int pass, int kind, uint64
 }
 constexpr int kRsOwn = 1, kRsUpTo = 2;         // the tile's own count; all up to it
 constexpr int kRsWaitPolls = 1 << 20;          // some tenths of a second
+constexpr int kRsWindow = 8;
 
 // One stable pass.  Each warp ranks its rows in order (the lanes of equal
 // digit by eight ballots, per-warp running counts); the tile's items are then
@@ -188,12 +192,12 @@ constexpr int kRsWaitPolls = 1 << 20;          // some tenths of a second
 // memory at the largest sizes and the launch at the smallest; against a
 // histogram, a scan and a scatter kernel per pass it reads the keys once less
 // and takes one launch instead of four.
-template <class K>
-__global__ void __launch_bounds__(kRsThreads, 3) rs_pass_kernel(
+template <class K, int kRows>
+__global__ void __launch_bounds__(kRsThreads, kRows <= 8 ? 5 : 4) rs_pass_kernel(
     const K* __restrict__ kin, const int32_t* __restrict__ vin, K* __restrict__ kout,
     int32_t* __restrict__ vout, int64_t n, int shift, int pass, const uint32_t* __restrict__ hist,
     uint32_t* __restrict__ counter, unsigned long long* __restrict__ state) {
-    constexpr int kRows = rs_rows<K>(), kTile = rs_tile<K>();
+    constexpr int kTile = rs_tile<kRows>();
     __shared__ uint32_t wcnt[kRsWarps][256];
     __shared__ uint32_t tstart[256];
     __shared__ int64_t gbase[256];
@@ -239,6 +243,12 @@ __global__ void __launch_bounds__(kRsThreads, 3) rs_pass_kernel(
     for (int c = 0; c < kRows; ++c)
         pos[c] = __shfl_sync(kFull, pos[c], max(__ffs(peers[c]) - 1, 0)) +
                  __popc(peers[c] & lt_mask);
+    int32_t val[kRows];  // (on their way while the block scans its counts)
+#pragma unroll
+    for (int c = 0; c < kRows; ++c) {
+        const int64_t idx = base + c * 32 + lane;
+        val[c] = idx < n ? vin[idx] : 0;
+    }
     __syncthreads();
     const int d = threadIdx.x;  // this thread's digit
     uint32_t count = 0;
@@ -258,28 +268,40 @@ __global__ void __launch_bounds__(kRsThreads, 3) rs_pass_kernel(
             const unsigned dg = (unsigned)(key[c] >> shift) & 255u;
             const uint32_t lp = tstart[dg] + wcnt[w][dg] + pos[c];
             skey[lp] = key[c];
-            sval[lp] = vin[base + c * 32 + lane];
+            sval[lp] = val[c];
         }
     }
     // ---- the digit's items in the tiles before this one
+    // (kRsWindow words at a time: tiles that run side by side have published
+    // their own counts only, and a walk over them one by one is one read's
+    // latency each)
     uint64_t before = 0;
-    bool lost = false;
-    for (int64_t t = tile - 1; t >= 0 && !lost;) {
-        const volatile unsigned long long* from = state + t * 256 + d;
-        unsigned long long x = *from;
-        int polls = 0;
-        while ((int)(x >> 56) <= 2 * pass) {  // not published in this pass yet
+    bool lost = false, done = tile == 0;
+    int polls = 0;
+    for (int64_t t = tile - 1; !done;) {
+        unsigned long long x[kRsWindow];
+#pragma unroll
+        for (int j = 0; j < kRsWindow; ++j)
+            x[j] = t - j >= 0 ? *(const volatile unsigned long long*)(state + (t - j) * 256 + d)
+                              : 0ull;
+        int taken = 0;
+#pragma unroll
+        for (int j = 0; j < kRsWindow; ++j) {
+            // in order, up to one not published in this pass yet
+            if (!done && taken == j && (int)(x[j] >> 56) > 2 * pass) {
+                before += x[j] & ((1ull << 56) - 1ull);
+                done = (int)(x[j] >> 56) == 2 * pass + kRsUpTo;
+                ++taken;
+            }
+        }
+        t -= taken;
+        if (!done && taken == 0) {
             if (++polls > kRsWaitPolls) {
                 lost = true;
                 break;
             }
             if (polls > 16) __nanosleep(64);
-            x = *from;
         }
-        if (lost) break;
-        before += x & ((1ull << 56) - 1ull);
-        if ((int)(x >> 56) == 2 * pass + kRsUpTo) break;
-        --t;
     }
     if (__syncthreads_or(lost)) {  // count them from the keys
         wcnt[0][d] = 0;
@@ -364,7 +386,9 @@ int radix_sort(Workspace& ws, K* keys, int32_t* vals, int64_t n, int begin_bit, 
         return FHG_OK;
     }
     const int passes = (end_bit - begin_bit + 7) / 8;
-    const int64_t tiles = (n + rs_tile<K>() - 1) / rs_tile<K>();
+    const bool many = n > kRsMany;
+    const int tile = many ? rs_tile<kRsRowsMany>() : rs_tile<kRsRowsFew>();
+    const int64_t tiles = (n + tile - 1) / tile;
     Workspace tmp(ws);
     // an odd number of passes over two buffers would end in the other one
     K* kb[3] = {keys, nullptr, nullptr};
@@ -382,14 +406,16 @@ int radix_sort(Workspace& ws, K* keys, int32_t* vals, int64_t n, int begin_bit, 
     unsigned long long* state = reinterpret_cast<unsigned long long*>(head + kHead);
     FHG_CUDA(cudaMemsetAsync(head, 0, words * sizeof(uint32_t), s));
     ::fhg::note_launch();
-    rs_hist_kernel<K><<<(unsigned)std::min<int64_t>(tiles, 4 * 152), kRsThreads, 0, s>>>(
+    rs_hist_kernel<K><<<(unsigned)std::min<int64_t>((n + 1023) / 1024, 6 * 152), kRsThreads, 0,
+                        s>>>(
         keys, n, begin_bit, passes, head + kRsMaxPasses);
     FHG_CUDA(cudaGetLastError());
     int cur = 0;
     for (int p = 0; p < passes; ++p) {
         const int to = p + 1 == passes && passes > 1 ? 0 : (cur == 1 ? (spare == 2 ? 2 : 0) : 1);
         ::fhg::note_launch();
-        rs_pass_kernel<K><<<(unsigned)tiles, kRsThreads, 0, s>>>(
+        const auto pass = many ? rs_pass_kernel<K, kRsRowsMany> : rs_pass_kernel<K, kRsRowsFew>;
+        pass<<<(unsigned)tiles, kRsThreads, 0, s>>>(
             kb[cur], vb[cur], kb[to], vb[to], n, begin_bit + 8 * p, p,
             head + kRsMaxPasses + 256 * p, head + p, state);
         FHG_CUDA(cudaGetLastError());

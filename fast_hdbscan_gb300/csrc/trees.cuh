@@ -21,8 +21,11 @@ struct Linkage {
 // Sorts MST rows by (weight, src, dst) (hdbscan.py:511) and builds the
 // linkage tree (cluster_trees.py:65).  w may be the float64 weight column or,
 // when w2 is given instead, the squared float32 weights (sqrt is applied).
+// `order`: what is known of the rows' order.
+enum class EdgeOrder { any, by_weight, sorted };
 int sort_and_link(Workspace& ws, int64_t n, const int32_t* src, const int32_t* dst,
-                  const double* w, const float* w2, Linkage* out, bool presorted = false);
+                  const double* w, const float* w2, Linkage* out,
+                  EdgeOrder order = EdgeOrder::any);
 
 // Column views of the reference's float64 arrays.
 int split_mst_f64(Workspace& ws, const double* mst, int64_t m, int32_t** src, int32_t** dst,

@@ -70,3 +70,19 @@ def test_mst_sort_sizes(engine, m, weights):
     mst = mst[rng.permutation(m)]
     expect = mst[np.lexsort((mst[:, 1], mst[:, 0], mst[:, 2]))]
     np.testing.assert_array_equal(sort_mst(mst), expect)
+
+
+@pytest.mark.parametrize("mcs", [1, 2, 31, 511, 512, 513, 2500])
+@pytest.mark.parametrize("n", [7000, 20_000])
+def test_condense_segments_vs_oracle(engine, n, mcs):
+    """Condensed rows ordered by counting (short segments) and by sorting."""
+    from fast_hdbscan_gb300 import synthetic
+    from fast_hdbscan_gb300.cluster_trees import condense_tree, mst_to_linkage_tree, sort_mst
+    from oracle import oracle as O
+
+    X = synthetic.varying_density(n, seed=mcs)
+    mst = O.parallel_boruvka(O.build_kdtree(X), 5, mode=1)[0]
+    linkage = mst_to_linkage_tree(sort_mst(mst))
+    got, expect = condense_tree(linkage, min_cluster_size=mcs), O.condense_tree(linkage, mcs)
+    for a, b in zip(got, expect):
+        np.testing.assert_array_equal(a, b)
