@@ -49,6 +49,7 @@ constexpr int kHdChunk = 64;    // points per streamed chunk
 constexpr int kHdCap = 192;     // largest candidate buffer per query (L + kHdChunk)
 constexpr int kHdMaxL = 128;    // candidates kept (k + 32)
 constexpr int kHdSmemMax = 227 * 1024;
+constexpr int kLandmarks = 256;
 
 __device__ __forceinline__ unsigned long long hd_key(float dist, int32_t j) {
     return ((unsigned long long)__float_as_uint(dist) << 32) | (uint32_t)j;
@@ -57,37 +58,45 @@ __device__ __forceinline__ float hd_dist(unsigned long long key) {
     return __uint_as_float((uint32_t)(key >> 32));
 }
 
-// Column means (one block per dimension, a fixed summation order).
-__global__ void __launch_bounds__(256) hd_mean_kernel(const float* __restrict__ X, int64_t n,
-                                                      int d, float* __restrict__ mu) {
-    __shared__ double part[256];
-    const int col = blockIdx.x;
+// Column means: every block sums its rows (consecutive threads take consecutive
+// columns), then one block the partial sums, each in a fixed order.
+constexpr int kMeanBlocks = 304;
+__global__ void __launch_bounds__(256) hd_mean_part_kernel(const float* __restrict__ X, int64_t n,
+                                                           int d, double* __restrict__ part) {
+    __shared__ double s_part[256];
+    const int lanes = 256 / d;  // rows side by side
+    const int col = threadIdx.x % d, row = threadIdx.x / d;
     double a = 0.0;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) a += X[i * d + col];
-    part[threadIdx.x] = a;
+    if (row < lanes)
+        for (int64_t i = (int64_t)blockIdx.x * lanes + row; i < n; i += (int64_t)gridDim.x * lanes)
+            a += X[i * d + col];
+    s_part[threadIdx.x] = a;
     __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
-        __syncthreads();
+    if (row == 0) {
+        for (int r = 1; r < lanes; ++r) a += s_part[r * d + col];
+        part[(int64_t)blockIdx.x * d + col] = a;
     }
-    if (threadIdx.x == 0) mu[col] = (float)(part[0] / (double)n);
+}
+__global__ void __launch_bounds__(kHighdMaxDim) hd_mean_kernel(const double* __restrict__ part,
+                                                               int blocks, int64_t n, int d,
+                                                               float* __restrict__ mu) {
+    const int col = threadIdx.x;
+    if (col >= d) return;
+    double a = 0.0;
+    for (int b = 0; b < blocks; ++b) a += part[(int64_t)b * d + col];
+    mu[col] = (float)(a / (double)n);
 }
 
 // Per point: the operand rows A = [hi, hi, lo] and B = [hi, lo, hi] (dp
 // columns each, zero-padded), |y|^2 (float32, dimension order), |c|, and the
 // running maxima of |y| and |c| (float bit patterns, non-negative).
-// Rows are kw >= 3 dp elements long (zero-padded: the tensor-core pipeline
-// takes whole 64-element row segments).
-__global__ void hd_split_kernel(const float* __restrict__ X, int64_t n, int d, int dp, int kw,
+__global__ void hd_split_kernel(const float* __restrict__ X, int64_t n, int d, int dp,
                                 const float* __restrict__ mu, __nv_bfloat16* __restrict__ A,
                                 __nv_bfloat16* __restrict__ B, float* __restrict__ ny,
                                 float* __restrict__ cn, unsigned* __restrict__ maxes) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    for (int k = 3 * dp; k < kw; ++k) {
-        A[i * kw + k] = __float2bfloat16_rn(0.0f);
-        B[i * kw + k] = __float2bfloat16_rn(0.0f);
-    }
+    const int kw = 3 * dp;
     float y2 = 0.0f, c2 = 0.0f;
     for (int k = 0; k < dp; ++k) {
         __nv_bfloat16 hi = __float2bfloat16_rn(0.0f), lo = hi;
@@ -362,38 +371,240 @@ __device__ __forceinline__ float hd_rdist(const float* __restrict__ q,
     return r;
 }
 
+// The same sum, read four coordinates at a time (d a multiple of 4, both rows
+// on 16-byte boundaries): a lane per row wants few, wide loads.
+__device__ __forceinline__ float hd_rdist4(const float* __restrict__ q,
+                                           const float* __restrict__ x, int d) {
+    float r = 0.0f;
+#pragma unroll 4
+    for (int k = 0; k < d; k += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(q + k);
+        const float4 b = __ldg(reinterpret_cast<const float4*>(x + k));
+        const float dx = __fsub_rn(a.x, b.x), dy = __fsub_rn(a.y, b.y);
+        const float dz = __fsub_rn(a.z, b.z), dw = __fsub_rn(a.w, b.w);
+        r = __fadd_rn(r, __fmul_rn(dx, dx));
+        r = __fadd_rn(r, __fmul_rn(dy, dy));
+        r = __fadd_rn(r, __fmul_rn(dz, dz));
+        r = __fadd_rn(r, __fmul_rn(dw, dw));
+    }
+    return r;
+}
+
 // ------------------------------------------------- tcgen05 candidate GEMM
 // The same candidates as hd_cand_kernel, from a Blackwell pipeline: a CTA of
 // 128 queries holds their operand rows in shared memory (one TMA load), and
 // every point tile of 128 rows streams through a two-stage ring of shared
 // memory by TMA (cp.async.bulk.tensor, 128-byte swizzle); one thread issues
 // the 128 x 128 x 16 bf16 tcgen05.mma steps into a float32 accumulator in
-// tensor memory (two accumulators, so the next tile's products accumulate
-// while the last one is read); four warps read the accumulator rows
-// (tcgen05.ld, lane = query) and run the selection of hd_cand_kernel on them.
+// tensor memory (four accumulators, so that the products run ahead of the
+// warps that read them); four warps read the accumulator rows (tcgen05.ld,
+// lane = query) and select.
 //   warp 0  TMA producer        warp 1  MMA issuer (allocates TMEM)
 //   warps 4-7  epilogue: query row = 32 (warp - 4) + lane, the TMEM lane
-// Operand rows are padded to a multiple of 64 bf16 (KA atoms of 128 bytes).
-// The points' |y|^2 travel in their own four-slot ring, released by the
-// epilogue (the operand ring is released by the MMA, which runs ahead).
+// Queries and points are the same rows [hi | lo]: the three products hi.hi,
+// hi.lo and lo.hi address the two halves of a row in turn, so a row is a third
+// shorter than [hi, hi, lo] beside [hi, lo, hi] and stands in memory once.
+// A tile's |y|^2, and the least of each 32 of them, travel in their own ring,
+// released by the epilogue (the operand ring is released by the MMA).
+//
+// What bounds it: the estimates of 32 columns that hold a candidate of some row
+// of a warp ("open" columns, ~1,600 cycles) against those that provably do not
+// (a maximum of 32 products, ~200).  So the rows stand grouped by their nearest
+// landmark, and by |y|^2 inside a group: the points close to a warp's queries
+// are neighbours in few columns, and every CTA starts with the tiles around its
+// own, which leave its thresholds close to their final values.  With the points
+// in order of |y|^2 alone most columns were open below a million points.
+// Candidate kernel, k = 31, 150k x 64-D: 30.5 -> 9.3 ms (5.2 with no selection).
 constexpr int kTcBM = 128;       // queries per CTA (TMEM lanes)
 constexpr int kTcBN = 128;       // points per tile (accumulator columns)
 constexpr int kTcStages = 2;     // operand ring (gated by the MMA)
-constexpr int kTcNyStages = 4;   // |y|^2 ring (gated by the epilogue, which trails the MMA by
-                                 // at most two tiles: it never holds the producer back)
-constexpr int kTcSub = 8;        // estimates inserted between buffer checks
+constexpr int kTcAcc = 4;        // accumulators (512 tensor-memory columns)
+constexpr int kTcNyStages = 8;   // |y|^2 ring (gated by the epilogue, which trails the MMA by
+                                 // at most five tiles: it never holds the producer back)
+constexpr int kTcChunk = 32;     // columns read and tested together
+constexpr int kTcRec = kTcBN + kTcBN / kTcChunk;  // a tile's |y|^2 and its chunks' least
+constexpr int kTcBack = 4;       // tiles before its own that a CTA starts with
+constexpr int kTcWarm = 8;       // tiles looked at first for thresholds, and
+constexpr int kTcWarmTiles = 32; // the fewest tiles of an input for which they are;
+constexpr int kTcLooks = kTcWarm * kTcBN / 16; // the estimates that this leaves per query
 constexpr int kTcStatic = 1024;  // room for the kernel's static shared memory (barriers)
 constexpr int kTcThreads = 256;
-constexpr int kTcTmemCols = 2 * kTcBN;
+constexpr int kTcTmemCols = kTcAcc * kTcBN;
 constexpr int kTcAtom = 128;     // bytes per swizzled operand row segment (64 bf16)
 
-__host__ __device__ constexpr int tc_cap(int L) { return (L + kTcSub + 7) / 8 * 8; }
+// A buffer cut back to at most L + kTcSlack takes all of a chunk's columns.
+constexpr int kTcSlack = 8;
+__host__ __device__ constexpr int tc_cap(int L) { return (L + kTcSlack + kTcChunk + 7) / 8 * 8; }
+static_assert(tc_cap(1 + 32) >= kTcLooks, "the first estimates fit in a buffer");
 __host__ __device__ constexpr size_t tc_smem(int ka, int L) {
     return (size_t)ka * kTcBM * kTcAtom                       // A
            + (size_t)kTcStages * ka * kTcBN * kTcAtom         // B ring
-           + (size_t)kTcNyStages * kTcBN * sizeof(float)      // |y|^2 of the ring's points
+           + (size_t)kTcNyStages * kTcRec * sizeof(float)     // |y|^2 of the ring's points
            + (size_t)kTcBM * tc_cap(L) * sizeof(unsigned long long)  // candidate buffers
            + 1024;                                            // 1024-byte alignment slack
+}
+
+// |y|^2 and |c| of every point, and the running maxima of |y| and |c| (float
+// bit patterns, non-negative): a warp per point, y = hi + lo as the rows hold
+// it.  The sums' order is the warp's; the certificate's bounds hold for any.
+__global__ void __launch_bounds__(256) hd_norms_kernel(const float* __restrict__ X, int64_t n,
+                                                       int d, const float* __restrict__ mu,
+                                                       float* __restrict__ ny,
+                                                       float* __restrict__ cn,
+                                                       unsigned* __restrict__ maxes) {
+    __shared__ unsigned s_max[2];
+    if (threadIdx.x < 2) s_max[threadIdx.x] = 0u;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    unsigned my = 0, mc = 0;
+    const int64_t warps = (int64_t)gridDim.x * 8;
+    for (int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); i < n; i += warps) {
+        float y2 = 0.0f, c2 = 0.0f;
+        for (int k = lane; k < d; k += 32) {
+            const float c = __fsub_rn(X[i * d + k], mu[k]);
+            const __nv_bfloat16 hi = __float2bfloat16_rn(c);
+            const __nv_bfloat16 lo = __float2bfloat16_rn(__fsub_rn(c, __bfloat162float(hi)));
+            const float y = __fadd_rn(__bfloat162float(hi), __bfloat162float(lo));
+            y2 = __fadd_rn(y2, __fmul_rn(y, y));
+            c2 = __fadd_rn(c2, __fmul_rn(c, c));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            y2 += __shfl_xor_sync(0xffffffffu, y2, o);
+            c2 += __shfl_xor_sync(0xffffffffu, c2, o);
+        }
+        const float c = sqrtf(c2);
+        if (lane == 0) {
+            ny[i] = y2;
+            cn[i] = c;
+        }
+        my = max(my, __float_as_uint(sqrtf(y2)));
+        mc = max(mc, __float_as_uint(c));
+    }
+    if (lane == 0) {
+        atomicMax(&s_max[0], my);
+        atomicMax(&s_max[1], mc);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) atomicMax(maxes + threadIdx.x, s_max[threadIdx.x]);
+}
+
+// Row r = [hi | lo] (dp columns each, zero-padded) of point perm[r]; |y|^2 of
+// every row and the least of each 32 in the tiles' records.  A block writes 32
+// rows; rows past the points have infinite |y|^2.
+__global__ void __launch_bounds__(256) hd_rows_kernel(const float* __restrict__ X, int64_t n,
+                                                      int d, int dp, const float* __restrict__ mu,
+                                                      const int32_t* __restrict__ perm,
+                                                      const float* __restrict__ ny,
+                                                      __nv_bfloat16* __restrict__ P,
+                                                      float* __restrict__ rec) {
+    __shared__ unsigned s_min;
+    if (threadIdx.x == 0) s_min = 0x7f800000u;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t r0 = (int64_t)blockIdx.x * kTcChunk;
+    float* out = rec + r0 / kTcBN * kTcRec;
+    const int col0 = (int)(r0 % kTcBN);
+    for (int t = w; t < kTcChunk; t += 8) {
+        const int64_t r = r0 + t;
+        float h = INFINITY;
+        if (r < n) {
+            const int64_t i = perm[r];
+            h = ny[i];
+            for (int k = 2 * lane; k < dp; k += 64) {
+                const float c0 = k < d ? __fsub_rn(X[i * d + k], mu[k]) : 0.0f;
+                const float c1 = k + 1 < d ? __fsub_rn(X[i * d + k + 1], mu[k + 1]) : 0.0f;
+                __nv_bfloat162 hi, lo;
+                hi.x = __float2bfloat16_rn(c0);
+                hi.y = __float2bfloat16_rn(c1);
+                lo.x = __float2bfloat16_rn(__fsub_rn(c0, __bfloat162float(hi.x)));
+                lo.y = __float2bfloat16_rn(__fsub_rn(c1, __bfloat162float(hi.y)));
+                *reinterpret_cast<__nv_bfloat162*>(P + r * 2 * dp + k) = hi;
+                *reinterpret_cast<__nv_bfloat162*>(P + r * 2 * dp + dp + k) = lo;
+            }
+        }
+        if (lane == 0) {
+            out[col0 + t] = h;
+            atomicMin(&s_min, __float_as_uint(h));
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) out[kTcBN + col0 / kTcChunk] = __uint_as_float(s_min);
+}
+// The landmarks' points, a warp per point: sums by atomics, then each
+// landmark's mean (the landmark itself where no point is nearest to it).  The
+// sums' order is not fixed, so neither is the last bit of a mean, nor which
+// group a point half way between two joins; no result depends on the groups.
+__global__ void __launch_bounds__(256) hd_mark_sums_kernel(int64_t n, int d,
+                                                           const float* __restrict__ X,
+                                                           const uint32_t* __restrict__ mark,
+                                                           float* __restrict__ sums,
+                                                           uint32_t* __restrict__ count) {
+    const int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const uint32_t m = mark[i];
+    for (int k = lane; k < d; k += 32) atomicAdd(&sums[(int64_t)m * d + k], X[i * d + k]);
+    if (lane == 0) atomicAdd(&count[m], 1u);
+}
+__global__ void hd_mark_means_kernel(int marks, int d, int64_t stride,
+                                     const float* __restrict__ X,
+                                     const uint32_t* __restrict__ count,
+                                     float* __restrict__ sums) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= marks * d) return;
+    const int m = t / d;
+    sums[t] = count[m] ? sums[t] / (float)count[m] : X[(int64_t)m * stride * d + (t - m * d)];
+}
+// place[m] = landmark m's place in a chain that goes on to the nearest landmark
+// not yet in it: groups of points that lie together stand together.  One block,
+// a thread per landmark with its coordinates in registers.
+__global__ void __launch_bounds__(kLandmarks) hd_chain_kernel(int marks, int d,
+                                                              const float* __restrict__ C,
+                                                              uint32_t* __restrict__ place) {
+    __shared__ float s_cur[kHighdMaxDim];
+    __shared__ uint32_t s_best[kLandmarks / 32];
+    const int m = threadIdx.x;
+    float own[kHighdMaxDim];
+#pragma unroll
+    for (int k = 0; k < kHighdMaxDim; ++k) own[k] = m < marks && k < d ? C[m * d + k] : 0.0f;
+    bool open = m < marks;
+    int cur = 0;
+    for (int step = 0; step < marks; ++step) {
+        if (m == cur) {
+            place[m] = (uint32_t)step;
+            open = false;
+#pragma unroll
+            for (int k = 0; k < kHighdMaxDim; ++k) s_cur[k] = own[k];
+        }
+        __syncthreads();
+        float a = 0.0f;
+#pragma unroll
+        for (int k = 0; k < kHighdMaxDim; k += 4) {
+            const float4 c = *reinterpret_cast<const float4*>(s_cur + k);
+            const float x = own[k] - c.x, y = own[k + 1] - c.y;
+            const float z = own[k + 2] - c.z, w = own[k + 3] - c.w;
+            a += x * x + y * y + z * z + w * w;
+        }
+        // the distance's leading bits above the landmark's number
+        const uint32_t key =
+            open ? (__float_as_uint(a) & ~(uint32_t)(kLandmarks - 1)) | (uint32_t)m : 0xffffffffu;
+        const uint32_t least = __reduce_min_sync(0xffffffffu, key);
+        if ((m & 31) == 0) s_best[m >> 5] = least;
+        __syncthreads();
+        uint32_t best = 0xffffffffu;
+#pragma unroll
+        for (int w = 0; w < kLandmarks / 32; ++w) best = min(best, s_best[w]);
+        cur = best == 0xffffffffu ? -1 : (int)(best & (kLandmarks - 1));
+    }
+}
+// key[j] = the place of the landmark of point perm[j].
+__global__ void hd_gather_key_kernel(int64_t n, const uint32_t* __restrict__ mark,
+                                     const uint32_t* __restrict__ place,
+                                     const int32_t* __restrict__ perm,
+                                     uint32_t* __restrict__ key) {
+    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < n) key[j] = place[mark[perm[j]]];
 }
 
 // Sort keys of the points by |y|^2 (non-negative: its float bits order it).
@@ -406,12 +617,13 @@ __global__ void hd_norm_keys_kernel(int64_t n, const float* __restrict__ ny,
 }
 
 // The nearest of `marks` landmarks (points 0, stride, 2 stride, ...) of every
-// point, in float32 (first landmark wins ties), with perm = identity.
-constexpr int kLandmarks = 256;
+// point, in float32 (first landmark wins ties).  marked: the landmarks
+// themselves, else points 0, stride, 2 stride, ...
 __global__ void __launch_bounds__(256) hd_landmark_kernel(int64_t n, int d,
                                                           const float* __restrict__ X, int marks,
-                                                          int64_t stride, uint32_t* __restrict__ key,
-                                                          int32_t* __restrict__ perm) {
+                                                          int64_t stride,
+                                                          const float* __restrict__ marked,
+                                                          uint32_t* __restrict__ key) {
     __shared__ float lm[32][kHighdMaxDim];
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     float best = INFINITY;
@@ -420,7 +632,9 @@ __global__ void __launch_bounds__(256) hd_landmark_kernel(int64_t n, int d,
         __syncthreads();
         for (int t = threadIdx.x; t < 32 * d; t += blockDim.x) {
             const int l = t / d, j = t - (t / d) * d;
-            lm[l][j] = c0 + l < marks ? X[(int64_t)(c0 + l) * stride * d + j] : 0.0f;
+            lm[l][j] = c0 + l >= marks ? 0.0f
+                       : marked        ? marked[(int64_t)(c0 + l) * d + j]
+                                       : X[(int64_t)(c0 + l) * stride * d + j];
         }
         __syncthreads();
         if (p < n) {
@@ -443,83 +657,116 @@ __global__ void __launch_bounds__(256) hd_landmark_kernel(int64_t n, int d,
                 }
         }
     }
-    if (p < n) {
-        key[p] = (uint32_t)bi;
-        perm[p] = (int32_t)p;
-    }
+    if (p < n) key[p] = (uint32_t)bi;
 }
 
-// Row r of Bp (vw 16-byte vectors) and nyp[r] from point perm[r].
-__global__ void hd_permute_kernel(int64_t n, int vw, const int32_t* __restrict__ perm,
-                                  const uint4* __restrict__ B, const float* __restrict__ ny,
-                                  uint4* __restrict__ Bp, float* __restrict__ nyp) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * vw) return;
-    const int64_t r = t / vw;
-    const int c = (int)(t - r * vw);
-    const int64_t j = perm[r];
-    Bp[t] = B[j * vw + c];
-    if (c == 0) nyp[r] = ny[j];
-}
-
-// hd_cut for buffers of up to 32 * PER entries (kept out of line: the
-// epilogue calls it rarely, from several places).
+// Cuts a buffer of cnt <= 32 * PER keys back to its smallest by estimate: at
+// least `keep` of them (when there are as many), at most keep + slack; which of
+// several equal estimates stay does not matter.  Returns their number; *last =
+// the estimate that no key left out is below.  That estimate is found by bitwise
+// descent from the highest bit in which the buffer's extremes differ, a ballot
+// per 32 entries and bit, and with some slack five or six bits settle it.
+// (Kept out of line: the epilogue calls it rarely.)
 template <int PER>
-__device__ __noinline__ int tc_cut(unsigned long long* buf, int cnt, int keep, int lane) {
+__device__ __noinline__ int tc_cut(unsigned long long* buf, int cnt, int keep, int slack,
+                                   int lane, float* last) {
+    if (cnt < keep) return cnt;
     unsigned long long mine[PER];
-    int rank[PER];
+    uint32_t lo = 0xffffffffu, hi = 0u;
 #pragma unroll
     for (int m = 0; m < PER; ++m) {
         const int e = lane + 32 * m;
         mine[m] = e < cnt ? buf[e] : ~0ull;
-        rank[m] = 0;
+        const uint32_t v = (uint32_t)(mine[m] >> 32);
+        if (e < cnt) {
+            lo = min(lo, v);
+            hi = max(hi, v);
+        }
     }
-    for (int e = 0; e < cnt; ++e) {
-        const unsigned long long o = buf[e];
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    uint32_t res = lo;
+    if (lo != hi) {
+        const int top = 31 - __clz(lo ^ hi);
+        res = lo & ~((2u << top) - 1u);
+        for (int b = top; b >= 0; --b) {
+            const uint32_t trial = res | (1u << b);
+            int c = 0;
 #pragma unroll
-        for (int m = 0; m < PER; ++m) rank[m] += o < mine[m] ? 1 : 0;
+            for (int m = 0; m < PER; ++m)
+                c += __popc(__ballot_sync(0xffffffffu, (uint32_t)(mine[m] >> 32) < trial));
+            if (c < keep) {
+                res = trial;
+            } else if (c <= keep + slack) {
+                res = trial;  // enough below it: no key at it is wanted
+                break;
+            }
+        }
     }
-    __syncwarp();
+    int below = 0;
 #pragma unroll
     for (int m = 0; m < PER; ++m)
-        if (lane + 32 * m < cnt && rank[m] < keep) buf[rank[m]] = mine[m];
+        below += __popc(__ballot_sync(0xffffffffu, (uint32_t)(mine[m] >> 32) < res));
+    int ties = max(keep - below, 0), at = 0;
+    const unsigned lt = (1u << lane) - 1u;
     __syncwarp();
-    return cnt < keep ? cnt : keep;
+#pragma unroll
+    for (int m = 0; m < PER; ++m) {
+        const uint32_t v = (uint32_t)(mine[m] >> 32);
+        const unsigned eq = __ballot_sync(0xffffffffu, v == res && lane + 32 * m < cnt);
+        const bool on = v < res || (((eq >> lane) & 1u) && __popc(eq & lt) < ties);
+        ties -= min(ties, __popc(eq));
+        const unsigned kept = __ballot_sync(0xffffffffu, on);
+        if (on) buf[at + __popc(kept & lt)] = mine[m];
+        at += __popc(kept);
+    }
+    __syncwarp();
+    *last = __uint_as_float(res);
+    return at;
 }
 
 template <int KA, int PER>
 __global__ void __launch_bounds__(kTcThreads, 1) hd_cand_tc_kernel(
-    const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-    int64_t n, int L, int cap, const float* __restrict__ ny, const float* __restrict__ nyq,
-    const int32_t* __restrict__ perm, const int32_t* __restrict__ qperm,
-    int32_t* __restrict__ cand, float* __restrict__ T, int* __restrict__ err) {
+    const __grid_constant__ CUtensorMap map, int64_t n, int L, int cap,
+    const float* __restrict__ rec, const int32_t* __restrict__ perm, int32_t* __restrict__ cand,
+    float* __restrict__ T, int* __restrict__ err) {
     constexpr int kABytes = KA * kTcBM * kTcAtom;
     constexpr int kBBytes = KA * kTcBN * kTcAtom;  // one stage
+    constexpr uint32_t kRecBytes = kTcRec * (uint32_t)sizeof(float);
+    constexpr int kSteps = 2 * KA;  // 16-element steps of one half of a row
     constexpr uint32_t kIdesc = tc::idesc_bf16_f32(kTcBM, kTcBN);
     extern __shared__ unsigned char tc_smem_raw[];
-    // full: a stage's operand rows and |y|^2 landed; empty: the MMA read the
-    // stage's rows; nempty: the epilogue read a slot's |y|^2; tfull /
+    // full: a stage's operand rows and record landed; empty: the MMA read the
+    // stage's rows; nempty: the epilogue read a slot's record; tfull /
     // tempty: an accumulator was written / read
     __shared__ __align__(8) uint64_t full[kTcStages], empty[kTcStages], nempty[kTcNyStages],
-        tfull[2], tempty[2], afull, done;
+        tfull[kTcAcc], tempty[kTcAcc], afull, done;
     __shared__ uint32_t tmem_slot;
     unsigned char* base = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* As = base;
     unsigned char* Bs = As + kABytes;
-    float* nys = reinterpret_cast<float*>(Bs + kTcStages * kBBytes);
-    unsigned long long* bufs = reinterpret_cast<unsigned long long*>(nys + kTcNyStages * kTcBN);
+    float* recs = reinterpret_cast<float*>(Bs + kTcStages * kBBytes);
+    unsigned long long* bufs = reinterpret_cast<unsigned long long*>(recs + kTcNyStages * kTcRec);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t q0 = (int64_t)blockIdx.x * kTcBM;
     const int64_t ntiles = (n + kTcBN - 1) / kTcBN;
+    // The sweep starts kTcBack tiles before the CTA's own and wraps around; the
+    // first `warm` steps look at its first tiles for thresholds.
+    const int64_t first = (blockIdx.x + ntiles - min((int64_t)kTcBack, ntiles - 1)) % ntiles;
+    const int64_t warm = ntiles >= kTcWarmTiles ? kTcWarm : 0, steps = ntiles + warm;
+    auto tile_of = [&](int64_t t) {
+        const int64_t x = first + (t < warm ? t : t - warm);
+        return x < ntiles ? x : x - ntiles;
+    };
     if (threadIdx.x == 0) {
         for (int s = 0; s < kTcStages; ++s) {
             tc::mbar_init(&full[s], 1);
             tc::mbar_init(&empty[s], 1);
         }
         for (int u = 0; u < kTcNyStages; ++u) tc::mbar_init(&nempty[u], 4 * 32);
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < kTcAcc; ++b) {
             tc::mbar_init(&tfull[b], 1);
             tc::mbar_init(&tempty[b], 4 * 32);
         }
@@ -539,30 +786,28 @@ __global__ void __launch_bounds__(kTcThreads, 1) hd_cand_tc_kernel(
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
         if (tc::elect_one()) {
-            tc::prefetch_tmap(&mapA);
-            tc::prefetch_tmap(&mapB);
+            tc::prefetch_tmap(&map);
             tc::mbar_arrive_expect_tx(&afull, kABytes);
             for (int a = 0; a < KA; ++a)
-                tc::tma_load_2d(As + a * kTcBM * kTcAtom, &mapA, a * 64, (int32_t)q0, &afull);
+                tc::tma_load_2d(As + a * kTcBM * kTcAtom, &map, a * 64, (int32_t)q0, &afull);
             int64_t issued = 0;
-            for (int64_t t = 0; t < ntiles; ++t) {
+            for (int64_t t = 0; t < steps; ++t) {
                 const int s = (int)(t % kTcStages);
                 const int u = (int)(t % kTcNyStages);
                 const uint32_t ph = (uint32_t)((t / kTcStages) & 1);
-                // the operand stage is free once the MMA has read tile
-                // t - kTcStages; the |y|^2 slot once the epilogue has read
-                // tile t - kTcNyStages
+                // the operand stage is free once the MMA has read step
+                // t - kTcStages; the record's slot once the epilogue has read
+                // that of step t - kTcNyStages
                 if (!tc::mbar_wait(&empty[s], ph ^ 1u, err, 1)) break;
                 if (!tc::mbar_wait(&nempty[u], (uint32_t)(((t / kTcNyStages) & 1) ^ 1), err, 7))
                     break;
-                tc::mbar_arrive_expect_tx(&full[s], kBBytes + kTcBN * (uint32_t)sizeof(float));
+                const int64_t tile = tile_of(t);
+                tc::mbar_arrive_expect_tx(&full[s], kBBytes + kRecBytes);
                 unsigned char* dst = Bs + s * kBBytes;
                 for (int a = 0; a < KA; ++a)
-                    tc::tma_load_2d(dst + a * kTcBN * kTcAtom, &mapB, a * 64,
-                                    (int32_t)(t * kTcBN), &full[s]);
-                // |y|^2 of the tile's points (ny is padded to whole tiles)
-                tc::bulk_load(nys + u * kTcBN, ny + t * kTcBN, kTcBN * (uint32_t)sizeof(float),
-                              &full[s]);
+                    tc::tma_load_2d(dst + a * kTcBN * kTcAtom, &map, a * 64,
+                                    (int32_t)(tile * kTcBN), &full[s]);
+                tc::bulk_load(recs + u * kTcRec, rec + tile * kTcRec, kRecBytes, &full[s]);
                 issued = t + 1;
             }
             // no copy may still be in flight when the block exits
@@ -574,22 +819,28 @@ __global__ void __launch_bounds__(kTcThreads, 1) hd_cand_tc_kernel(
         // ------------------------------------------------------- MMA issuer
         if (tc::elect_one()) {
             if (tc::mbar_wait(&afull, 0, err, 2)) {
-                for (int64_t t = 0; t < ntiles; ++t) {
+                for (int64_t t = 0; t < steps; ++t) {
                     const int s = (int)(t % kTcStages);
-                    const int b = (int)(t & 1);
+                    const int b = (int)(t % kTcAcc);
                     if (!tc::mbar_wait(&full[s], (uint32_t)((t / kTcStages) & 1), err, 3)) break;
-                    if (!tc::mbar_wait(&tempty[b], (uint32_t)(((t >> 1) & 1) ^ 1), err, 4)) break;
+                    if (!tc::mbar_wait(&tempty[b], (uint32_t)(((t / kTcAcc) & 1) ^ 1), err, 4))
+                        break;
                     tc::tc_fence_after();
                     const uint32_t d = tmem + (uint32_t)(b * kTcBN);
                     const uint32_t a0 = tc::smem_u32(As), b0 = tc::smem_u32(Bs + s * kBBytes);
+                    // hi.hi, hi.lo, lo.hi: step x of a row is 32 bytes of its
+                    // 64-element segment x / 4
+                    auto at = [](uint32_t rows, int x) {
+                        return tc::smem_desc_sw128(rows + (x >> 2) * kTcBM * kTcAtom +
+                                                   (x & 3) * 32);
+                    };
 #pragma unroll
-                    for (int a = 0; a < KA; ++a)
+                    for (int pair = 0; pair < 3; ++pair)
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
-                            tc::mma_bf16(d,
-                                         tc::smem_desc_sw128(a0 + a * kTcBM * kTcAtom + kk * 32),
-                                         tc::smem_desc_sw128(b0 + a * kTcBN * kTcAtom + kk * 32),
-                                         kIdesc, (a | kk) != 0);
+                        for (int x = 0; x < kSteps; ++x)
+                            tc::mma_bf16(d, at(a0, (pair == 2 ? kSteps : 0) + x),
+                                         at(b0, (pair == 1 ? kSteps : 0) + x), kIdesc,
+                                         (pair | x) != 0);
                     tc::mma_commit(&empty[s]);
                     tc::mma_commit(&tfull[b]);
                 }
@@ -603,106 +854,154 @@ __global__ void __launch_bounds__(kTcThreads, 1) hd_cand_tc_kernel(
         const int quarter = warp & 3;
         const int r = quarter * 32 + lane;
         const int64_t q = q0 + r;
-        const float nq = q < n ? nyq[q] : 0.0f;
+        const float nq = q < n ? rec[q / kTcBN * kTcRec + q % kTcBN] : 0.0f;
         unsigned long long* row = bufs + (size_t)r * cap;
-        float tq = INFINITY;
+        float tq = q < n ? INFINITY : -INFINITY;  // estimates below it are wanted
         int cnt = 0;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-        for (int64_t t = 0; t < ntiles; ++t) {
-            const int b = (int)(t & 1);
-            if (!tc::mbar_wait(&tfull[b], (uint32_t)((t >> 1) & 1), err, 6)) break;
+        // Cuts the rows in `rows` (one bit each) to their `keep` to keep + slack
+        // smallest entries; the largest of these is a threshold.
+        auto cut = [&](unsigned rows, int keep, int slack) {
+            __syncwarp();  // every lane's buffer writes visible to the warp
+            for (; rows; rows &= rows - 1u) {
+                const int rr = __ffs(rows) - 1;
+                const int cc = __shfl_sync(0xffffffffu, cnt, rr);
+                float last = INFINITY;
+                const int kept =
+                    tc_cut<PER>(bufs + (size_t)(quarter * 32 + rr) * cap, cc, keep, slack, lane, &last);
+                if (lane == rr) {
+                    cnt = kept;
+                    tq = fminf(tq, last);  // (keys at the old one may be gone)
+                }
+            }
+        };
+        // 32 columns in registers: h >= hmin for each, and, rounding being
+        // monotone, no estimate is below fl(fl(nq + hmin) - 2 max dot): columns
+        // whose bound reaches every row's threshold hold no candidate.
+        auto least = [&](const uint32_t (&acc)[kTcChunk], float hmin) {
+            float m0 = __uint_as_float(acc[0]), m1 = __uint_as_float(acc[1]);
+            float m2 = __uint_as_float(acc[2]), m3 = __uint_as_float(acc[3]);
+#pragma unroll
+            for (int i = 4; i < kTcChunk; i += 4) {
+                m0 = fmaxf(m0, __uint_as_float(acc[i]));
+                m1 = fmaxf(m1, __uint_as_float(acc[i + 1]));
+                m2 = fmaxf(m2, __uint_as_float(acc[i + 2]));
+                m3 = fmaxf(m3, __uint_as_float(acc[i + 3]));
+            }
+            const float dmax = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+            return __fsub_rn(__fadd_rn(nq, hmin), __fmul_rn(2.0f, dmax));
+        };
+        // The warm-up keeps the least estimate of every 16 columns of the tiles
+        // around the query, 64 in all, in the row's buffer: the k + 2 smallest of
+        // them lie below the first threshold, so no row is left short of k
+        // candidates, and the buffer fills once instead of with every estimate
+        // that is among the least so far (150k x 64-D: 9.3 ms; with the k + 10
+        // smallest of 64 in half the tiles 11.4, the k + 2 smallest there 9.9).
+        auto look = [&](const uint32_t (&acc)[kTcChunk], const float* h) {
+            float m[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
+#pragma unroll
+            for (int i = 0; i < kTcChunk; i += 4) {
+                const float4 hv = *reinterpret_cast<const float4*>(h + i);
+                m[0] = fminf(m[0], fmaf(-2.0f, __uint_as_float(acc[i]), hv.x));
+                m[1] = fminf(m[1], fmaf(-2.0f, __uint_as_float(acc[i + 1]), hv.y));
+                m[2] = fminf(m[2], fmaf(-2.0f, __uint_as_float(acc[i + 2]), hv.z));
+                m[3] = fminf(m[3], fmaf(-2.0f, __uint_as_float(acc[i + 3]), hv.w));
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                row[cnt++] = hd_key(fmaxf(nq + fminf(m[i], m[i + 2]), 0.0f), 0);
+        };
+        auto columns = [&](uint32_t (&acc)[kTcChunk], const float* h, float hmin, int64_t j0) {
+            const float lb = least(acc, hmin);
+            if (!__any_sync(0xffffffffu, lb < tq)) return;
+            unsigned in = 0;
+#pragma unroll
+            for (int i = 0; i < kTcChunk; ++i) {
+                const float e = fmaxf(
+                    __fsub_rn(__fadd_rn(nq, h[i]), __fmul_rn(2.0f, __uint_as_float(acc[i]))), 0.0f);
+                acc[i] = __float_as_uint(e);
+                in |= (e < tq ? 1u : 0u) << i;
+            }
+            // a row whose buffer cannot take these is first cut back to its L
+            // smallest (which only tightens its threshold)
+            const unsigned rows = __ballot_sync(0xffffffffu, cnt + __popc(in) > cap);
+            if (rows) cut(rows, L, kTcSlack);
+            // most columns are wanted by no row
+            const unsigned some = __reduce_or_sync(0xffffffffu, in);
+            if (some) {
+#pragma unroll
+                for (int i = 0; i < kTcChunk; ++i)
+                    if ((some >> i) & 1u) {
+                        if ((in >> i) & 1u)
+                            row[cnt++] = hd_key(__uint_as_float(acc[i]), (int32_t)(j0 + i));
+                    }
+            }
+            __syncwarp();  // (the loads of tensor memory want the whole warp)
+        };
+        for (int64_t t = 0; t < steps; ++t) {
+            const int b = (int)(t % kTcAcc);
+            if (!tc::mbar_wait(&tfull[b], (uint32_t)((t / kTcAcc) & 1), err, 6)) break;
+            __syncwarp();
             tc::tc_fence_after();
             const int u = (int)(t % kTcNyStages);
-            const float* hy = nys + u * kTcBN;
-            const int64_t jb = t * kTcBN;
-            // 32 accumulator columns at a time; the accumulator is handed back
-            // to the MMA as soon as its last columns are in registers
+            const float* h = recs + u * kTcRec;
+            const int64_t jb = tile_of(t) * kTcBN;
+            const uint32_t from = tmem + lane_base + (uint32_t)(b * kTcBN);
+            // the next columns are on their way while these are tested; the
+            // accumulator is handed back as soon as its last ones are here
+            uint32_t acc0[kTcChunk], acc1[kTcChunk];
+            if (t < warm) {
 #pragma unroll 1
-            for (int c = 0; c < kTcBN / 32; ++c) {
-                uint32_t acc[32];
-                tc::tmem_ld32(tmem + lane_base + (uint32_t)(b * kTcBN + c * 32), acc);
-                tc::tmem_wait_ld();
-                if (c == kTcBN / 32 - 1) {
+                for (int c = 0; c < kTcBN / kTcChunk; ++c) {
+                    tc::tmem_ld32(from + c * kTcChunk, acc0);
+                    tc::tmem_wait_ld32(acc0);
+                    look(acc0, h + c * kTcChunk);
+                }
+                if (t + 1 == warm) {
+                    const int k = L - 32;
+                    cut(__ballot_sync(0xffffffffu, q < n), min(k + 2, kTcLooks - kTcSlack),
+                        0);
+                    if (!(tq > 0.0f) && q < n) tq = INFINITY;  // (nothing is below 0)
+                    cnt = 0;
+                }
+                tc::tc_fence_before();
+                tc::mbar_arrive(&tempty[b]);
+                tc::mbar_arrive(&nempty[u]);
+                continue;
+            }
+            tc::tmem_ld32(from, acc0);
+            // (two copies of the test and of the insertion, not four: they are
+            // run from the instruction cache)
+#pragma unroll 1
+            for (int c = 0; c < kTcBN / kTcChunk; c += 2) {
+                tc::tmem_wait_ld32(acc0);
+                tc::tmem_ld32(from + (c + 1) * kTcChunk, acc1);
+                columns(acc0, h + c * kTcChunk, h[kTcBN + c], jb + c * kTcChunk);
+                tc::tmem_wait_ld32(acc1);
+                if (c + 2 < kTcBN / kTcChunk) {
+                    tc::tmem_ld32(from + (c + 2) * kTcChunk, acc0);
+                } else {
                     tc::tc_fence_before();
                     tc::mbar_arrive(&tempty[b]);
                 }
-                // estimates of 32 columns, 8 between buffer checks; only the
-                // last tile has columns past the points
-                auto columns = [&](auto whole_tag) {
-                    constexpr bool whole = decltype(whole_tag)::value;
-                    const float* h = hy + c * 32;
-                    const int64_t j0 = jb + c * 32;
-#pragma unroll
-                    for (int sub = 0; sub < 32 / kTcSub; ++sub) {
-                        float e[kTcSub];
-                        int pass = 0;
-#pragma unroll
-                        for (int i = 0; i < kTcSub; ++i) {
-                            const int col = sub * kTcSub + i;
-                            const float dot = __uint_as_float(acc[col]);
-                            e[i] = fmaxf(__fsub_rn(__fadd_rn(nq, h[col]), __fmul_rn(2.0f, dot)),
-                                         0.0f);
-                            if (!whole && j0 + col >= n) e[i] = INFINITY;
-                            pass += e[i] < tq ? 1 : 0;
-                        }
-                        // a row whose buffer cannot take these is first cut
-                        // back to its L smallest (which only tightens its
-                        // threshold)
-                        unsigned rows = __ballot_sync(0xffffffffu, cnt + pass > cap);
-                        if (rows) {
-                            __syncwarp();  // every lane's buffer writes visible to the warp
-                            do {
-                                const int rr = __ffs(rows) - 1;
-                                rows &= rows - 1u;
-                                const int cc = __shfl_sync(0xffffffffu, cnt, rr);
-                                unsigned long long* rb = bufs + (size_t)(quarter * 32 + rr) * cap;
-                                const int kept = tc_cut<PER>(rb, cc, L, lane);
-                                if (lane == rr) {
-                                    cnt = kept;
-                                    tq = kept >= L ? hd_dist(rb[L - 1]) : INFINITY;
-                                }
-                            } while (rows);
-                        }
-                        if (pass) {
-#pragma unroll
-                            for (int i = 0; i < kTcSub; ++i)
-                                if (e[i] < tq)
-                                    row[cnt++] = hd_key(e[i], (int32_t)(j0 + sub * kTcSub + i));
-                        }
-                    }
-                };
-                if (jb + kTcBN <= n) {
-                    // the points run in increasing |y|^2, so h[c * 32] is the
-                    // least of the chunk and, rounding being monotone, no
-                    // estimate of the chunk is below
-                    // fl(fl(nq + h[c * 32]) - 2 max dot): a chunk whose bound
-                    // reaches every row's threshold holds no candidate
-                    float dmax = __uint_as_float(acc[0]);
-#pragma unroll
-                    for (int i = 1; i < 32; ++i) dmax = fmaxf(dmax, __uint_as_float(acc[i]));
-                    const float lb =
-                        __fsub_rn(__fadd_rn(nq, hy[c * 32]), __fmul_rn(2.0f, dmax));
-                    if (__any_sync(0xffffffffu, lb < tq)) columns(std::true_type{});
-                } else {
-                    columns(std::false_type{});
-                }
+                columns(acc1, h + (c + 1) * kTcChunk, h[kTcBN + c + 1], jb + (c + 1) * kTcChunk);
             }
-            tc::mbar_arrive(&nempty[u]);  // this tile's |y|^2 are read
+            tc::mbar_arrive(&nempty[u]);  // this tile's record is read
         }
-        // the L smallest estimates of every row, and its L-th estimate
+        // L of the smallest estimates of every row, and its L-th estimate
+        cut(__ballot_sync(0xffffffffu, cnt >= L), L, 0);
         __syncwarp();
         for (int rr = 0; rr < 32; ++rr) {
-            const int cc = __shfl_sync(0xffffffffu, cnt, rr);
-            unsigned long long* rb = bufs + (size_t)(quarter * 32 + rr) * cap;
-            const int kept = tc_cut<PER>(rb, cc, L, lane);
+            const int kept = __shfl_sync(0xffffffffu, cnt, rr);
+            const float last = __shfl_sync(0xffffffffu, tq, rr);
+            const unsigned long long* rb = bufs + (size_t)(quarter * 32 + rr) * cap;
             const int64_t qr = q0 + quarter * 32 + rr;
             if (qr < n) {
-                const int64_t qq = qperm[qr];
+                const int64_t qq = perm[qr];
                 for (int e2 = lane; e2 < L; e2 += 32)
                     cand[qq * L + e2] = e2 < kept ? perm[(uint32_t)rb[e2]] : -1;
-                if (lane == 0) T[qq] = kept >= L ? hd_dist(rb[L - 1]) : INFINITY;
+                if (lane == 0) T[qq] = last;
             }
-            __syncwarp();
         }
     }
     tc::tc_fence_before();
@@ -711,15 +1010,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) hd_cand_tc_kernel(
     if (warp == 1) tc::tmem_dealloc(tmem, kTcTmemCols);
 }
 
-// Re-rank: a warp per query.  Writes the certified queries' k nearest (rows
+// Re-rank: a warp per query (150k x 64-D, k = 31: 2.07 ms by single coordinates,
+// 0.63 by four).  Writes the certified queries' k nearest (rows
 // of k, (distance, index) order) and lists the others.
+template <bool WIDE>
 __global__ void __launch_bounds__(128) hd_rerank_kernel(
     int64_t n, int d, int dp, int k, int L, const float* __restrict__ X,
     const int32_t* __restrict__ cand, const float* __restrict__ T, const float* __restrict__ ny,
     const float* __restrict__ cn, const unsigned* __restrict__ maxes, float* __restrict__ rd_o,
     int32_t* __restrict__ ix_o, int32_t* __restrict__ fail_list,
     unsigned long long* __restrict__ fail_count) {
-    __shared__ float qs[4][96];
+    __shared__ __align__(16) float qs[4][96];
     __shared__ unsigned long long keys[4][kHdMaxL];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t q = (int64_t)blockIdx.x * 4 + warp;
@@ -729,7 +1030,9 @@ __global__ void __launch_bounds__(128) hd_rerank_kernel(
     int cntc = 0;
     for (int e = lane; e < L; e += 32) {
         const int32_t j = cand[q * L + e];
-        keys[warp][e] = j >= 0 ? hd_key(hd_rdist(qs[warp], X + (int64_t)j * d, d), j) : ~0ull;
+        const float* x = X + (int64_t)j * d;
+        keys[warp][e] =
+            j >= 0 ? hd_key(WIDE ? hd_rdist4(qs[warp], x, d) : hd_rdist(qs[warp], x, d), j) : ~0ull;
     }
     __syncwarp();
     for (int e = 0; e < L; ++e) cntc += keys[warp][e] != ~0ull ? 1 : 0;
@@ -908,12 +1211,11 @@ int tensor_map_rows(CUtensorMap* map, const __nv_bfloat16* base, int64_t rows, i
 }
 
 template <int KA, int PER>
-int launch_cand_tc(int64_t n, int L, const __nv_bfloat16* A, const __nv_bfloat16* B,
-                   const float* ny_padded, const float* nyq, const int32_t* perm,
-                   const int32_t* qperm, int32_t* cand, float* T, int* err, cudaStream_t s) {
-    CUtensorMap ma, mb;
-    FHG_TRY(tensor_map_rows(&ma, A, n, KA * 64, kTcBM));
-    FHG_TRY(tensor_map_rows(&mb, B, n, KA * 64, kTcBN));
+int launch_cand_tc(int64_t n, int L, const __nv_bfloat16* P, const float* rec,
+                   const int32_t* perm, int32_t* cand, float* T, int* err, cudaStream_t s) {
+    static_assert(kTcBM == kTcBN, "one tensor map serves queries and points");
+    CUtensorMap map;
+    FHG_TRY(tensor_map_rows(&map, P, n, KA * 64, kTcBM));
     const size_t smem = tc_smem(KA, L);
     FHG_CUDA(cudaFuncSetAttribute(hd_cand_tc_kernel<KA, PER>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -921,34 +1223,30 @@ int launch_cand_tc(int64_t n, int L, const __nv_bfloat16* A, const __nv_bfloat16
     Stage stage(s, "hd_cand_kernel");
     ::fhg::note_launch();
     hd_cand_tc_kernel<KA, PER><<<(unsigned)blocks, kTcThreads, smem, s>>>(
-        ma, mb, n, L, tc_cap(L), ny_padded, nyq, perm, qperm, cand, T, err);
+        map, n, L, tc_cap(L), rec, perm, cand, T, err);
     FHG_CUDA(cudaGetLastError());
     return FHG_OK;
 }
 
-// The tensor-core pipeline's operand atoms for (dp, L), or 0 when the
-// mma.sync kernel must run (rows of 96 dimensions, or buffers too large for
-// shared memory).
+// The tensor-core pipeline's 64-element segments of a row [hi | lo] for (dp,
+// L), or 0 when the mma.sync kernel must run (rows of 96 dimensions, or
+// buffers too large for shared memory: k > 56 at 64 dimensions).
 int tc_atoms(int dp, int L) {
-    const int ka = dp == 32 ? 2 : (dp == 64 ? 3 : 0);
+    const int ka = dp == 32 ? 1 : (dp == 64 ? 2 : 0);
     if (ka == 0 || tc_cap(L) > 32 * 4 || tc_smem(ka, L) + kTcStatic > (size_t)kHdSmemMax)
         return 0;
     return ka;
 }
 
-int launch_cand_tc_any(int ka, int64_t n, int L, const __nv_bfloat16* A, const __nv_bfloat16* B,
-                       const float* ny_padded, const float* nyq, const int32_t* perm,
-                       const int32_t* qperm, int32_t* cand, float* T, int* err,
-                       cudaStream_t s) {
+int launch_cand_tc_any(int ka, int64_t n, int L, const __nv_bfloat16* P, const float* rec,
+                       const int32_t* perm, int32_t* cand, float* T, int* err, cudaStream_t s) {
     const int per = (tc_cap(L) + 31) / 32;
-#define FHG_TC(KA, PER)                                                                     \
-    if (ka == KA && per == PER)                                                             \
-        return launch_cand_tc<KA, PER>(n, L, A, B, ny_padded, nyq, perm, qperm, cand, T, err, \
-                                       s);
-    FHG_TC(2, 1) FHG_TC(2, 2) FHG_TC(2, 3) FHG_TC(2, 4)
-    FHG_TC(3, 1) FHG_TC(3, 2) FHG_TC(3, 3) FHG_TC(3, 4)
+#define FHG_TC(KA, PER) \
+    if (ka == KA && per == PER) return launch_cand_tc<KA, PER>(n, L, P, rec, perm, cand, T, err, s);
+    FHG_TC(1, 3) FHG_TC(1, 4)
+    FHG_TC(2, 3) FHG_TC(2, 4)
 #undef FHG_TC
-    set_error("tensor-core kNN: no pipeline for %d atoms, %d-entry buffers", ka, tc_cap(L));
+    set_error("tensor-core kNN: no pipeline for %d segments, %d-entry buffers", ka, tc_cap(L));
     return FHG_ERR_UNSUPPORTED;
 }
 
@@ -983,76 +1281,80 @@ int highd_knn(const float* X, int64_t n, int d, int k, float* rd_o, int32_t* ix_
     const int dp = d <= 32 ? 32 : (d <= 64 ? 64 : 96);
     const int L = k + 32;
     const int ka = t_hd_legacy ? 0 : tc_atoms(dp, L);
-    const int kw = ka ? 64 * ka : 3 * dp;
-    const int64_t n_pad = (n + kTcBN - 1) / kTcBN * kTcBN;
     Workspace ws(s);
     float *mu, *ny, *cn, *T;
+    double* part;
     unsigned* maxes;
-    __nv_bfloat16 *A, *B;
     int32_t *cand, *flist;
     unsigned long long* fcount;
     FHG_TRY(ws.alloc(&mu, (size_t)d));
-    FHG_TRY(ws.alloc(&ny, (size_t)n_pad));  // whole point tiles for the bulk copies
+    FHG_TRY(ws.alloc(&part, (size_t)kMeanBlocks * d));
+    FHG_TRY(ws.alloc(&ny, (size_t)n));
     FHG_TRY(ws.alloc(&cn, (size_t)n));
     FHG_TRY(ws.alloc(&T, (size_t)n));
     FHG_TRY(ws.alloc(&maxes, 2));
-    FHG_TRY(ws.alloc(&A, (size_t)(n * kw)));
-    FHG_TRY(ws.alloc(&B, (size_t)(n * kw)));
     FHG_TRY(ws.alloc(&cand, (size_t)(n * L)));
     FHG_TRY(ws.alloc(&flist, (size_t)n));
     FHG_TRY(ws.alloc(&fcount, 1));
     FHG_CUDA(cudaMemsetAsync(maxes, 0, 2 * sizeof(unsigned), s));
     FHG_CUDA(cudaMemsetAsync(fcount, 0, sizeof(unsigned long long), s));
-    if (n_pad > n) FHG_CUDA(cudaMemsetAsync(ny + n, 0, sizeof(float) * (size_t)(n_pad - n), s));
     ::fhg::note_launch();
-    hd_mean_kernel<<<d, 256, 0, s>>>(X, n, d, mu);
+    hd_mean_part_kernel<<<kMeanBlocks, 256, 0, s>>>(X, n, d, part);
     ::fhg::note_launch();
-    hd_split_kernel<<<grid_for(n, 128), 128, 0, s>>>(X, n, d, dp, kw, mu, A, B, ny, cn, maxes);
+    hd_mean_kernel<<<1, kHighdMaxDim, 0, s>>>(part, kMeanBlocks, n, d, mu);
     FHG_CUDA(cudaGetLastError());
     if (ka) {
-        // the points (B rows, |y|^2) in increasing |y|^2, for the chunk
-        // bound of the epilogue; candidates map back through perm.  The
-        // queries (A rows) grouped by their nearest landmark, so that the
-        // rows of a CTA tend to need the same chunks; results go back to
-        // the query's own row through qperm.
-        uint32_t *nkey, *qkey;
-        int32_t *perm, *qperm;
-        float *nyp, *nyq;
-        __nv_bfloat16 *Ap, *Bp;
+        // the rows grouped by their nearest landmark, by |y|^2 inside a group;
+        // candidates and results go back through perm
+        uint32_t *key, *mark, *place;
+        int32_t* perm;
+        float* rec;
+        __nv_bfloat16* P;
         int* err;
-        FHG_TRY(ws.alloc(&nkey, (size_t)n));
-        FHG_TRY(ws.alloc(&qkey, (size_t)n));
+        const int64_t tiles = (n + kTcBN - 1) / kTcBN;
+        FHG_TRY(ws.alloc(&key, (size_t)n));
+        FHG_TRY(ws.alloc(&mark, (size_t)n));
+        FHG_TRY(ws.alloc(&place, (size_t)kLandmarks));
         FHG_TRY(ws.alloc(&perm, (size_t)n));
-        FHG_TRY(ws.alloc(&qperm, (size_t)n));
-        FHG_TRY(ws.alloc(&nyp, (size_t)n_pad));
-        FHG_TRY(ws.alloc(&nyq, (size_t)n));
-        FHG_TRY(ws.alloc(&Ap, (size_t)(n * kw)));
-        FHG_TRY(ws.alloc(&Bp, (size_t)(n * kw)));
+        FHG_TRY(ws.alloc(&rec, (size_t)(tiles * kTcRec)));
+        FHG_TRY(ws.alloc(&P, (size_t)(n * 2 * dp)));
         FHG_TRY(ws.alloc(&err, 1));
+        FHG_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
         ::fhg::note_launch();
-        hd_norm_keys_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, ny, nkey, perm);
+        hd_norms_kernel<<<(unsigned)std::min<int64_t>((n + 7) / 8, 152 * 8), 256, 0, s>>>(
+            X, n, d, mu, ny, cn, maxes);
+        ::fhg::note_launch();
+        hd_norm_keys_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, ny, key, perm);
         FHG_CUDA(cudaGetLastError());
-        FHG_TRY(radix_sort_u32(ws, nkey, perm, n, 0, 32));
+        FHG_TRY(radix_sort_u32(ws, key, perm, n, 0, 32));
         const int marks = (int)std::min<int64_t>(kLandmarks, n);
         ::fhg::note_launch();
-        hd_landmark_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, d, X, marks, n / marks, qkey,
-                                                             qperm);
-        FHG_CUDA(cudaGetLastError());
-        FHG_TRY(radix_sort_u32(ws, qkey, qperm, n, 0, 8));
-        const int64_t vecs = n * (kw / 8);
+        // landmarks: every (n / marks)-th point, then the means of their points
+        float* sums;
+        uint32_t* count;
+        FHG_TRY(ws.alloc(&sums, (size_t)(marks * (d + 1))));
+        count = reinterpret_cast<uint32_t*>(sums + (size_t)marks * d);
+        FHG_CUDA(cudaMemsetAsync(sums, 0, sizeof(float) * marks * (d + 1), s));
+        hd_landmark_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, d, X, marks, n / marks, nullptr,
+                                                             mark);
         ::fhg::note_launch();
-        hd_permute_kernel<<<grid_for(vecs, 256), 256, 0, s>>>(
-            n, kw / 8, perm, reinterpret_cast<const uint4*>(B), ny,
-            reinterpret_cast<uint4*>(Bp), nyp);
+        hd_mark_sums_kernel<<<grid_for(n, 8), 256, 0, s>>>(n, d, X, mark, sums, count);
         ::fhg::note_launch();
-        hd_permute_kernel<<<grid_for(vecs, 256), 256, 0, s>>>(
-            n, kw / 8, qperm, reinterpret_cast<const uint4*>(A), ny,
-            reinterpret_cast<uint4*>(Ap), nyq);
+        hd_mark_means_kernel<<<grid_for(marks * d, 256), 256, 0, s>>>(marks, d, n / marks, X,
+                                                                       count, sums);
+        ::fhg::note_launch();
+        hd_landmark_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, d, X, marks, n / marks, sums, mark);
+        ::fhg::note_launch();
+        hd_chain_kernel<<<1, kLandmarks, 0, s>>>(marks, d, sums, place);
+        ::fhg::note_launch();
+        hd_gather_key_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, mark, place, perm, key);
         FHG_CUDA(cudaGetLastError());
-        if (n_pad > n)
-            FHG_CUDA(cudaMemsetAsync(nyp + n, 0, sizeof(float) * (size_t)(n_pad - n), s));
-        FHG_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
-        FHG_TRY(launch_cand_tc_any(ka, n, L, Ap, Bp, nyp, nyq, perm, qperm, cand, T, err, s));
+        FHG_TRY(radix_sort_u32(ws, key, perm, n, 0, 8));
+        ::fhg::note_launch();
+        hd_rows_kernel<<<(unsigned)(tiles * (kTcBN / kTcChunk)), 256, 0, s>>>(X, n, d, dp, mu,
+                                                                              perm, ny, P, rec);
+        FHG_CUDA(cudaGetLastError());
+        FHG_TRY(launch_cand_tc_any(ka, n, L, P, rec, perm, cand, T, err, s));
         int h_err = 0;
         FHG_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, s));
         FHG_CUDA(cudaStreamSynchronize(s));
@@ -1061,6 +1363,13 @@ int highd_knn(const float* X, int64_t n, int d, int k, float* rd_o, int32_t* ix_
             return FHG_ERR_CUDA;
         }
     } else {
+        __nv_bfloat16 *A, *B;
+        const int kw = 3 * dp;
+        FHG_TRY(ws.alloc(&A, (size_t)(n * kw)));
+        FHG_TRY(ws.alloc(&B, (size_t)(n * kw)));
+        ::fhg::note_launch();
+        hd_split_kernel<<<grid_for(n, 128), 128, 0, s>>>(X, n, d, dp, mu, A, B, ny, cn, maxes);
+        FHG_CUDA(cudaGetLastError());
         switch (dp) {
             case 32: FHG_TRY(launch_cand<6>(n, L, A, B, ny, cand, T, s)); break;
             case 64: FHG_TRY(launch_cand<12>(n, L, A, B, ny, cand, T, s)); break;
@@ -1070,7 +1379,9 @@ int highd_knn(const float* X, int64_t n, int d, int k, float* rd_o, int32_t* ix_
     {
         Stage st(s, "hd_rerank_kernel");
         ::fhg::note_launch();
-        hd_rerank_kernel<<<(unsigned)((n + 3) / 4), 128, 0, s>>>(
+        const bool wide = d % 4 == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0;
+        (wide ? hd_rerank_kernel<true> : hd_rerank_kernel<false>)<<<(unsigned)((n + 3) / 4), 128, 0,
+                                                                    s>>>(
             n, d, dp, k, L, X, cand, T, ny, cn, maxes, rd_o, ix_o, flist, fcount);
         FHG_CUDA(cudaGetLastError());
     }

@@ -141,3 +141,23 @@ def test_tcgen05_pipeline_equals_mma_sync_kernel(engine, n, d, k):
     np.testing.assert_array_equal(ix_tc, ix_o)
     np.testing.assert_array_equal(rd_tc, rd_o)
     print("n=%d d=%d k=%d: fallbacks tcgen05 %d, mma.sync %d" % (n, d, k, fb_tc, fb_ms))
+
+
+@pytest.mark.parametrize("n,d,k", [(127, 33, 31), (128, 64, 31), (129, 32, 31), (3969, 31, 4),
+                                   (4096, 64, 1), (4097, 63, 31), (6000, 33, 31), (6001, 32, 56),
+                                   (6000, 32, 57), (4200, 30, 56)])
+def test_tcgen05_tiles_and_thresholds_equal_oracle(engine, n, d, k):
+    """Around a tile of 128, around the 32 tiles from which first thresholds
+    are taken, dimensions that fill their segment or leave one over (with and
+    without 16-byte rows), and the lists around the largest buffers: the
+    oracle's lists exactly.  A tight group far from the rest, and a row of
+    duplicates, want candidates that first thresholds must not cut off."""
+    from oracle import oracle as O
+
+    X = synthetic.aniso_highdim(n=n, seed=70 + d, dim=d, n_comp=5)
+    X[: n // 20] = X[0] * 3 + 0.01 * X[: n // 20]
+    X[n // 2: n // 2 + min(k, 40)] = X[n // 2]
+    rd, ix, _ = _highd(X, k)
+    rd_o, ix_o = O.tree_query(O.build_kdtree(X), k, mode=1, nthreads=NTH)
+    np.testing.assert_array_equal(ix, ix_o)
+    np.testing.assert_array_equal(rd, rd_o)
