@@ -868,7 +868,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) hd_cand_tc_kernel(
                 const int cc = __shfl_sync(0xffffffffu, cnt, rr);
                 float last = INFINITY;
                 const int kept =
-                    tc_cut<PER>(bufs + (size_t)(quarter * 32 + rr) * cap, cc, keep, slack, lane, &last);
+                    tc_cut<PER>(bufs + (size_t)(quarter * 32 + rr) * cap, cc, keep, slack, lane,
+                                &last);
                 if (lane == rr) {
                     cnt = kept;
                     tq = fminf(tq, last);  // (keys at the old one may be gone)
@@ -1230,7 +1231,7 @@ int launch_cand_tc(int64_t n, int L, const __nv_bfloat16* P, const float* rec,
 
 // The tensor-core pipeline's 64-element segments of a row [hi | lo] for (dp,
 // L), or 0 when the mma.sync kernel must run (rows of 96 dimensions, or
-// buffers too large for shared memory: k > 56 at 64 dimensions).
+// buffers too large for shared memory: k > 48 at 64 dimensions, 56 at 32).
 int tc_atoms(int dp, int L) {
     const int ka = dp == 32 ? 1 : (dp == 64 ? 2 : 0);
     if (ka == 0 || tc_cap(L) > 32 * 4 || tc_smem(ka, L) + kTcStatic > (size_t)kHdSmemMax)

@@ -408,7 +408,7 @@ int fhg_hdbscan_fit_precomputed(const int32_t* rows_dev, const int32_t* cols_dev
  *   FHG_HD_TCGEN05 (default): a Blackwell pipeline -- TMA loads of the
  *     operand tiles into shared memory, tcgen05.mma into tensor-memory
  *     accumulators, candidate selection in the epilogue warps -- for padded
- *     depths of 32 and 64 with k <= 32 (the others fall back);
+ *     depths of 32 (k <= 56) and 64 (k <= 48; the others fall back);
  *   FHG_HD_MMA_SYNC: the warp-level mma.sync kernel.
  * Both give the same certified kNN. */
 #define FHG_HD_TCGEN05 0

@@ -145,7 +145,8 @@ def test_tcgen05_pipeline_equals_mma_sync_kernel(engine, n, d, k):
 
 @pytest.mark.parametrize("n,d,k", [(127, 33, 31), (128, 64, 31), (129, 32, 31), (3969, 31, 4),
                                    (4096, 64, 1), (4097, 63, 31), (6000, 33, 31), (6001, 32, 56),
-                                   (6000, 32, 57), (4200, 30, 56)])
+                                   (6000, 32, 57), (4200, 30, 56), (4100, 64, 48),
+                                   (4100, 64, 49)])
 def test_tcgen05_tiles_and_thresholds_equal_oracle(engine, n, d, k):
     """Around a tile of 128, around the 32 tiles from which first thresholds
     are taken, dimensions that fill their segment or leave one over (with and

@@ -53,6 +53,31 @@ def test_knn_list_lengths_vs_oracle(engine, n, k, kind):
     np.testing.assert_array_equal(ix, oix)
 
 
+@pytest.mark.parametrize("n", [5, 600, 1025, 2600, 40_001])
+@pytest.mark.parametrize("k,d", [(65, 3), (112, 2), (128, 4), (129, 1), (700, 3), (1150, 2),
+                                 (2048, 3), (101, 11), (90, 20)])
+@pytest.mark.parametrize("kind", ["normal", "grid", "same"])
+def test_long_knn_lists_vs_oracle(engine, n, k, d, kind):
+    """Lists longer than 64, from fewer points than k to trees of several
+    levels of 32, with many points at the k-th distance (grid) and, in the
+    buffer's cuts, keys that differ in their index alone (same)."""
+    from fast_hdbscan_gb300.numba_kdtree import build_kdtree, parallel_tree_query
+    from oracle import oracle as O
+
+    if n > 3000 and (kind == "same" or d > 4 or k > 1200):
+        pytest.skip("covered by the smaller sizes")
+    rng = np.random.default_rng(n + 7 * k + d)
+    if kind == "normal":
+        X = (rng.normal(size=(n, d)) * np.exp(rng.normal(size=(n, 1)))).astype(np.float32)
+    else:
+        X = rng.integers(0, 9 if kind == "grid" else 2, size=(n, d)).astype(np.float32)
+    tree = build_kdtree(X)
+    rd, ix = parallel_tree_query(tree, tree.data, k=k, output_rdist=True)
+    ord_, oix = O.tree_query(O.build_kdtree(X), k, mode=1)
+    np.testing.assert_array_equal(rd, ord_)
+    np.testing.assert_array_equal(ix, oix)
+
+
 @pytest.mark.parametrize("m", [2, 2048, 2049, 2816, 2817, 4096, 4097, 8192, 8193, 100_001,
                                1_000_000])
 @pytest.mark.parametrize("weights", ["random", "few", "equal"])
