@@ -10,15 +10,19 @@
 // tile; in the second each block adds up the counts of the tiles before its
 // own (at most a few thousand words, from L2) and places its indices.  Against
 // flags, a three-launch scan of them and a gather this halves the launches and
-// leaves out two passes over n words.
+// leaves out two passes over n words.  Past kCompactScan tiles (8M indices) the
+// blocks' sums grow to a good part of what the indices themselves take (their
+// reads with the square of n), and a scan of the counts takes their place.
 #pragma once
 #include "fhg_common.cuh"
+#include "primitives.cuh"
 
 namespace fhg {
 
 constexpr int kCompactThreads = 256;
 constexpr int kCompactRows = 16;  // indices of a thread, kCompactThreads apart
 constexpr int kCompactTile = kCompactThreads * kCompactRows;
+constexpr int64_t kCompactScan = 2048;
 
 template <class F>
 __global__ void __launch_bounds__(kCompactThreads) compact_count_kernel(F f, int64_t n,
@@ -44,6 +48,7 @@ __global__ void __launch_bounds__(kCompactThreads) compact_count_kernel(F f, int
 template <class F>
 __global__ void __launch_bounds__(kCompactThreads) compact_emit_kernel(F f, int64_t n,
                                                                        const uint32_t* counts,
+                                                                       bool scanned,
                                                                        uint32_t* total) {
     constexpr int kWarps = kCompactThreads / 32;
     __shared__ uint32_t s_cell[kCompactRows][kWarps];  // marked indices per row and warp
@@ -52,8 +57,12 @@ __global__ void __launch_bounds__(kCompactThreads) compact_emit_kernel(F f, int6
     if (threadIdx.x == 0) s_before = 0;
     __syncthreads();
     uint32_t before = 0;
-    for (int64_t b = threadIdx.x; b < (int64_t)blockIdx.x; b += kCompactThreads)
-        before += counts[b];
+    if (scanned) {
+        before = threadIdx.x == 0 ? counts[blockIdx.x] : 0u;
+    } else {
+        for (int64_t b = threadIdx.x; b < (int64_t)blockIdx.x; b += kCompactThreads)
+            before += counts[b];
+    }
     before = __reduce_add_sync(kFull, before);
     if (lane == 0 && before) atomicAdd(&s_before, before);
     const int64_t base = (int64_t)blockIdx.x * kCompactTile + threadIdx.x;
@@ -109,15 +118,19 @@ int compact(Workspace& ws, const F& f, int64_t n, uint32_t* total) {
     }
     const int64_t tiles = (n + kCompactTile - 1) / kCompactTile;
     Workspace tmp(ws);
-    uint32_t* counts = nullptr;
+    uint32_t *counts = nullptr, *starts = nullptr;
+    const bool scanned = tiles > kCompactScan;
     if (tiles > 1) {
         FHG_TRY(tmp.alloc(&counts, (size_t)tiles));
+        if (scanned) FHG_TRY(tmp.alloc(&starts, (size_t)tiles));
         ::fhg::note_launch();
         compact_count_kernel<F><<<(unsigned)tiles, kCompactThreads, 0, s>>>(f, n, counts);
         FHG_CUDA(cudaGetLastError());
+        if (scanned) FHG_TRY(scan_exclusive_u32(tmp, counts, starts, tiles, nullptr));
     }
     ::fhg::note_launch();
-    compact_emit_kernel<F><<<(unsigned)tiles, kCompactThreads, 0, s>>>(f, n, counts, total);
+    compact_emit_kernel<F><<<(unsigned)tiles, kCompactThreads, 0, s>>>(f, n, scanned ? starts : counts,
+                                                                     scanned, total);
     FHG_CUDA(cudaGetLastError());
     return FHG_OK;
 }

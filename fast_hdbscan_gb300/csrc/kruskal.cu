@@ -28,6 +28,7 @@
 // that value (non-negative floats order like their bits).
 #include <memory>
 
+#include "compact.cuh"
 #include "highd.cuh"
 #include "index.cuh"
 #include "mst.cuh"
@@ -48,14 +49,20 @@ namespace {
 
 // kruskal.py:995-1015: float64 core distances from the kNN lists (rows of kq,
 // the point itself first; min_samples <= 1: zero) and the float32 value the
-// edge keys take the maximum of (the squared core distance).
+// edge keys take the maximum of (the squared core distance), beside the squared
+// distance of the point's last neighbour (+inf when the row is not full).
+__device__ __forceinline__ float kr_last(int64_t i, int kq, const float* __restrict__ rd,
+                                         const int32_t* __restrict__ ix) {
+    return ix[i * kq + kq - 1] >= 0 ? rd[i * kq + kq - 1] : INFINITY;
+}
 __global__ void kr_core_kernel(int64_t n, int kq, int ms, const float* __restrict__ rd,
-                               double* __restrict__ core, float* __restrict__ ck) {
+                               const int32_t* __restrict__ ix, double* __restrict__ core,
+                               float2* __restrict__ ck) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float c2 = ms > 1 ? rd[i * kq + ms] : 0.0f;
     core[i] = ms > 1 ? __dsqrt_rn((double)c2) : 0.0;
-    ck[i] = c2;
+    ck[i] = make_float2(c2, kr_last(i, kq, rd, ix));
 }
 // kruskal.py:981-990 with boruvka.py:528 sample_weight_core_distance: the
 // first list position at which the running float64 weight (the point's own
@@ -63,7 +70,7 @@ __global__ void kr_core_kernel(int64_t n, int kq, int ms, const float* __restric
 // distances are the float32 square roots the reference's tree query returns.
 __global__ void kr_core_w_kernel(int64_t n, int kq, int ms, const float* __restrict__ rd,
                                  const int32_t* __restrict__ ix, const float* __restrict__ w,
-                                 double* __restrict__ core, float* __restrict__ ck) {
+                                 double* __restrict__ core, float2* __restrict__ ck) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double total = 0.0;
@@ -75,131 +82,139 @@ __global__ void kr_core_w_kernel(int64_t n, int kq, int ms, const float* __restr
     }
     const float c = __fsqrt_rn(rd[i * kq + (j > 0 ? j - 1 : 0)]);
     core[i] = (double)c;
-    ck[i] = c;
+    ck[i] = make_float2(c, kr_last(i, kq, rd, ix));
 }
 // kruskal.py:456 _build_mrd_edges_knn and the filter of :1022, as each edge's
-// float32 key.  Edge e is the (e % kk)-th neighbour of point e / kk
-// (kk = kq - 1).
+// float32 key (kNoEdge: filtered out).  Edge e is the (e % kk)-th neighbour of
+// point e / kk (kk = kq - 1).  An edge from i to a smaller j that lies within
+// j's last distance stands in j's row too: with the same weight and, the rows
+// being in order, an earlier place, so the later one is never accepted and is
+// left out here (3-D, 16 neighbours: two thirds of the edges are left to sort).
+constexpr uint32_t kNoEdge = 0xffffffffu;  // (a NaN: no key of a finite weight)
 __global__ void kr_edges_kernel(int64_t n, int kq, int weighted, const float* __restrict__ rd,
-                                const int32_t* __restrict__ ix, const float* __restrict__ ck,
-                                uint32_t* __restrict__ key, uint32_t* __restrict__ flag) {
-    const int64_t kk = kq - 1;
+                                const int32_t* __restrict__ ix, const float2* __restrict__ ck,
+                                uint32_t* __restrict__ key) {
+    const uint32_t kk = (uint32_t)(kq - 1);
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n * kk) return;
-    const int64_t i = e / kk, jp = e - i * kk;
-    const int32_t j = ix[i * kq + jp + 1];
-    float v = INFINITY;
-    if (j >= 0) {
-        const float r = rd[i * kq + jp + 1];
-        v = fmaxf(fmaxf(ck[i], ck[j]), weighted ? __fsqrt_rn(r) : r);
+    if (e >= n * kk) return;  // (at most 2^31 - 1 edges)
+    const int64_t i = (uint32_t)e / kk, at = i * kq + (e - i * kk) + 1;
+    const int32_t j = ix[at];
+    uint32_t out = kNoEdge;
+    if (j >= 0 && j != (int32_t)i) {
+        const float r = rd[at];
+        const float2 cj = ck[j];
+        const float v = fmaxf(fmaxf(ck[i].x, cj.x), weighted ? __fsqrt_rn(r) : r);
+        if (isfinite(v) && !(j < (int32_t)i && r < cj.y)) out = __float_as_uint(v);
     }
-    key[e] = __float_as_uint(v);
-    flag[e] = (j >= 0 && j != (int32_t)i && isfinite(v)) ? 1u : 0u;
+    key[e] = out;
 }
-__global__ void kr_compact_kernel(int64_t E, const uint32_t* __restrict__ flag,
-                                  const uint32_t* __restrict__ pos, const uint32_t* __restrict__ k0,
-                                  uint32_t* __restrict__ key, int32_t* __restrict__ eid) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E || !flag[e]) return;
-    key[pos[e]] = k0[e];
-    eid[pos[e]] = (int32_t)e;
-}
-// Endpoints of every sorted edge, and the initial active list (all ranks).
+// The edges that are left, in order.
+struct KeptEdges {
+    const uint32_t* k0;
+    uint32_t* key;
+    int32_t* eid;
+    __device__ bool test(int64_t e) const { return k0[e] != kNoEdge; }
+    __device__ void emit(int64_t e, uint32_t at) const {
+        key[at] = k0[e];
+        eid[at] = (int32_t)e;
+    }
+    __device__ void each(int64_t) const {}
+};
+// Endpoints of every sorted edge.
 __global__ void kr_ends_kernel(int64_t m, int kq, const int32_t* __restrict__ eid,
-                               const int32_t* __restrict__ ix, int2* __restrict__ uv,
-                               int32_t* __restrict__ act, int2* __restrict__ act_uv) {
+                               const int32_t* __restrict__ ix, int2* __restrict__ uv) {
     const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= m) return;
-    const int64_t kk = kq - 1, e = eid[r], i = e / kk;
-    const int2 p = make_int2((int32_t)i, ix[i * kq + (e - i * kk) + 1]);
-    uv[r] = p;
-    act[r] = (int32_t)r;
-    act_uv[r] = p;
+    const uint32_t kk = (uint32_t)(kq - 1), e = (uint32_t)eid[r], i = e / kk;
+    uv[r] = make_int2((int32_t)i, ix[(int64_t)i * kq + (e - i * kk) + 1]);
 }
-__global__ void kr_iota_kernel(int32_t* a, int64_t n) {
+__global__ void kr_init_kernel(int64_t n, int32_t* __restrict__ par, uint32_t* __restrict__ best) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = (int32_t)i;
+    if (i >= n) return;
+    par[i] = (int32_t)i;
+    best[i] = 0xffffffffu;
 }
-__global__ void kr_fill_u32_kernel(uint32_t* a, int64_t n, uint32_t v) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = v;
-}
-// One Boruvka round, step 1: every component's lowest outgoing rank.  Active
-// ranks come in increasing order, so a component's best is mostly set by its
-// first edge and later ones only read it.
+// One Boruvka round over the active edges (rank act[t], or t in the first
+// round; act_uv their components).  What bounds it is the gathers by component:
+// endpoints are looked up once a round, by the compaction that ends it, the
+// picked edges are joined by a pass over the points, and a round takes five
+// launches (16M edges of 1M points: 2.2 -> 0.8 ms; 4.5M pairs of 300k points,
+// twice as many entries before: 1.5 -> 0.5).
+// Step 1: every component's lowest outgoing rank.  Active ranks come in
+// increasing order, so a component's best is mostly set by its first edge and
+// later ones only read it.
 __global__ void kr_best_kernel(int64_t na, const int32_t* __restrict__ act,
-                               const int2* __restrict__ act_uv, int32_t* par,
-                               uint32_t* __restrict__ best) {
+                               const int2* __restrict__ act_uv, uint32_t* __restrict__ best) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= na) return;
-    const uint32_t r = (uint32_t)act[t];
+    const uint32_t r = act ? (uint32_t)act[t] : (uint32_t)t;
     const int2 p = act_uv[t];
-    const int32_t cu = uf_find(par, p.x), cv = uf_find(par, p.y);
-    if (cu == cv) return;
-    if (r < *(volatile uint32_t*)&best[cu]) atomicMin(&best[cu], r);
-    if (r < *(volatile uint32_t*)&best[cv]) atomicMin(&best[cv], r);
+    if (p.x == p.y) return;
+    if (r < *(volatile uint32_t*)&best[p.x]) atomicMin(&best[p.x], r);
+    if (r < *(volatile uint32_t*)&best[p.y]) atomicMin(&best[p.y], r);
 }
-// Step 2 (no union yet, so the roots are those of step 1): an edge picked by
-// either of its components is marked with the round.
-__global__ void kr_pick_kernel(int64_t na, const int32_t* __restrict__ act,
-                               const int2* __restrict__ act_uv, int32_t* par,
-                               const uint32_t* __restrict__ best, int32_t* __restrict__ mark,
-                               int round, uint32_t* __restrict__ picked) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= na) return;
-    const uint32_t r = (uint32_t)act[t];
-    const int2 p = act_uv[t];
-    const int32_t cu = uf_find(par, p.x), cv = uf_find(par, p.y);
-    if (cu != cv && (best[cu] == r || best[cv] == r)) {
-        mark[r] = round;
-        atomicAdd(picked, 1u);
-    }
-}
-// Step 3: hook the picked edges.
-__global__ void kr_hook_kernel(int64_t na, const int32_t* __restrict__ act,
-                               const int2* __restrict__ act_uv, int32_t* par,
-                               const int32_t* __restrict__ mark, int round) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= na) return;
-    if (mark[act[t]] != round) return;
-    const int2 p = act_uv[t];
+// Step 2: the picked edges are marked and hooked (an edge that both of its
+// components pick, twice: the second union finds nothing to do).
+__global__ void kr_join_kernel(int64_t n, uint32_t* __restrict__ best,
+                               const int2* __restrict__ uv, uint8_t* __restrict__ mark,
+                               int32_t* par) {
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n) return;
+    const uint32_t r = best[c];
+    if (r == 0xffffffffu) return;
+    best[c] = 0xffffffffu;
+    mark[r] = 1;
+    const int2 p = uv[r];
     uf_union(par, p.x, p.y);
 }
-// Step 4: edges now inside one component leave the list.
-__global__ void kr_keep_kernel(int64_t na, const int2* __restrict__ act_uv, int32_t* par,
-                               uint32_t* __restrict__ keep) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= na) return;
-    const int2 p = act_uv[t];
-    keep[t] = uf_find(par, p.x) != uf_find(par, p.y) ? 1u : 0u;
+// Step 3: every point's parent is its root.  (Reads the chains only: a find that
+// halves paths could put an inner point back behind another thread's root.)
+__global__ void kr_flatten_kernel(int64_t n, int32_t* par) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int32_t first = par[i];
+    int32_t root = first, up;
+    while ((up = par[root]) != root) root = up;
+    if (root != first) par[i] = root;
 }
-__global__ void kr_scatter_active_kernel(int64_t na, const int32_t* __restrict__ act,
-                                         const int2* __restrict__ act_uv,
-                                         const uint32_t* __restrict__ keep,
-                                         const uint32_t* __restrict__ pos,
-                                         int32_t* __restrict__ act2, int2* __restrict__ act_uv2) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= na || !keep[t]) return;
-    act2[pos[t]] = act[t];
-    act_uv2[pos[t]] = act_uv[t];
-}
-__global__ void kr_mark_flags_kernel(int64_t m, const int32_t* __restrict__ mark,
-                                     uint32_t* __restrict__ flag) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < m) flag[r] = mark[r] > 0 ? 1u : 0u;
-}
-// kruskal.py:104-107: picked edges in rank order as (row point, neighbour,
-// float64 weight); the weight is the rank's float32 key (kNN graph) or its
-// float64 weight.
-__global__ void kr_emit_kernel(int64_t m, int weighted, const uint32_t* __restrict__ flag,
-                               const uint32_t* __restrict__ pos, const int2* __restrict__ uv,
-                               const uint32_t* __restrict__ key, const double* __restrict__ w64,
-                               double* __restrict__ edges) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= m || !flag[r]) return;
-    const int64_t o = pos[r];
-    edges[3 * o + 0] = (double)uv[r].x;
-    edges[3 * o + 1] = (double)uv[r].y;
+// Step 4: edges between two components stay.
+struct EdgesApart {
+    const int32_t* act;
+    const int2* act_uv;
+    const int32_t* par;
+    int32_t* act2;
+    int2* act_uv2;
+    __device__ bool test(int64_t t) const {
+        const int2 p = act_uv[t];
+        return par[p.x] != par[p.y];
+    }
+    __device__ void emit(int64_t t, uint32_t at) const {
+        const int2 p = act_uv[t];
+        act2[at] = act ? act[t] : (int32_t)t;
+        act_uv2[at] = make_int2(par[p.x], par[p.y]);
+    }
+    __device__ void each(int64_t) const {}
+};
+// The picked ranks in order, and kruskal.py:104-107: their edges as (row point,
+// neighbour, float64 weight); the weight is the rank's float32 key (kNN graph)
+// or its float64 weight.  (The float64 square roots want full warps: taken in
+// the compaction, a few lanes at a time, they made it 250 us at 1M points.)
+struct PickedRanks {
+    const uint8_t* mark;
+    int32_t* ranks;
+    __device__ bool test(int64_t r) const { return mark[r] != 0; }
+    __device__ void emit(int64_t r, uint32_t at) const { ranks[at] = (int32_t)r; }
+    __device__ void each(int64_t) const {}
+};
+__global__ void kr_emit_kernel(int64_t nf, int weighted, const int32_t* __restrict__ ranks,
+                               const int2* __restrict__ uv, const uint32_t* __restrict__ key,
+                               const double* __restrict__ w64, double* __restrict__ edges) {
+    const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= nf) return;
+    const int32_t r = ranks[o];
+    const int2 p = uv[r];
+    edges[3 * o + 0] = (double)p.x;
+    edges[3 * o + 1] = (double)p.y;
     if (w64) {
         edges[3 * o + 2] = w64[r];
     } else {
@@ -207,23 +222,22 @@ __global__ void kr_emit_kernel(int64_t m, int weighted, const uint32_t* __restri
         edges[3 * o + 2] = weighted ? (double)v : __dsqrt_rn((double)v);
     }
 }
-__global__ void kr_root_flags_kernel(int64_t n, int32_t* par, uint32_t* __restrict__ flag) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) flag[i] = uf_find(par, (int32_t)i) == (int32_t)i ? 1u : 0u;
-}
+struct ForestRoots {
+    const int32_t* par;
+    int32_t* roots;
+    __device__ bool test(int64_t i) const { return par[i] == (int32_t)i; }
+    __device__ void emit(int64_t i, uint32_t at) const { roots[at] = (int32_t)i; }
+    __device__ void each(int64_t) const {}
+};
 // kruskal.py:723 / precomputed.py:308: +inf bridges between consecutive
 // component representatives (the roots, each its component's smallest point).
-__global__ void kr_bridge_kernel(int64_t n, int64_t nc, const uint32_t* __restrict__ flag,
-                                 const uint32_t* __restrict__ pos, int64_t base,
+__global__ void kr_bridge_kernel(int64_t nb, const int32_t* __restrict__ roots,
                                  double* __restrict__ edges) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !flag[i]) return;
-    const int64_t c = pos[i];  // this root's place among the roots
-    if (c > 0) {               // bridge c - 1 ends here
-        edges[3 * (base + c - 1) + 1] = (double)i;
-        edges[3 * (base + c - 1) + 2] = INFINITY;
-    }
-    if (c + 1 < nc) edges[3 * (base + c) + 0] = (double)i;  // bridge c starts here
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= nb) return;
+    edges[3 * c + 0] = (double)roots[c];
+    edges[3 * c + 1] = (double)roots[c + 1];
+    edges[3 * c + 2] = INFINITY;
 }
 __global__ void kr_neighbors_kernel(int64_t n, int kq, int cols, const int32_t* __restrict__ ix,
                                     int32_t* __restrict__ out) {
@@ -270,7 +284,8 @@ int kruskal_mst_of_lists(int64_t n, int min_samples, int query_k, const float* w
     }
     Stage stage(s, "kruskal_knn");
     Workspace ws(s);
-    float *rd, *ck;
+    float* rd;
+    float2* ck;
     int32_t* ix;
     FHG_TRY(ws.alloc(&rd, (size_t)(n * kq)));
     FHG_TRY(ws.alloc(&ix, (size_t)(n * kq)));
@@ -278,7 +293,7 @@ int kruskal_mst_of_lists(int64_t n, int min_samples, int query_k, const float* w
     if (index) FHG_TRY(index_knn(*index, kq, nullptr, nullptr, rd, ix, s));
     else FHG_TRY(highd_knn(X, n, d, kq, rd, ix, nullptr, s));
     if (weights) LAUNCH(kr_core_w_kernel, n, n, kq, min_samples, rd, ix, weights, core, ck);
-    else LAUNCH(kr_core_kernel, n, n, kq, min_samples, rd, core, ck);
+    else LAUNCH(kr_core_kernel, n, n, kq, min_samples, rd, ix, core, ck);
     if (neighbors) {
         const int cols = weights ? kq - 1 : (min_samples > 1 ? min_samples : 1);
         LAUNCH(kr_neighbors_kernel, n * cols, n, kq, cols, ix, neighbors);
@@ -287,23 +302,18 @@ int kruskal_mst_of_lists(int64_t n, int min_samples, int query_k, const float* w
     // ---- valid edges, stably sorted by weight
     std::unique_ptr<Stage> sub(new Stage(s, "kruskal_edges"));
     const int64_t E = n * kk;
-    uint32_t *k0, *flag, *pos, *cnt;
+    uint32_t *k0, *key, *cnt;
+    int32_t* eid;
     FHG_TRY(ws.alloc(&k0, (size_t)E));
-    FHG_TRY(ws.alloc(&flag, (size_t)E));
-    FHG_TRY(ws.alloc(&pos, (size_t)E));
-    FHG_TRY(ws.alloc(&cnt, 2));
-    LAUNCH(kr_edges_kernel, E, n, kq, weights ? 1 : 0, rd, ix, ck, k0, flag);
-    FHG_TRY(scan_exclusive_u32(ws, flag, pos, E, cnt));
+    FHG_TRY(ws.alloc(&key, (size_t)E));
+    FHG_TRY(ws.alloc(&eid, (size_t)E));
+    FHG_TRY(ws.alloc(&cnt, 1));
+    LAUNCH(kr_edges_kernel, E, n, kq, weights ? 1 : 0, rd, ix, ck, k0);
+    FHG_TRY(compact(ws, KeptEdges{k0, key, eid}, E, cnt));
     uint32_t h_m = 0;
     FHG_CUDA(cudaMemcpyAsync(&h_m, cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     FHG_CUDA(cudaStreamSynchronize(s));
     const int64_t m = h_m;
-    const size_t mm = (size_t)(m > 0 ? m : 1);
-    uint32_t* key;
-    int32_t* eid;
-    FHG_TRY(ws.alloc(&key, mm));
-    FHG_TRY(ws.alloc(&eid, mm));
-    LAUNCH(kr_compact_kernel, E, E, flag, pos, k0, key, eid);
     sub.reset(new Stage(s, "kruskal_sort"));
     if (m > 1) {
         Workspace tmp(ws);
@@ -324,77 +334,69 @@ int sorted_forest_edges(Workspace& ws, int64_t n, int64_t m, int kq, const int32
     const size_t mm = (size_t)(m > 0 ? m : 1);
     // ---- minimum spanning forest: Boruvka rounds over the ranks
     std::unique_ptr<Stage> sub(new Stage(s, "kruskal_forest"));
-    int32_t *par, *act, *act2, *mark;
-    int2 *uv, *act_uv, *act_uv2;
-    uint32_t *best, *keep, *picked, *pos, *cnt;
+    int32_t *par, *act = nullptr, *act_a, *act_b;
+    int2 *uv_a, *uv_b;
+    const int2 *uv = uv_in, *act_uv;
+    uint32_t *best, *cnt;
+    uint8_t* mark;
     FHG_TRY(ws.alloc(&par, (size_t)n));
     FHG_TRY(ws.alloc(&best, (size_t)n));
-    FHG_TRY(ws.alloc(&uv, mm));
-    FHG_TRY(ws.alloc(&act, mm));
-    FHG_TRY(ws.alloc(&act2, mm));
-    FHG_TRY(ws.alloc(&act_uv, mm));
-    FHG_TRY(ws.alloc(&act_uv2, mm));
-    FHG_TRY(ws.alloc(&keep, mm));
-    FHG_TRY(ws.alloc(&pos, mm));
+    FHG_TRY(ws.alloc(&act_a, mm));
+    FHG_TRY(ws.alloc(&act_b, mm));
+    FHG_TRY(ws.alloc(&uv_a, mm));
+    FHG_TRY(ws.alloc(&uv_b, mm));
     FHG_TRY(ws.alloc(&mark, mm));
-    FHG_TRY(ws.alloc(&picked, 1));
-    FHG_TRY(ws.alloc(&cnt, 2));
-    LAUNCH(kr_iota_kernel, n, par, n);
-    if (uv_in) {
-        FHG_CUDA(cudaMemcpyAsync(uv, uv_in, sizeof(int2) * m, cudaMemcpyDeviceToDevice, s));
-        FHG_CUDA(cudaMemcpyAsync(act_uv, uv_in, sizeof(int2) * m, cudaMemcpyDeviceToDevice, s));
-        LAUNCH(kr_iota_kernel, m, act, m);
-    } else {
-        LAUNCH(kr_ends_kernel, m, m, kq, eid, ix, uv, act, act_uv);
+    FHG_TRY(ws.alloc(&cnt, 1));
+    LAUNCH(kr_init_kernel, n, n, par, best);
+    if (!uv_in) {
+        int2* ends;
+        FHG_TRY(ws.alloc(&ends, mm));
+        LAUNCH(kr_ends_kernel, m, m, kq, eid, ix, ends);
+        uv = ends;
     }
-    if (m > 0) FHG_CUDA(cudaMemsetAsync(mark, 0, sizeof(int32_t) * m, s));
+    act_uv = uv;
+    if (m > 0) FHG_CUDA(cudaMemsetAsync(mark, 0, (size_t)m, s));
+    uint32_t h = 0;
     int64_t na = m;
     for (int round = 1; na > 0; ++round) {
         if (round > 64) {  // each round at least halves the components
             set_error("kruskal: the spanning forest did not converge");
             return FHG_ERR_NO_CONVERGENCE;
         }
-        LAUNCH(kr_fill_u32_kernel, n, best, n, 0xffffffffu);
-        FHG_CUDA(cudaMemsetAsync(picked, 0, sizeof(uint32_t), s));
-        LAUNCH(kr_best_kernel, na, na, act, act_uv, par, best);
-        LAUNCH(kr_pick_kernel, na, na, act, act_uv, par, best, mark, round, picked);
-        LAUNCH(kr_hook_kernel, na, na, act, act_uv, par, mark, round);
-        LAUNCH(kr_keep_kernel, na, na, act_uv, par, keep);
-        FHG_TRY(scan_exclusive_u32(ws, keep, pos, na, cnt));
-        LAUNCH(kr_scatter_active_kernel, na, na, act, act_uv, keep, pos, act2, act_uv2);
-        uint32_t h[2] = {0, 0};
-        FHG_CUDA(cudaMemcpyAsync(&h[0], picked, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        FHG_CUDA(cudaMemcpyAsync(&h[1], cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        LAUNCH(kr_best_kernel, na, na, act, act_uv, best);
+        LAUNCH(kr_join_kernel, n, n, best, uv, mark, par);
+        LAUNCH(kr_flatten_kernel, n, n, par);
+        FHG_TRY(compact(ws, EdgesApart{act, act_uv, par, act_a, uv_a}, na, cnt));
+        FHG_CUDA(cudaMemcpyAsync(&h, cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         FHG_CUDA(cudaStreamSynchronize(s));
-        std::swap(act, act2);
-        std::swap(act_uv, act_uv2);
-        na = h[0] == 0 ? 0 : (int64_t)h[1];
+        act = act_a;
+        act_uv = uv_a;
+        std::swap(act_a, act_b);
+        std::swap(uv_a, uv_b);
+        na = (int64_t)h;
     }
 
     // ---- the forest in Kruskal's acceptance order, then the bridges
     sub.reset(new Stage(s, "kruskal_emit"));
-    uint32_t *flag, *rflag, *rpos;
-    FHG_TRY(ws.alloc(&flag, mm));
-    FHG_TRY(ws.alloc(&rflag, (size_t)n));
-    FHG_TRY(ws.alloc(&rpos, (size_t)n));
-    uint32_t h_f = 0, h_c = 0;
-    if (m > 0) {
-        LAUNCH(kr_mark_flags_kernel, m, m, mark, flag);
-        FHG_TRY(scan_exclusive_u32(ws, flag, pos, m, cnt));
-        FHG_CUDA(cudaMemcpyAsync(&h_f, cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    }
-    LAUNCH(kr_root_flags_kernel, n, n, par, rflag);
-    FHG_TRY(scan_exclusive_u32(ws, rflag, rpos, n, cnt + 1));
-    FHG_CUDA(cudaMemcpyAsync(&h_c, cnt + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    int32_t* ranks = act_a;  // (room for all m)
+    FHG_TRY(compact(ws, PickedRanks{mark, ranks}, m, cnt));
+    FHG_CUDA(cudaMemcpyAsync(&h, cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     FHG_CUDA(cudaStreamSynchronize(s));
-    const int64_t nf = h_f, nc = h_c;
-    if (nc < 1 || nf + nc != n) {  // a forest over n points in nc components
+    const int64_t nf = h, nc = n - nf;
+    if (nc >= 1) LAUNCH(kr_emit_kernel, nf, nf, key_weighted, ranks, uv, key32, w64, edges);
+    if (nc > 1) {
+        int32_t* roots;
+        FHG_TRY(ws.alloc(&roots, (size_t)n));
+        FHG_TRY(compact(ws, ForestRoots{par, roots}, n, cnt));
+        FHG_CUDA(cudaMemcpyAsync(&h, cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        FHG_CUDA(cudaStreamSynchronize(s));
+        if ((int64_t)h == nc) LAUNCH(kr_bridge_kernel, nc - 1, nc - 1, roots, edges + 3 * nf);
+    }
+    if (nc < 1 || (nc > 1 && (int64_t)h != nc)) {  // a forest over n points in nc components
         set_error("kruskal: %lld forest edges for %lld points in %lld components", (long long)nf,
-                  (long long)n, (long long)nc);
+                  (long long)n, (long long)(nc < 1 ? nc : (int64_t)h));
         return FHG_ERR_NO_CONVERGENCE;
     }
-    if (m > 0) LAUNCH(kr_emit_kernel, m, m, key_weighted, flag, pos, uv, key32, w64, edges);
-    if (nc > 1) LAUNCH(kr_bridge_kernel, n, n, nc, rflag, rpos, nf, edges);
     *n_components = nc;
     return FHG_OK;
 }

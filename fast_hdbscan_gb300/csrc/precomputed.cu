@@ -10,15 +10,21 @@
 // spanning forest -- Kruskal over a stable argsort of the entries, or its
 // float32 Boruvka -- then joins the components with +inf bridges.
 //
-// Here every step is a sort or a pass over the entries: the symmetrised
-// graph by a stable radix sort of the (min, max) pair keys with a segmented
-// minimum, its CSR order (pairs (i, j) with i < j first, then the mirrored
-// ones, each stably by row, as the reference's two concatenated halves) by a
-// stable radix sort of the row; row order by weight by a two-key LSD sort;
-// the forest by the Boruvka rounds over sorted ranks of kruskal.cu.  The
-// forest is Kruskal's (float64 weight, then entry position) for both
-// algorithms: the reference's Boruvka returns a forest of the same weights,
-// whose equal-weight choices and edge order are its own.
+// Here: the least weight of every pair by a stable radix sort of the (min, max)
+// pair keys with a segmented minimum.  A row of the symmetric matrix is then its
+// pairs (i, j) with i < j, which stand together in pair order, and the mirrored
+// ones, stably by row, as the reference's two concatenated halves: only these
+// are sorted.  A warp per row ranks its entries by (weight, position) for the
+// core distance and the neighbours.  A pair's two entries have one weight and
+// the one with i < j comes first, so the other is never accepted: the pairs
+// alone are sorted by weight, and the forest comes from the Boruvka rounds over
+// sorted ranks of kruskal.cu.  The forest is Kruskal's (float64 weight, then
+// entry position) for both algorithms: the reference's Boruvka returns a forest
+// of the same weights, whose equal-weight choices and edge order are its own.
+//
+// What bounds it is the sorts' digit passes: 5 over the entries and 3 + 8 over
+// the pairs (before: 5, and 3 + 8 + 3 + 8 over both entries of every pair).
+// 300k rows, 15 neighbours each: 4.5 -> 1.9 ms with the forest.
 #include "mst.cuh"
 #include "primitives.cuh"
 
@@ -84,7 +90,80 @@ __global__ void pc_group_min_kernel(int64_t m0, int64_t n, const uint64_t* __res
         gv[g] = (int32_t)(key[j] % (uint64_t)n);
     }
 }
-// The symmetric entries: pairs (u, v) in pair order, then (v, u) likewise.
+// The mirrored entries (v, u), in pair order.
+__global__ void pc_mirror_kernel(int64_t mu, const int32_t* __restrict__ gv,
+                                 uint32_t* __restrict__ rowkey, int32_t* __restrict__ perm) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= mu) return;
+    rowkey[t] = (uint32_t)gv[t];
+    perm[t] = (int32_t)t;
+}
+template <class T>
+__device__ __forceinline__ int64_t pc_lower_bound(const T* __restrict__ a, int64_t n, T v) {
+    int64_t lo = 0, hi = n;
+    while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (a[mid] < v) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+// Where row r's pairs (among gu) and mirrored entries (among the sorted vrow)
+// start, r in [0, n]; longest = the longest row.
+__global__ void pc_rows_kernel(int64_t n, int64_t mu, const int32_t* __restrict__ gu,
+                               const uint32_t* __restrict__ vrow, uint32_t* __restrict__ ubeg,
+                               uint32_t* __restrict__ lbeg, uint32_t* __restrict__ longest) {
+    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t len = 0;
+    if (r <= n) {
+        const int64_t u = pc_lower_bound(gu, mu, (int32_t)r);
+        const int64_t l = pc_lower_bound(vrow, mu, (uint32_t)r);
+        ubeg[r] = (uint32_t)u;
+        lbeg[r] = (uint32_t)l;
+        if (r < n)
+            len = (uint32_t)(pc_lower_bound(gu, mu, (int32_t)r + 1) - u +
+                             pc_lower_bound(vrow, mu, (uint32_t)r + 1) - l);
+    }
+    len = __reduce_max_sync(kFull, len);
+    if ((threadIdx.x & 31) == 0 && len > *(volatile uint32_t*)longest) atomicMax(longest, len);
+}
+// :148 _core_distances_csr, a warp per row of up to kPcRow entries: an entry's
+// place is the number of entries of the row before it in (weight, position).
+// Longer rows are ordered by sorting all entries by weight and by row, eleven
+// digit passes however long the rows; ranking takes len^2 / 32 steps a row (4M
+// entries, rows of 16 / 64 / 256: 1.40 / 1.29 / 1.54 ms for the whole tree, by
+// sorting 2.26 / 2.07 / 2.24).
+constexpr int kPcRow = 256, kPcWarps = 4;
+__global__ void __launch_bounds__(kPcWarps * 32) pc_rank_rows_kernel(
+    int64_t n, int k, int ms, const int32_t* __restrict__ gu, const int32_t* __restrict__ gv,
+    const unsigned long long* __restrict__ gmin, const int32_t* __restrict__ lperm,
+    const uint32_t* __restrict__ ubeg, const uint32_t* __restrict__ lbeg,
+    int32_t* __restrict__ nbrs, double* __restrict__ core) {
+    __shared__ unsigned long long s_w[kPcWarps][kPcRow];
+    __shared__ int32_t s_col[kPcWarps][kPcRow];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t r = (int64_t)blockIdx.x * kPcWarps + warp;
+    if (r >= n) return;
+    const uint32_t u0 = ubeg[r], l0 = lbeg[r];
+    const int nu = (int)(ubeg[r + 1] - u0), len = nu + (int)(lbeg[r + 1] - l0);
+    for (int e = lane; e < len; e += 32) {
+        const int64_t g = e < nu ? u0 + e : lperm[l0 + (e - nu)];
+        s_w[warp][e] = gmin[g];
+        s_col[warp][e] = e < nu ? gv[g] : gu[g];
+    }
+    __syncwarp();
+    for (int e = lane; e < len; e += 32) {
+        const unsigned long long w = s_w[warp][e];
+        int at = 0;
+        for (int o = 0; o < len; ++o) {
+            const unsigned long long x = s_w[warp][o];
+            at += x < w || (x == w && o < e) ? 1 : 0;
+        }
+        if (at < k) nbrs[r * k + at] = s_col[warp][e];
+        if (ms > 1 && at == ms - 1) core[r] = __longlong_as_double((long long)w);
+    }
+}
+// Both halves one behind the other, for rows too long to rank.
 __global__ void pc_sym_kernel(int64_t mu, const int32_t* __restrict__ gu,
                               const int32_t* __restrict__ gv, uint32_t* __restrict__ rowkey,
                               int32_t* __restrict__ perm) {
@@ -139,29 +218,70 @@ __global__ void pc_core_kernel(int64_t M, int k, int ms, const int32_t* __restri
     if (j < k) nbrs[(int64_t)r * k + j] = scol[p];
     if (ms > 1 && j == ms - 1) core[r] = sd[p];
 }
-// kruskal.py:421 _compute_mrd_csr_flat.
-__global__ void pc_mrd_kernel(int64_t M, const int32_t* __restrict__ srow,
-                              const int32_t* __restrict__ scol, const double* __restrict__ sd,
+// kruskal.py:421 _compute_mrd_csr_flat, of every pair's first entry.
+__global__ void pc_mrd_kernel(int64_t mu, const int32_t* __restrict__ gu,
+                              const int32_t* __restrict__ gv,
+                              const unsigned long long* __restrict__ gmin,
                               const double* __restrict__ core, uint64_t* __restrict__ key,
                               int32_t* __restrict__ perm) {
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= M) return;
-    double mrd = core[srow[p]];
-    const double cj = core[scol[p]];
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= mu) return;
+    double mrd = core[gu[g]];
+    const double cj = core[gv[g]], d = __longlong_as_double((long long)gmin[g]);
     if (cj > mrd) mrd = cj;
-    if (sd[p] > mrd) mrd = sd[p];
-    key[p] = f64_bits(mrd);
-    perm[p] = (int32_t)p;
+    if (d > mrd) mrd = d;
+    key[g] = f64_bits(mrd);
+    perm[g] = (int32_t)g;
 }
-__global__ void pc_ranks_kernel(int64_t M, const int32_t* __restrict__ perm,
-                                const int32_t* __restrict__ srow, const int32_t* __restrict__ scol,
-                                const uint64_t* __restrict__ key, int2* __restrict__ uv,
-                                double* __restrict__ w) {
+__global__ void pc_ranks_kernel(int64_t mu, const int32_t* __restrict__ perm,
+                                const int32_t* __restrict__ gu, const int32_t* __restrict__ gv,
+                                int2* __restrict__ uv) {
     const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= M) return;
-    const int32_t p = perm[r];
-    uv[r] = make_int2(srow[p], scol[p]);
-    w[r] = __longlong_as_double((long long)key[r]);
+    if (r >= mu) return;
+    const int32_t g = perm[r];
+    uv[r] = make_int2(gu[g], gv[g]);
+}
+
+// _core_distances_csr by sorting: the symmetric CSR, every row by weight, ties
+// by position.
+int core_by_sorting(Workspace& outer, int64_t n, int64_t mu, int k, int ms, const int32_t* gu,
+                    const int32_t* gv, const unsigned long long* gmin, int32_t* neighbors,
+                    double* core) {
+    cudaStream_t s = outer.stream();
+    Workspace ws(outer);
+    const int64_t M = 2 * mu;
+    uint32_t *rowkey, *count, *indptr;
+    int32_t *perm, *srow, *scol;
+    double* sd;
+    uint64_t* wkey;
+    FHG_TRY(ws.alloc(&rowkey, (size_t)M));
+    FHG_TRY(ws.alloc(&perm, (size_t)M));
+    FHG_TRY(ws.alloc(&srow, (size_t)M));
+    FHG_TRY(ws.alloc(&scol, (size_t)M));
+    FHG_TRY(ws.alloc(&sd, (size_t)M));
+    FHG_TRY(ws.alloc(&count, (size_t)n));
+    FHG_TRY(ws.alloc(&indptr, (size_t)n));
+    FHG_TRY(ws.alloc(&wkey, (size_t)M));
+    FHG_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t) * n, s));
+    LAUNCH(pc_sym_kernel, M, mu, gu, gv, rowkey, perm);
+    {
+        Workspace tmp(ws);
+        FHG_TRY(radix_sort_u32(tmp, rowkey, perm, M, 0, bits_for(n)));
+    }
+    LAUNCH(pc_csr_kernel, M, M, mu, perm, gu, gv, gmin, srow, scol, sd, count);
+    FHG_TRY(scan_exclusive_u32(ws, count, indptr, n, nullptr));
+    LAUNCH(pc_weight_keys_kernel, M, M, sd, wkey, perm);
+    {
+        Workspace tmp(ws);
+        FHG_TRY(radix_sort_u64(tmp, wkey, perm, M, 0, 64));
+    }
+    LAUNCH(pc_row_keys_kernel, M, M, perm, srow, rowkey);
+    {
+        Workspace tmp(ws);
+        FHG_TRY(radix_sort_u32(tmp, rowkey, perm, M, 0, bits_for(n)));
+    }
+    LAUNCH(pc_core_kernel, M, M, k, ms, perm, srow, scol, sd, indptr, neighbors, core);
+    return FHG_OK;
 }
 
 }  // namespace
@@ -224,67 +344,53 @@ int precomputed_mst(const int32_t* rows, const int32_t* cols, const double* data
     LAUNCH(pc_fill_u64_kernel, mu, reinterpret_cast<uint64_t*>(gmin), mu, ~0ull);
     LAUNCH(pc_group_min_kernel, m0, m0, n, key, at, d0, gflag, gpos, gmin, gu, gv);
 
-    // ---- the symmetric CSR: both halves, stably by row
-    const int64_t M = 2 * mu;
-    if (M > 0x7fffffffLL) {
+    // ---- _core_distances_csr
+    if (2 * mu > 0x7fffffffLL) {
         set_error("precomputed: %lld symmetric entries exceed the int32 entry index",
-                  (long long)M);
+                  (long long)(2 * mu));
         return FHG_ERR_UNSUPPORTED;
     }
-    const size_t Mz = (size_t)(M > 0 ? M : 1);
-    uint32_t *rowkey, *count, *indptr;
-    int32_t *perm, *srow, *scol;
-    double* sd;
-    FHG_TRY(ws.alloc(&rowkey, Mz));
-    FHG_TRY(ws.alloc(&perm, Mz));
-    FHG_TRY(ws.alloc(&srow, Mz));
-    FHG_TRY(ws.alloc(&scol, Mz));
-    FHG_TRY(ws.alloc(&sd, Mz));
-    FHG_TRY(ws.alloc(&count, (size_t)n));
-    FHG_TRY(ws.alloc(&indptr, (size_t)n));
-    FHG_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t) * n, s));
-    LAUNCH(pc_sym_kernel, M, mu, gu, gv, rowkey, perm);
-    if (M > 1) {
+    int32_t* perm;
+    FHG_TRY(ws.alloc(&perm, gz));
+    if (mu > 0) {
         Workspace tmp(ws);
-        FHG_TRY(radix_sort_u32(tmp, rowkey, perm, M, 0, bits_for(n)));
-    }
-    LAUNCH(pc_csr_kernel, M, M, mu, perm, gu, gv, gmin, srow, scol, sd, count);
-    FHG_TRY(scan_exclusive_u32(ws, count, indptr, n, cnt));
-
-    // ---- _core_distances_csr: every row by weight, ties by position
-    if (M > 0) {
-        uint64_t* wkey;
-        FHG_TRY(ws.alloc(&wkey, Mz));
-        LAUNCH(pc_weight_keys_kernel, M, M, sd, wkey, perm);
-        {
-            Workspace tmp(ws);
-            if (M > 1) FHG_TRY(radix_sort_u64(tmp, wkey, perm, M, 0, 64));
+        uint32_t *vrow, *ubeg, *lbeg;
+        FHG_TRY(tmp.alloc(&vrow, gz));
+        FHG_TRY(tmp.alloc(&ubeg, (size_t)(n + 1)));
+        FHG_TRY(tmp.alloc(&lbeg, (size_t)(n + 1)));
+        LAUNCH(pc_mirror_kernel, mu, mu, gv, vrow, perm);
+        if (mu > 1) {
+            Workspace sort(tmp);
+            FHG_TRY(radix_sort_u32(sort, vrow, perm, mu, 0, bits_for(n)));
         }
-        LAUNCH(pc_row_keys_kernel, M, M, perm, srow, rowkey);
-        {
-            Workspace tmp(ws);
-            if (M > 1) FHG_TRY(radix_sort_u32(tmp, rowkey, perm, M, 0, bits_for(n)));
+        FHG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t), s));
+        LAUNCH(pc_rows_kernel, n + 1, n, mu, gu, vrow, ubeg, lbeg, cnt);
+        FHG_CUDA(cudaMemcpyAsync(&h, cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        FHG_CUDA(cudaStreamSynchronize(s));
+        if (h <= (uint32_t)kPcRow) {
+            ::fhg::note_launch();
+            pc_rank_rows_kernel<<<grid_for(n, kPcWarps), kPcWarps * 32, 0, s>>>(
+                n, k, min_samples, gu, gv, gmin, perm, ubeg, lbeg, neighbors, core);
+            FHG_CUDA(cudaGetLastError());
+        } else {
+            FHG_TRY(core_by_sorting(tmp, n, mu, k, min_samples, gu, gv, gmin, neighbors, core));
         }
-        LAUNCH(pc_core_kernel, M, M, k, min_samples, perm, srow, scol, sd, indptr, neighbors,
-               core);
     }
 
     // ---- mutual-reachability weights, stably sorted, and the forest
     uint64_t* mkey;
     int2* uv;
-    double* w;
-    FHG_TRY(ws.alloc(&mkey, Mz));
-    FHG_TRY(ws.alloc(&uv, Mz));
-    FHG_TRY(ws.alloc(&w, Mz));
-    LAUNCH(pc_mrd_kernel, M, M, srow, scol, sd, core, mkey, perm);
-    if (M > 1) {
+    FHG_TRY(ws.alloc(&mkey, gz));
+    FHG_TRY(ws.alloc(&uv, gz));
+    LAUNCH(pc_mrd_kernel, mu, mu, gu, gv, gmin, core, mkey, perm);
+    if (mu > 1) {
         Workspace tmp(ws);
-        FHG_TRY(radix_sort_u64(tmp, mkey, perm, M, 0, 64));
+        FHG_TRY(radix_sort_u64(tmp, mkey, perm, mu, 0, 64));
     }
-    LAUNCH(pc_ranks_kernel, M, M, perm, srow, scol, mkey, uv, w);
+    LAUNCH(pc_ranks_kernel, mu, mu, perm, gu, gv, uv);
     if (n < 2) return FHG_OK;
-    return sorted_forest_edges(ws, n, M, 0, nullptr, nullptr, uv, nullptr, 0, edges,
-                               n_components, w);
+    return sorted_forest_edges(ws, n, mu, 0, nullptr, nullptr, uv, nullptr, 0, edges,
+                               n_components, reinterpret_cast<const double*>(mkey));
 }
 
 }  // namespace fhg

@@ -87,3 +87,24 @@ def test_kruskal_estimator_and_trees(engine):
     np.testing.assert_array_equal(res[5], g["neighbors"])
     np.testing.assert_array_equal(res[6], g["core"])
     assert np.isinf(res[4][:, 2]).sum() == np.isinf(g["mst"][:, 2]).sum()
+
+
+@pytest.mark.parametrize("n,knn_k", [(600_000, 15), (30_000, 2), (512, 8), (241, 17),
+                                     (77_823, 16), (77_824, 16)])
+def test_kruskal_edge_counts_vs_oracle(engine, n, knn_k):
+    """Nine million edges (more tiles than a compaction sums by itself), a graph
+    of many components, and edge lists on both sides of what one block takes
+    and of where its tiles grow; points at most five times repeated, so that
+    neighbours at the last distance and at distance zero are common."""
+    from fast_hdbscan_gb300.hdbscan import compute_minimum_spanning_tree
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(n)
+    side = int((n / 2) ** 0.5)
+    X = rng.integers(0, side, size=(n, 2)).astype(np.float32)
+    mst, nbrs, core = compute_minimum_spanning_tree(X, min_samples=2, algorithm="kruskal",
+                                                    knn_k=knn_k)
+    omst, onb, ocore = O.kruskal_knn(O.build_kdtree(X), 2, knn_k, mode=1, nthreads=8)
+    np.testing.assert_array_equal(core, ocore)
+    np.testing.assert_array_equal(nbrs, onb)
+    np.testing.assert_array_equal(mst, omst)

@@ -88,6 +88,39 @@ def test_precomputed_vs_oracle_synthetic(engine, n, k, ms):
     np.testing.assert_array_equal(mst, omst)
 
 
+@pytest.mark.parametrize("longest", [255, 256, 257, 1100])
+@pytest.mark.parametrize("ms", [1, 7, 300])
+def test_precomputed_row_lengths_vs_oracle(engine, longest, ms):
+    """Rows on both sides of the longest that is ranked by one warp, many equal
+    weights in a row, rows shorter than min_samples, some of one entry."""
+    import scipy.sparse
+
+    from fast_hdbscan_gb300.hdbscan import compute_minimum_spanning_tree
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(longest + ms)
+    n, hub = 1500, 700
+    near = rng.permutation(np.setdiff1d(np.arange(n), [hub]))[:longest]
+    rows, cols = [np.full(longest, hub)], [near]
+    i = np.arange(1, n)
+    rows.append(i)  # a chain keeps it connected, but for the hub's entries
+    cols.append(i - 1)
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
+    keep = ~(((rows == hub) | (cols == hub)) & (np.abs(rows - cols) == 1)
+             & (np.arange(rows.size) >= longest))
+    rows, cols = rows[keep], cols[keep]
+    flip = rng.random(rows.size) < 0.5
+    rows, cols = np.where(flip, cols, rows), np.where(flip, rows, cols)
+    data = rng.integers(1, 6, size=rows.size).astype(np.float64)
+    G = scipy.sparse.csr_matrix((data, (rows, cols)), shape=(n, n))
+    mst, nbrs, core = compute_minimum_spanning_tree(G, min_samples=ms, metric="precomputed",
+                                                    algorithm="kruskal")
+    omst, onb, ocore = O.precomputed_kruskal(G, ms)
+    np.testing.assert_array_equal(core, ocore)
+    np.testing.assert_array_equal(nbrs, onb)
+    np.testing.assert_array_equal(mst, omst)
+
+
 def test_precomputed_validation(engine):
     import scipy.sparse
 
