@@ -1,4 +1,4 @@
-// Stable stream compaction in two launches (one for up to kCompactTile
+// Stable stream compaction in two launches (one for up to kCompactOne
 // indices): the indices i of [0, n) with f.test(i), in order, get the places
 // 0, 1, ... by f.emit(i, place).
 //
@@ -19,39 +19,43 @@
 
 namespace fhg {
 
-constexpr int kCompactThreads = 256;
-constexpr int kCompactRows = 16;  // indices of a thread, kCompactThreads apart
-constexpr int kCompactTile = kCompactThreads * kCompactRows;
+// A thread's indices, THREADS apart.  A tile of 256 x 16 reads its counts least
+// often; but test and emit are chains of gathers, and below kCompactFew indices
+// (two rounds of blocks) its few blocks are latency: there a thread takes 2 (200k
+// components, the round's edges: 182 -> 32 us).  One block takes what fits in it.
+constexpr int kCompactThreads = 256, kCompactRows = 16, kCompactFewRows = 2;
+constexpr int kCompactOneThreads = 1024, kCompactOneRows = 4;
+constexpr int64_t kCompactFew = (int64_t)2 * 152 * kCompactThreads * kCompactRows;
+constexpr int64_t kCompactOne = kCompactOneThreads * kCompactOneRows;
 constexpr int64_t kCompactScan = 2048;
 
-template <class F>
-__global__ void __launch_bounds__(kCompactThreads) compact_count_kernel(F f, int64_t n,
-                                                                        uint32_t* counts) {
-    const int64_t base = (int64_t)blockIdx.x * kCompactTile + threadIdx.x;
+template <class F, int THREADS, int ROWS>
+__global__ void __launch_bounds__(THREADS) compact_count_kernel(F f, int64_t n,
+                                                                uint32_t* counts) {
+    const int64_t base = (int64_t)blockIdx.x * (THREADS * ROWS) + threadIdx.x;
     int c = 0;
 #pragma unroll
-    for (int t = 0; t < kCompactRows; ++t) {
-        const int64_t i = base + t * kCompactThreads;
+    for (int t = 0; t < ROWS; ++t) {
+        const int64_t i = base + t * THREADS;
         c += i < n && f.test(i) ? 1 : 0;
     }
-    __shared__ int s_c[kCompactThreads / 32];
+    __shared__ int s_c[THREADS / 32];
     c = __reduce_add_sync(kFull, c);
     if ((threadIdx.x & 31) == 0) s_c[threadIdx.x >> 5] = c;
     __syncthreads();
     if (threadIdx.x == 0) {
         int sum = 0;
-        for (int w = 0; w < kCompactThreads / 32; ++w) sum += s_c[w];
+        for (int w = 0; w < THREADS / 32; ++w) sum += s_c[w];
         counts[blockIdx.x] = (uint32_t)sum;
     }
 }
 
-template <class F>
-__global__ void __launch_bounds__(kCompactThreads) compact_emit_kernel(F f, int64_t n,
-                                                                       const uint32_t* counts,
-                                                                       bool scanned,
-                                                                       uint32_t* total) {
-    constexpr int kWarps = kCompactThreads / 32;
-    __shared__ uint32_t s_cell[kCompactRows][kWarps];  // marked indices per row and warp
+template <class F, int THREADS, int ROWS>
+__global__ void __launch_bounds__(THREADS) compact_emit_kernel(F f, int64_t n,
+                                                               const uint32_t* counts,
+                                                               bool scanned, uint32_t* total) {
+    constexpr int kWarps = THREADS / 32;
+    __shared__ uint32_t s_cell[ROWS][kWarps];  // marked indices per row and warp
     __shared__ uint32_t s_before;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_before = 0;
@@ -60,27 +64,28 @@ __global__ void __launch_bounds__(kCompactThreads) compact_emit_kernel(F f, int6
     if (scanned) {
         before = threadIdx.x == 0 ? counts[blockIdx.x] : 0u;
     } else {
-        for (int64_t b = threadIdx.x; b < (int64_t)blockIdx.x; b += kCompactThreads)
+        for (int64_t b = threadIdx.x; b < (int64_t)blockIdx.x; b += THREADS)
             before += counts[b];
     }
     before = __reduce_add_sync(kFull, before);
     if (lane == 0 && before) atomicAdd(&s_before, before);
-    const int64_t base = (int64_t)blockIdx.x * kCompactTile + threadIdx.x;
-    unsigned mine[kCompactRows];
+    const int64_t base = (int64_t)blockIdx.x * (THREADS * ROWS) + threadIdx.x;
+    unsigned mine[ROWS];
 #pragma unroll
-    for (int t = 0; t < kCompactRows; ++t) {
-        const int64_t i = base + t * kCompactThreads;
+    for (int t = 0; t < ROWS; ++t) {
+        const int64_t i = base + t * THREADS;
         mine[t] = __ballot_sync(kFull, i < n && f.test(i));
         if (lane == 0) s_cell[t][w] = __popc(mine[t]);
     }
     __syncthreads();
     if (w == 0) {  // exclusive prefix of the cells, in index order
-        constexpr int kCells = kCompactRows * kWarps, kPer = kCells / 32;
+        constexpr int kCells = ROWS * kWarps, kPer = (kCells + 31) / 32;
         uint32_t v[kPer], sum = 0;
         uint32_t* cell = &s_cell[0][0] + lane * kPer;
+        const bool mine_too = lane * kPer < kCells;
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
-            v[j] = cell[j];
+            v[j] = mine_too ? cell[j] : 0u;
             sum += v[j];
         }
         uint32_t x = sum;
@@ -92,15 +97,15 @@ __global__ void __launch_bounds__(kCompactThreads) compact_emit_kernel(F f, int6
         uint32_t run = s_before + x - sum;
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
-            cell[j] = run;
+            if (mine_too) cell[j] = run;
             run += v[j];
         }
         if (lane == 31 && total && blockIdx.x == gridDim.x - 1) *total = run;
     }
     __syncthreads();
 #pragma unroll
-    for (int t = 0; t < kCompactRows; ++t) {
-        const int64_t i = base + t * kCompactThreads;
+    for (int t = 0; t < ROWS; ++t) {
+        const int64_t i = base + t * THREADS;
         if (i >= n) break;
         f.each(i);
         if ((mine[t] >> lane) & 1u)
@@ -108,15 +113,11 @@ __global__ void __launch_bounds__(kCompactThreads) compact_emit_kernel(F f, int6
     }
 }
 
-// total (device, nullable) receives the number of marked indices.
-template <class F>
-int compact(Workspace& ws, const F& f, int64_t n, uint32_t* total) {
+template <class F, int THREADS, int ROWS>
+int compact_tiles(Workspace& ws, const F& f, int64_t n, uint32_t* total) {
+    static_assert(ROWS * THREADS / 32 <= 32 || ROWS * THREADS / 32 % 32 == 0, "whole lanes");
     cudaStream_t s = ws.stream();
-    if (n <= 0) {
-        if (total) FHG_CUDA(cudaMemsetAsync(total, 0, sizeof(uint32_t), s));
-        return FHG_OK;
-    }
-    const int64_t tiles = (n + kCompactTile - 1) / kCompactTile;
+    const int64_t tiles = (n + THREADS * ROWS - 1) / (THREADS * ROWS);
     Workspace tmp(ws);
     uint32_t *counts = nullptr, *starts = nullptr;
     const bool scanned = tiles > kCompactScan;
@@ -124,15 +125,29 @@ int compact(Workspace& ws, const F& f, int64_t n, uint32_t* total) {
         FHG_TRY(tmp.alloc(&counts, (size_t)tiles));
         if (scanned) FHG_TRY(tmp.alloc(&starts, (size_t)tiles));
         ::fhg::note_launch();
-        compact_count_kernel<F><<<(unsigned)tiles, kCompactThreads, 0, s>>>(f, n, counts);
+        compact_count_kernel<F, THREADS, ROWS><<<(unsigned)tiles, THREADS, 0, s>>>(f, n, counts);
         FHG_CUDA(cudaGetLastError());
         if (scanned) FHG_TRY(scan_exclusive_u32(tmp, counts, starts, tiles, nullptr));
     }
     ::fhg::note_launch();
-    compact_emit_kernel<F><<<(unsigned)tiles, kCompactThreads, 0, s>>>(f, n, scanned ? starts : counts,
-                                                                     scanned, total);
+    compact_emit_kernel<F, THREADS, ROWS><<<(unsigned)tiles, THREADS, 0, s>>>(
+        f, n, scanned ? starts : counts, scanned, total);
     FHG_CUDA(cudaGetLastError());
     return FHG_OK;
+}
+
+// total (device, nullable) receives the number of marked indices.
+template <class F>
+int compact(Workspace& ws, const F& f, int64_t n, uint32_t* total) {
+    if (n <= 0) {
+        if (total) FHG_CUDA(cudaMemsetAsync(total, 0, sizeof(uint32_t), ws.stream()));
+        return FHG_OK;
+    }
+    if (n <= kCompactOne)
+        return compact_tiles<F, kCompactOneThreads, kCompactOneRows>(ws, f, n, total);
+    if (n < kCompactFew)
+        return compact_tiles<F, kCompactThreads, kCompactFewRows>(ws, f, n, total);
+    return compact_tiles<F, kCompactThreads, kCompactRows>(ws, f, n, total);
 }
 
 }  // namespace fhg
