@@ -23,47 +23,72 @@ namespace {
 
 constexpr int kEomThreads = 1024;
 
-// Maximum of non-negative floats as bits, with an atomic only where it grows:
-// most warps find a value at or above theirs (reading first took this from
-// 1.25 to 0.1 ms at 10M rows, of which a few clusters have most).
+// Maximum of non-negative floats as bits, with an atomic only where it grows.
 __device__ __forceinline__ void max_bits(unsigned int* to, unsigned int b) {
     if (b > *(volatile unsigned int*)to) atomicMax(to, b);
 }
 // One pass over the rows: the row of every point and cluster, the largest
 // lambda under the root (root_max) and of every cluster's points (death), and
 // -- with key -- the parent keys and the row numbers to be sorted by them.
-__global__ void row_facts_kernel(int64_t rows, int64_t n, const int32_t* __restrict__ parent,
-                                 const int32_t* __restrict__ child, const float* __restrict__ lam,
-                                 const float* __restrict__ csize,
-                                 int32_t* __restrict__ row_of_point,
-                                 int32_t* __restrict__ row_of_cluster, unsigned int* root_max,
-                                 unsigned int* death, uint32_t* __restrict__ key,
-                                 int32_t* __restrict__ order) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    const int32_t c = parent[r] - (int32_t)n, x = child[r];
-    if (x >= n) row_of_cluster[x - n] = (int32_t)r;
-    else row_of_point[x] = (int32_t)r;
-    if (key) {
-        key[r] = (uint32_t)c;
-        order[r] = (int32_t)r;
-    }
-    const unsigned int b = __float_as_uint(lam[r]);
+// A few clusters have most rows, and what bounds this is how many warps turn to
+// the same words: a block brings the maxima of its rows together first, in a
+// small table by cluster (rows of a cluster stand together; a cluster whose
+// place is taken goes to its word directly), and takes them on once (10M rows:
+// 1.48 -> 0.83 ms, 1M: 98 -> 54 us, with a maximum per warp before).
+constexpr int kFactsThreads = 256, kFactsRows = 4, kFactsSlots = 64;
+__global__ void __launch_bounds__(kFactsThreads) row_facts_kernel(
+    int64_t rows, int64_t n, const int32_t* __restrict__ parent,
+    const int32_t* __restrict__ child, const float* __restrict__ lam,
+    const float* __restrict__ csize, int32_t* __restrict__ row_of_point,
+    int32_t* __restrict__ row_of_cluster, unsigned int* root_max, unsigned int* death,
+    uint32_t* __restrict__ key, int32_t* __restrict__ order) {
+    __shared__ int32_t s_cluster[kFactsSlots];
+    __shared__ unsigned int s_max[kFactsSlots], s_root;
     const int lane = threadIdx.x & 31;
-    const unsigned act = __activemask();
-    // non-negative floats order like their bits; lanes combine first
-    const unsigned roots = __ballot_sync(act, c == 0);
-    if (c == 0) {
-        const unsigned m = __reduce_max_sync(roots, b);
-        if (lane == __ffs(roots) - 1) max_bits(root_max, m);
+    if (threadIdx.x < kFactsSlots) {
+        s_cluster[threadIdx.x] = -1;
+        s_max[threadIdx.x] = 0u;
     }
-    const bool pt = csize[r] == 1.0f;
-    const unsigned pts = __ballot_sync(act, pt);
-    if (pt) {
-        const unsigned peers = __match_any_sync(pts, c);
-        const unsigned m = __reduce_max_sync(peers, b);
-        if (lane == __ffs(peers) - 1) max_bits(&death[c], m);
+    if (threadIdx.x == 0) s_root = 0u;
+    __syncthreads();
+    const int64_t base = (int64_t)blockIdx.x * (kFactsThreads * kFactsRows) + threadIdx.x;
+#pragma unroll
+    for (int t = 0; t < kFactsRows; ++t) {
+        const int64_t r = base + t * kFactsThreads;
+        const bool here = r < rows;
+        int32_t c = -1;
+        unsigned int b = 0u;  // (non-negative floats order like their bits)
+        bool pt = false;
+        if (here) {
+            c = parent[r] - (int32_t)n;
+            b = __float_as_uint(lam[r]);
+            pt = csize[r] == 1.0f;
+            const int32_t x = child[r];
+            if (x >= n) row_of_cluster[x - n] = (int32_t)r;
+            else row_of_point[x] = (int32_t)r;
+            if (key) {
+                key[r] = (uint32_t)c;
+                order[r] = (int32_t)r;
+            }
+        }
+        const unsigned top = __reduce_max_sync(kFull, c == 0 ? b : 0u);
+        if (lane == 0 && top) atomicMax(&s_root, top);
+        const unsigned pts = __ballot_sync(kFull, pt);
+        if (pt) {
+            const unsigned peers = __match_any_sync(pts, c);
+            const unsigned m = __reduce_max_sync(peers, b);
+            if (lane == __ffs(peers) - 1) {
+                const int slot = c & (kFactsSlots - 1);
+                const int32_t was = atomicCAS(&s_cluster[slot], -1, c);
+                if (was == -1 || was == c) atomicMax(&s_max[slot], m);
+                else max_bits(&death[c], m);
+            }
+        }
     }
+    __syncthreads();
+    if (threadIdx.x < kFactsSlots && s_cluster[threadIdx.x] >= 0)
+        max_bits(&death[s_cluster[threadIdx.x]], s_max[threadIdx.x]);
+    if (threadIdx.x == 0 && s_root) max_bits(root_max, s_root);
 }
 // lambda * size of every row, in parent-grouped row order (contiguous per
 // cluster), so that each cluster's sequential sum below streams its addends.
@@ -81,10 +106,13 @@ __global__ void products_kernel(int64_t rows, const uint32_t* __restrict__ key,
     if (j == 0 || key[j - 1] != c) start[c] = j;
     if (j + 1 == rows || key[j + 1] != c) end[c] = j + 1;
 }
-// One thread per cluster: the float32 sum of its rows' products, strictly in
-// row order (a float32 sum is not associative, so the order is the result).
-// Clusters of kBigRows rows or more are summed by score_big_kernel.
-constexpr int32_t kBigRows = 8192;
+// One warp per cluster: the float32 sum of its rows' products, strictly in row
+// order (a float32 sum is not associative, so the order is the result).  The
+// lanes read 32 products together, the next ones while these are added, and all
+// add the same chain; a thread per cluster waited for each of its loads (1M
+// points, min_cluster_size 500: 218 -> 29 us).  Clusters of kBigRows rows or
+// more are summed by score_big_kernel.
+constexpr int32_t kBigRows = 2048;
 __device__ __forceinline__ float score_start(int64_t c, const int32_t* __restrict__ row_of_cluster,
                                              const float* __restrict__ lam,
                                              const float* __restrict__ csize) {
@@ -100,20 +128,25 @@ __global__ void score_kernel(int64_t C, const int64_t* __restrict__ start,
                              const int32_t* __restrict__ row_of_cluster,
                              const float* __restrict__ lam, const float* __restrict__ csize,
                              float* __restrict__ score) {
-    int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C || end[c] - start[c] >= kBigRows) return;
+    const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (c >= C) return;
+    const int64_t b = start[c];
+    const int len = (int)min(end[c] - b, (int64_t)kBigRows);
+    if (len >= kBigRows) return;
     float s = score_start(c, row_of_cluster, lam, csize);
-    const int64_t b = start[c], e = end[c];
-    int64_t j = b;
-    for (; j + 8 <= e; j += 8) {
-        float v[8];
+    float v = lane < len ? __ldg(prod + b + lane) : 0.0f;
+    for (int j = 0; j < len; j += 32) {
+        const float next = j + 32 + lane < len ? __ldg(prod + b + j + 32 + lane) : 0.0f;
+        if (len - j >= 32) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = __ldg(prod + j + u);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) s = __fadd_rn(s, v[u]);
+            for (int u = 0; u < 32; ++u) s = __fadd_rn(s, __shfl_sync(kFull, v, u));
+        } else {
+            for (int u = 0; u < len - j; ++u) s = __fadd_rn(s, __shfl_sync(kFull, v, u));
+        }
+        v = next;
     }
-    for (; j < e; ++j) s = __fadd_rn(s, __ldg(prod + j));
-    score[c] = s;
+    if (lane == 0) score[c] = s;
 }
 // One block per cluster of kBigRows rows or more: the same sequential sum by
 // one thread, fed from shared memory -- the other warps stage the next chunk
@@ -199,36 +232,49 @@ __global__ void cluster_info_kernel(int64_t C, int64_t n, const int32_t* __restr
     in_tree[c] = ok ? 1 : 0;
 }
 
+// Exclusive scan by one block of kEomThreads (len small).
 __device__ void block_scan_excl(int32_t* a, int64_t len, int32_t* tmp_total) {
-    // simple single-block exclusive scan over global memory (len small)
-    __shared__ int32_t part[kEomThreads];
-    const int t = threadIdx.x;
-    int64_t per = (len + blockDim.x - 1) / blockDim.x;
-    int64_t b = t * per, e = b + per < len ? b + per : len;
+    __shared__ int32_t part[kEomThreads / 32];
+    const int t = threadIdx.x, lane = t & 31;
+    const int64_t per = (len + blockDim.x - 1) / blockDim.x;
+    const int64_t b = t * per, e = b + per < len ? b + per : len;
     int32_t s = 0;
     for (int64_t i = b; i < e; ++i) s += a[i];
-    part[t] = s;
+    int32_t x = s;  // inclusive over the warp, then over the warps
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int32_t y = __shfl_up_sync(kFull, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) part[t >> 5] = x;
     __syncthreads();
-    if (t == 0) {
-        int32_t run = 0;
-        for (int i = 0; i < (int)blockDim.x; ++i) {
-            int32_t v = part[i];
-            part[i] = run;
-            run += v;
+    if (t < 32) {
+        int32_t y = part[t];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t z = __shfl_up_sync(kFull, y, o);
+            if (lane >= o) y += z;
         }
-        *tmp_total = run;
+        part[t] = y;
+        if (t == 31) *tmp_total = y;
     }
     __syncthreads();
-    int32_t run = part[t];
+    int32_t run = (t >= 32 ? part[(t >> 5) - 1] : 0) + x - s;
     for (int64_t i = b; i < e; ++i) {
-        int32_t v = a[i];
+        const int32_t v = a[i];
         a[i] = run;
         run += v;
     }
     __syncthreads();
 }
 
-// Single-block EOM.  Scratch arrays are C entries each.
+// Single-block EOM.  What bounds it is the latency of one level after another,
+// leaves to root and back: up to kEomShared clusters, everything that the levels
+// read and write is first brought into shared memory (1M points, min_cluster_size
+// 500: 310 -> 136 us).  Above, the scratch arrays are C entries each (dcount C +
+// 2) in global memory.
+constexpr int64_t kEomShared = 4096;
+constexpr size_t kEomBytes = 47;  // a cluster's, and 16 for dcount
 __global__ void __launch_bounds__(kEomThreads) eom_kernel(
     int64_t C, const int32_t* __restrict__ cpar, const float* __restrict__ nsize,
     const int8_t* __restrict__ in_tree, const float* __restrict__ score,
@@ -239,11 +285,44 @@ __global__ void __launch_bounds__(kEomThreads) eom_kernel(
     double* ret, int8_t* chose, int8_t* blocked, int32_t* flags, int32_t* sel, int64_t* n_sel) {
     const int t = threadIdx.x;
     __shared__ int32_t s_maxd, s_total;
+    extern __shared__ double s_eom[];
+    const bool here = C <= kEomShared;
+    int32_t *kid0 = nullptr, *kids = nullptr, *nkid = nullptr;
+    float* own = nullptr;
+    const int32_t* up = cpar;
+    const int8_t* tree = in_tree;
+    if (here) {
+        ret = s_eom;
+        int32_t* at = reinterpret_cast<int32_t*>(s_eom + C);
+        depth = at;
+        depth2 = at + C;
+        jmp = at + 2 * C;
+        jmp2 = at + 3 * C;
+        kid0 = at + 4 * C;
+        nkid = at + 5 * C;
+        int32_t* s_up = at + 6 * C;
+        own = reinterpret_cast<float*>(at + 7 * C);
+        dcount = at + 8 * C;  // C + 2
+        chose = reinterpret_cast<int8_t*>(at + 9 * C + 4);
+        blocked = chose + C;
+        int8_t* s_tree = chose + 2 * C;
+        for (int64_t c = t; c < C; c += blockDim.x) {
+            s_up[c] = cpar[c];
+            kid0[c] = (int32_t)start[c];
+            nkid[c] = cnt[c];
+            s_tree[c] = in_tree[c];
+            // (larger than the caller's maximum: never chosen)
+            own[c] = (double)nsize[c] > max_cs ? -1.0f : fmaxf(score[c], 0.0f);
+        }
+        up = s_up;
+        tree = s_tree;
+        __syncthreads();
+    }
     // depth of every cluster by pointer doubling (root = 0)
     for (int64_t c = t; c < C; c += blockDim.x) {
-        const bool inner = c != 0 && in_tree[c];
+        const bool inner = c != 0 && tree[c];
         depth[c] = inner ? 1 : 0;
-        jmp[c] = inner ? cpar[c] : 0;
+        jmp[c] = inner ? up[c] : 0;
     }
     __syncthreads();
     int rounds = 1;
@@ -259,20 +338,30 @@ __global__ void __launch_bounds__(kEomThreads) eom_kernel(
         tp = jmp; jmp = jmp2; jmp2 = tp;
     }
     if (t == 0) s_maxd = 0;
+    if (here) {  // the doubling's arrays serve again
+        byd = depth2;
+        kids = jmp;
+        flags = jmp2;
+        for (int64_t c = t; c < C; c += blockDim.x)
+            for (int32_t q = 0; q < nkid[c]; ++q)
+                if (kid0[c] + q < C) kids[kid0[c] + q] = (int32_t)(child[order[kid0[c] + q]] - n);
+    }
     __syncthreads();
-    for (int64_t c = t; c < C; c += blockDim.x)
-        if (in_tree[c]) atomicMax(&s_maxd, depth[c]);
+    for (int64_t c = t; c < C; c += blockDim.x) {
+        depth[c] = min(depth[c], (int32_t)C);  // (rows that form a cycle)
+        if (tree[c]) atomicMax(&s_maxd, depth[c]);
+    }
     __syncthreads();
     const int32_t maxd = s_maxd;
     // bucket clusters by depth (counting sort)
     for (int64_t d = t; d <= maxd + 1; d += blockDim.x) dcount[d] = 0;
     __syncthreads();
     for (int64_t c = t; c < C; c += blockDim.x)
-        if (in_tree[c]) atomicAdd(&dcount[depth[c]], 1);
+        if (tree[c]) atomicAdd(&dcount[depth[c]], 1);
     __syncthreads();
     block_scan_excl(dcount, maxd + 2, &s_total);
     for (int64_t c = t; c < C; c += blockDim.x)
-        if (in_tree[c]) byd[atomicAdd(&dcount[depth[c]], 1)] = (int32_t)c;
+        if (tree[c]) byd[atomicAdd(&dcount[depth[c]], 1)] = (int32_t)c;
     __syncthreads();
     // dcount[d] is now the end of level d; level d spans [end(d-1), end(d))
     for (int32_t d = maxd; d >= 0; --d) {
@@ -284,11 +373,21 @@ __global__ void __launch_bounds__(kEomThreads) eom_kernel(
                 ret[c] = 0.0;
                 continue;
             }
-            const double cur = (double)score[c] > 0.0 ? (double)score[c] : 0.0;
-            double tot = 0.0;
-            for (int32_t q = 0; q < cnt[c]; ++q)
-                tot += ret[child[order[start[c] + (uint32_t)q]] - n];
-            if (tot > cur || (double)nsize[c] > max_cs) {
+            double cur, tot = 0.0;
+            bool too_big = false;
+            if (here) {
+                cur = (double)own[c];
+                for (int32_t q = kid0[c]; q < kid0[c] + nkid[c]; ++q) {
+                    const int64_t x = q < C ? kids[q] : child[order[q]] - n;
+                    tot += x >= 0 && x < C ? ret[x] : 0.0;
+                }
+            } else {
+                cur = (double)score[c] > 0.0 ? (double)score[c] : 0.0;
+                too_big = (double)nsize[c] > max_cs;
+                for (int32_t q = 0; q < cnt[c]; ++q)
+                    tot += ret[child[order[start[c] + (uint32_t)q]] - n];
+            }
+            if (tot > cur || too_big) {
                 ret[c] = tot;
             } else {
                 ret[c] = cur;
@@ -305,18 +404,18 @@ __global__ void __launch_bounds__(kEomThreads) eom_kernel(
                 blocked[c] = 0;
                 continue;
             }
-            const int32_t p = cpar[c];
+            const int32_t p = up[c];
             blocked[c] = blocked[p] || (chose[p] && (p != 0 || allow_single));
         }
         __syncthreads();
     }
     // selected ids in label order (the reference dict's insertion order)
     for (int64_t c = t; c < C; c += blockDim.x)
-        flags[c] = (in_tree[c] && chose[c] && !blocked[c]) ? 1 : 0;
+        flags[c] = (tree[c] && chose[c] && !blocked[c]) ? 1 : 0;
     __syncthreads();
     block_scan_excl(flags, C, &s_total);
     for (int64_t c = t; c < C; c += blockDim.x) {
-        const bool on = in_tree[c] && chose[c] && !blocked[c];
+        const bool on = tree[c] && chose[c] && !blocked[c];
         if (on) sel[flags[c]] = (int32_t)(n + c);
     }
     if (t == 0) *n_sel = s_total;
@@ -525,9 +624,12 @@ int prepare(Workspace& ws, const Condensed& ct, LabelPre* pre, Prepared* P) {
         FHG_TRY(ws.alloc(&P->corder, (size_t)rows));
         FHG_TRY(ws.alloc(&P->score, (size_t)C));
     }
-    LAUNCH(row_facts_kernel, rows, rows, n, ct.parent, ct.child, ct.lambda, ct.csize,
-           pre->row_of_point, pre->row_of_cluster, pre->root_max, pre->death,
-           P ? P->key : (uint32_t*)nullptr, P ? P->order : (int32_t*)nullptr);
+    ::fhg::note_launch();
+    row_facts_kernel<<<grid_for(rows, kFactsThreads * kFactsRows), kFactsThreads, 0, s>>>(
+        rows, n, ct.parent, ct.child, ct.lambda, ct.csize, pre->row_of_point, pre->row_of_cluster,
+        pre->root_max, pre->death, P ? P->key : (uint32_t*)nullptr,
+        P ? P->order : (int32_t*)nullptr);
+    FHG_CUDA(cudaGetLastError());
     if (P) {
         FHG_TRY(radix_sort_u32(ws, P->key, P->order, rows, 0, bits_for(C)));
         LAUNCH(products_kernel, rows, rows, P->key, P->order, ct.lambda, ct.csize, P->prod,
@@ -563,7 +665,7 @@ int prepare(Workspace& ws, const Condensed& ct, LabelPre* pre, Prepared* P) {
                 FHG_CUDA(cudaGetLastError());
             }
             ::fhg::note_launch();
-            score_kernel<<<grid_for(C, 256), 256, 0, ss>>>(C, P->start, P->end, P->prod,
+            score_kernel<<<grid_for(C, 8), 256, 0, ss>>>(C, P->start, P->end, P->prod,
                                                            pre->row_of_cluster, ct.lambda,
                                                            ct.csize, P->score);
             FHG_CUDA(cudaGetLastError());
@@ -646,11 +748,14 @@ int select_eom(Workspace& ws, const Condensed& ct, double max_cs, bool allow_sin
     FHG_TRY(ws.alloc(&chose, (size_t)C));
     FHG_TRY(ws.alloc(&blocked, (size_t)C));
     FHG_TRY(ws.alloc(&nsel_dev, 1));
+    const size_t smem = C <= kEomShared ? kEomBytes * (size_t)C + 16 : 0;
+    FHG_CUDA(cudaFuncSetAttribute(eom_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(kEomBytes * kEomShared + 16)));
     ::fhg::note_launch();
-    eom_kernel<<<1, kEomThreads, 0, s>>>(C, pre->cpar, pre->nsize, pre->in_tree, P.score, P.cstart,
-                                         P.ccnt, P.corder, ct.child, ct.n, max_cs,
-                                         allow_single ? 1 : 0, depth, depth2, jmp, jmp2, dcount,
-                                         byd, ret, chose, blocked, flags, sel, nsel_dev);
+    eom_kernel<<<1, kEomThreads, smem, s>>>(C, pre->cpar, pre->nsize, pre->in_tree, P.score,
+                                            P.cstart, P.ccnt, P.corder, ct.child, ct.n, max_cs,
+                                            allow_single ? 1 : 0, depth, depth2, jmp, jmp2, dcount,
+                                            byd, ret, chose, blocked, flags, sel, nsel_dev);
     FHG_CUDA(cudaGetLastError());
     FHG_CUDA(cudaMemcpyAsync(n_sel, nsel_dev, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     FHG_CUDA(cudaStreamSynchronize(s));

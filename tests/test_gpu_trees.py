@@ -175,3 +175,35 @@ def test_clusters_from_spanning_tree_weight_shape(engine):
     labels, probs, *_ = clusters_from_spanning_tree(mst, min_cluster_size=2,
                                                     sample_weights=np.ones(4, np.float32))
     assert labels.shape == (4,) and probs.shape == (4,)
+
+
+@pytest.mark.parametrize("C", [2, 33, 4095, 4096, 4097])
+@pytest.mark.parametrize("shape", ["bushy", "chain"])
+@pytest.mark.parametrize("big", [2047, 2048, 8192])
+def test_eom_cluster_counts_vs_oracle(engine, C, shape, big):
+    """Cluster trees on both sides of what the EOM kernel keeps in shared
+    memory, wide and as deep as they have clusters, with clusters of 0 to 40
+    rows and one on either side of the rows that a warp sums."""
+    from fast_hdbscan_gb300.cluster_trees import (
+        CondensedTree, cluster_tree_from_condensed_tree, extract_eom_clusters)
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(C + big)
+    lens = rng.integers(0, 41, size=C)
+    lens[0] = max(lens[0], 1)
+    lens[C // 2] = big
+    n = int(lens.sum())
+    up = np.maximum(np.arange(1, C) - 1, 0) if shape == "chain" else (
+        rng.random(C - 1) * np.arange(1, C)).astype(np.int64)
+    parent = np.concatenate([n + np.repeat(np.arange(C), lens), n + up])
+    child = np.concatenate([np.arange(n), n + np.arange(1, C)])
+    lam = (rng.random(n + C - 1) * 10).astype(np.float32)
+    size = np.concatenate([np.ones(n), rng.integers(2, 1000, size=C - 1)]).astype(np.float32)
+    # as in any condensed tree, a cluster's row comes before the rows under it
+    order = np.concatenate([n + np.arange(C - 1), rng.permutation(n)])
+    ct = CondensedTree(*[np.ascontiguousarray(a[order]) for a in (
+        parent.astype(np.int64), child.astype(np.int64), lam, size)])
+    for max_size in (np.inf, 500.0):
+        for single in (False, True):
+            sel = extract_eom_clusters(ct, cluster_tree_from_condensed_tree(ct), max_size, single)
+            np.testing.assert_array_equal(sel, O.extract_eom_clusters(ct, max_size, single))
