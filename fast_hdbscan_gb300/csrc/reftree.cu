@@ -35,11 +35,14 @@
 namespace fhg {
 namespace {
 
-constexpr int kSelThreads = 512;
+constexpr int kSelThreads = 512, kSelFewThreads = 64;
 constexpr int kSelV = 8;                          // consecutive keys per thread and tile
 constexpr int kSelTile = kSelThreads * kSelV;     // keys per scan tile
 constexpr int kBlockSortMax = 4096;               // ranges a block sorts in shared memory
-constexpr int64_t kWideMin = 32768;               // longer ranges partition device-wide
+// Longer ranges partition device-wide: a step of four launches takes 25 to 35 us,
+// a block as long for 32k keys (1M points, the whole tree: 3.5 ms with a line at
+// 32768, 3.6 at 16384, 4.0 at 8192, where a block works in shared memory next).
+constexpr int64_t kWideMin = 32768;
 
 // The saved introselect state of a node partitioned device-wide.
 constexpr int kWideActive = 0, kWideBlock = 1, kWideDone = 2;
@@ -47,7 +50,7 @@ struct WideNode {
     int64_t l, r, B;
     uint64_t pivot;
     int32_t depth, state;
-    uint32_t c, K;
+    uint32_t K;
 };
 
 #define LAUNCH(kernel, count, ...)                                                   \
@@ -243,6 +246,7 @@ __device__ __forceinline__ void swap_keys(uint64_t* k, int64_t a, int64_t b) {
 }
 
 // Exclusive block prefix of one value per thread; returns the block total.
+template <int THREADS = kSelThreads>
 __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* out, uint32_t* s_warp) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     uint32_t incl = v;
@@ -254,14 +258,14 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* out, u
     if (lane == 31) s_warp[w] = incl;
     __syncthreads();
     if (w == 0) {
-        uint32_t x = lane < kSelThreads / 32 ? s_warp[lane] : 0u;
+        uint32_t x = lane < THREADS / 32 ? s_warp[lane] : 0u;
         uint32_t y = x;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t t = __shfl_up_sync(kFull, y, o);
             if (lane >= o) y += t;
         }
-        if (lane < kSelThreads / 32) s_warp[32 + lane] = y - x;  // exclusive warp offsets
+        if (lane < THREADS / 32) s_warp[32 + lane] = y - x;  // exclusive warp offsets
         if (lane == 31) s_warp[64] = y;
     }
     __syncthreads();
@@ -317,9 +321,10 @@ __device__ __forceinline__ int wide_node_of(const int64_t* __restrict__ tile_off
     return lo;
 }
 
-// One block: per node, start (init) or continue a partition step; tiles of
-// the step's range, their prefix over nodes, and in ctl the total of tiles
-// and the number of nodes partitioned in this step.
+// One block: per node, start (init) or finish a partition step -- the pivot goes
+// to its place and the range narrows to the side that holds the median -- and
+// begin the next; tiles of the step's range, their prefix over nodes, and in ctl
+// the total of tiles and the number of nodes partitioned in this step.
 __global__ void __launch_bounds__(kSelThreads) wide_setup_kernel(
     int64_t first, int count, const int64_t* __restrict__ rs, const int64_t* __restrict__ re,
     int64_t n_nodes, int init, uint64_t* keys, WideNode* wide, int64_t* __restrict__ tile_off,
@@ -343,6 +348,12 @@ __global__ void __launch_bounds__(kSelThreads) wide_setup_kernel(
                 w.r = e0;
                 w.depth = m > 16 ? 2 * (63 - __clzll((unsigned long long)m)) : 0;
                 w.state = (2 * v + 1 >= n_nodes || m < 2) ? kWideDone : kWideActive;
+            } else if (w.state == kWideActive) {
+                swap_keys(keys, w.B, w.r - 1);
+                const int64_t v = first + t, nth = rs[v] + (re[v] - rs[v]) / 2;
+                if (nth < w.B) w.r = w.B;
+                else if (nth > w.B) w.l = w.B + 1;
+                else w.state = kWideDone;
             }
             if (w.state == kWideActive) {
                 const int64_t l = w.l, r = w.r, m = r - l;
@@ -379,11 +390,14 @@ __global__ void __launch_bounds__(kSelThreads) wide_setup_kernel(
 }
 
 // Elements below the pivot in one tile of a node's step range [l, r - 1).
+// (The grids of a step's kernels cover at least its ctl[0] tiles.)
 __global__ void __launch_bounds__(kSelThreads) wide_count_kernel(
-    int count, const int64_t* __restrict__ tile_off, const WideNode* __restrict__ wide,
-    const uint64_t* __restrict__ keys, uint32_t* __restrict__ tile_small) {
+    int count, const int64_t* __restrict__ tile_off, const int64_t* __restrict__ ctl,
+    const WideNode* __restrict__ wide, const uint64_t* __restrict__ keys,
+    uint32_t* __restrict__ tile_small) {
     __shared__ uint32_t s_warp[65];
     const int64_t tile = blockIdx.x;
+    if (tile >= ctl[0]) return;
     const int t = wide_node_of(tile_off, count, tile);
     const WideNode w = wide[t];
     const int64_t p0 = w.l + (tile - tile_off[t]) * kSelTile + (int64_t)threadIdx.x * kSelV;
@@ -398,43 +412,39 @@ __global__ void __launch_bounds__(kSelThreads) wide_count_kernel(
     if (threadIdx.x == 0) tile_small[tile] = total;
 }
 
-// One block per node: the tiles' exclusive prefix of their counts, the
-// node's count c and the pivot's final place B = l + c.
-__global__ void __launch_bounds__(kSelThreads) wide_scan_kernel(
-    int count, const int64_t* __restrict__ tile_off, const int64_t* __restrict__ ctl,
-    WideNode* wide, const uint32_t* __restrict__ tile_small, uint32_t* __restrict__ tile_base) {
-    __shared__ uint32_t s_warp[65];
-    const int t = blockIdx.x;
-    const WideNode w = wide[t];
-    if (w.state != kWideActive) return;
-    const int64_t a = tile_off[t], b = t + 1 < count ? tile_off[t + 1] : ctl[0];
-    uint32_t carry = 0;
-    for (int64_t i0 = a; i0 < b; i0 += kSelThreads) {
-        const int64_t i = i0 + threadIdx.x;
-        uint32_t before;
-        const uint32_t sum = block_exclusive(i < b ? tile_small[i] : 0u, &before, s_warp);
-        if (i < b) tile_base[i] = carry + before;
-        carry += sum;
-    }
-    if (threadIdx.x == 0) {
-        wide[t].c = carry;
-        wide[t].B = w.l + carry;
-    }
-}
-
 // select_level_kernel's pairing, over tiles: elements above the pivot left
 // of B, ranked from the left, and elements below it from B on, ranked from
-// the right; K counts the pairs.
+// the right; K counts the pairs.  Every block adds up the counts of its node's
+// tiles: those before its own, and all of them (c, which gives B = l + c).
 __global__ void __launch_bounds__(kSelThreads) wide_rank_kernel(
-    int count, const int64_t* __restrict__ tile_off, WideNode* wide,
-    const uint64_t* __restrict__ keys, const uint32_t* __restrict__ tile_base,
+    int count, const int64_t* __restrict__ tile_off, const int64_t* __restrict__ ctl,
+    WideNode* wide, const uint64_t* __restrict__ keys, const uint32_t* __restrict__ tile_small,
     int32_t* __restrict__ pos_big, int32_t* __restrict__ pos_small) {
     __shared__ uint32_t s_warp[65];
+    __shared__ uint32_t s_before, s_all;
     const int64_t tile = blockIdx.x;
+    if (tile >= ctl[0]) return;
+    if (threadIdx.x == 0) s_before = s_all = 0;
+    __syncthreads();
     const int t = wide_node_of(tile_off, count, tile);
+    const int64_t t0 = tile_off[t], t1 = t + 1 < count ? tile_off[t + 1] : ctl[0];
+    uint32_t mine = 0, all = 0;
+    for (int64_t i = t0 + threadIdx.x; i < t1; i += kSelThreads) {
+        const uint32_t v = tile_small[i];
+        all += v;
+        if (i < tile) mine += v;
+    }
+    mine = __reduce_add_sync(kFull, mine);
+    all = __reduce_add_sync(kFull, all);
+    if ((threadIdx.x & 31) == 0) {
+        if (mine) atomicAdd(&s_before, mine);
+        if (all) atomicAdd(&s_all, all);
+    }
+    __syncthreads();
     const WideNode w = wide[t];
-    const int64_t l = w.l, r = w.r, B = w.B;
-    const uint32_t c = w.c;
+    const uint32_t c = s_all;
+    const int64_t l = w.l, r = w.r, B = l + c;
+    if (tile == t0 && threadIdx.x == 0) wide[t].B = B;  // (read by the next setup)
     const int64_t p0 = l + (tile - tile_off[t]) * kSelTile + (int64_t)threadIdx.x * kSelV;
     uint64_t kv[kSelV];
     uint32_t cnt = 0;
@@ -446,7 +456,7 @@ __global__ void __launch_bounds__(kSelThreads) wide_rank_kernel(
     }
     uint32_t before;
     block_exclusive(cnt, &before, s_warp);
-    before += tile_base[tile];
+    before += s_before;
     uint32_t kb = 0;
 #pragma unroll
     for (int j = 0; j < kSelV; ++j) {
@@ -466,9 +476,11 @@ __global__ void __launch_bounds__(kSelThreads) wide_rank_kernel(
 }
 
 __global__ void __launch_bounds__(kSelThreads) wide_swap_kernel(
-    int count, const int64_t* __restrict__ tile_off, const WideNode* __restrict__ wide,
-    uint64_t* keys, const int32_t* __restrict__ pos_big, const int32_t* __restrict__ pos_small) {
+    int count, const int64_t* __restrict__ tile_off, const int64_t* __restrict__ ctl,
+    const WideNode* __restrict__ wide, uint64_t* keys, const int32_t* __restrict__ pos_big,
+    const int32_t* __restrict__ pos_small) {
     const int64_t tile = blockIdx.x;
+    if (tile >= ctl[0]) return;
     const int t = wide_node_of(tile_off, count, tile);
     const WideNode w = wide[t];
     const int64_t k0 = (tile - tile_off[t]) * kSelTile;
@@ -476,26 +488,12 @@ __global__ void __launch_bounds__(kSelThreads) wide_swap_kernel(
         swap_keys(keys, pos_big[w.l + k], pos_small[w.l + k]);
 }
 
-// The pivot to its place; the range narrows to the side holding the median.
-__global__ void wide_finish_kernel(int count, WideNode* wide, uint64_t* keys, int64_t first,
-                                   const int64_t* __restrict__ rs, const int64_t* __restrict__ re) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    WideNode w = wide[t];
-    if (w.state != kWideActive) return;
-    swap_keys(keys, w.B, w.r - 1);
-    const int64_t v = first + t, nth = rs[v] + (re[v] - rs[v]) / 2;
-    if (nth < w.B) w.r = w.B;
-    else if (nth > w.B) w.l = w.B + 1;
-    else w.state = kWideDone;
-    wide[t] = w;
-}
-
 // The introselect of keys[l, r) around nth (l <= nth < r), continued in
 // shared memory once the active range fits (r - l <= kBlockSortMax): the
 // range is read once, every later partition and the final sort run on s_buf,
 // and it is written back once.  The pairing positions are 12-bit offsets in
 // s_big / s_small (a partition pairs at most (r - l - 1) / 2 elements).
+template <int THREADS>
 __device__ void select_in_smem(uint64_t* keys, int64_t l, int64_t r, int64_t nth, int depth,
                                uint64_t* s_buf, uint16_t* s_big, uint16_t* s_small,
                                uint32_t* s_warp, uint32_t* s_K) {
@@ -552,7 +550,7 @@ __device__ void select_in_smem(uint64_t* keys, int64_t l, int64_t r, int64_t nth
             cnt += (p < R - 1 && kv[j] < pivot) ? 1u : 0u;
         }
         uint32_t before;
-        const uint32_t c = block_exclusive(cnt, &before, s_warp);
+        const uint32_t c = block_exclusive<THREADS>(cnt, &before, s_warp);
         const int B = L + (int)c;
         uint32_t kb = 0;
 #pragma unroll
@@ -599,13 +597,17 @@ __device__ void select_in_smem(uint64_t* keys, int64_t l, int64_t r, int64_t nth
 // reaches the depth limit while longer than a block can sort is recorded in
 // big_sort (its bounds) for a device-wide sort after the launch.  wide
 // (nullable): the state the device-wide partitions left for each node.
-__global__ void __launch_bounds__(kSelThreads) select_level_kernel(
+// A level whose ranges fit in 512 keys takes blocks of 64 threads: what bounds
+// these levels is the steps' barriers and the 41 KB that let five blocks of 512
+// threads share an SM (1M points, the last three levels: 97 + 152 + 234 -> 30 + 37 + 47 us).
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) select_level_kernel(
     int64_t first, const int64_t* __restrict__ rs, const int64_t* __restrict__ re,
     int64_t n_nodes, uint64_t* keys, int32_t* __restrict__ pos_big,
     int32_t* __restrict__ pos_small, int64_t* __restrict__ big_sort, int* big_sort_count,
     const WideNode* __restrict__ wide) {
-    __shared__ uint64_t s_buf[kBlockSortMax];
-    __shared__ uint16_t s_big[kBlockSortMax / 2], s_small[kBlockSortMax / 2];
+    __shared__ uint64_t s_buf[THREADS * kSelV];
+    __shared__ uint16_t s_big[THREADS * kSelV / 2], s_small[THREADS * kSelV / 2];
     __shared__ uint32_t s_warp[65];
     __shared__ int64_t s_l, s_r;
     __shared__ uint64_t s_pivot;
@@ -636,8 +638,8 @@ __global__ void __launch_bounds__(kSelThreads) select_level_kernel(
     __syncthreads();
     while (true) {
         const int64_t l = s_l, r = s_r;
-        if (r - l <= kBlockSortMax) {
-            select_in_smem(keys, l, r, nth, depth, s_buf, s_big, s_small, s_warp, &s_K);
+        if (r - l <= THREADS * kSelV) {
+            select_in_smem<THREADS>(keys, l, r, nth, depth, s_buf, s_big, s_small, s_warp, &s_K);
             return;
         }
         if (depth == 0) {
@@ -670,12 +672,12 @@ __global__ void __launch_bounds__(kSelThreads) select_level_kernel(
         uint32_t c_loc = 0;
         for (int64_t p = l + threadIdx.x; p < r - 1; p += blockDim.x) c_loc += keys[p] < pivot;
         uint32_t dummy;
-        const uint32_t c = block_exclusive(c_loc, &dummy, s_warp);
+        const uint32_t c = block_exclusive<THREADS>(c_loc, &dummy, s_warp);
         const int64_t B = l + c;
         // pair the elements above the pivot left of B (ranked from the left)
         // with those below it from B on (ranked from the right)
         uint32_t carry = 0;
-        for (int64_t base = l; base < r - 1; base += kSelTile) {
+        for (int64_t base = l; base < r - 1; base += THREADS * kSelV) {
             const int64_t p0 = base + (int64_t)threadIdx.x * kSelV;
             uint64_t kv[kSelV];
             uint32_t cnt = 0;
@@ -686,7 +688,7 @@ __global__ void __launch_bounds__(kSelThreads) select_level_kernel(
                 cnt += (p < r - 1 && kv[j] < pivot) ? 1u : 0u;
             }
             uint32_t before;
-            const uint32_t tile_total = block_exclusive(cnt, &before, s_warp);
+            const uint32_t tile_total = block_exclusive<THREADS>(cnt, &before, s_warp);
             before += carry;
             uint32_t kb = 0;
 #pragma unroll
@@ -969,7 +971,7 @@ int ref_tree_build(Workspace& ws, const fhg_index& ix, RefTree* out) {
         ++wide_levels;
     WideNode* wide = nullptr;
     int64_t *tile_off = nullptr, *ctl = nullptr;
-    uint32_t *tile_small = nullptr, *tile_base = nullptr;
+    uint32_t* tile_small = nullptr;
     if (wide_levels > 0) {
         const int64_t wide_nodes = (int64_t)1 << (wide_levels - 1);
         const size_t max_tiles = (size_t)(n / kSelTile + wide_nodes + 1);
@@ -977,7 +979,6 @@ int ref_tree_build(Workspace& ws, const fhg_index& ix, RefTree* out) {
         FHG_TRY(tmp.alloc(&tile_off, (size_t)wide_nodes));
         FHG_TRY(tmp.alloc(&ctl, 2));
         FHG_TRY(tmp.alloc(&tile_small, max_tiles));
-        FHG_TRY(tmp.alloc(&tile_base, max_tiles));
     }
     float* ptsc;
     FHG_TRY(tmp.alloc(&ptsc, (size_t)(n * pad)));
@@ -1003,43 +1004,54 @@ int ref_tree_build(Workspace& ws, const fhg_index& ix, RefTree* out) {
         const bool wide_level = lvl < wide_levels;  // some node longer than kWideMin
         if (wide_level) {
             Stage sel(s, "ref_tree_select_wide");
+            // A step leaves about 0.6 of a range.  As many steps as that takes
+            // follow one another before the host looks whether any node is
+            // left (a look costs as much as three steps that find nothing to
+            // do); grids cover the tiles of the last look, which only shrink.
+            const double size = (double)((n + count - 1) / count);
+            int ahead = 1 + (int)(1.4 * std::log2(std::max(1.0, size / (double)kWideMin)));
+            unsigned tiles = (unsigned)(n / kSelTile + count);
             for (int init = 1;; init = 0) {
                 ::fhg::note_launch();
                 wide_setup_kernel<<<1, kSelThreads, 0, s>>>(first, (int)count, rs, re, nodes, init,
                                                            keys, wide, tile_off, ctl);
                 FHG_CUDA(cudaGetLastError());
-                int64_t h_ctl[2];
-                FHG_CUDA(cudaMemcpyAsync(h_ctl, ctl, sizeof(h_ctl), cudaMemcpyDeviceToHost, s));
-                FHG_CUDA(cudaStreamSynchronize(s));
-                if (h_ctl[1] == 0) break;
-                const unsigned tiles = (unsigned)h_ctl[0];
+                if (ahead-- == 0) {
+                    int64_t h_ctl[2];
+                    FHG_CUDA(cudaMemcpyAsync(h_ctl, ctl, sizeof(h_ctl), cudaMemcpyDeviceToHost, s));
+                    FHG_CUDA(cudaStreamSynchronize(s));
+                    if (h_ctl[1] == 0) break;
+                    tiles = (unsigned)h_ctl[0];
+                    ahead = 1;
+                }
                 ::fhg::note_launch();
-                wide_count_kernel<<<tiles, kSelThreads, 0, s>>>((int)count, tile_off, wide, keys,
-                                                                tile_small);
+                wide_count_kernel<<<tiles, kSelThreads, 0, s>>>((int)count, tile_off, ctl, wide,
+                                                                keys, tile_small);
                 ::fhg::note_launch();
-                wide_scan_kernel<<<(unsigned)count, kSelThreads, 0, s>>>((int)count, tile_off, ctl,
-                                                                         wide, tile_small, tile_base);
+                wide_rank_kernel<<<tiles, kSelThreads, 0, s>>>((int)count, tile_off, ctl, wide,
+                                                               keys, tile_small, pos_big,
+                                                               pos_small);
                 ::fhg::note_launch();
-                wide_rank_kernel<<<tiles, kSelThreads, 0, s>>>((int)count, tile_off, wide, keys,
-                                                               tile_base, pos_big, pos_small);
-                ::fhg::note_launch();
-                wide_swap_kernel<<<tiles, kSelThreads, 0, s>>>((int)count, tile_off, wide, keys,
-                                                               pos_big, pos_small);
+                wide_swap_kernel<<<tiles, kSelThreads, 0, s>>>((int)count, tile_off, ctl, wide,
+                                                               keys, pos_big, pos_small);
                 FHG_CUDA(cudaGetLastError());
-                LAUNCH(wide_finish_kernel, count, (int)count, wide, keys, first, rs, re);
             }
         }
         {
             Stage sel(s, wide_level ? "ref_tree_select_top" : "ref_tree_select_deep");
             ::fhg::note_launch();
-            select_level_kernel<<<(unsigned)count, kSelThreads, 0, s>>>(
+            const bool few = (n + count - 1) / count <= kSelFewThreads * kSelV;
+            (few ? select_level_kernel<kSelFewThreads> : select_level_kernel<kSelThreads>)<<<
+                (unsigned)count, few ? kSelFewThreads : kSelThreads, 0, s>>>(
                 first, rs, re, nodes, keys, pos_big, pos_small, big_sort, big_count,
                 wide_level ? wide : nullptr);
             FHG_CUDA(cudaGetLastError());
         }
         int h_big = 0;
-        FHG_CUDA(cudaMemcpyAsync(&h_big, big_count, sizeof(int), cudaMemcpyDeviceToHost, s));
-        FHG_CUDA(cudaStreamSynchronize(s));
+        if ((n + count - 1) / count > kBlockSortMax) {  // (the level's longest range)
+            FHG_CUDA(cudaMemcpyAsync(&h_big, big_count, sizeof(int), cudaMemcpyDeviceToHost, s));
+            FHG_CUDA(cudaStreamSynchronize(s));
+        }
         if (h_big > 0) {
             // ranges that hit the depth limit while longer than a block sorts:
             // sorted ascending on the device (the heapsort's result)

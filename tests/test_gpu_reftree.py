@@ -61,3 +61,22 @@ def test_reference_kdtree_vs_oracle(engine, case):
     name, X = _cases()[case]
     tree = build_reference_kdtree(X)
     _assert_tree_equal(tree, O.build_kdtree(X).arrays())
+
+
+@pytest.mark.parametrize("n", [8191, 8192, 8193, 8194, 16_385, 32_768, 32_769, 33_001,
+                               65_537, 150_000])
+@pytest.mark.parametrize("kind", ["normal", "organ", "few"])
+def test_reference_kdtree_wide_ranges_vs_oracle(engine, n, kind):
+    """Ranges on both sides of what one block partitions alone, on inputs that a
+    median of three splits badly (organ pipes: steps up to the depth limit) and
+    with coordinates that differ in their index alone."""
+    from fast_hdbscan_gb300.numba_kdtree import build_reference_kdtree
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(n)
+    X = rng.standard_normal((n, 2)).astype(np.float32)
+    if kind == "organ":
+        X[:, 0] = 10 * np.minimum(np.arange(n), np.arange(n)[::-1])
+    elif kind == "few":
+        X = rng.integers(0, 3, size=(n, 2)).astype(np.float32)
+    _assert_tree_equal(build_reference_kdtree(X), O.build_kdtree(X).arrays())
