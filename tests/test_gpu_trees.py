@@ -207,3 +207,23 @@ def test_eom_cluster_counts_vs_oracle(engine, C, shape, big):
         for single in (False, True):
             sel = extract_eom_clusters(ct, cluster_tree_from_condensed_tree(ct), max_size, single)
             np.testing.assert_array_equal(sel, O.extract_eom_clusters(ct, max_size, single))
+
+
+@pytest.mark.parametrize("m", [1, 511, 512, 513, 1024, 1025, 2049, 4096, 4097, 8193, 70_001])
+@pytest.mark.parametrize("shape", ["random", "chain", "star", "pairs"])
+def test_linkage_intervals_vs_oracle(engine, m, shape):
+    """Edge counts around the intervals that one thread and one block take, on
+    spanning trees with long chains, one hub, and many components to the end."""
+    from fast_hdbscan_gb300.cluster_trees import mst_to_linkage_tree
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(m)
+    child = np.arange(1, m + 1)
+    parent = {"random": (rng.random(m) * child).astype(np.int64), "chain": child - 1,
+              "star": np.zeros(m, np.int64), "pairs": np.where(child % 2 == 1, child - 1,
+                                                               child // 4)}[shape]
+    w = rng.random(m) + (child % 2 == 0 if shape == "pairs" else 0)
+    relabel = rng.permutation(m + 1)
+    mst = np.stack([relabel[parent], relabel[child], w], axis=1).astype(np.float64)
+    mst = mst[np.argsort(w, kind="stable")]
+    np.testing.assert_array_equal(mst_to_linkage_tree(mst), O.mst_to_linkage_tree(mst))
