@@ -361,17 +361,29 @@ __device__ __forceinline__ void seed_body(const BorState& S, int64_t p) {
     int32_t bq = -1, bo = INT32_MAX;
     if (!S.exhausted[p]) {
         const float cp = S.core2[p];
-        for (int j = 1; j < k; ++j) {
-            const int32_t qs = S.knn_s[p * k + j];
-            if (qs < 0) break;
-            if (S.comp[qs] == c) continue;
-            const float w = fmaxf(fmaxf(S.knn_d[p * k + j], cp), S.core2[qs]);
-            const int32_t o = S.orig[qs];
-            if (w < bw || (w == bw && o < bo)) {
-                bw = w;
-                bq = qs;
-                bo = o;
+        // kSeedAhead neighbours and their components are read together: one at
+        // a time, each waited for two gathers (10M points, k = 16, all rounds:
+        // 2.12 -> 2.07 ms; 2M x 5-D, k = 11: 381 -> 318 us; 300k, k = 101: 417 -> 286)
+        constexpr int kSeedAhead = 4;
+        for (int j = 1; j < k; j += kSeedAhead) {
+            int32_t qs[kSeedAhead], cq[kSeedAhead];
+#pragma unroll
+            for (int u = 0; u < kSeedAhead; ++u)
+                qs[u] = j + u < k ? S.knn_s[p * k + j + u] : -1;
+#pragma unroll
+            for (int u = 0; u < kSeedAhead; ++u) cq[u] = qs[u] >= 0 ? S.comp[qs[u]] : c;
+#pragma unroll
+            for (int u = 0; u < kSeedAhead; ++u) {
+                if (cq[u] == c) continue;
+                const float w = fmaxf(fmaxf(S.knn_d[p * k + j + u], cp), S.core2[qs[u]]);
+                const int32_t o = S.orig[qs[u]];
+                if (w < bw || (w == bw && o < bo)) {
+                    bw = w;
+                    bq = qs[u];
+                    bo = o;
+                }
             }
+            if (qs[kSeedAhead - 1] < 0) break;  // (an empty slot: the list ends)
         }
         if (bq < 0) S.exhausted[p] = 1;  // no other component in the kNN list
     }
