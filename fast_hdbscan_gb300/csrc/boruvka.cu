@@ -758,7 +758,8 @@ __global__ void __launch_bounds__(kSW * 32) search_kernel(
                 int64_t node = 0;  // the node to expand
                 int at = 0;        // its depth
                 for (;;) {
-                    const int step = at == 0 && depth % kWideLevels ? depth % kWideLevels : kWideLevels;
+                    const int step =
+                        at == 0 && depth % kWideLevels ? depth % kWideLevels : kWideLevels;
                     const int64_t first = ((node + 1) << step) - 1;
                     if (at + step == depth) {
                         const int64_t group = (first - first_leaf_node) >> kWideLevels;
@@ -1200,8 +1201,10 @@ __global__ void finalize_edges_kernel(int64_t m, const int32_t* __restrict__ src
 }
 
 // Warps per bucket (or per 32 listed points), as for the kNN: with few of
-// them the latency of one walk is the search's time.
-constexpr int64_t kSearchWarpsWanted = 20 * 152;
+// them the latency of one walk is the search's time.  (All searches, ms with 20 /
+// 40 / 80 / 160 warps wanted per SM: 60k x 13-D 3.85 / 3.59 / 4.36 / 6.07, 200k x
+// 4-D 1.50 / 1.33 / 1.24 / 1.29, 20k x 2-D 0.142 / 0.131 / 0.139 / 0.162.)
+constexpr int64_t kSearchWarpsWanted = 40 * 152;
 int search_split(int64_t groups) {
     int split = 1;
     while (split < 32 && 2 * split * groups <= kSearchWarpsWanted) split *= 2;
@@ -1220,8 +1223,8 @@ int launch_search(Workspace& ws, const fhg_index& ix, const int8_t* knn_open, co
         Stage stage(s, "search_kernel");
         ::fhg::note_launch();
         search_kernel<DIM, SP><<<grid_for(groups * split, kSW), kSW * 32, 0, s>>>(
-            view_of(ix), knn_open, S.core2, S.comp, S.nc, S.keyA, S.cand_w, S.cand_q, pass, list, len,
-            S.ref_ties, split, S.stat);
+            view_of(ix), knn_open, S.core2, S.comp, S.nc, S.keyA, S.cand_w, S.cand_q, pass, list,
+            len, S.ref_ties, split, S.stat);
         FHG_CUDA(cudaGetLastError());
         return FHG_OK;
     };
