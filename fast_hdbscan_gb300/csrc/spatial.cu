@@ -1,7 +1,8 @@
 // Spatial index build: Hilbert keys -> radix sort -> median splits of chunks
-// (low dimensions) -> bucketed points -> bottom-up bounding boxes.  Replaces the reference's single-threaded
-// median-split KD-tree build (numba_kdtree.py:410-521); the tree here only
-// serves as a pruning structure, so its shape does not affect results.
+// (low dimensions) -> bucketed points -> bottom-up bounding boxes.  Replaces
+// the reference's single-threaded median-split KD-tree build
+// (numba_kdtree.py:410-521); the tree here only serves as a pruning structure,
+// so its shape does not affect results.
 #include "index.cuh"
 #include "primitives.cuh"
 
