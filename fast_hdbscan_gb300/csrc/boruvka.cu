@@ -1201,13 +1201,15 @@ __global__ void finalize_edges_kernel(int64_t m, const int32_t* __restrict__ src
 }
 
 // Warps per bucket (or per 32 listed points), as for the kNN: with few of
-// them the latency of one walk is the search's time.  (All searches, ms with 20 /
-// 40 / 80 / 160 warps wanted per SM: 60k x 13-D 3.85 / 3.59 / 4.36 / 6.07, 200k x
-// 4-D 1.50 / 1.33 / 1.24 / 1.29, 20k x 2-D 0.142 / 0.131 / 0.139 / 0.162.)
+// them the latency of one walk is the search's time.  Listed points, each
+// walking from the root, have the least to share and take twice as many.  (All
+// searches, ms with 20 / 40 / 80 / 160 warps wanted per SM: 60k x 13-D 3.85 / 3.59
+// / 4.36 / 6.07, 20k x 2-D 0.142 / 0.131 / 0.139 / 0.162; the lists alone, 40 / 80 /
+// 160: 200k x 4-D 1.35 / 1.24 / 1.33, 20k x 2-D 0.130 / 0.126 / 0.129.)
 constexpr int64_t kSearchWarpsWanted = 40 * 152;
-int search_split(int64_t groups) {
+int search_split(int64_t groups, int64_t wanted) {
     int split = 1;
-    while (split < 32 && 2 * split * groups <= kSearchWarpsWanted) split *= 2;
+    while (split < 32 && 2 * split * groups <= wanted) split *= 2;
     return split;
 }
 
@@ -1219,7 +1221,7 @@ int launch_search(Workspace& ws, const fhg_index& ix, const int8_t* knn_open, co
     cudaStream_t s = ws.stream();
     auto run = [&](int pass, const int32_t* list, int64_t len) -> int {
         const int64_t groups = list ? (len + 31) / 32 : ix.nleaves;
-        const int split = search_split(groups);
+        const int split = search_split(groups, list ? 2 * kSearchWarpsWanted : kSearchWarpsWanted);
         Stage stage(s, "search_kernel");
         ::fhg::note_launch();
         search_kernel<DIM, SP><<<grid_for(groups * split, kSW), kSW * 32, 0, s>>>(
