@@ -406,14 +406,15 @@ __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>()
 // list is the k smallest keys of all points and the tie flag has knn_kernel's
 // meaning, so both kernels give the same outputs bit for bit.
 //
-// What bounds it is instruction issue (75 % before and after).  Sorting each
+// What bounds it is instruction issue (75 % of the slots before).  Sorting each
 // bucket's candidates and merging them into a sorted list took most of it, one
-// node at a time most of the rest.  300k x 3-D, k = 101: 4.06 -> 1.94 ms.
-constexpr int kCutSlack = 16;
+// node at a time most of the rest.  300k x 3-D, k = 101: 4.06 -> 1.88 ms
+// (room for 64 / 96 / 160 / 256 keys between cuts: 2.11 / 1.95 / 1.88 / 1.93).
+constexpr int kCutSlack = 8;
 // An expansion leaves at most 31 nodes besides the one that goes on, and a tree
 // of 2^26 buckets has four expansions on a path.
 constexpr int kLargeStack = 5 * 32;
-constexpr int kLargeGrowth = 96;  // what a buffer takes between two cuts, at least
+constexpr int kLargeGrowth = 160;  // what a buffer takes between two cuts, at least
 __host__ __device__ constexpr int large_pow2(int k) {
     int p = 64;
     while (p < k) p *= 2;
