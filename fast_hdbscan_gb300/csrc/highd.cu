@@ -923,6 +923,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) hd_cand_tc_kernel(
                 acc[i] = __float_as_uint(e);
                 in |= (e < tq ? 1u : 0u) << i;
             }
+            // Columns past the points are never candidates: |y|^2 is infinite
+            // there, but beside a query or a product that is no number (rows near
+            // the largest float32) the sum is none either, and fmaxf makes it 0.
+            if (n - j0 < kTcChunk) in &= n > j0 ? (1u << (int)(n - j0)) - 1u : 0u;
             // a row whose buffer cannot take these is first cut back to its L
             // smallest (which only tightens its threshold)
             const unsigned rows = __ballot_sync(0xffffffffu, cnt + __popc(in) > cap);

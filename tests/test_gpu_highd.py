@@ -162,3 +162,22 @@ def test_tcgen05_tiles_and_thresholds_equal_oracle(engine, n, d, k):
     rd_o, ix_o = O.tree_query(O.build_kdtree(X), k, mode=1, nthreads=NTH)
     np.testing.assert_array_equal(ix, ix_o)
     np.testing.assert_array_equal(rd, rd_o)
+
+
+@pytest.mark.parametrize("n,d,k", [(1000, 40, 5), (4201, 33, 31), (4097, 64, 16)])
+def test_rows_near_the_largest_float_equal_brute_force(engine, n, d, k):
+    """Finite rows whose bfloat16 parts are infinite give estimates that are no
+    numbers, in the columns past the last point too: these are no candidates."""
+    rng = np.random.default_rng(n)
+    X = rng.normal(size=(n, d)).astype(np.float32)
+    big = np.finfo(np.float32).max
+    X[[3, n // 3, n // 2, n - 1]] = np.array([[big], [-big], [big], [-big]], np.float32)
+    rd, ix, _ = _highd(X, k)
+    with np.errstate(over="ignore"):
+        for i in np.concatenate([[3, n // 3, n // 2, n - 1], rng.choice(n, 60, replace=False)]):
+            dd = np.zeros(n, np.float32)
+            for j in range(d):
+                dd += (X[i, j] - X[:, j]) ** 2
+            order = np.lexsort((np.arange(n), dd))[:k]
+            np.testing.assert_array_equal(ix[i], order)
+            np.testing.assert_array_equal(rd[i], dd[order])
