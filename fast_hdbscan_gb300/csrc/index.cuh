@@ -102,6 +102,11 @@ __device__ __forceinline__ void load_box(const float* __restrict__ box, int64_t 
     }
 }
 
+// A box without points (lo = +inf, hi = -inf): its bound to any point is +inf,
+// which a box of points can have too, when squared distances overflow.
+template <int SP>
+__device__ __forceinline__ bool box_empty(const float* box) { return box[0] > box[SP]; }
+
 int index_build(const float* X, int64_t n, int32_t d, cudaStream_t s, fhg_index** out);
 int index_free(fhg_index* ix, cudaStream_t s);
 

@@ -198,6 +198,16 @@ __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>()
     int sp = 0;
     bool right_side = false;
     float later_lb = 0.0f;
+    // Slots past the last bucket have boxes without points, whose bound, +inf, is
+    // within reach of a list that is not full yet, or holds points at infinite
+    // (overflowed) distances: only then are nodes looked at for it.  (2^20 + 1
+    // points, whose last bucket holds one, scanned every empty slot: 131 ms.)
+    bool unfilled = true;
+    auto empty = [&](int32_t v) {
+        float b[2 * SP];
+        load_box<SP>(ix.box, v, b);
+        return box_empty<SP>(b);
+    };
     int64_t lf = leaf;  // the bucket to scan, -1 when the walk has ended
     bool need = valid;
     for (bool home = true;; home = false) {
@@ -305,6 +315,7 @@ __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>()
                     merge8<K>(key, v, rejected);
                 }
                 if (valid) thr = entry_dist(key[K - 1]);
+                unfilled = __any_sync(kFull, thr == INFINITY);
                 __syncwarp();
             }
             if (room) break;
@@ -328,7 +339,7 @@ __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>()
                 float b[2 * SP];
                 load_box<SP>(ix.box, node, b);
                 need = box_lb_n<DIM, SP>(b, q) <= thr;
-                if (!__any_sync(kFull, need)) continue;
+                if (!__any_sync(kFull, need) || (unfilled && empty(node))) continue;
                 if (node >= first_leaf_node) {
                     lf = node - first_leaf_node;
                     break;
@@ -344,7 +355,11 @@ __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>()
                 load_box<SP>(ix.box, nearc, bn);
                 load_box<SP>(ix.box, farc, bf);
                 const float lbn = box_lb_n<DIM, SP>(bn, q), lbf = box_lb_n<DIM, SP>(bf, q);
-                const bool an = __any_sync(kFull, lbn <= thr), af = __any_sync(kFull, lbf <= thr);
+                bool an = __any_sync(kFull, lbn <= thr), af = __any_sync(kFull, lbf <= thr);
+                if (unfilled) {
+                    an = an && !empty(nearc);
+                    af = af && !empty(farc);
+                }
                 if (!an && !af) break;
                 if (l >= first_leaf_node) {
                     lf = (an ? nearc : farc) - first_leaf_node;

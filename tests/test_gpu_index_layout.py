@@ -111,3 +111,61 @@ def test_condense_segments_vs_oracle(engine, n, mcs):
     got, expect = condense_tree(linkage, min_cluster_size=mcs), O.condense_tree(linkage, mcs)
     for a, b in zip(got, expect):
         np.testing.assert_array_equal(a, b)
+
+
+def _far_groups(n, d, far, seed):
+    """n points, `far` of them 1e20 from the rest: finite rows whose squared
+    distances overflow float32."""
+    X = np.random.default_rng(seed).normal(size=(n, d)).astype(np.float32)
+    X[-far:, 0] += np.float32(1e20)
+    return X[np.random.default_rng(seed + 1).permutation(n)]
+
+
+@pytest.mark.parametrize("n,far", [(65, 3), (90, 5), (129, 64), (1000, 7), (2049, 20),
+                                   (4097, 2000), (5000, 9)])
+@pytest.mark.parametrize("d", [1, 3, 5, 7, 20])
+@pytest.mark.parametrize("k", [2, 11, 24, 40])
+def test_knn_at_infinite_distances_vs_oracle(engine, n, far, d, k):
+    """Lists that must be filled with points at infinite distances, where the
+    tree has slots without points: by index, each point once."""
+    from fast_hdbscan_gb300.numba_kdtree import build_kdtree, parallel_tree_query
+    from oracle import oracle as O
+
+    X = _far_groups(n, d, far, 10 * n + d)
+    tree = build_kdtree(X)
+    rd, ix = parallel_tree_query(tree, tree.data, k=k, output_rdist=True)
+    ord_, oix = O.tree_query(O.build_kdtree(X), k, mode=1)
+    np.testing.assert_array_equal(rd, ord_)
+    np.testing.assert_array_equal(ix, oix)
+
+
+def test_knn_does_not_scan_empty_slots(engine):
+    """One point in the last bucket, beside as many slots without points as the
+    tree can have: the walk that fills its list costs no more than others."""
+    import ctypes
+
+    import torch
+
+    from fast_hdbscan_gb300 import _native
+
+    V, lib, k = _native.vptr, _native.load(), 16
+
+    def knn_ms(n):
+        g = torch.Generator(device="cuda").manual_seed(3)
+        X = torch.randn(n, 3, generator=g, device="cuda")
+        rd = torch.empty(n, k, device="cuda")
+        ix = torch.empty(n, k, dtype=torch.int32, device="cuda")
+        h = ctypes.c_void_p()
+        _native.check(lib.fhg_index_build(V(X), n, 3, _native.stream_ptr(), ctypes.byref(h)))
+        times = []
+        for _ in range(4):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            _native.check(lib.fhg_index_knn(h, k, V(rd), V(ix), _native.stream_ptr()))
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        _native.check(lib.fhg_index_free(h, _native.stream_ptr()))
+        return min(times)
+
+    assert knn_ms(2**20 + 1) < 3 * knn_ms(2**20)
