@@ -706,8 +706,11 @@ __global__ void __launch_bounds__(kSW * 32) search_kernel(
                     __reduce_max_sync(kFull, S.active ? __float_as_uint(S.thr) : 0u));
             };
             float T = largest_thr();
-            auto box_key = [&](int64_t node, int2 ncn) {  // lane's node against the points' box
-                if (ncn.x == kEmpty || ncn.x == c0 || __int_as_float(ncn.y) > T) return INFINITY;
+            // Lane's node against the points' box; NaN for a node to leave out (+inf is
+            // a bound like any other: squared distances overflow, core distances
+            // are infinite where there are fewer points than neighbours).
+            auto box_key = [&](int64_t node, int2 ncn) {
+                if (ncn.x == kEmpty || ncn.x == c0 || __int_as_float(ncn.y) > T) return NAN;
                 float b[2 * SP];
                 load_box<SP>(ix.box, node, b);
                 float r = 0.0f;
@@ -726,12 +729,12 @@ __global__ void __launch_bounds__(kSW * 32) search_kernel(
                 const int size = ix.slots < 32 ? (int)ix.slots : 32;
                 const int64_t node = first_leaf_node + group * 32 + lane;
                 int2 ncn = make_int2(kEmpty, 0);
-                float key = INFINITY;
+                float key = NAN;
                 if (lane < size) {
                     ncn = nc[node];
                     key = box_key(node, ncn);
                 }
-                unsigned left = __ballot_sync(kFull, key <= T && key < INFINITY);
+                unsigned left = __ballot_sync(kFull, key <= T);
                 while (left) {
                     const uint32_t mine = (left >> lane) & 1u ? __float_as_uint(key) : 0xffffffffu;
                     const uint32_t least = __reduce_min_sync(kFull, mine);
@@ -766,9 +769,9 @@ __global__ void __launch_bounds__(kSW * 32) search_kernel(
                         if (group != home_group) scan_group(group);
                     } else {
                         const int64_t mine = first + lane;
-                        float key = INFINITY;
+                        float key = NAN;
                         if (lane < (1 << step)) key = box_key(mine, nc[mine]);
-                        const unsigned in = __ballot_sync(kFull, key <= T && key < INFINITY);
+                        const unsigned in = __ballot_sync(kFull, key <= T);
                         if (in) {  // the nearest on top of the stack
                             const bool on = (in >> lane) & 1u;
                             const uint32_t bits = on ? __float_as_uint(key) : 0xffffffffu;

@@ -128,3 +128,27 @@ def test_boruvka_vs_oracle_synthetic(engine, gen, n, ms):
     np.testing.assert_array_equal(core, oc)
     np.testing.assert_array_equal(nbrs, onb)
     np.testing.assert_array_equal(edges, oe)
+
+
+@pytest.mark.parametrize("sizes", [(64, 64), (32, 96), (33, 90), (1, 2, 130), (700, 300, 64),
+                                   (4096, 4000), (6000, 5000), (8192, 4096, 32), (11_000, 7)])
+@pytest.mark.parametrize("d", [1, 3, 7, 20])
+@pytest.mark.parametrize("ms", [1, 5, 20])
+def test_boruvka_across_infinite_distances(engine, sizes, d, ms):
+    """Groups of finite points 1e20 apart, whose squared distances overflow:
+    joined by edges of infinite weight, in the oracle's order, whether one
+    bucket holds points of two groups or none does."""
+    from fast_hdbscan_gb300.numba_kdtree import build_kdtree
+    from fast_hdbscan_gb300.boruvka import parallel_boruvka
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(sum(sizes) + d)
+    X = np.concatenate([rng.normal(size=(m, d)) + 1e20 * i * np.eye(1, d)
+                        for i, m in enumerate(sizes)])
+    X = rng.permutation(X).astype(np.float32)
+    edges, nbrs, core = parallel_boruvka(build_kdtree(X), 1, min_samples=ms)
+    oe, onb, oc, _ = O.parallel_boruvka(O.build_kdtree(X), ms, mode=1)
+    assert np.isinf(oe[:, 2]).sum() >= len(sizes) - 1
+    np.testing.assert_array_equal(edges, oe)
+    np.testing.assert_array_equal(nbrs, onb)
+    np.testing.assert_array_equal(core, oc)
