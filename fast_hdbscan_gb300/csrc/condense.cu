@@ -34,17 +34,20 @@ __device__ __forceinline__ float lambda_of(double d) {
 }
 
 // Per internal node: case, lambda, and the child flags written into the
-// node-indexed arrays of its two children.
+// node-indexed arrays of its two children.  *odd is cleared when a node's size
+// is not the sum of its children's.
 __global__ void cases_kernel(int64_t m, int64_t n, const int32_t* __restrict__ left,
                              const int32_t* __restrict__ right, const double* __restrict__ w,
                              const int32_t* __restrict__ size, const float* __restrict__ wsize,
                              double mcs, double max_cs, int8_t* __restrict__ kase,
                              float* __restrict__ lam,
                              int32_t* __restrict__ par, int8_t* __restrict__ cont,
-                             int8_t* __restrict__ birth, int8_t* __restrict__ side) {
+                             int8_t* __restrict__ birth, int8_t* __restrict__ side,
+                             int32_t* __restrict__ odd) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     const int32_t L = left[i], R = right[i];
+    if ((int64_t)size[n + i] != (int64_t)size[L] + size[R]) *odd = 0;
     // counts: leaves, or the points' sample weights (cluster_trees.py:253-262)
     const double lc = wsize ? (double)wsize[L] : (double)(float)size[L];
     const double rc = wsize ? (double)wsize[R] : (double)(float)size[R];
@@ -140,8 +143,8 @@ __global__ void pj_step_kernel(int64_t m, const PjRec* __restrict__ R, PjRec* __
     pj_store(R2, i, x);
 }
 
-// node_at: the node at every place of the preorder (-1 where the sizes given
-// with a linkage tree are not its own and leave or overstep a place).
+// node_at: the node at every place of the preorder (sizes given with a linkage
+// tree that are not its own leave or overstep places: condense_tree starts over).
 __global__ void pj_split_kernel(int64_t m, int64_t n, const PjRec* __restrict__ R,
                                 int32_t* __restrict__ dep, int64_t* __restrict__ pre,
                                 int32_t* __restrict__ top, int32_t* __restrict__ bth,
@@ -383,6 +386,13 @@ constexpr int64_t kCountedRun = 512;
         }                                                                   \
     } while (0)
 
+// Sizes as the weights that the cases go by.
+__global__ void sizes_as_weights_kernel(int64_t nodes, const int32_t* __restrict__ size,
+                                        float* __restrict__ wsize) {
+    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v < nodes) wsize[v] = (float)size[v];
+}
+
 template <class T>
 int read1(const T* dev, T* host, cudaStream_t s) {
     FHG_CUDA(cudaMemcpyAsync(host, dev, sizeof(T), cudaMemcpyDeviceToHost, s));
@@ -411,16 +421,19 @@ int condense_tree(Workspace& ws, const Linkage& lk, int64_t mcs, double max_cs, 
     FHG_TRY(ws.alloc(&cont, (size_t)nodes));
     FHG_TRY(ws.alloc(&birth, (size_t)nodes));
     FHG_TRY(ws.alloc(&side, (size_t)nodes));
+    // the nodes in preorder, a flag (-1: every size is its children's sum) and the
+    // number of reached nodes
+    FHG_TRY(ws.alloc(&node_at, (size_t)(nodes + 2)));
+    int32_t* odd = node_at + nodes;
+    FHG_CUDA(cudaMemsetAsync(node_at, 0xff, sizeof(int32_t) * (nodes + 1), s));
     LAUNCH(cases_kernel, m, m, n, lk.left, lk.right, lk.w, lk.size, lk.wsize, (double)mcs, max_cs,
            kase, lam,
-           par, cont, birth, side);
+           par, cont, birth, side, odd);
 
     FHG_TRY(ws.alloc(&dep, (size_t)m));
     FHG_TRY(ws.alloc(&pre, (size_t)m));
     FHG_TRY(ws.alloc(&top, (size_t)m));
     FHG_TRY(ws.alloc(&bth, (size_t)m));
-    FHG_TRY(ws.alloc(&node_at, (size_t)nodes));
-    FHG_CUDA(cudaMemsetAsync(node_at, 0xff, sizeof(int32_t) * nodes, s));
     {
         Workspace tmp(ws);
         PjRec *R, *R2;
@@ -454,15 +467,30 @@ int condense_tree(Workspace& ws, const Linkage& lk, int64_t mcs, double max_cs, 
 
     // ---- reached internal nodes in breadth-first order: by depth, stably from
     // the preorder
-    uint32_t *cnt_dev, *kd;
+    uint32_t* kd;
     int32_t *reached, *bfs_pos, *label;
-    FHG_TRY(ws.alloc(&cnt_dev, 2));
     FHG_TRY(ws.alloc(&reached, (size_t)m));
     FHG_TRY(ws.alloc(&kd, (size_t)m));
-    FHG_TRY(compact(ws, ReachedNodes{n, node_at, top, dep, reached, kd}, nodes, cnt_dev));
-    uint32_t h_cnt = 0;
-    FHG_TRY(read1(cnt_dev, &h_cnt, s));
-    const int64_t cnt = h_cnt;
+    FHG_TRY(compact(ws, ReachedNodes{n, node_at, top, dep, reached, kd}, nodes,
+                    reinterpret_cast<uint32_t*>(odd + 1)));
+    int2 h_cnt = make_int2(0, 0);
+    FHG_CUDA(cudaMemcpyAsync(&h_cnt, odd, sizeof(h_cnt), cudaMemcpyDeviceToHost, s));
+    FHG_CUDA(cudaStreamSynchronize(s));
+    if (h_cnt.x != -1) {
+        // Sizes of the caller's (weight sums without their weights, say): the
+        // cases and the rows' sizes go by them, as the reference's do, but places
+        // and numbers of rows by the leaves that there are.
+        if (lk.wsize) {
+            set_error("condense: the linkage is not a tree over its points");
+            return FHG_ERR_INVALID;
+        }
+        Linkage own = lk;
+        FHG_TRY(ws.alloc(&own.wsize, (size_t)nodes));
+        LAUNCH(sizes_as_weights_kernel, nodes, nodes, lk.size, own.wsize);
+        FHG_TRY(linkage_leaf_counts(ws, own));
+        return condense_tree(ws, own, mcs, max_cs, out);
+    }
+    const int64_t cnt = h_cnt.y;
     // (every node above a reached one is reached: no depth is cnt or more)
     FHG_TRY(radix_sort_u32(ws, kd, reached, cnt, 0, bits_for(cnt)));
     int64_t *count, *off, *tot;

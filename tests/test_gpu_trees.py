@@ -227,3 +227,29 @@ def test_linkage_intervals_vs_oracle(engine, m, shape):
     mst = np.stack([relabel[parent], relabel[child], w], axis=1).astype(np.float64)
     mst = mst[np.argsort(w, kind="stable")]
     np.testing.assert_array_equal(mst_to_linkage_tree(mst), O.mst_to_linkage_tree(mst))
+
+
+@pytest.mark.parametrize("kind", ["weights", "random", "root", "zero", "large"])
+@pytest.mark.parametrize("n", [40, 3000, 20_000])
+@pytest.mark.parametrize("mcs", [2, 5, 40, 600])
+def test_condense_sizes_that_are_no_counts(engine, kind, n, mcs):
+    """A linkage tree whose size column is not the number of leaves (weight
+    sums condensed without their weights, among others): the cases go by it,
+    the rows by the points that there are, as in the reference."""
+    from fast_hdbscan_gb300.cluster_trees import condense_tree
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(n + mcs)
+    child = np.arange(1, n)
+    parent = np.where(rng.random(n - 1) < 0.5, child - 1, (rng.random(n - 1) * child).astype(int))
+    w = np.sort(rng.integers(1, n, size=n - 1).astype(np.float64))
+    mst = np.stack([parent, child, rng.permutation(w)], axis=1).astype(np.float64)
+    weights = rng.integers(1, 5, size=n).astype(np.float32)
+    linkage = O.mst_to_linkage_tree(O.sort_mst(mst), weights if kind == "weights" else None)
+    size = linkage[:, 3]
+    linkage[:, 3] = {"weights": size, "random": size * rng.integers(1, 4, size=n - 1),
+                     "root": np.where(np.arange(n - 1) == n - 2, 3, size),
+                     "zero": 0 * size, "large": size + 1000}[kind]
+    got, expect = condense_tree(linkage, min_cluster_size=mcs), O.condense_tree(linkage, mcs)
+    for a, b in zip(got, expect):
+        np.testing.assert_array_equal(a, b)
