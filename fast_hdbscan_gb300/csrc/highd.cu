@@ -562,7 +562,7 @@ __global__ void hd_mark_means_kernel(int marks, int d, int64_t stride,
 __global__ void __launch_bounds__(kLandmarks) hd_chain_kernel(int marks, int d,
                                                               const float* __restrict__ C,
                                                               uint32_t* __restrict__ place) {
-    __shared__ float s_cur[kHighdMaxDim];
+    __shared__ __align__(16) float s_cur[kHighdMaxDim];
     __shared__ uint32_t s_best[kLandmarks / 32];
     const int m = threadIdx.x;
     float own[kHighdMaxDim];

@@ -247,3 +247,20 @@ def test_ctypes_signatures_match_the_header():
         assert _c_kind(ret + " x") == _ctypes_kind(restype), name
         checked += 1
     assert checked == len(_native.SIGNATURES)
+
+
+def test_shared_arrays_read_as_vectors_are_aligned():
+    """A shared array that a kernel reads or writes through a wider vector type
+    says so in its declaration: nothing else puts it on such a boundary."""
+    src = os.path.join(ROOT, "fast_hdbscan_gb300", "csrc")
+    vector = r"reinterpret_cast<(?:const\s+)?(?:float|int|uint)[24]\s*\*>\(\s*&?(\w+)"
+    checked = 0
+    for fn in sorted(os.listdir(src)):
+        text = open(os.path.join(src, fn)).read()
+        wide = set(re.findall(vector, text))
+        for align, names in re.findall(r"__shared__\s+(__align__\(\d+\)\s+)?\w+\s+([^;]*);", text):
+            for name in re.findall(r"(\w+)\s*\[", names):
+                if name in wide:
+                    checked += 1
+                    assert align, "%s: %s" % (fn, name)
+    assert checked
