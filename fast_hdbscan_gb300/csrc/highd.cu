@@ -893,11 +893,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) hd_cand_tc_kernel(
             return __fsub_rn(__fadd_rn(nq, hmin), __fmul_rn(2.0f, dmax));
         };
         // The warm-up keeps the least estimate of every 16 columns of the tiles
-        // around the query, 64 in all, in the row's buffer: the k + 2 smallest of
-        // them lie below the first threshold, so no row is left short of k
-        // candidates, and the buffer fills once instead of with every estimate
-        // that is among the least so far (150k x 64-D: 9.3 ms; with the k + 10
-        // smallest of 64 in half the tiles 11.4, the k + 2 smallest there 9.9).
+        // around the query, 64 in all, in the row's buffer, and takes the (k + 2)nd
+        // smallest (at most the 56th) as the first threshold, so that the buffer
+        // fills once instead of with every estimate that is among the least so far
+        // (150k x 64-D: 9.3 ms; with the k + 10 smallest of 64 in half the tiles
+        // 11.4, the k + 2 smallest there 9.9).  Nearly always at least k points lie
+        // below it; where fewer do (equal estimates at the threshold), the row has
+        // no certificate and is searched exactly, as for any other reason.
         auto look = [&](const uint32_t (&acc)[kTcChunk], const float* h) {
             float m[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
 #pragma unroll

@@ -181,3 +181,24 @@ def test_rows_near_the_largest_float_equal_brute_force(engine, n, d, k):
             order = np.lexsort((np.arange(n), dd))[:k]
             np.testing.assert_array_equal(ix[i], order)
             np.testing.assert_array_equal(rd[i], dd[order])
+
+
+@pytest.mark.parametrize("n,d,k", [(4096, 64, 1), (4097, 63, 31), (6001, 32, 56), (4100, 64, 48)])
+def test_first_thresholds_leave_rows_certified(engine, n, d, k):
+    """A first threshold that cut off candidates would show in the rows that
+    are searched again, not in the lists.  Both kernels certify a row by its
+    L-th smallest estimate, computed from the same products: only rows within
+    rounding of the bound may differ, 1 % of them at most."""
+    from fast_hdbscan_gb300 import _native
+
+    X = synthetic.aniso_highdim(n=n, seed=70 + d, dim=d, n_comp=5)
+    X[: n // 20] = X[0] * 3 + 0.01 * X[: n // 20]
+    lib = _native.load()
+    _, _, fb_tc = _highd(X, k)
+    lib.fhg_set_highd_kernel(1)
+    try:
+        _, _, fb_ms = _highd(X, k)
+    finally:
+        lib.fhg_set_highd_kernel(0)
+    print("n=%d d=%d k=%d: fallbacks tcgen05 %d, mma.sync %d" % (n, d, k, fb_tc, fb_ms))
+    assert fb_tc <= fb_ms + n // 100
