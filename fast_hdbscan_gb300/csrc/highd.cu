@@ -925,10 +925,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) hd_cand_tc_kernel(
                 acc[i] = __float_as_uint(e);
                 in |= (e < tq ? 1u : 0u) << i;
             }
-            // Columns past the points are never candidates: |y|^2 is infinite
-            // there, but beside a query or a product that is no number (rows near
-            // the largest float32) the sum is none either, and fmaxf makes it 0.
-            if (n - j0 < kTcChunk) in &= n > j0 ? (1u << (int)(n - j0)) - 1u : 0u;
             // a row whose buffer cannot take these is first cut back to its L
             // smallest (which only tightens its threshold)
             const unsigned rows = __ballot_sync(0xffffffffu, cnt + __popc(in) > cap);
@@ -995,7 +991,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) hd_cand_tc_kernel(
             }
             tc::mbar_arrive(&nempty[u]);  // this tile's record is read
         }
-        // L of the smallest estimates of every row, and its L-th estimate
+        // L of the smallest estimates of every row, and its L-th estimate.  Columns
+        // past the points have an infinite |y|^2; they join a list only where a query
+        // is no number (a row near the largest float32, its bfloat16 parts infinite),
+        // whose estimates fmaxf makes 0.  Such entries are left out here, and the
+        // certificate holds for no row then: the largest |y| is no number either.
+        // (Masked where they join instead: 1 % of the kernel.)
         cut(__ballot_sync(0xffffffffu, cnt >= L), L, 0);
         __syncwarp();
         for (int rr = 0; rr < 32; ++rr) {
@@ -1005,8 +1006,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) hd_cand_tc_kernel(
             const int64_t qr = q0 + quarter * 32 + rr;
             if (qr < n) {
                 const int64_t qq = perm[qr];
-                for (int e2 = lane; e2 < L; e2 += 32)
-                    cand[qq * L + e2] = e2 < kept ? perm[(uint32_t)rb[e2]] : -1;
+                for (int e2 = lane; e2 < L; e2 += 32) {
+                    const uint32_t at = (uint32_t)rb[e2];
+                    cand[qq * L + e2] = e2 < kept && at < n ? perm[at] : -1;
+                }
                 if (lane == 0) T[qq] = last;
             }
         }
