@@ -35,6 +35,16 @@ constexpr int kTransposeMax = 16;
 // larger lists take what they need.
 template <int DIM, int K>
 constexpr int knn_min_blocks() { return K > 16 || DIM > 8 ? 1 : DIM <= 4 ? 6 : 5; }
+// Candidates at a lane's k-th distance that come after its k-th entry never join
+// its list.  A few of them cost least where they are queued and merged like the
+// others, but among many equal points a bucket holds nothing else.  Scans query
+// by query drop them where a queue would overflow; the others drop each of them
+// for lists of up to 24 (2 % of the kernel at 10M x 3-D; for 64 it would be 7).
+// 300 points 1,000 times each, k = 6 / 16 / 24 / 40, ms: 0.71 / 1.16 / 1.87 / 5.6
+// by insertion one by one, 2.2 / 3.5 / 3.9 / 8.9 queued and merged, 0.93 / 1.20 /
+// 1.55 / 4.6 here.  (20,000 equal points, k = 6 / 31: 2.5 / 7.2, 23 / 52, 6.1 /
+// 9.4: every bucket before the query's replaces its whole list.)
+constexpr int kDropLateMax = 24;
 // A lane's queue of candidates not yet in its list (see knn_kernel): the fill
 // at which the warp empties its queues, and the row stride (odd, in 8-byte
 // words: no bank conflicts across lanes).
@@ -120,6 +130,7 @@ __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>()
                const uint8_t* __restrict__ redo, uint8_t* __restrict__ fail,
                unsigned long long* fail_count, unsigned long long* scan_count, int split) {
     constexpr int kKnnWarps = knn_warps<SP>();
+    constexpr bool kDropLate = K <= kDropLateMax;
     __shared__ float4 s_cand[kKnnWarps][32 * (SP / 4)];
     __shared__ float4 s_query[kKnnWarps][32 * (SP / 4)];
     __shared__ int32_t s_corig[kKnnWarps][32];
@@ -236,8 +247,9 @@ __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>()
             corig[lane] = own_o;
             __syncwarp();
         }
-        unsigned open = cnt >= 32 ? kFull : (1u << cnt) - 1u;  // candidates of the current query
-        const unsigned every = open;
+        const unsigned every = cnt >= 32 ? kFull : (1u << cnt) - 1u;
+        unsigned left = 0;    // by_query: candidates this lane's query had no room for,
+        bool again = false;   // and whether these are looked at now
         int t0 = 0;
         // the queues are emptied at a fill of kQueueFull; after the home
         // bucket and at the end always
@@ -246,9 +258,12 @@ __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>()
             bool room = true;  // false: a queue must be emptied to go on
             if (by_query) {
                 // Few lanes need the bucket: each lane takes its own candidate
-                // and the warp visits only the needing queries.
+                // and the warp visits only the needing queries.  What a query's
+                // queue has no room for waits until all queues are emptied.
+                unsigned more = 0;
                 while (todo) {
                     const int i = __ffs(todo) - 1;
+                    todo &= todo - 1u;
                     float y[SP];
 #pragma unroll
                     for (int h = 0; h < SP / 4; ++h) {
@@ -257,26 +272,34 @@ __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>()
                     }
                     const float lim = __shfl_sync(kFull, thr, i);
                     const float dd = rdist_rn<DIM>(y, own);
-                    unsigned in = __ballot_sync(kFull, dd <= lim) & open;
-                    if (in) {
-                        const int have = __shfl_sync(kFull, waiting, i);
-                        if (have + __popc(in) > kQueue) {
-                            room = false;
-                            if (have > 0) break;
-                            if (in & 0xffffu) in &= 0xffffu;  // at most 16 at a time
+                    unsigned in = __ballot_sync(kFull, dd <= lim);
+                    if (!in) continue;
+                    in &= again ? __shfl_sync(kFull, left, i) : every;
+                    const int have = __shfl_sync(kFull, waiting, i);
+                    int place = have + __popc(in & ((1u << lane) - 1u));
+                    if (have + __popc(in) > kQueue) {
+                        // Many at once, mostly at equal distances: at the k-th only
+                        // candidates before the k-th entry join, and what then has
+                        // no room waits.
+                        const int32_t last = __shfl_sync(kFull, entry_orig(key[K - 1]), i);
+                        const unsigned late = __ballot_sync(kFull, dd == lim && own_o > last) & in;
+                        in &= ~late;
+                        place = have + __popc(in & ((1u << lane) - 1u));
+                        const unsigned fit = __ballot_sync(kFull, place < kQueue) & in;
+                        if (lane == i) {
+                            left = in & ~fit;
+                            if (late) rejected = min(rejected, pack_entry(lim, 0));
                         }
-                        if ((in >> lane) & 1u)
-                            queue[i * kQueueStride + have + __popc(in & ((1u << lane) - 1u))] =
-                                pack_entry(dd, own_o);
-                        if (lane == i) waiting += __popc(in);
-                        if (!room) {
-                            open &= ~in;
-                            break;
-                        }
+                        if (in != fit) more |= 1u << i;
+                        in = fit;
                     }
-                    open = every;
-                    todo &= todo - 1u;
+                    if ((in >> lane) & 1u)
+                        queue[i * kQueueStride + place] = pack_entry(dd, own_o);
+                    if (lane == i) waiting += __popc(in);
                 }
+                todo = more;
+                again = true;
+                room = more == 0;
             } else {
                 // Every lane reads candidate t from shared memory.
                 const float lim = need ? thr : -1.0f;
@@ -294,8 +317,15 @@ __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>()
                             c[4 * h + 2] = v.z; c[4 * h + 3] = v.w;
                         }
                         const float dd = rdist_rn<DIM>(q, c);
-                        if (dd <= lim && t < cnt)
-                            queue[lane * kQueueStride + waiting++] = pack_entry(dd, corig[t]);
+                        if (dd <= lim && t < cnt) {
+                            const unsigned long long e = pack_entry(dd, corig[t]);
+                            queue[lane * kQueueStride + waiting] = e;
+                            if (!kDropLate || dd < lim ||
+                                entry_orig(e) < entry_orig(key[K - 1]))
+                                ++waiting;
+                            else
+                                rejected = min(rejected, e);
+                        }
                     }
                 }
             }

@@ -169,3 +169,57 @@ def test_knn_does_not_scan_empty_slots(engine):
         return min(times)
 
     assert knn_ms(2**20 + 1) < 3 * knn_ms(2**20)
+
+
+@pytest.mark.parametrize("n", [70, 3000, 50_000])
+@pytest.mark.parametrize("copies", [20, 200])
+@pytest.mark.parametrize("order", ["together", "mixed"])
+@pytest.mark.parametrize("k", [2, 8, 11, 16, 24, 31, 40, 64])
+def test_knn_among_equal_points_vs_oracle(engine, n, copies, order, k):
+    """Buckets of nothing but equal points: more candidates at once than a
+    query's queue has room for, before and after its list."""
+    from fast_hdbscan_gb300.numba_kdtree import build_kdtree, parallel_tree_query
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(n + copies + k)
+    d = 2 + k % 5
+    X = np.repeat(rng.normal(size=(n // copies + 1, d)), copies, axis=0)[:n].astype(np.float32)
+    if order == "mixed":
+        X = X[rng.permutation(n)]
+    tree = build_kdtree(X)
+    rd, ix = parallel_tree_query(tree, tree.data, k=k, output_rdist=True)
+    ord_, oix = O.tree_query(O.build_kdtree(X), k, mode=1)
+    np.testing.assert_array_equal(rd, ord_)
+    np.testing.assert_array_equal(ix, oix)
+
+
+def test_knn_time_among_equal_points(engine):
+    """Equal points cost what their distances cost, not a merge for every eight
+    that could join no list (7.5 times the kNN of distinct points before)."""
+    import torch
+
+    from fast_hdbscan_gb300 import _native
+
+    V, lib, k, n = _native.vptr, _native.load(), 16, 300_000
+
+    def knn_ms(X):
+        import ctypes
+
+        rd = torch.empty(n, k, device="cuda")
+        ix = torch.empty(n, k, dtype=torch.int32, device="cuda")
+        h = ctypes.c_void_p()
+        _native.check(lib.fhg_index_build(V(X), n, 3, _native.stream_ptr(), ctypes.byref(h)))
+        times = []
+        for _ in range(5):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            _native.check(lib.fhg_index_knn(h, k, V(rd), V(ix), _native.stream_ptr()))
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        _native.check(lib.fhg_index_free(h, _native.stream_ptr()))
+        return min(times)
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    X = torch.randn(n, 3, generator=g, device="cuda")
+    assert knn_ms(X[:300].repeat_interleave(1000, 0).contiguous()) < 4.5 * knn_ms(X)
