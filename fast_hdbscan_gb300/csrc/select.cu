@@ -106,12 +106,15 @@ __global__ void products_kernel(int64_t rows, const uint32_t* __restrict__ key,
     if (j == 0 || key[j - 1] != c) start[c] = j;
     if (j + 1 == rows || key[j + 1] != c) end[c] = j + 1;
 }
-// One warp per cluster: the float32 sum of its rows' products, strictly in row
-// order (a float32 sum is not associative, so the order is the result).  The
+// The float32 sum of a cluster's products, strictly in row order (a float32 sum
+// is not associative, so the order is the result): one warp per cluster.  The
 // lanes read 32 products together, the next ones while these are added, and all
 // add the same chain; a thread per cluster waited for each of its loads (1M
 // points, min_cluster_size 500: 218 -> 29 us).  Clusters of kBigRows rows or
-// more are summed by score_big_kernel.
+// more are summed by score_big_kernel.  Above kScoreWarps clusters a warp takes
+// 32 of them, a lane each where they have up to kLaneRows rows: most are small
+// then, and a warp for each leaves its lanes idle (1M clusters of 10 rows on
+// average: 286 -> 24 us).
 constexpr int32_t kBigRows = 2048;
 __device__ __forceinline__ float score_start(int64_t c, const int32_t* __restrict__ row_of_cluster,
                                              const float* __restrict__ lam,
@@ -123,21 +126,12 @@ __device__ __forceinline__ float score_start(int64_t c, const int32_t* __restric
     }
     return s;
 }
-__global__ void score_kernel(int64_t C, const int64_t* __restrict__ start,
-                             const int64_t* __restrict__ end, const float* __restrict__ prod,
-                             const int32_t* __restrict__ row_of_cluster,
-                             const float* __restrict__ lam, const float* __restrict__ csize,
-                             float* __restrict__ score) {
-    const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// s + v[0] + v[1] + ... + v[len - 1] by one warp.
+__device__ __forceinline__ float warp_sum(float s, const float* __restrict__ p, int len) {
     const int lane = threadIdx.x & 31;
-    if (c >= C) return;
-    const int64_t b = start[c];
-    const int len = (int)min(end[c] - b, (int64_t)kBigRows);
-    if (len >= kBigRows) return;
-    float s = score_start(c, row_of_cluster, lam, csize);
-    float v = lane < len ? __ldg(prod + b + lane) : 0.0f;
+    float v = lane < len ? __ldg(p + lane) : 0.0f;
     for (int j = 0; j < len; j += 32) {
-        const float next = j + 32 + lane < len ? __ldg(prod + b + j + 32 + lane) : 0.0f;
+        const float next = j + 32 + lane < len ? __ldg(p + j + 32 + lane) : 0.0f;
         if (len - j >= 32) {
 #pragma unroll
             for (int u = 0; u < 32; ++u) s = __fadd_rn(s, __shfl_sync(kFull, v, u));
@@ -146,7 +140,56 @@ __global__ void score_kernel(int64_t C, const int64_t* __restrict__ start,
         }
         v = next;
     }
-    if (lane == 0) score[c] = s;
+    return s;
+}
+__global__ void score_kernel(int64_t C, const int64_t* __restrict__ start,
+                             const int64_t* __restrict__ end, const float* __restrict__ prod,
+                             const int32_t* __restrict__ row_of_cluster,
+                             const float* __restrict__ lam, const float* __restrict__ csize,
+                             float* __restrict__ score) {
+    const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (c >= C) return;
+    const int64_t b = start[c];
+    const int len = (int)min(end[c] - b, (int64_t)kBigRows);
+    if (len >= kBigRows) return;
+    const float s = warp_sum(score_start(c, row_of_cluster, lam, csize), prod + b, len);
+    if ((threadIdx.x & 31) == 0) score[c] = s;
+}
+constexpr int64_t kScoreWarps = 16384;
+constexpr int kLaneRows = 64;
+__global__ void score_many_kernel(int64_t C, const int64_t* __restrict__ start,
+                                  const int64_t* __restrict__ end, const float* __restrict__ prod,
+                                  const int32_t* __restrict__ row_of_cluster,
+                                  const float* __restrict__ lam, const float* __restrict__ csize,
+                                  float* __restrict__ score) {
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    int64_t b = 0;
+    int len = kBigRows;  // (past the clusters: nothing to do)
+    float s = 0.0f;
+    if (c < C) {
+        b = start[c];
+        len = (int)min(end[c] - b, (int64_t)kBigRows);
+        s = score_start(c, row_of_cluster, lam, csize);
+        if (len <= kLaneRows) {
+            int j = 0;
+            for (; j + 8 <= len; j += 8) {
+                float v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] = __ldg(prod + b + j + u);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) s = __fadd_rn(s, v[u]);
+            }
+            for (; j < len; ++j) s = __fadd_rn(s, __ldg(prod + b + j));
+            score[c] = s;
+        }
+    }
+    for (unsigned m = __ballot_sync(kFull, len > kLaneRows && len < kBigRows); m; m &= m - 1u) {
+        const int i = __ffs(m) - 1;
+        const float t = warp_sum(__shfl_sync(kFull, s, i), prod + __shfl_sync(kFull, b, i),
+                                 __shfl_sync(kFull, len, i));
+        if (lane == i) score[c] = t;
+    }
 }
 // One block per cluster of kBigRows rows or more: the same sequential sum by
 // one thread, fed from shared memory -- the other warps stage the next chunk
@@ -154,43 +197,61 @@ __global__ void score_kernel(int64_t C, const int64_t* __restrict__ start,
 // dependent additions never waits for memory.
 constexpr int kScoreThreads = 256;
 constexpr int kScoreChunk = 4096;
+// The first bit set from i on, or kScoreThreads.
+__device__ __forceinline__ int next_large(const unsigned* bits, int i) {
+    for (; i < kScoreThreads; i = (i | 31) + 1) {
+        const unsigned m = bits[i >> 5] >> (i & 31);
+        if (m) return i + __ffs(m) - 1;
+    }
+    return kScoreThreads;
+}
 __global__ void __launch_bounds__(kScoreThreads) score_big_kernel(
     int64_t C, const int64_t* __restrict__ start, const int64_t* __restrict__ end,
     const float* __restrict__ prod, const int32_t* __restrict__ row_of_cluster,
     const float* __restrict__ lam, const float* __restrict__ csize, float* __restrict__ score) {
     __shared__ float buf[2][kScoreChunk];
-    for (int64_t c = blockIdx.x; c < C; c += gridDim.x) {
-        const int64_t b = start[c], len = end[c] - b;
-        if (len < kBigRows) continue;  // uniform over the block
-        const int64_t chunks = (len + kScoreChunk - 1) / kScoreChunk;
-        for (int64_t j = threadIdx.x; j < kScoreChunk && j < len; j += blockDim.x)
-            buf[0][j] = __ldg(prod + b + j);
+    __shared__ unsigned s_large[kScoreThreads / 32];
+    const int64_t stride = gridDim.x;
+    for (int64_t c0 = blockIdx.x; c0 < C; c0 += stride * kScoreThreads) {
+        // (every stride-th cluster is this block's: a look at kScoreThreads at once)
+        const int64_t mine = c0 + threadIdx.x * stride;
+        const unsigned large =
+            __ballot_sync(kFull, mine < C && end[mine] - start[mine] >= kBigRows);
+        if ((threadIdx.x & 31) == 0) s_large[threadIdx.x >> 5] = large;
         __syncthreads();
-        float s = threadIdx.x == 0 ? score_start(c, row_of_cluster, lam, csize) : 0.0f;
-        for (int64_t k = 0; k < chunks; ++k) {
-            const int cur = (int)(k & 1);
-            const int64_t base = k * kScoreChunk;
-            const int cl = (int)(len - base < kScoreChunk ? len - base : kScoreChunk);
-            if (threadIdx.x >= 32) {  // warps 1.. stage chunk k + 1
-                const int64_t nb = base + kScoreChunk;
-                for (int64_t j = threadIdx.x - 32; j < kScoreChunk && nb + j < len;
-                     j += blockDim.x - 32)
-                    buf[cur ^ 1][j] = __ldg(prod + b + nb + j);
-            } else if (threadIdx.x == 0) {
-                const float* v = buf[cur];
-                int t = 0;
-                for (; t + 8 <= cl; t += 8) {
-                    float x[8];
+        for (int i = next_large(s_large, 0); i < kScoreThreads; i = next_large(s_large, i + 1)) {
+            const int64_t c = c0 + i * stride, b = start[c], len = end[c] - b;
+            const int64_t chunks = (len + kScoreChunk - 1) / kScoreChunk;
+            for (int64_t j = threadIdx.x; j < kScoreChunk && j < len; j += blockDim.x)
+                buf[0][j] = __ldg(prod + b + j);
+            __syncthreads();
+            float s = threadIdx.x == 0 ? score_start(c, row_of_cluster, lam, csize) : 0.0f;
+            for (int64_t k = 0; k < chunks; ++k) {
+                const int cur = (int)(k & 1);
+                const int64_t base = k * kScoreChunk;
+                const int cl = (int)(len - base < kScoreChunk ? len - base : kScoreChunk);
+                if (threadIdx.x >= 32) {  // warps 1.. stage chunk k + 1
+                    const int64_t nb = base + kScoreChunk;
+                    for (int64_t j = threadIdx.x - 32; j < kScoreChunk && nb + j < len;
+                         j += blockDim.x - 32)
+                        buf[cur ^ 1][j] = __ldg(prod + b + nb + j);
+                } else if (threadIdx.x == 0) {
+                    const float* v = buf[cur];
+                    int t = 0;
+                    for (; t + 8 <= cl; t += 8) {
+                        float x[8];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) x[u] = v[t + u];
+                        for (int u = 0; u < 8; ++u) x[u] = v[t + u];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) s = __fadd_rn(s, x[u]);
+                        for (int u = 0; u < 8; ++u) s = __fadd_rn(s, x[u]);
+                    }
+                    for (; t < cl; ++t) s = __fadd_rn(s, v[t]);
                 }
-                for (; t < cl; ++t) s = __fadd_rn(s, v[t]);
+                __syncthreads();  // chunk k summed, chunk k + 1 staged
             }
-            __syncthreads();  // chunk k summed, chunk k + 1 staged
+            if (threadIdx.x == 0) score[c] = s;
         }
-        if (threadIdx.x == 0) score[c] = s;
+        __syncthreads();
     }
 }
 
@@ -275,6 +336,7 @@ __device__ void block_scan_excl(int32_t* a, int64_t len, int32_t* tmp_total) {
 // 2) in global memory.
 constexpr int64_t kEomShared = 4096;
 constexpr size_t kEomBytes = 47;  // a cluster's, and 16 for dcount
+template <bool HERE>
 __global__ void __launch_bounds__(kEomThreads) eom_kernel(
     int64_t C, const int32_t* __restrict__ cpar, const float* __restrict__ nsize,
     const int8_t* __restrict__ in_tree, const float* __restrict__ score,
@@ -286,12 +348,11 @@ __global__ void __launch_bounds__(kEomThreads) eom_kernel(
     const int t = threadIdx.x;
     __shared__ int32_t s_maxd, s_total;
     extern __shared__ double s_eom[];
-    const bool here = C <= kEomShared;
     int32_t *kid0 = nullptr, *kids = nullptr, *nkid = nullptr;
     float* own = nullptr;
     const int32_t* up = cpar;
     const int8_t* tree = in_tree;
-    if (here) {
+    if constexpr (HERE) {
         ret = s_eom;
         int32_t* at = reinterpret_cast<int32_t*>(s_eom + C);
         depth = at;
@@ -338,7 +399,7 @@ __global__ void __launch_bounds__(kEomThreads) eom_kernel(
         tp = jmp; jmp = jmp2; jmp2 = tp;
     }
     if (t == 0) s_maxd = 0;
-    if (here) {  // the doubling's arrays serve again
+    if constexpr (HERE) {  // the doubling's arrays serve again
         byd = depth2;
         kids = jmp;
         flags = jmp2;
@@ -375,7 +436,7 @@ __global__ void __launch_bounds__(kEomThreads) eom_kernel(
             }
             double cur, tot = 0.0;
             bool too_big = false;
-            if (here) {
+            if constexpr (HERE) {
                 cur = (double)own[c];
                 for (int32_t q = kid0[c]; q < kid0[c] + nkid[c]; ++q) {
                     const int64_t x = q < C ? kids[q] : child[order[q]] - n;
@@ -384,8 +445,8 @@ __global__ void __launch_bounds__(kEomThreads) eom_kernel(
             } else {
                 cur = (double)score[c] > 0.0 ? (double)score[c] : 0.0;
                 too_big = (double)nsize[c] > max_cs;
-                for (int32_t q = 0; q < cnt[c]; ++q)
-                    tot += ret[child[order[start[c] + (uint32_t)q]] - n];
+                const uint32_t b0 = start[c], e0 = b0 + (uint32_t)cnt[c];
+                for (uint32_t q = b0; q < e0; ++q) tot += ret[child[order[q]] - n];
             }
             if (tot > cur || too_big) {
                 ret[c] = tot;
@@ -665,9 +726,9 @@ int prepare(Workspace& ws, const Condensed& ct, LabelPre* pre, Prepared* P) {
                 FHG_CUDA(cudaGetLastError());
             }
             ::fhg::note_launch();
-            score_kernel<<<grid_for(C, 8), 256, 0, ss>>>(C, P->start, P->end, P->prod,
-                                                           pre->row_of_cluster, ct.lambda,
-                                                           ct.csize, P->score);
+            const bool many = C > kScoreWarps;
+            (many ? score_many_kernel : score_kernel)<<<grid_for(C, many ? 256 : 8), 256, 0, ss>>>(
+                C, P->start, P->end, P->prod, pre->row_of_cluster, ct.lambda, ct.csize, P->score);
             FHG_CUDA(cudaGetLastError());
         }
         if (P->side) FHG_CUDA(cudaEventRecord(P->done, P->side));
@@ -748,14 +809,15 @@ int select_eom(Workspace& ws, const Condensed& ct, double max_cs, bool allow_sin
     FHG_TRY(ws.alloc(&chose, (size_t)C));
     FHG_TRY(ws.alloc(&blocked, (size_t)C));
     FHG_TRY(ws.alloc(&nsel_dev, 1));
-    const size_t smem = C <= kEomShared ? kEomBytes * (size_t)C + 16 : 0;
-    FHG_CUDA(cudaFuncSetAttribute(eom_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const bool here = C <= kEomShared;
+    const size_t smem = here ? kEomBytes * (size_t)C + 16 : 0;
+    FHG_CUDA(cudaFuncSetAttribute(eom_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(kEomBytes * kEomShared + 16)));
     ::fhg::note_launch();
-    eom_kernel<<<1, kEomThreads, smem, s>>>(C, pre->cpar, pre->nsize, pre->in_tree, P.score,
-                                            P.cstart, P.ccnt, P.corder, ct.child, ct.n, max_cs,
-                                            allow_single ? 1 : 0, depth, depth2, jmp, jmp2, dcount,
-                                            byd, ret, chose, blocked, flags, sel, nsel_dev);
+    (here ? eom_kernel<true> : eom_kernel<false>)<<<1, kEomThreads, smem, s>>>(
+        C, pre->cpar, pre->nsize, pre->in_tree, P.score, P.cstart, P.ccnt, P.corder, ct.child,
+        ct.n, max_cs, allow_single ? 1 : 0, depth, depth2, jmp, jmp2, dcount, byd, ret, chose,
+        blocked, flags, sel, nsel_dev);
     FHG_CUDA(cudaGetLastError());
     FHG_CUDA(cudaMemcpyAsync(n_sel, nsel_dev, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     FHG_CUDA(cudaStreamSynchronize(s));

@@ -253,3 +253,33 @@ def test_condense_sizes_that_are_no_counts(engine, kind, n, mcs):
     got, expect = condense_tree(linkage, min_cluster_size=mcs), O.condense_tree(linkage, mcs)
     for a, b in zip(got, expect):
         np.testing.assert_array_equal(a, b)
+
+
+def _cluster_tree(C, rng, big=0):
+    """A condensed tree of C clusters of 0 to 100 rows, one of `big`, every
+    cluster's row before the rows under it."""
+    from fast_hdbscan_gb300.cluster_trees import CondensedTree
+
+    lens = rng.integers(0, rng.integers(1, 101, size=C))
+    lens[0] += 1
+    lens[C // 3] += big
+    n = int(lens.sum())
+    up = (rng.random(C - 1) * np.arange(1, C)).astype(np.int64)
+    parent = np.concatenate([n + up, n + np.repeat(np.arange(C), lens)])
+    child = np.concatenate([n + np.arange(1, C), rng.permutation(n)])
+    lam = (rng.random(n + C - 1) * 10).astype(np.float32)
+    size = np.concatenate([rng.integers(2, 1000, size=C - 1), np.ones(n)]).astype(np.float32)
+    return CondensedTree(parent.astype(np.int64), child.astype(np.int64), lam, size), n
+
+
+@pytest.mark.parametrize("C", [16_384, 16_385, 40_000, 300_000])
+@pytest.mark.parametrize("big", [0, 2047, 9000])
+def test_eom_of_many_clusters_vs_oracle(engine, C, big):
+    """A warp to a cluster's sum, and a lane or a warp each for 32 clusters."""
+    from fast_hdbscan_gb300.cluster_trees import (
+        cluster_tree_from_condensed_tree, extract_eom_clusters)
+    from oracle import oracle as O
+
+    ct, _ = _cluster_tree(C, np.random.default_rng(C + big), big)
+    sel = extract_eom_clusters(ct, cluster_tree_from_condensed_tree(ct))
+    np.testing.assert_array_equal(sel, O.extract_eom_clusters(ct))
