@@ -16,6 +16,7 @@
 // touched by an interval is no longer a root in any later interval), so one
 // global parent array serves every interval of a level at once.  Work is
 // O(n log n), depth O(log^2 n), whatever the height of the dendrogram.
+#include "compact.cuh"
 #include "primitives.cuh"
 #include "trees.cuh"
 
@@ -31,11 +32,6 @@ __device__ __forceinline__ uint64_t f64_key(double x) {
 __global__ void iota_kernel(int32_t* a, int64_t n) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) a[i] = (int32_t)i;
-}
-__global__ void gather_key32_kernel(const int32_t* __restrict__ v, const int32_t* __restrict__ perm,
-                                    uint32_t* __restrict__ keys, int64_t m) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m) keys[i] = (uint32_t)v[perm[i]];
 }
 __global__ void gather_wkey_kernel(const double* __restrict__ w, const float* __restrict__ w2,
                                    const int32_t* __restrict__ perm, uint64_t* __restrict__ k64,
@@ -55,44 +51,163 @@ __global__ void gather_ends_kernel(const int32_t* __restrict__ perm,
     s0[i] = src[perm[i]];
     d0[i] = dst[perm[i]];
 }
-// Runs of equal weight ordered by (src, dst), then as they came: every edge
-// counts the edges of its run that precede it.  A run longer than `most` sets
-// *too_long and leaves the order unfinished.
+// Runs of equal weight of up to kTieRun edges ordered by (src, dst), then as they
+// came: every edge counts the edges of its run that precede it.  The edges of
+// longer runs are marked, and their number and that of their runs go to longs[0]
+// and longs[1].
 //
-// Equal weights come in short runs (one core distance shared by a few edges),
-// so this takes the place of the sorts by dst and src: six of ten digits.
-// Sort of 10M edges 1.41 -> 0.65 ms, of 20k 114 -> 70 us.
+// Equal weights mostly come in short runs (one core distance shared by a few
+// edges), so this takes the place of the sorts by dst and src: six of ten digits.
+// Sort of 10M edges 1.41 -> 0.65 ms, of 20k 114 -> 70 us.  Sorting and linking 10M
+// edges of weights in runs of 200 / 300 / all equal, ms: ten or fourteen digits for
+// all 9.3 / 9.3 / 9.0; here 8.9 / 9.4 / 9.2 (a line at 64 or 128: 9.4 for 200).
+constexpr int kTieRun = 256;
+constexpr int kTieWalk = 8;  // neighbours looked at one by one
+// One past the edges equal to i on the side `step`, as their distance from i: up
+// to kTieRun, or kTieRun + 1 for more.
+template <class K>
+__device__ __forceinline__ int equal_side(const K* __restrict__ key, int64_t m, int64_t i, K k,
+                                          int step) {
+    auto same = [&](int d) {
+        const int64_t j = i + (int64_t)step * d;
+        return j >= 0 && j < m && key[j] == k;
+    };
+    for (int d = 1; d <= kTieWalk; ++d)
+        if (!same(d)) return d;
+    if (same(kTieRun)) return kTieRun + 1;
+    int lo = kTieWalk, hi = kTieRun;  // same(lo), not same(hi)
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (same(mid)) lo = mid;
+        else hi = mid;
+    }
+    return hi;
+}
 template <class K>
 __global__ void order_ties_kernel(int64_t m, const K* __restrict__ key,
                                   const int32_t* __restrict__ perm,
                                   const int32_t* __restrict__ s0, const int32_t* __restrict__ d0,
                                   const double* __restrict__ w, const float* __restrict__ w2,
-                                  int most, int32_t* __restrict__ ssrc,
-                                  int32_t* __restrict__ sdst, double* __restrict__ sw,
-                                  int32_t* __restrict__ A, int32_t* __restrict__ B,
-                                  int* __restrict__ too_long) {
+                                  int32_t* __restrict__ ssrc, int32_t* __restrict__ sdst,
+                                  double* __restrict__ sw, int32_t* __restrict__ A,
+                                  int32_t* __restrict__ B, uint8_t* __restrict__ mark,
+                                  uint32_t* __restrict__ longs) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     const K k = key[i];
-    const int32_t a = s0[i], b = d0[i];
-    int64_t at = i;
-    int seen = 0;
-    for (int64_t j = i - 1; j >= 0 && key[j] == k; --j) {
-        if (++seen > most) break;
-        if (s0[j] > a || (s0[j] == a && d0[j] > b)) --at;
-    }
-    for (int64_t j = i + 1; j < m && key[j] == k && seen <= most; ++j) {
-        ++seen;
-        if (s0[j] < a || (s0[j] == a && d0[j] < b)) ++at;
-    }
-    if (seen > most) {
-        *too_long = 1;
+    const int before = equal_side(key, m, i, k, -1) - 1, after = equal_side(key, m, i, k, 1) - 1;
+    const bool is_long = before + after + 1 > kTieRun;
+    mark[i] = is_long ? 1 : 0;
+    if (is_long) {
+        if (before > 0) return;
+        // the run's first edge finds its end: (lo is in the run, hi is not)
+        int64_t lo = i + after, hi = lo + 1;
+        while (hi < m && key[hi] == k) {
+            lo = hi;
+            hi = i + 2 * (hi - i);
+        }
+        hi = hi < m ? hi : m;
+        while (hi - lo > 1) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (key[mid] == k) lo = mid;
+            else hi = mid;
+        }
+        atomicAdd(&longs[0], (uint32_t)(hi - i));
+        atomicAdd(&longs[1], 1u);
         return;
     }
+    const int32_t a = s0[i], b = d0[i];
+    int64_t at = i - before;
+    for (int64_t j = i - before; j < i; ++j)
+        at += s0[j] < a || (s0[j] == a && d0[j] <= b) ? 1 : 0;
+    for (int64_t j = i + 1; j <= i + after; ++j)
+        at += s0[j] < a || (s0[j] == a && d0[j] < b) ? 1 : 0;
     const int32_t e = perm[i];
     ssrc[at] = A[at] = a;
     sdst[at] = B[at] = b;
     sw[at] = w ? w[e] : __dsqrt_rn((double)w2[e]);
+}
+// The edges of long runs, in order, and where their runs start.
+template <class K>
+struct LongRuns {
+    const uint8_t* mark;
+    const K* key;
+    int32_t* pos;
+    uint32_t* first;
+    __device__ bool test(int64_t i) const { return mark[i] != 0; }
+    __device__ void emit(int64_t i, uint32_t at) const {
+        pos[at] = (int32_t)i;
+        first[at] = i == 0 || key[i - 1] != key[i] ? 1u : 0u;
+    }
+    __device__ void each(int64_t) const {}
+};
+// Sort keys of the edges of long runs, in the order so far: an end of theirs, or
+// (v NULL) their run's number.
+__global__ void long_keys_kernel(int64_t cnt, const int32_t* __restrict__ order,
+                                 const int32_t* __restrict__ pos, const int32_t* __restrict__ v,
+                                 const uint32_t* __restrict__ first,
+                                 const uint32_t* __restrict__ before, uint32_t* __restrict__ key) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= cnt) return;
+    const int32_t o = order[t];
+    key[t] = v ? (uint32_t)v[pos[o]] : before[o] + first[o];
+}
+__global__ void place_long_kernel(int64_t cnt, const int32_t* __restrict__ order,
+                                  const int32_t* __restrict__ pos, const int32_t* __restrict__ perm,
+                                  const int32_t* __restrict__ s0, const int32_t* __restrict__ d0,
+                                  const double* __restrict__ w, const float* __restrict__ w2,
+                                  int32_t* __restrict__ ssrc, int32_t* __restrict__ sdst,
+                                  double* __restrict__ sw, int32_t* __restrict__ A,
+                                  int32_t* __restrict__ B) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= cnt) return;
+    const int32_t at = pos[t], j = pos[order[t]], e = perm[j];
+    ssrc[at] = A[at] = s0[j];
+    sdst[at] = B[at] = d0[j];
+    sw[at] = w ? w[e] : __dsqrt_rn((double)w2[e]);
+}
+// All of a small input by one block: a bitonic sort by (weight, src, dst, place).
+constexpr int kSmallSort = 2048, kSmallSortThreads = 1024;
+__global__ void __launch_bounds__(kSmallSortThreads) sort_small_kernel(
+    int m, const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
+    const double* __restrict__ w, const float* __restrict__ w2, int32_t* __restrict__ ssrc,
+    int32_t* __restrict__ sdst, double* __restrict__ sw, int32_t* __restrict__ A,
+    int32_t* __restrict__ B) {
+    __shared__ uint64_t s_key[kSmallSort], s_ends[kSmallSort];
+    __shared__ uint16_t s_at[kSmallSort];
+    int m2 = 1;
+    while (m2 < m) m2 <<= 1;
+    for (int i = threadIdx.x; i < m2; i += kSmallSortThreads) {
+        s_key[i] = i >= m ? ~0ull : w ? f64_key(w[i]) : __float_as_uint(w2[i]);
+        s_ends[i] = i >= m ? ~0ull : ((uint64_t)(uint32_t)src[i] << 32) | (uint32_t)dst[i];
+        s_at[i] = (uint16_t)i;  // (places past the edges come last)
+    }
+    __syncthreads();
+    for (int size = 2; size <= m2; size <<= 1) {
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            for (int p = threadIdx.x; p < m2 / 2; p += kSmallSortThreads) {
+                const int i = 2 * p - (p & (stride - 1)), j = i + stride;
+                const uint64_t ki = s_key[i], kj = s_key[j], ei = s_ends[i], ej = s_ends[j];
+                const uint16_t ai = s_at[i], aj = s_at[j];
+                const bool greater = ki != kj ? ki > kj : ei != ej ? ei > ej : ai > aj;
+                if (greater == ((i & size) == 0)) {
+                    s_key[i] = kj;
+                    s_key[j] = ki;
+                    s_ends[i] = ej;
+                    s_ends[j] = ei;
+                    s_at[i] = aj;
+                    s_at[j] = ai;
+                }
+            }
+            __syncthreads();
+        }
+    }
+    for (int i = threadIdx.x; i < m; i += kSmallSortThreads) {
+        const int e = s_at[i];
+        ssrc[i] = A[i] = (int32_t)(s_ends[i] >> 32);
+        sdst[i] = B[i] = (int32_t)(uint32_t)s_ends[i];
+        sw[i] = w ? w[e] : __dsqrt_rn((double)w2[e]);
+    }
 }
 __global__ void apply_perm_kernel(const int32_t* __restrict__ perm, const int32_t* __restrict__ src,
                                   const int32_t* __restrict__ dst, const double* __restrict__ w,
@@ -494,10 +609,54 @@ __global__ void sorted_mst_f64_kernel(int64_t m, const int32_t* __restrict__ ssr
         }                                                                   \
     } while (0)
 
-// Longest run of equal weights ordered by counting, and the input size up to
-// which every run is.
-constexpr int kTieRun = 256;
-constexpr int64_t kTieRunSmall = 2048;
+// Edges after the sort by weight (perm, key): runs of equal weight settled, the
+// long ones by stable sorts of their edges alone over dst, src and run.
+template <class K>
+int settle_ties(Workspace& outer, int64_t n, int64_t m, const K* key, const int32_t* perm,
+                const int32_t* src, const int32_t* dst, const double* w, const float* w2,
+                Linkage* out, int32_t* A, int32_t* B) {
+    cudaStream_t s = outer.stream();
+    Workspace ws(outer);
+    int32_t *s0, *d0;
+    uint8_t* mark;
+    uint32_t* longs;
+    FHG_TRY(ws.alloc(&s0, (size_t)m));
+    FHG_TRY(ws.alloc(&d0, (size_t)m));
+    FHG_TRY(ws.alloc(&mark, (size_t)m));
+    FHG_TRY(ws.alloc(&longs, 2));
+    LAUNCH(gather_ends_kernel, m, perm, src, dst, s0, d0, m);
+    FHG_CUDA(cudaMemsetAsync(longs, 0, 2 * sizeof(uint32_t), s));
+    LAUNCH(order_ties_kernel<K>, m, m, key, perm, s0, d0, w, w2, out->ssrc, out->sdst, out->w, A,
+           B, mark, longs);
+    uint32_t h[2] = {0, 0};
+    FHG_CUDA(cudaMemcpyAsync(h, longs, sizeof(h), cudaMemcpyDeviceToHost, s));
+    FHG_CUDA(cudaStreamSynchronize(s));
+    const int64_t cnt = h[0];
+    if (cnt == 0) return FHG_OK;
+    int32_t *pos, *order;
+    uint32_t *first, *before, *k32;
+    FHG_TRY(ws.alloc(&pos, (size_t)cnt));
+    FHG_TRY(ws.alloc(&order, (size_t)cnt));
+    FHG_TRY(ws.alloc(&first, (size_t)cnt));
+    FHG_TRY(ws.alloc(&before, (size_t)cnt));
+    FHG_TRY(ws.alloc(&k32, (size_t)cnt));
+    FHG_TRY(compact(ws, LongRuns<K>{mark, key, pos, first}, m, nullptr));
+    const int32_t* none = nullptr;
+    const int ibits = bits_for(n);
+    LAUNCH(iota_kernel, cnt, order, cnt);
+    LAUNCH(long_keys_kernel, cnt, cnt, order, pos, d0, first, before, k32);
+    FHG_TRY(radix_sort_u32(ws, k32, order, cnt, 0, ibits));
+    LAUNCH(long_keys_kernel, cnt, cnt, order, pos, s0, first, before, k32);
+    FHG_TRY(radix_sort_u32(ws, k32, order, cnt, 0, ibits));
+    if (h[1] > 1) {
+        FHG_TRY(scan_exclusive_u32(ws, first, before, cnt, nullptr));
+        LAUNCH(long_keys_kernel, cnt, cnt, order, pos, none, first, before, k32);
+        FHG_TRY(radix_sort_u32(ws, k32, order, cnt, 0, bits_for(h[1])));
+    }
+    LAUNCH(place_long_kernel, cnt, cnt, order, pos, perm, s0, d0, w, w2, out->ssrc, out->sdst,
+           out->w, A, B);
+    return FHG_OK;
+}
 
 // The whole contraction over m > 0 sorted edges with endpoint labels A, B.
 // The leaf interval length L = ceil(m / 2^K) <= kLeafRanks makes the top
@@ -551,15 +710,7 @@ int sort_and_link(Workspace& ws, int64_t n, const int32_t* src, const int32_t* d
     }
 
     // ---- sort by (weight, src, dst): a stable radix sort by weight (left out
-    // where the edges come in that order), then the runs of equal weight; a long
-    // run sends all of it to stable sorts over dst, src and weight instead
-    int32_t* perm;
-    uint32_t* k32;
-    uint64_t* k64 = nullptr;
-    FHG_TRY(ws.alloc(&perm, (size_t)m));
-    FHG_TRY(ws.alloc(&k32, (size_t)m));
-    if (w) FHG_TRY(ws.alloc(&k64, (size_t)m));
-    LAUNCH(iota_kernel, m, perm, m);
+    // where the edges come in that order), then the runs of equal weight
     int32_t *A, *B;
     FHG_TRY(ws.alloc(&out->ssrc, (size_t)m));
     FHG_TRY(ws.alloc(&out->sdst, (size_t)m));
@@ -567,49 +718,34 @@ int sort_and_link(Workspace& ws, int64_t n, const int32_t* src, const int32_t* d
     FHG_TRY(ws.alloc(&A, (size_t)m));
     FHG_TRY(ws.alloc(&B, (size_t)m));
     if (order == EdgeOrder::sorted) {
+        Workspace tmp(ws);
+        int32_t* perm;
+        FHG_TRY(tmp.alloc(&perm, (size_t)m));
+        LAUNCH(iota_kernel, m, perm, m);
         LAUNCH(apply_perm_kernel, m, perm, src, dst, w, w2, out->ssrc, out->sdst, out->w, A, B, m);
+    } else if (m <= kSmallSort) {
+        Stage stage(s, "mst_sort");
+        ::fhg::note_launch();
+        sort_small_kernel<<<1, kSmallSortThreads, 0, s>>>((int)m, src, dst, w, w2, out->ssrc,
+                                                          out->sdst, out->w, A, B);
+        FHG_CUDA(cudaGetLastError());
     } else {
         Stage stage(s, "mst_sort");
         Workspace tmp(ws);
+        int32_t* perm;
+        uint32_t* k32;
+        uint64_t* k64 = nullptr;
+        FHG_TRY(tmp.alloc(&perm, (size_t)m));
+        FHG_TRY(tmp.alloc(&k32, (size_t)m));
+        if (w) FHG_TRY(tmp.alloc(&k64, (size_t)m));
+        LAUNCH(iota_kernel, m, perm, m);
         LAUNCH(gather_wkey_kernel, m, w, w2, perm, k64, k32, m);
         if (order == EdgeOrder::any) {
             if (w) FHG_TRY(radix_sort_u64(tmp, k64, perm, m, 0, 64));
             else FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, 32));
         }
-        int32_t *s0, *d0;
-        int* too_long;
-        FHG_TRY(tmp.alloc(&s0, (size_t)m));
-        FHG_TRY(tmp.alloc(&d0, (size_t)m));
-        FHG_TRY(tmp.alloc(&too_long, 1));
-        LAUNCH(gather_ends_kernel, m, perm, src, dst, s0, d0, m);
-        // (no run of a small input is too long, so its flag is not read)
-        const bool small = m <= kTieRunSmall;
-        const int most = small ? (int)kTieRunSmall : kTieRun;
-        if (!small) FHG_CUDA(cudaMemsetAsync(too_long, 0, sizeof(int), s));
-        if (w)
-            LAUNCH(order_ties_kernel<uint64_t>, m, m, k64, perm, s0, d0, w, w2, most, out->ssrc,
-                   out->sdst, out->w, A, B, too_long);
-        else
-            LAUNCH(order_ties_kernel<uint32_t>, m, m, k32, perm, s0, d0, w, w2, most, out->ssrc,
-                   out->sdst, out->w, A, B, too_long);
-        int h_long = 0;
-        if (!small) {
-            FHG_CUDA(cudaMemcpyAsync(&h_long, too_long, sizeof(int), cudaMemcpyDeviceToHost, s));
-            FHG_CUDA(cudaStreamSynchronize(s));
-        }
-        if (h_long) {
-            const int ibits = bits_for(n);
-            LAUNCH(iota_kernel, m, perm, m);
-            LAUNCH(gather_key32_kernel, m, dst, perm, k32, m);
-            FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, ibits));
-            LAUNCH(gather_key32_kernel, m, src, perm, k32, m);
-            FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, ibits));
-            LAUNCH(gather_wkey_kernel, m, w, w2, perm, k64, k32, m);
-            if (w) FHG_TRY(radix_sort_u64(tmp, k64, perm, m, 0, 64));
-            else FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, 32));
-            LAUNCH(apply_perm_kernel, m, perm, src, dst, w, w2, out->ssrc, out->sdst, out->w, A, B,
-                   m);
-        }
+        if (w) FHG_TRY(settle_ties(tmp, n, m, k64, perm, src, dst, w, w2, out, A, B));
+        else FHG_TRY(settle_ties(tmp, n, m, k32, perm, src, dst, w, w2, out, A, B));
     }
 
     Stage stage(s, "linkage");
