@@ -33,6 +33,11 @@ __global__ void iota_kernel(int32_t* a, int64_t n) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) a[i] = (int32_t)i;
 }
+__global__ void gather_key32_kernel(const int32_t* __restrict__ v, const int32_t* __restrict__ perm,
+                                    uint32_t* __restrict__ keys, int64_t m) {
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < m) keys[i] = (uint32_t)v[perm[i]];
+}
 __global__ void gather_wkey_kernel(const double* __restrict__ w, const float* __restrict__ w2,
                                    const int32_t* __restrict__ perm, uint64_t* __restrict__ k64,
                                    uint32_t* __restrict__ k32, int64_t m) {
@@ -658,6 +663,24 @@ int settle_ties(Workspace& outer, int64_t n, int64_t m, const K* key, const int3
     return FHG_OK;
 }
 
+// The order by stable sorts over dst, src and weight: nothing is read back, as a
+// stream that is being captured wants it.
+int sort_all(Workspace& ws, int64_t n, int64_t m, const int32_t* src, const int32_t* dst,
+             const double* w, const float* w2, int32_t* perm, uint64_t* k64, uint32_t* k32,
+             Linkage* out, int32_t* A, int32_t* B) {
+    cudaStream_t s = ws.stream();
+    const int ibits = bits_for(n);
+    LAUNCH(gather_key32_kernel, m, dst, perm, k32, m);
+    FHG_TRY(radix_sort_u32(ws, k32, perm, m, 0, ibits));
+    LAUNCH(gather_key32_kernel, m, src, perm, k32, m);
+    FHG_TRY(radix_sort_u32(ws, k32, perm, m, 0, ibits));
+    LAUNCH(gather_wkey_kernel, m, w, w2, perm, k64, k32, m);
+    if (w) FHG_TRY(radix_sort_u64(ws, k64, perm, m, 0, 64));
+    else FHG_TRY(radix_sort_u32(ws, k32, perm, m, 0, 32));
+    LAUNCH(apply_perm_kernel, m, perm, src, dst, w, w2, out->ssrc, out->sdst, out->w, A, B, m);
+    return FHG_OK;
+}
+
 // The whole contraction over m > 0 sorted edges with endpoint labels A, B.
 // The leaf interval length L = ceil(m / 2^K) <= kLeafRanks makes the top
 // interval L * 2^K just cover m, so every level splits its intervals at their
@@ -739,13 +762,19 @@ int sort_and_link(Workspace& ws, int64_t n, const int32_t* src, const int32_t* d
         FHG_TRY(tmp.alloc(&k32, (size_t)m));
         if (w) FHG_TRY(tmp.alloc(&k64, (size_t)m));
         LAUNCH(iota_kernel, m, perm, m);
-        LAUNCH(gather_wkey_kernel, m, w, w2, perm, k64, k32, m);
-        if (order == EdgeOrder::any) {
-            if (w) FHG_TRY(radix_sort_u64(tmp, k64, perm, m, 0, 64));
-            else FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, 32));
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        FHG_CUDA(cudaStreamIsCapturing(s, &capture));
+        if (capture != cudaStreamCaptureStatusNone) {
+            FHG_TRY(sort_all(tmp, n, m, src, dst, w, w2, perm, k64, k32, out, A, B));
+        } else {
+            LAUNCH(gather_wkey_kernel, m, w, w2, perm, k64, k32, m);
+            if (order == EdgeOrder::any) {
+                if (w) FHG_TRY(radix_sort_u64(tmp, k64, perm, m, 0, 64));
+                else FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, 32));
+            }
+            if (w) FHG_TRY(settle_ties(tmp, n, m, k64, perm, src, dst, w, w2, out, A, B));
+            else FHG_TRY(settle_ties(tmp, n, m, k32, perm, src, dst, w, w2, out, A, B));
         }
-        if (w) FHG_TRY(settle_ties(tmp, n, m, k64, perm, src, dst, w, w2, out, A, B));
-        else FHG_TRY(settle_ties(tmp, n, m, k32, perm, src, dst, w, w2, out, A, B));
     }
 
     Stage stage(s, "linkage");

@@ -387,3 +387,36 @@ def test_mst_sort_time_of_equal_weights(engine, m, most):
         return min(times)
 
     assert sort_ms(True) < most * sort_ms(False)
+
+
+@pytest.mark.parametrize("m", [100, 5000, 100_000])
+@pytest.mark.parametrize("weights", ["random", "few"])
+def test_sort_mst_in_a_graph(engine, m, weights):
+    """fhg_sort_mst asks the host for nothing, so that a CUDA graph can hold it:
+    captured on one input, replayed on another."""
+    import torch
+
+    from fast_hdbscan_gb300 import _native
+
+    rng = np.random.default_rng(m)
+
+    def tree():
+        child = np.arange(1, m + 1)
+        w = rng.integers(0, 5, size=m) if weights == "few" else rng.normal(size=m) ** 2
+        return np.stack([(rng.random(m) * child).astype(np.int64), child, w],
+                        axis=1).astype(np.float64)
+
+    V, lib = _native.vptr, _native.load()
+    first, second = tree(), tree()
+    d = torch.from_numpy(first).cuda()
+    out = torch.empty_like(d)
+    _native.check(lib.fhg_sort_mst(V(d), m, V(out), _native.stream_ptr()))  # kernels loaded
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        _native.check(lib.fhg_sort_mst(V(d), m, V(out), _native.stream_ptr()))
+    for mst in (first, second):
+        d.copy_(torch.from_numpy(mst))
+        graph.replay()
+        expect = mst[np.lexsort((mst[:, 1], mst[:, 0], mst[:, 2]))]
+        np.testing.assert_array_equal(out.cpu().numpy(), expect)
