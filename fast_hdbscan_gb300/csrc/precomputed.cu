@@ -49,7 +49,9 @@ __global__ void pc_offdiag_kernel(int64_t nnz, const int32_t* __restrict__ rows,
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < nnz) flag[t] = rows[t] != cols[t] ? 1u : 0u;
 }
-// (min, max) pair key of every off-diagonal entry, in input order.
+// (min, max) pair key of every off-diagonal entry, in input order, and its
+// weight, with -0.0 as 0.0: from here on weights are ordered by their bits, and
+// the forest's edges are taken to come in ascending order.
 __global__ void pc_pairs_kernel(int64_t nnz, int64_t n, const int32_t* __restrict__ rows,
                                 const int32_t* __restrict__ cols, const double* __restrict__ data,
                                 const uint32_t* __restrict__ flag, const uint32_t* __restrict__ pos,
@@ -61,7 +63,7 @@ __global__ void pc_pairs_kernel(int64_t nnz, int64_t n, const int32_t* __restric
     const uint32_t o = pos[t];
     key[o] = (uint64_t)u * (uint64_t)n + (uint64_t)v;
     at[o] = (int32_t)o;
-    d0[o] = data[t];
+    d0[o] = data[t] + 0.0;
 }
 __global__ void pc_group_flags_kernel(int64_t m0, const uint64_t* __restrict__ key,
                                       uint32_t* __restrict__ flag) {

@@ -160,3 +160,31 @@ def test_graph_to_device_matches_tocoo(engine):
     bad.data[3] = -1.0
     with pytest.raises(ValueError, match="non-negative"):
         HDBSCAN(metric="precomputed").fit(bad)
+
+
+@pytest.mark.parametrize("ms", [1, 2, 4, 9])
+@pytest.mark.parametrize("n", [60, 4000])
+def test_precomputed_negative_zero_weights(engine, ms, n):
+    """-0.0 is a weight like 0.0: the forest's order, the core distances and the
+    labels are the oracle's, which compares values."""
+    import scipy.sparse
+
+    from fast_hdbscan_gb300.hdbscan import compute_minimum_spanning_tree, fast_hdbscan
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(n + ms)
+    rows, cols = np.repeat(np.arange(n), 8), rng.integers(0, n, 8 * n)
+    data = rng.integers(0, 4, 8 * n).astype(np.float64)
+    data[rng.random(8 * n) < 0.3] = -0.0
+    G = scipy.sparse.coo_matrix((data, (rows, cols)), shape=(n, n))
+    mst, nbrs, core = compute_minimum_spanning_tree(G, min_samples=ms, metric="precomputed",
+                                                    algorithm="kruskal")
+    omst, onb, ocore = O.precomputed_kruskal(G, ms)
+    np.testing.assert_array_equal(core, ocore)
+    np.testing.assert_array_equal(nbrs, onb)
+    np.testing.assert_array_equal(mst, omst)
+    labels, probs = fast_hdbscan(G, min_samples=ms, min_cluster_size=5, metric="precomputed",
+                                 algorithm="kruskal")
+    olabels, oprobs, *_ = O.clusters_from_spanning_tree(omst, min_cluster_size=5)
+    np.testing.assert_array_equal(labels, olabels)
+    np.testing.assert_array_equal(probs, oprobs)
