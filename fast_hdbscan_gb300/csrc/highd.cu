@@ -1068,12 +1068,14 @@ __global__ void __launch_bounds__(128) hd_rerank_kernel(
     __syncwarp();
     // certificate
     const float Tq = T[q];
+    const float ymax = __uint_as_float(maxes[0]), cmax = __uint_as_float(maxes[1]);
     bool ok = true;
-    if (cntc < k) {
+    if (!(ymax < INFINITY && cmax < INFINITY)) {
+        ok = false;  // estimates overflow float32 and may have left out any point
+    } else if (cntc < k) {
         ok = !(Tq < INFINITY);  // fewer than k points exist only when every point is a candidate
     } else if (Tq < INFINITY) {
         const float dk = hd_dist(keys[warp][k - 1]);
-        const float ymax = __uint_as_float(maxes[0]), cmax = __uint_as_float(maxes[1]);
         const float yq = sqrtf(ny[q]), cq = cn[q];
         const float kw = 3.0f * (float)dp;
         const float eta = (2.0f * kw + 4.0f * (float)dp + 16.0f) * 5.9604645e-8f *

@@ -202,3 +202,31 @@ def test_first_thresholds_leave_rows_certified(engine, n, d, k):
         lib.fhg_set_highd_kernel(0)
     print("n=%d d=%d k=%d: fallbacks tcgen05 %d, mma.sync %d" % (n, d, k, fb_tc, fb_ms))
     assert fb_tc <= fb_ms + n // 100
+
+
+@pytest.mark.parametrize("kernel", [0, 1])
+@pytest.mark.parametrize("scale", [1e19, 1e20, 1e38])
+@pytest.mark.parametrize("n,d,k", [(90, 33, 16), (1000, 40, 11), (4500, 64, 31), (3000, 70, 5)])
+def test_overflowing_estimates_equal_brute_force(engine, kernel, scale, n, d, k):
+    """Groups of finite rows so far apart that |y|^2 overflows: no estimate says
+    anything, so no row may be certified by them."""
+    from fast_hdbscan_gb300 import _native
+
+    rng = np.random.default_rng(n + d)
+    X = rng.normal(size=(n, d))
+    X[:, 3] += scale * rng.integers(0, 3, n)
+    X = X.astype(np.float32)
+    lib = _native.load()
+    lib.fhg_set_highd_kernel(kernel)
+    try:
+        rd, ix, _ = _highd(X, k)
+    finally:
+        lib.fhg_set_highd_kernel(0)
+    with np.errstate(over="ignore"):
+        for i in rng.choice(n, 60, replace=False):
+            dd = np.zeros(n, np.float32)
+            for j in range(d):
+                dd += (X[i, j] - X[:, j]) ** 2
+            order = np.lexsort((np.arange(n), dd))[:k]
+            np.testing.assert_array_equal(ix[i], order)
+            np.testing.assert_array_equal(rd[i], dd[order])
