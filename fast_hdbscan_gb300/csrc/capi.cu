@@ -1034,7 +1034,7 @@ int fit_impl(const float* X_dev, int64_t n, int32_t d, int32_t min_samples,
     int32_t* sel;
     FHG_TRY(ws.alloc(&sel, (size_t)(ct.n_clusters > 0 ? ct.n_clusters : 1)));
     int64_t k = 0;
-    LabelPre lpre;  // labelling work that overlaps the stabilities
+    LabelPre lpre;  // rows and clusters as the selection found them, for the labels
     if (selection_method == 0)
         FHG_TRY(select_eom(ws, ct, max_cluster_size, allow_single_cluster != 0, sel, &k, &lpre));
     else

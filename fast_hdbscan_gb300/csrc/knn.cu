@@ -30,9 +30,10 @@ __host__ __device__ constexpr int knn_warps() { return SP <= 8 ? 4 : 2; }
 // counters for the queues: 13.3 against 13.2 ms at 10M x 3-D, 11.7 against 9.3
 // at 2M x 5-D.)
 constexpr int kTransposeMax = 16;
-// Resident blocks asked of the register allocator: small lists fit in 80
-// registers (100 above four dimensions), which keeps 24 (20) warps per SM;
-// larger lists take what they need.
+// Resident blocks asked of the register allocator: small lists get 80 registers
+// (100 above four dimensions), which keeps 24 (20) warps per SM, at the price of
+// a few spilled words at K = 16 (12 stored and 15 loaded a thread in 3-D); larger
+// lists take what they need.
 template <int DIM, int K>
 constexpr int knn_min_blocks() { return K > 16 || DIM > 8 ? 1 : DIM <= 4 ? 6 : 5; }
 // Candidates at a lane's k-th distance that come after its k-th entry never join
@@ -108,20 +109,21 @@ __device__ __forceinline__ void merge8(unsigned long long (&key)[K],
     if constexpr (!kPow2) out = c[K] < out ? c[K] : out;
 }
 
-// What bounds this kernel is instruction issue.  A bucket's candidates within
-// a lane's k-th distance go into that lane's queue in shared memory; when some
-// lane's queue fills up, every lane sorts its queue eight at a time and merges
-// it into its sorted list, by networks that run the same instructions on all
-// lanes.  (Inserting each candidate as it came made the warp wait for its
-// busiest lane in every bucket: about 150 insertions per warp at 1M x 3-D, k =
-// 16, where a lane inserts 41; now about 20 merges.)  Until its queue is
-// emptied a lane's k-th distance is out of date, i.e. larger: it queues some
-// more candidates, and no result changes.  Measured (one GB300, lists inserted
-// one by one -> this): 10M x 3-D, k = 16: 15.3 -> 12.5 ms; 2M x 5-D, k = 11:
-// 10.4 -> 9.2; 60k x 13-D, k = 11: 2.3 -> 1.7; 1M x 3-D, k = 31: 5.9 -> 3.4
-// (this one before the index order changed), 63 % of issue slots busy.  (All
-// nodes of a level at once against the bucket's box, as the Boruvka search
-// does: 16.1 ms at 10M -- one outlying query makes its bucket walk everything.)
+// What bounds this kernel is instruction issue and, next to it, the latency of a
+// walk: 65 % of the issue slots are busy at 4M x 3-D, k = 16; stalls are fixed
+// latencies first, then loads.  A bucket's candidates within a lane's k-th
+// distance go into that lane's queue in shared memory; when some lane's queue
+// fills up, every lane sorts its queue eight at a time and merges it into its
+// sorted list, by networks that run the same instructions on all lanes.
+// (Inserting each candidate as it came made the warp wait for its busiest lane in
+// every bucket: about 150 insertions per warp at 1M x 3-D, k = 16, where a lane
+// inserts 41; now about 20 merges.)  Until its queue is emptied a lane's k-th
+// distance is out of date, i.e. larger: it queues some more candidates, and no
+// result changes.  Measured (one GB300, lists inserted one by one -> this): 10M x
+// 3-D, k = 16: 15.3 -> 12.6 ms; 2M x 5-D, k = 11: 10.4 -> 9.2; 60k x 13-D, k = 11:
+// 2.3 -> 1.7.  (All nodes of a level at once against the bucket's box, as the
+// Boruvka search does: 16.1 ms at 10M -- one outlying query makes its bucket walk
+// everything.)
 template <int DIM, int SP, int K>
 __global__ void __launch_bounds__(knn_warps<SP>() * 32, knn_min_blocks<DIM, K>())
     knn_kernel(IndexView ix, int k, float* __restrict__ d_s, int32_t* __restrict__ i_s,
@@ -474,7 +476,9 @@ __host__ __device__ constexpr int large_cap(int k) {
 // and keep + slack of them, and lowers `below` to a key that these are below
 // and the others are not; out = min(out, distance of each key left out).  The
 // key is found by bitwise descent from the highest bit in which the buffer's
-// extremes differ; with some slack five or six bits settle it.
+// extremes differ: the keys are distinct, so the number below a key grows by one
+// at a time and the descent meets one within the slack; five or six bits do with
+// some of it.
 __device__ __forceinline__ int large_cut(unsigned long long* buf, int cnt, int keep, int slack,
                                          int lane, unsigned long long& below, float& out) {
     __syncwarp();
@@ -502,8 +506,6 @@ __device__ __forceinline__ int large_cut(unsigned long long* buf, int cnt, int k
         if (c <= keep + slack) res = trial;
         settled = c >= keep && c <= keep + slack;
     }
-    // (not settled: res is the keep-th smallest key itself)
-    if (!settled) ++res;
     int at = 0;
     const unsigned lt = (1u << lane) - 1u;
     for (int e0 = 0; e0 < cnt; e0 += 32) {

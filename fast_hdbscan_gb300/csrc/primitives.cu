@@ -3,8 +3,9 @@
 // Radix sort: one kernel counts every digit of every key, then one kernel per
 // digit ranks, places and writes its tiles.  A tile learns how many items of
 // each digit lie in the tiles before it from the words those tiles publish
-// (decoupled look-back: their own count first, then the count up to and
-// including them).  Tiles are numbered as blocks start, so every tile before
+// (decoupled look-back, D. Merrill and M. Garland, "Single-pass Parallel Prefix
+// Scan with Decoupled Look-back", 2016: their own count first, then the count up
+// to and including them).  Tiles are numbered as blocks start, so every tile before
 // a running one has started; a wait that still goes on too long ends with the
 // block counting the keys of the tiles before it itself.
 //

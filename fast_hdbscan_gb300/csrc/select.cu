@@ -652,10 +652,10 @@ __global__ void fill_i64_kernel(int64_t* a, int64_t n, int64_t v) {
 //
 // The scores are one sequential float32 sum per cluster, so a large cluster's
 // sum is a long chain of dependent additions on a single thread.  For many
-// rows they are computed on a side stream while the stream goes on with the
-// work that does not read them; join() (also run by the destructor) orders the
-// stream after them.  Every buffer the side stream touches belongs to the
-// caller's Workspace, which outlives the join.
+// rows they are computed on a side stream while the stream lists the cluster
+// rows and their parents; join() (also run by the destructor) orders the stream
+// after them.  Every buffer the side stream touches belongs to the caller's
+// Workspace, which outlives the join.
 struct Prepared {
     int32_t *order = nullptr, *corder = nullptr, *ccnt = nullptr;
     uint32_t *key = nullptr, *cstart = nullptr;

@@ -69,8 +69,8 @@ int select_leaf(Workspace& ws, const Condensed& ct, int32_t* sel, int64_t* n_sel
                 LabelPre* pre = nullptr);
 
 // Labels and membership strengths (cluster_trees.py:944, :1011).  Returns
-// FHG_ERR_INVALID where the reference raises a KeyError.  `pre`: the
-// label_prework of the same tree, or NULL.
+// FHG_ERR_INVALID where the reference raises a KeyError.  `pre`: what the
+// selection of the same tree left, or NULL.
 int label_points(Workspace& ws, const Condensed& ct, const int32_t* sel, int64_t n_sel,
                  double epsilon, int64_t* labels, float* probs, const LabelPre* pre = nullptr);
 // Membership strengths for given labels (cluster_trees.py:1011).
