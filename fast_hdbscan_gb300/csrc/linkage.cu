@@ -58,8 +58,9 @@ __global__ void gather_ends_kernel(const int32_t* __restrict__ perm,
 }
 // Runs of equal weight of up to kTieRun edges ordered by (src, dst), then as they
 // came: every edge counts the edges of its run that precede it.  The edges of
-// longer runs are marked, and their number and that of their runs go to longs[0]
-// and longs[1].
+// longer runs are marked.  told: how many such runs there are, and whether the
+// keys are not in order (a forest's edges are only said to be, and negative
+// weights of a caller's graph are not), which leaves everything to be sorted.
 //
 // Equal weights mostly come in short runs (one core distance shared by a few
 // edges), so this takes the place of the sorts by dst and src: six of ten digits.
@@ -68,6 +69,7 @@ __global__ void gather_ends_kernel(const int32_t* __restrict__ perm,
 // all 9.3 / 9.3 / 9.0; here 8.9 / 9.4 / 9.2 (a line at 64 or 128: 9.4 for 200).
 constexpr int kTieRun = 256;
 constexpr int kTieWalk = 8;  // neighbours looked at one by one
+enum { kToldRuns = 0, kToldUnsorted, kToldWords };
 // One past the edges equal to i on the side `step`, as their distance from i: up
 // to kTieRun, or kTieRun + 1 for more.
 template <class K>
@@ -96,29 +98,16 @@ __global__ void order_ties_kernel(int64_t m, const K* __restrict__ key,
                                   int32_t* __restrict__ ssrc, int32_t* __restrict__ sdst,
                                   double* __restrict__ sw, int32_t* __restrict__ A,
                                   int32_t* __restrict__ B, uint8_t* __restrict__ mark,
-                                  uint32_t* __restrict__ longs) {
+                                  uint32_t* __restrict__ told) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     const K k = key[i];
     const int before = equal_side(key, m, i, k, -1) - 1, after = equal_side(key, m, i, k, 1) - 1;
     const bool is_long = before + after + 1 > kTieRun;
     mark[i] = is_long ? 1 : 0;
+    if (i > 0 && key[i - 1] > k) told[kToldUnsorted] = 1u;
     if (is_long) {
-        if (before > 0) return;
-        // the run's first edge finds its end: (lo is in the run, hi is not)
-        int64_t lo = i + after, hi = lo + 1;
-        while (hi < m && key[hi] == k) {
-            lo = hi;
-            hi = i + 2 * (hi - i);
-        }
-        hi = hi < m ? hi : m;
-        while (hi - lo > 1) {
-            const int64_t mid = (lo + hi) >> 1;
-            if (key[mid] == k) lo = mid;
-            else hi = mid;
-        }
-        atomicAdd(&longs[0], (uint32_t)(hi - i));
-        atomicAdd(&longs[1], 1u);
+        if (before == 0) atomicAdd(&told[kToldRuns], 1u);
         return;
     }
     const int32_t a = s0[i], b = d0[i];
@@ -615,37 +604,42 @@ __global__ void sorted_mst_f64_kernel(int64_t m, const int32_t* __restrict__ ssr
     } while (0)
 
 // Edges after the sort by weight (perm, key): runs of equal weight settled, the
-// long ones by stable sorts of their edges alone over dst, src and run.
+// long ones by stable sorts of their edges alone over dst, src and run; or
+// *unsorted set and nothing settled.
 template <class K>
 int settle_ties(Workspace& outer, int64_t n, int64_t m, const K* key, const int32_t* perm,
                 const int32_t* src, const int32_t* dst, const double* w, const float* w2,
-                Linkage* out, int32_t* A, int32_t* B) {
+                Linkage* out, int32_t* A, int32_t* B, bool* unsorted) {
     cudaStream_t s = outer.stream();
     Workspace ws(outer);
     int32_t *s0, *d0;
     uint8_t* mark;
-    uint32_t* longs;
+    uint32_t* told;
     FHG_TRY(ws.alloc(&s0, (size_t)m));
     FHG_TRY(ws.alloc(&d0, (size_t)m));
     FHG_TRY(ws.alloc(&mark, (size_t)m));
-    FHG_TRY(ws.alloc(&longs, 2));
+    FHG_TRY(ws.alloc(&told, (size_t)kToldWords));
     LAUNCH(gather_ends_kernel, m, perm, src, dst, s0, d0, m);
-    FHG_CUDA(cudaMemsetAsync(longs, 0, 2 * sizeof(uint32_t), s));
+    FHG_CUDA(cudaMemsetAsync(told, 0, kToldWords * sizeof(uint32_t), s));
     LAUNCH(order_ties_kernel<K>, m, m, key, perm, s0, d0, w, w2, out->ssrc, out->sdst, out->w, A,
-           B, mark, longs);
-    uint32_t h[2] = {0, 0};
-    FHG_CUDA(cudaMemcpyAsync(h, longs, sizeof(h), cudaMemcpyDeviceToHost, s));
+           B, mark, told);
+    uint32_t h[kToldWords] = {};
+    FHG_CUDA(cudaMemcpyAsync(h, told, sizeof(h), cudaMemcpyDeviceToHost, s));
     FHG_CUDA(cudaStreamSynchronize(s));
-    const int64_t cnt = h[0];
-    if (cnt == 0) return FHG_OK;
+    *unsorted = h[kToldUnsorted] != 0;
+    const int64_t runs = h[kToldRuns];
+    if (*unsorted || runs == 0) return FHG_OK;
     int32_t *pos, *order;
     uint32_t *first, *before, *k32;
-    FHG_TRY(ws.alloc(&pos, (size_t)cnt));
+    FHG_TRY(ws.alloc(&pos, (size_t)m));
+    FHG_TRY(ws.alloc(&first, (size_t)m));
+    FHG_TRY(compact(ws, LongRuns<K>{mark, key, pos, first}, m, told));
+    FHG_CUDA(cudaMemcpyAsync(h, told, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    FHG_CUDA(cudaStreamSynchronize(s));
+    const int64_t cnt = h[0];
     FHG_TRY(ws.alloc(&order, (size_t)cnt));
-    FHG_TRY(ws.alloc(&first, (size_t)cnt));
     FHG_TRY(ws.alloc(&before, (size_t)cnt));
     FHG_TRY(ws.alloc(&k32, (size_t)cnt));
-    FHG_TRY(compact(ws, LongRuns<K>{mark, key, pos, first}, m, nullptr));
     const int32_t* none = nullptr;
     const int ibits = bits_for(n);
     LAUNCH(iota_kernel, cnt, order, cnt);
@@ -653,10 +647,10 @@ int settle_ties(Workspace& outer, int64_t n, int64_t m, const K* key, const int3
     FHG_TRY(radix_sort_u32(ws, k32, order, cnt, 0, ibits));
     LAUNCH(long_keys_kernel, cnt, cnt, order, pos, s0, first, before, k32);
     FHG_TRY(radix_sort_u32(ws, k32, order, cnt, 0, ibits));
-    if (h[1] > 1) {
+    if (runs > 1) {
         FHG_TRY(scan_exclusive_u32(ws, first, before, cnt, nullptr));
         LAUNCH(long_keys_kernel, cnt, cnt, order, pos, none, first, before, k32);
-        FHG_TRY(radix_sort_u32(ws, k32, order, cnt, 0, bits_for(h[1])));
+        FHG_TRY(radix_sort_u32(ws, k32, order, cnt, 0, bits_for(runs)));
     }
     LAUNCH(place_long_kernel, cnt, cnt, order, pos, perm, s0, d0, w, w2, out->ssrc, out->sdst,
            out->w, A, B);
@@ -764,17 +758,18 @@ int sort_and_link(Workspace& ws, int64_t n, const int32_t* src, const int32_t* d
         LAUNCH(iota_kernel, m, perm, m);
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         FHG_CUDA(cudaStreamIsCapturing(s, &capture));
-        if (capture != cudaStreamCaptureStatusNone) {
-            FHG_TRY(sort_all(tmp, n, m, src, dst, w, w2, perm, k64, k32, out, A, B));
-        } else {
+        bool all = capture != cudaStreamCaptureStatusNone;
+        if (!all) {
             LAUNCH(gather_wkey_kernel, m, w, w2, perm, k64, k32, m);
             if (order == EdgeOrder::any) {
                 if (w) FHG_TRY(radix_sort_u64(tmp, k64, perm, m, 0, 64));
                 else FHG_TRY(radix_sort_u32(tmp, k32, perm, m, 0, 32));
             }
-            if (w) FHG_TRY(settle_ties(tmp, n, m, k64, perm, src, dst, w, w2, out, A, B));
-            else FHG_TRY(settle_ties(tmp, n, m, k32, perm, src, dst, w, w2, out, A, B));
+            if (w) FHG_TRY(settle_ties(tmp, n, m, k64, perm, src, dst, w, w2, out, A, B, &all));
+            else FHG_TRY(settle_ties(tmp, n, m, k32, perm, src, dst, w, w2, out, A, B, &all));
+            if (all) LAUNCH(iota_kernel, m, perm, m);
         }
+        if (all) FHG_TRY(sort_all(tmp, n, m, src, dst, w, w2, perm, k64, k32, out, A, B));
     }
 
     Stage stage(s, "linkage");

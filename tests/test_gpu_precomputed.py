@@ -188,3 +188,42 @@ def test_precomputed_negative_zero_weights(engine, ms, n):
     olabels, oprobs, *_ = O.clusters_from_spanning_tree(omst, min_cluster_size=5)
     np.testing.assert_array_equal(labels, olabels)
     np.testing.assert_array_equal(probs, oprobs)
+
+
+@pytest.mark.parametrize("n", [500, 3000, 40_000])
+def test_precomputed_fit_sorts_what_is_not_in_order(engine, n):
+    """The forest of a graph of negative weights (the C entry point does not look
+    at them) comes by magnitude, in descending order: the fused fit still gives
+    the tree of the forest that fhg_precomputed_mst returns."""
+    import ctypes
+
+    import torch
+
+    from fast_hdbscan_gb300 import _native
+    from fast_hdbscan_gb300.hdbscan import clusters_from_spanning_tree
+
+    rng = np.random.default_rng(n)
+    nnz, ms, mcs = 8 * n, 3, 10
+    rows = torch.from_numpy(np.repeat(np.arange(n), 8).astype(np.int32)).cuda()
+    cols = torch.from_numpy(rng.integers(0, n, nnz).astype(np.int32)).cuda()
+    data = torch.from_numpy(-rng.integers(1, 400, nnz).astype(np.float64)).cuda()
+    V, lib = _native.vptr, _native.load()
+    edges = torch.empty(n - 1, 3, dtype=torch.float64, device="cuda")
+    nbrs = torch.empty(n, ms, dtype=torch.int32, device="cuda")
+    core = torch.empty(n, dtype=torch.float64, device="cuda")
+    ncomp = ctypes.c_int64(0)
+    _native.check(lib.fhg_precomputed_mst(V(rows), V(cols), V(data), nnz, n, ms, 1, V(edges),
+                                          V(nbrs), V(core), ctypes.byref(ncomp),
+                                          _native.stream_ptr()))
+    e = edges.cpu().numpy()
+    assert (np.diff(e[:, 2]) < 0).any()
+    labels = torch.empty(n, dtype=torch.int64, device="cuda")
+    probs = torch.empty(n, device="cuda")
+    linkage = torch.empty(n - 1, 4, dtype=torch.float64, device="cuda")
+    rows_n, sel_n = ctypes.c_int64(0), ctypes.c_int64(0)
+    _native.check(lib.fhg_hdbscan_fit_precomputed(
+        V(rows), V(cols), V(data), nnz, n, ms, 1, mcs, 0, float("inf"), 0, 0.0, 0.0, V(labels),
+        V(probs), None, V(linkage), None, None, None, None, ctypes.byref(rows_n), None, None, None,
+        ctypes.byref(sel_n), _native.stream_ptr()))
+    _, _, expect, _, _ = clusters_from_spanning_tree(e, min_cluster_size=mcs)
+    np.testing.assert_array_equal(linkage.cpu().numpy(), expect)
